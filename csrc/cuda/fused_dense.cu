@@ -4,12 +4,20 @@
 //   ring : N hops of  poll incoming partial sum -> decode -> merge with the local
 //          chunk and its residual -> re-encode -> store the payload straight into
 //          the successor GPU's inbox over NVLink; the last hop stores the fully
-//          reduced payload into every rank's inbox, and every rank decodes all N
-//          chunks into the gradient (averaged).
-//   PS   : encode each of the N chunks and store chunk j into owner j's inbox;
-//          the owner decodes and sums the N payloads in rank order, re-encodes
-//          with its server residual and stores the result into every inbox;
-//          every rank decodes all N chunks.
+//          reduced payload into every peer's inbox and decodes its own copy from
+//          registers, and every rank decodes the other N-1 chunks into the gradient
+//          (averaged).
+//   PS   : encode the N-1 chunks that other ranks own and store chunk j into owner
+//          j's inbox; then, tile by tile, encode the own chunk, decode and sum the N
+//          payloads in rank order (the own one from registers), re-encode with the
+//          server residual, store the result into every peer's inbox and decode it;
+//          every rank decodes the other N-1 chunks.
+//
+// What a rank owns never goes through its own inbox: the tile is still in registers
+// when its final codes exist, so the 8-byte slots, the poll and a second visit of the
+// tile are saved for 1/N of the gradient (for all of it on one rank, where VGG-19's
+// gradients took 416 us instead of 443 through TBQ + ring and a base Transformer's
+// 278 us instead of 321 through TernGrad + PS).
 //
 // There is no NCCL call and no separate encode or decode launch.  Payloads are
 // plain 8-byte stores {codes, epoch} to peer-mapped memory; the receiver polls its
@@ -220,7 +228,7 @@ __device__ __forceinline__ void recv_finish(const uint8_t* base, uint32_t t, Til
 #pragma unroll
   for (int k = 0; k < MetaOf<ALG>::N; ++k)
     meta[k] = __uint_as_float(ll_finish(tb + k, rx.m[k], cm, status, code, ws));
-  if (ALG == kOnebit) meta[0] = meta[0] * meta_scale;  // see decode_phase
+  if (ALG == kOnebit) meta[0] = meta[0] * meta_scale;  // see decode_average
   uint32_t w[LL<B>::W], f[kIter];
 #pragma unroll
   for (int k = 0; k < LL<B>::W; ++k)
@@ -228,6 +236,24 @@ __device__ __forceinline__ void recv_finish(const uint8_t* base, uint32_t t, Til
   unpack_words<B>(w, f);
 #pragma unroll
   for (int j = 0; j < kIter; ++j) decode_frag<ALG, B>(f[j], meta, tau, d[j]);
+}
+
+// The averaged value of every element of a decoded tile.  onebit and TBQ decode to
+// +-level or 0, so level * (1/N) is the same float whether the level or the element is
+// scaled; TernGrad's min + q * gap is not.
+template <int ALG, int B>
+__device__ __forceinline__ void decode_average(const uint32_t (&frag)[kIter], float (&meta)[2],
+                                               const FusedParams& fp, float (&d)[kIter][4]) {
+  constexpr bool kFold = ALG != kTernGrad;
+  if (ALG == kOnebit) meta[0] = meta[0] * fp.inv_n;
+#pragma unroll
+  for (int j = 0; j < kIter; ++j) {
+    decode_frag<ALG, B>(frag[j], meta, kFold ? fp.P.tau * fp.inv_n : fp.P.tau, d[j]);
+    if (!kFold) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[j][e] = d[j][e] * fp.inv_n;
+    }
+  }
 }
 
 __device__ __forceinline__ uint32_t chunk_valid(uint32_t n, uint32_t chunk, int c) {
@@ -253,7 +279,7 @@ struct FusedSmem {
 struct PhaseSpec {
   int chunk;      // chunk of every tensor handled in this phase
   int in_slot;    // inbox slot to wait for and merge, or -1
-  int ndst;       // payload goes to ranks (dst0 + q) % N, q < ndst
+  int ndst;       // payload goes to ranks (dst0 + q) % N, q < ndst (the last phase: every peer)
   int dst0;
   int dst_slot;   // slot index inside the destination inbox
   uint32_t salt;
@@ -268,13 +294,17 @@ __device__ __forceinline__ PhaseSpec phase_spec(int ph, int N, int R) {
     if (ph < N - 1) {
       p.ndst = 1; p.dst0 = (R + 1) % N; p.dst_slot = ph;
     } else {
-      p.ndst = N; p.dst0 = R; p.dst_slot = N - 1 + R;
+      p.ndst = N - 1; p.dst0 = (R + 1) % N; p.dst_slot = N - 1 + R;
     }
     p.salt = (uint32_t)(R * 256 + ph);
-  } else {  // PS push: remote owners first, own chunk last
+  } else {  // PS: push to the remote owners first, own chunk (push and serve) last
     p.chunk = (R + 1 + ph) % N;
     p.in_slot = -1;
-    p.ndst = 1; p.dst0 = p.chunk; p.dst_slot = R;
+    if (ph < N - 1) {
+      p.ndst = 1; p.dst0 = p.chunk; p.dst_slot = R;
+    } else {
+      p.ndst = N - 1; p.dst0 = (R + 1) % N; p.dst_slot = N + R;
+    }
     p.salt = (uint32_t)(R * 256);
   }
   return p;
@@ -287,8 +317,8 @@ struct TileRef {
   size_t off;   // element offset of the tile inside the tensor
 };
 
-// Work distribution.  A launch is a sequence of phases (ring: N hops then N
-// gathers; PS: N pushes, the server pass, N pulls); every phase visits the
+// Work distribution.  A launch is a sequence of phases (N encode phases, the last of
+// which finishes the rank's own chunk, then N-1 gathers); every phase visits the
 // T = tiles_total tiles of one chunk of every tensor.  Tile i of phase ph is
 // work item ph * T + i, and item w belongs to CTA w % G: the assignment keeps
 // rotating across phases, so a bucket whose chunk has fewer tiles than there are
@@ -461,31 +491,66 @@ __device__ __forceinline__ void encode_phases(const BucketDev& bk, const HpComm&
 #pragma unroll
           for (int e = 0; e < 4; ++e) x[j][e] = x[j][e] + d[j][e];
       }
-      if (rp) {
-        float rr[kIter][4];
-        if (bulk) load_tile_smem(sm.r[st], rr);
-        else load_tile(rp, m, rr);
-#pragma unroll
-        for (int j = 0; j < kIter; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) x[j][e] = rr[j][e] + x[j][e];
-      }
       float meta[2];
       uint32_t frag[kIter];
-      encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt, sm.tile, meta, frag,
-                          rp != nullptr);
-      // after an expired wait the merged input is not a real partial sum: the error
-      // feedback state keeps its last good contents
-      const bool bad = *(volatile int*)&sm.ws.poisoned != 0;
-      if (rp && !bad) {
-        if (bulk) store_tile_full(rp, x);
-        else store_tile(rp, m, x);
+      bool bad = false;
+      const bool final_tile = ph == N - 1;  // this rank's own chunk gets its final codes here
+      // PS encodes a tile of the own chunk twice: what this rank pushes, and the sum of
+      // the N pushes (a rolled loop: one copy of the encoder's code)
+#pragma unroll 1
+      for (int pass = 0;; ++pass) {
+        if (rp) {
+          float rr[kIter][4];
+          if (bulk && pass == 0) load_tile_smem(sm.r[st], rr);
+          else load_tile(rp, m, rr);
+#pragma unroll
+          for (int j = 0; j < kIter; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[j][e] = rr[j][e] + x[j][e];
+        }
+        encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt + (uint32_t)pass, sm.tile,
+                            meta, frag, rp != nullptr);
+        // after an expired wait the merged input is not a real partial sum: the error
+        // feedback state keeps its last good contents
+        bad = *(volatile int*)&sm.ws.poisoned != 0;
+        if (rp && !bad) {
+          if (tile_is_full_aligned(rp, m)) store_tile_full(rp, x);
+          else store_tile(rp, m, x);
+        }
+        if (TOPO == HP_TOPO_RING || !final_tile || pass == 1) break;
+        // sum the N pushes of this tile in rank order.  The remote ones are polled one
+        // ahead: the loads of the next are in flight while the current one is decoded
+        TileRx<ALG, B> in[2];
+        if (N > 1 && !dbg_tile_ok<ALG, B>(bk, my_inbox, my_inbox + (size_t)(N - 1) * bk.slot_bytes + sg.pay_off,
+                                          t, status, 4u)) {
+          sm.ws.poisoned = 1;   // ll_finish returns at once, nothing is stored
+        } else if (R != 0) {
+          recv_issue<ALG, B>(my_inbox + sg.pay_off, t, in[0]);
+        }
+        for (int q = 0; q < N; ++q) {
+          if (q + 1 < N && q + 1 != R && !sm.ws.poisoned)
+            recv_issue<ALG, B>(my_inbox + (size_t)(q + 1) * bk.slot_bytes + sg.pay_off, t, in[(q + 1) & 1]);
+          float d[kIter][4];
+          if (q == R) {
+#pragma unroll
+            for (int j = 0; j < kIter; ++j) decode_frag<ALG, B>(frag[j], meta, fp.P.tau, d[j]);
+          } else {
+            recv_finish<ALG, B>(my_inbox + (size_t)q * bk.slot_bytes + sg.pay_off, t, in[q & 1], cm,
+                                status, HP_STATUS_TIMEOUT | (1u << 16) | ((uint32_t)q << 8) | (b & 255),
+                                sm.ws, fp.P.tau, d);
+          }
+#pragma unroll
+          for (int j = 0; j < kIter; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[j][e] = q > 0 ? x[j][e] + d[j][e] : d[j][e];
+        }
+        rp = sg.sr ? sg.sr + E * cm.emu_stride_sr + (size_t)t * kTile : nullptr;
       }
       uint32_t words[LL<B>::W];
       pack_words<B>(frag, words);
       const uint32_t ep = cm.epoch | (bad ? kGaveUp : 0u);
-      // one destination on a hop, every rank on the last one (a rolled loop: the
-      // broadcast is one phase in N)
+      // one destination on a hop or push, every peer in the last phase (a rolled loop:
+      // the broadcast is one phase in N)
 #pragma unroll 1
       for (int q = 0; q < ps.ndst; ++q) {
         int d = ps.dst0 + q;
@@ -493,6 +558,15 @@ __device__ __forceinline__ void encode_phases(const BucketDev& bk, const HpComm&
         uint8_t* dst = reinterpret_cast<uint8_t*>(cm.inbox[d]) + dst_off + sg.pay_off;
         if (dbg_tile_ok<ALG, B>(bk, cm.inbox[d], dst, t, status, 2u))
           send_tile<ALG, B>(dst, t, words, meta, ep);
+      }
+      // the own chunk is decoded from registers (a tile whose input never arrived is
+      // left as it was: the local gradient)
+      if (final_tile && !bad) {
+        float d[kIter][4];
+        decode_average<ALG, B>(frag, meta, fp, d);
+        float* op = sg.out + E * cm.emu_stride_out + tr.off;
+        if (tile_is_full_aligned(op, m)) store_tile_full(op, d);
+        else store_tile(op, m, d);
       }
       __syncthreads();  // the prefetch stage of this tile may be refilled from here on
     }
@@ -538,8 +612,7 @@ __device__ __forceinline__ void decode_phase(const BucketDev& bk, const HpComm& 
       if (u < cnt) {
         const SegDev& sg = bk.seg[tr[u].seg];
         float x[kIter][4];
-        // onebit and TBQ decode to +-level or 0, so level * (1/N) is the same float
-        // whether the level or the element is scaled; TernGrad's min + q * gap is not
+        // the scaling by 1/N is folded into the level where it can be (see decode_average)
         constexpr bool kFold = ALG != kTernGrad;
         recv_finish<ALG, B>(sp + sg.pay_off, tr[u].t, rx[u], cm, status, code, sm.ws,
                             kFold ? fp.P.tau * fp.inv_n : fp.P.tau, x, kFold ? fp.inv_n : 1.0f);
@@ -584,10 +657,11 @@ ring_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   trace_mark(cm, E, 0);
   encode_phases<ALG, B, HP_TOPO_RING>(bk, cm, fp, sm, R, E, status);
   trace_mark(cm, E, 1);
-  // gather: rank src finalised chunk src+1
-  for (int qq = 0; qq < N; ++qq) {
+  // gather: rank src finalised chunk src+1 (the own one is done)
+  trace_phase(cm, E, N, sm.ws);
+  for (int qq = 1; qq < N; ++qq) {
     const int src = (R + qq) % N;
-    decode_phase<ALG, B>(bk, cm, fp, sm, R, E, N + qq, N - 1 + src, (src + 1) % N, status);
+    decode_phase<ALG, B>(bk, cm, fp, sm, R, E, N + qq - 1, N - 1 + src, (src + 1) % N, status);
     trace_phase(cm, E, N + qq, sm.ws);
   }
   trace_mark(cm, E, 2);
@@ -599,93 +673,22 @@ __global__ void __launch_bounds__(kThreads, 3)
 ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FusedSmem& sm = *reinterpret_cast<FusedSmem*>(smem_raw);
-  TileSmem& s = sm.tile;
   const int N = cm.nranks;
   const int R = cm.emulate ? (int)blockIdx.y : cm.rank;
   const int E = cm.emulate ? (int)blockIdx.y : 0;
-  const int G = (int)gridDim.x;
-  const int b = (int)blockIdx.x;
   uint32_t* status = reinterpret_cast<uint32_t*>(cm.status) + 4 * E;
-  uint8_t* my_inbox = reinterpret_cast<uint8_t*>(cm.inbox[R]);
   fused_prologue(sm);
   trace_mark(cm, E, 0);
 
-  // phases 0 .. N-1: push
+  // phases 0 .. N-2: push; phase N-1: push and serve the own chunk
   encode_phases<ALG, B, HP_TOPO_PS>(bk, cm, fp, sm, R, E, status);
   trace_mark(cm, E, 1);
-
-  // phase N: server for chunk R: sum the N payloads in rank order, re-encode, broadcast
-  {
-    Cursor cur;
-    cursor_begin(bk, G, b, N, R, cur);
-    TileRef tr;
-    const size_t dst_off = (size_t)(N + R) * bk.slot_bytes;
-    while (cursor_next(bk, G, b, cur, tr)) {
-      const SegDev& sg = bk.seg[tr.seg];
-      const int m = tr.m;
-      const uint32_t t = tr.t;
-      const size_t coff = (size_t)t * kTile;  // offset inside the owned chunk
-      float x[kIter][4];
-      // the N pushes are polled two at a time: loads of the next source are in
-      // flight while the current one is decoded
-      TileRx<ALG, B> rx[2];
-      if (!dbg_tile_ok<ALG, B>(bk, my_inbox, my_inbox + (size_t)(N - 1) * bk.slot_bytes + sg.pay_off, t,
-                               status, 4u)) {
-        sm.ws.poisoned = 1;
-        continue;
-      }
-      recv_issue<ALG, B>(my_inbox + sg.pay_off, t, rx[0]);
-      for (int q = 0; q < N; ++q) {
-        if (q + 1 < N)
-          recv_issue<ALG, B>(my_inbox + (size_t)(q + 1) * bk.slot_bytes + sg.pay_off, t,
-                             rx[(q + 1) & 1]);
-        float d[kIter][4];
-        recv_finish<ALG, B>(my_inbox + (size_t)q * bk.slot_bytes + sg.pay_off, t, rx[q & 1], cm,
-                            status, HP_STATUS_TIMEOUT | (1u << 16) | ((uint32_t)q << 8) | (b & 255),
-                            sm.ws, fp.P.tau, d);
-#pragma unroll
-        for (int j = 0; j < kIter; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) x[j][e] = q > 0 ? x[j][e] + d[j][e] : d[j][e];
-      }
-      float* rp = sg.sr ? sg.sr + E * cm.emu_stride_sr + coff : nullptr;
-      if (rp) {
-        float rr[kIter][4];
-        load_tile(rp, m, rr);
-#pragma unroll
-        for (int jj = 0; jj < kIter; ++jj)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) x[jj][e] = rr[jj][e] + x[jj][e];
-      }
-      float meta[2];
-      uint32_t frag[kIter];
-      encode_tile<ALG, B>(x, m, fp.P, sg.id, (size_t)R * sg.chunk + coff,
-                          fp.P.salt + (uint32_t)(R * 256 + 1), s, meta, frag, rp != nullptr);
-      const bool bad = *(volatile int*)&sm.ws.poisoned != 0;
-      if (rp && !bad) {
-        if (tile_is_full_aligned(rp, m)) store_tile_full(rp, x);
-        else store_tile(rp, m, x);
-      }
-      uint32_t words[LL<B>::W];
-      pack_words<B>(frag, words);
-      const uint32_t ep = cm.epoch | (bad ? kGaveUp : 0u);
-#pragma unroll 1
-      for (int q = 0; q < N; ++q) {
-        int d = R + q;
-        if (d >= N) d -= N;
-        uint8_t* dst = reinterpret_cast<uint8_t*>(cm.inbox[d]) + dst_off + sg.pay_off;
-        if (dbg_tile_ok<ALG, B>(bk, cm.inbox[d], dst, t, status, 5u))
-          send_tile<ALG, B>(dst, t, words, meta, ep);
-      }
-    }
-    trace_phase(cm, E, N, sm.ws);
-  }
-
-  // phases N+1 .. 2N: pull: decode every owner's reduced chunk
-  for (int i = 0; i < N; ++i) {
+  trace_phase(cm, E, N, sm.ws);
+  // pull: decode every other owner's reduced chunk
+  for (int i = 1; i < N; ++i) {
     const int j = (R + i) % N;
-    decode_phase<ALG, B>(bk, cm, fp, sm, R, E, N + 1 + i, N + j, j, status);
-    trace_phase(cm, E, N + 1 + i, sm.ws);
+    decode_phase<ALG, B>(bk, cm, fp, sm, R, E, N + i - 1, N + j, j, status);
+    trace_phase(cm, E, N + i, sm.ws);
   }
   trace_mark(cm, E, 2);
 }
@@ -730,10 +733,8 @@ static int build_bucket(int alg, int bits, const HpSeg* segs, int nseg, int nran
 static int num_slots(int topo, int nranks) {
   return topo == HP_TOPO_RING ? 2 * nranks - 1 : 2 * nranks;
 }
-// phases of one launch (see Cursor)
-static int num_phases(int topo, int nranks) {
-  return topo == HP_TOPO_RING ? 2 * nranks : 2 * nranks + 1;
-}
+// phases of one launch that visit tiles (see Cursor)
+static int num_phases(int nranks) { return 2 * nranks - 1; }
 
 template <int ALG, int B>
 static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const FusedParams& fp,
@@ -836,7 +837,7 @@ int hp_cuda_fused_dense(int topo, int alg, int bits, const HpSeg* segs, int nseg
   bk.inbox_bytes = bk.slot_bytes * (uint64_t)num_slots(topo, comm->nranks);
   bk.dbg_limit = g_dbg_inbox_limit;
   {  // never more CTAs than work items
-    const uint64_t items = (uint64_t)bk.tiles_total * (uint64_t)num_phases(topo, comm->nranks);
+    const uint64_t items = (uint64_t)bk.tiles_total * (uint64_t)num_phases(comm->nranks);
     if ((uint64_t)ctas > items) ctas = (int)items;
   }
   FusedParams fp;

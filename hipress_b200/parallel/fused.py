@@ -63,7 +63,7 @@ class FusedDenseBucket:
         _lib.check(L.hp_fused_dense_layout(self.topo, spec.alg, spec.bits, arr, len(self.sizes),
                                            nranks, C.byref(ib), C.byref(sb), C.byref(tt)), "layout")
         self.inbox_bytes, self.slot_bytes, self.tiles_total = ib.value, sb.value, tt.value
-        phases = 2 * nranks + (1 if self.topo == _lib.TOPO_PS else 0)
+        phases = 2 * nranks - 1
         self.ctas = max(1, min(self.ctas, self.tiles_total * phases))   # never more CTAs than work items
         self.inbox_ptrs = None
         self.status = None
@@ -201,13 +201,14 @@ class FusedDenseBucket:
         return [((int(r[1]) - int(r[0])) * 1e-6, (int(r[2]) - int(r[0])) * 1e-6) for r in t]
 
     def last_trace_phases(self):
-        """Per rank played by the last launch: for every phase (ring: N hops then N
-        gathers; PS: N pushes, the server pass, N pulls) the time, in ms from the
-        first CTA's start, at which the last CTA finished it, and the mean time a CTA
-        spent polling for its input in that phase."""
+        """Per rank played by the last launch: for every phase (N hops or pushes, the
+        last of which finishes the rank's own chunk, then N gathers or pulls, the first
+        of which is that own chunk and does nothing) the time, in ms from the first
+        CTA's start, at which the last CTA finished it, and the mean time a CTA spent
+        polling for its input in that phase."""
         if self.trace is None:
             return None
-        phases = 2 * self.nranks + (1 if self.topo == _lib.TOPO_PS else 0)
+        phases = 2 * self.nranks
         out = []
         for r in self.trace.cpu().view(-1, TRACE_WORDS):
             t0 = int(r[0])
