@@ -62,6 +62,13 @@ __device__ __forceinline__ void store_tile(float* __restrict__ p, int m,
 }
 
 // a full tile at a 16-byte aligned address: no per-element checks
+__device__ __forceinline__ void load_tile_full(const float* __restrict__ p, float (&x)[kIter][4]) {
+#pragma unroll
+  for (int j = 0; j < kIter; ++j) {
+    const float4 v = reinterpret_cast<const float4*>(p)[j * kThreads + (int)threadIdx.x];
+    x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
+  }
+}
 __device__ __forceinline__ void store_tile_full(float* __restrict__ p, const float (&x)[kIter][4]) {
 #pragma unroll
   for (int j = 0; j < kIter; ++j)

@@ -693,6 +693,72 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   trace_mark(cm, E, 2);
 }
 
+// --------------------------------------------------------------------- one rank
+// A job of one rank has nobody to exchange with: a tile is encoded (twice through PS)
+// and decoded in registers, 16 bytes per element with error feedback (24 through PS).
+// Nothing waits, so the grid is one CTA per tile instead of what the GPU holds at once:
+// the hardware hands the next tile to whichever SM is free, and memory-bound SMs do not
+// run at one speed (a plain in-place streaming kernel reaches 6.15 TB/s with a fixed
+// share per CTA and 6.7 TB/s with one block per tile).  Bound by HBM
+// for onebit and TBQ: 102.8 M elements, TBQ ring 278 us (5.92 TB/s) in the persistent
+// kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us; TernGrad is bound by instruction
+// issue (ring 195 -> 146 us, PS 378 -> 214 us).
+template <int ALG, int B, int TOPO>
+__global__ void __launch_bounds__(kThreads, TOPO == HP_TOPO_PS && ALG != kTernGrad ? 3 : 4)
+local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
+  __shared__ TileSmem s;
+  int seg = 0;
+  while (seg + 1 < bk.nseg && blockIdx.x >= bk.seg[seg + 1].tile_prefix) ++seg;
+  const SegDev& sg = bk.seg[seg];
+  const uint32_t t = blockIdx.x - sg.tile_prefix;
+  const size_t off = (size_t)t * kTile;
+  const uint32_t left = sg.n - t * kTile;
+  const int m = (int)(left < (uint32_t)kTile ? left : (uint32_t)kTile);
+  const float* gp = sg.g + off;
+  float* rp = sg.r ? sg.r + off : nullptr;
+  float* sp = TOPO == HP_TOPO_PS && sg.sr ? sg.sr + off : nullptr;
+  float* op = sg.out + off;
+  const bool full = m == kTile && ((reinterpret_cast<uintptr_t>(gp) | reinterpret_cast<uintptr_t>(rp) |
+                                    reinterpret_cast<uintptr_t>(sp) | reinterpret_cast<uintptr_t>(op)) & 15) == 0;
+  trace_mark(cm, 0, 0);
+  // all loads of the tile go out before the first one is used
+  float x[kIter][4], rr[kIter][4], ss[kIter][4];
+  if (full) {
+    load_tile_full(gp, x);
+    if (rp) load_tile_full(rp, rr);
+    if (sp) load_tile_full(sp, ss);
+  } else {
+    load_tile(gp, m, x);
+    if (rp) load_tile(rp, m, rr);
+    if (sp) load_tile(sp, m, ss);
+  }
+  float meta[2];
+  uint32_t frag[kIter];
+#pragma unroll 1
+  for (int pass = 0;; ++pass) {
+    float* state = pass == 0 ? rp : sp;
+    if (state) {
+#pragma unroll
+      for (int j = 0; j < kIter; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[j][e] = (pass == 0 ? rr[j][e] : ss[j][e]) + x[j][e];
+    }
+    encode_tile<ALG, B>(x, m, fp.P, sg.id, off, fp.P.salt + (uint32_t)pass, s, meta, frag, state != nullptr);
+    if (state) {
+      if (full) store_tile_full(state, x);
+      else store_tile(state, m, x);
+    }
+    if (TOPO == HP_TOPO_RING || pass == 1) break;
+#pragma unroll
+    for (int j = 0; j < kIter; ++j) decode_frag<ALG, B>(frag[j], meta, fp.P.tau, x[j]);
+  }
+  decode_average<ALG, B>(frag, meta, fp, x);
+  if (full) store_tile_full(op, x);
+  else store_tile(op, m, x);
+  trace_mark(cm, 0, 1);
+  trace_mark(cm, 0, 2);
+}
+
 // ------------------------------------------------------------------ host side
 static int build_bucket(int alg, int bits, const HpSeg* segs, int nseg, int nranks,
                         BucketDev& bk) {
@@ -739,6 +805,11 @@ static int num_phases(int nranks) { return 2 * nranks - 1; }
 template <int ALG, int B>
 static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const FusedParams& fp,
                         int ctas, cudaStream_t st) {
+  if (cm.nranks == 1) {
+    if (topo == HP_TOPO_RING) local_dense_kernel<ALG, B, HP_TOPO_RING><<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
+    else local_dense_kernel<ALG, B, HP_TOPO_PS><<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
+    return (int)cudaGetLastError();
+  }
   void (*kern)(const BucketDev, const HpComm, const FusedParams) =
       topo == HP_TOPO_RING ? ring_dense_kernel<ALG, B> : ps_dense_kernel<ALG, B>;
   const size_t smem = sizeof(FusedSmem);
