@@ -170,17 +170,68 @@ __device__ __forceinline__ void decode_frag(uint32_t frag, const float (&meta)[2
   if (ALG == kTernGrad) gap = tern_gap(meta[0], meta[1], B);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    if (ALG == kTbq) {
+    if (ALG == kTernGrad) {
+      // the code as a float without a shift or a conversion (which run at an eighth of
+      // the rate of a multiply-add): its bits are or-ed in place into the mantissa of
+      // 2^23, and one exact multiply-add takes the place value and the 2^23 off again
+      const int sh = B == 8 ? 0 : e * B;
+      const uint32_t bits = B == 8 ? __byte_perm(frag, 0x4B000000u, 0x7650u | e)
+                                   : ((frag & (mask << sh)) | 0x4B000000u);
+      const float place = 1.0f / (float)(1u << sh);
+      const float q = fmaf(__uint_as_float(bits), place, -8388608.0f * place);
+      d[e] = fmaf(q, gap, meta[0]);   // tern_value
+    } else if (ALG == kTbq) {
       // tbq_value of the 2-bit code at bits 2e, 2e+1 by testing the bits in place
       // (bit 1: non-zero level, bit 0: positive)
       const bool nz = (frag & (2u << (e * B))) != 0u, pos = (frag & (1u << (e * B))) != 0u;
       d[e] = nz ? (pos ? tau : -tau) : 0.0f;
     } else {
-      const uint32_t c = (frag >> (e * B)) & mask;
-      if (ALG == kOnebit) d[e] = onebit_value(c, meta[0]);
-      else d[e] = tern_value(c, meta[0], gap);
+      d[e] = onebit_value((frag >> (e * B)) & mask, meta[0]);
     }
   }
+}
+
+// three-input minimum / maximum (sm_100a); like fminf / fmaxf they skip NaNs
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// Four TernGrad codes (tern_code of x[0..3] with the draws rnd16(v[e], half)) as the
+// fragment of one float4.  Bound by the integer pipe, which runs at half the rate of the
+// multiply-adds, and by the conversion unit at an eighth, so the work is moved off both:
+//   * up to 4 bits the position t = (x - min) * scale16 stays below 2^20, and its floor
+//     comes from adding 2^23 rounding down.  The product is taken 2^(16+B) smaller
+//     (exact), so that the saturating multiply maps NaN to 0 and infinity to a clamped
+//     code for free, and the multiply-add that adds 2^23 scales it back.  `scale` is
+//     scale16 / 2^(16+B) then.  8-bit positions need 24 bits: they are converted.
+//   * the draw is added and the sum clamped in one instruction; the code is byte 2
+//   * bytes are gathered with permutes, and for 1 and 2 bits packed with one dot product
+template <int B>
+__device__ __forceinline__ uint32_t tern_frag(const float (&x)[4], float mn, float scale, const Philox4& rnd,
+                                              uint32_t half) {
+  constexpr uint32_t qmax = (1u << B) - 1u;
+  uint32_t w[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const uint32_t u16 = rnd16(rnd.v[e], half);
+    if (B == 8) {
+      w[e] = __viaddmin_u32((uint32_t)f2i_floor_sat((x[e] - mn) * scale), u16, (qmax << 16) | 0xFFFFu);
+    } else {
+      const float y = __fmaf_rd(__saturatef((x[e] - mn) * scale), (float)(1u << (16 + B)), 8388608.0f);
+      w[e] = __viaddmin_u32(__float_as_uint(y), u16, 0x4B00FFFFu | (qmax << 16));
+    }
+  }
+  const uint32_t c = __byte_perm(__byte_perm(w[0], w[1], 0x0062), __byte_perm(w[2], w[3], 0x0062), 0x5410);
+  if (B == 8) return c;
+  if (B == 4) return __byte_perm(c | (c >> 4), 0u, 0x4420);
+  return __dp4a(c, B == 2 ? 0x40100401u : 0x08040201u, 0u);
 }
 
 // Quantise the register tile x (m valid elements).  On return frag[] holds the
@@ -208,19 +259,29 @@ __device__ __forceinline__ void encode_tile_impl(float (&x)[kIter][4], int m, co
 #pragma unroll
     for (int j = 0; j < kIter; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (FULL || 4 * (j * kThreads + (int)threadIdx.x) + e < m) {
+      for (int e = 0; e < 4; e += 2) {
+        const int i = 4 * (j * kThreads + (int)threadIdx.x) + e;
+        if (FULL || i + 1 < m) {
+          mn = fmin3(mn, x[j][e], x[j][e + 1]);
+          mx = fmax3(mx, x[j][e], x[j][e + 1]);
+        } else if (i < m) {
           mn = fminf(mn, x[j][e]);
           mx = fmaxf(mx, x[j][e]);
         }
+      }
     block_minmax(mn, mx, s);
     meta[0] = mn;
     meta[1] = mx;
   }
-  float gap = 0.0f, scale16 = 0.0f;
+  float gap = 0.0f, scale16 = 0.0f, scale = 0.0f;
+  bool fast = false;   // uniform over the tile: tern_frag applies
   if (ALG == kTernGrad) {
     gap = tern_gap(meta[0], meta[1], B);
     scale16 = tern_scale16(gap);
+    scale = B == 8 ? scale16 : scale16 * (1.0f / (float)(1u << (16 + B)));
+    // a scale that is no longer a normal number (a tile that spans more than about 2^120)
+    // would lose bits: such a tile takes the element-wise form below
+    fast = FULL && !ERR && (scale16 == 0.0f || scale >= 1.17549435e-38f);
   }
   // TernGrad: one Philox call per pair of rows (see rnd16_counter); a tile that does
   // not start on a 2048-element boundary of its tensor cannot share calls
@@ -235,6 +296,10 @@ __device__ __forceinline__ void encode_tile_impl(float (&x)[kIter][4], int m, co
       half = paired ? (uint32_t)(j & 1) : rnd16_half(ge);
       if (!paired || !(j & 1))
         rnd = philox4x32(rnd16_counter(ge), tensor_id, P.step, salt, P.seed_lo, P.seed_hi);
+    }
+    if (ALG == kTernGrad && fast) {
+      frag[j] = tern_frag<B>(x[j], meta[0], scale, rnd, half);
+      continue;
     }
     uint32_t f = 0u;
 #pragma unroll
