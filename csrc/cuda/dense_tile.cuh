@@ -22,10 +22,8 @@ constexpr int kIter = kTile / (kThreads * 4);  // float4 per thread per tile
 static_assert(kIter * kThreads * 4 == kTile, "tile must split evenly");
 
 struct TileSmem {
-  alignas(16) uint8_t codes[kTile];  // staged code bytes, up to 8 bits/element
-  double red_d[kThreads / 32];
-  float red_a[kThreads / 32];
-  float red_b[kThreads / 32];
+  double red_d[2][kThreads / 32];
+  float2 red_f[2][kThreads / 32];
 };
 
 // ------------------------------------------------------------------ memory ops
@@ -97,67 +95,57 @@ __device__ __forceinline__ uint32_t load_frag(const uint8_t* __restrict__ codes,
   }
 }
 
+__device__ __forceinline__ int tile_code_bytes(int m, int bits) {
+  return (int)align_up(((uint32_t)m * bits + 7) / 8, 16);
+}
+
+// The code bytes of one tile, straight from the registers: a warp's row is 16 to 128
+// consecutive bytes, so the stores are as wide as the codes allow and need no shared
+// memory and no barrier.  Bytes behind the last code of a partial tile are zero up to
+// the next multiple of 16.
 template <int B>
-__device__ __forceinline__ void stage_frags(uint8_t* sc, const uint32_t (&frag)[kIter]) {
+__device__ __forceinline__ void store_codes(uint8_t* __restrict__ dst, int m, const uint32_t (&frag)[kIter]) {
+  const int nbytes = tile_code_bytes(m, B);
 #pragma unroll
   for (int j = 0; j < kIter; ++j) {
     const int f = j * kThreads + (int)threadIdx.x;
     if (B == 1) {
       const uint32_t hi = __shfl_down_sync(0xffffffffu, frag[j], 1);
-      if (!(threadIdx.x & 1)) sc[f >> 1] = (uint8_t)(frag[j] | (hi << 4));
-    } else if (B == 2) {
-      sc[f] = (uint8_t)frag[j];
-    } else if (B == 4) {
-      reinterpret_cast<uint16_t*>(sc)[f] = (uint16_t)frag[j];
-    } else {
-      reinterpret_cast<uint32_t*>(sc)[f] = frag[j];
+      if (!(threadIdx.x & 1) && (f >> 1) < nbytes) dst[f >> 1] = (uint8_t)(frag[j] | (hi << 4));
+    } else if (f * B / 2 < nbytes) {
+      if (B == 2) dst[f] = (uint8_t)frag[j];
+      else if (B == 4) reinterpret_cast<uint16_t*>(dst)[f] = (uint16_t)frag[j];
+      else reinterpret_cast<uint32_t*>(dst)[f] = frag[j];
     }
   }
 }
 
-__device__ __forceinline__ int tile_code_bytes(int m, int bits) {
-  return (int)align_up(((uint64_t)m * bits + 7) / 8, 16);
-}
-
-// 16-byte stores; dst may be a peer GPU's memory (plain st.global over NVLink).
-__device__ __forceinline__ void copy_codes(uint8_t* __restrict__ dst, const uint8_t* sc,
-                                           int nbytes) {
-  for (int o = (int)threadIdx.x * 16; o < nbytes; o += kThreads * 16)
-    *reinterpret_cast<uint4*>(dst + o) = *reinterpret_cast<const uint4*>(sc + o);
-}
-
 // ------------------------------------------------------------- block reductions
-// All 256 threads must call; every thread returns the same value.
-__device__ __forceinline__ double block_sum(double v, TileSmem& s) {
+// All 256 threads must call; every thread returns the same value.  One barrier each:
+// `buf` (0 or 1) picks the shared array, and two calls with no other barrier in between
+// take different ones.
+__device__ __forceinline__ double block_sum(double v, TileSmem& s, int buf) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) s.red_d[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) s.red_d[buf][threadIdx.x >> 5] = v;
   __syncthreads();
   double t = 0.0;
 #pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) t += s.red_d[w];
-  __syncthreads();
+  for (int w = 0; w < kThreads / 32; ++w) t += s.red_d[buf][w];
   return t;
 }
 
 // Warp level: one redux.sync.{min,max}.f32 each (the fp32 forms of the warp
-// reduction are sm_100a instructions) instead of five shuffle + compare rounds.
-__device__ __forceinline__ void block_minmax(float& mn, float& mx, TileSmem& s) {
+// reduction are sm_100a instructions) instead of five shuffle + compare rounds; every
+// warp reduces the eight partial results the same way.
+__device__ __forceinline__ void block_minmax(float& mn, float& mx, TileSmem& s, int buf) {
   asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(mn) : "f"(mn));
   asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(mx));
-  if ((threadIdx.x & 31) == 0) {
-    s.red_a[threadIdx.x >> 5] = mn;
-    s.red_b[threadIdx.x >> 5] = mx;
-  }
+  if ((threadIdx.x & 31) == 0) s.red_f[buf][threadIdx.x >> 5] = make_float2(mn, mx);
   __syncthreads();
-  mn = s.red_a[0];
-  mx = s.red_b[0];
-#pragma unroll
-  for (int w = 1; w < kThreads / 32; ++w) {
-    mn = fminf(mn, s.red_a[w]);
-    mx = fmaxf(mx, s.red_b[w]);
-  }
-  __syncthreads();
+  const float2 v = s.red_f[buf][threadIdx.x & (kThreads / 32 - 1)];
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(mn) : "f"(v.x));
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(v.y));
 }
 
 // ------------------------------------------------------------------ algorithms
@@ -241,7 +229,7 @@ __device__ __forceinline__ uint32_t tern_frag(const float (&x)[4], float mn, flo
 template <int ALG, int B, bool FULL, bool ERR>
 __device__ __forceinline__ void encode_tile_impl(float (&x)[kIter][4], int m, const DenseParams& P,
                                                  uint32_t tensor_id, uint64_t elem0, uint32_t salt,
-                                                 TileSmem& s, float (&meta)[2],
+                                                 TileSmem& s, int buf, float (&meta)[2],
                                                  uint32_t (&frag)[kIter]) {
   meta[0] = 0.0f;
   meta[1] = 0.0f;
@@ -252,36 +240,26 @@ __device__ __forceinline__ void encode_tile_impl(float (&x)[kIter][4], int m, co
 #pragma unroll
       for (int e = 0; e < 4; ++e)
         if (FULL || 4 * (j * kThreads + (int)threadIdx.x) + e < m) part += (double)fabsf(x[j][e]);
-    const double tot = block_sum(part, s);
+    const double tot = block_sum(part, s, buf);
     meta[0] = (float)(tot / (double)m);
   } else if (ALG == kTernGrad) {
     float mn = INFINITY, mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < kIter; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const int i = 4 * (j * kThreads + (int)threadIdx.x) + e;
-        if (FULL || i + 1 < m) {
-          mn = fmin3(mn, x[j][e], x[j][e + 1]);
-          mx = fmax3(mx, x[j][e], x[j][e + 1]);
-        } else if (i < m) {
+      for (int e = 0; e < 4; ++e)
+        if (FULL || 4 * (j * kThreads + (int)threadIdx.x) + e < m) {
           mn = fminf(mn, x[j][e]);
           mx = fmaxf(mx, x[j][e]);
         }
-      }
-    block_minmax(mn, mx, s);
+    block_minmax(mn, mx, s, buf);
     meta[0] = mn;
     meta[1] = mx;
   }
-  float gap = 0.0f, scale16 = 0.0f, scale = 0.0f;
-  bool fast = false;   // uniform over the tile: tern_frag applies
+  float gap = 0.0f, scale16 = 0.0f;
   if (ALG == kTernGrad) {
     gap = tern_gap(meta[0], meta[1], B);
     scale16 = tern_scale16(gap);
-    scale = B == 8 ? scale16 : scale16 * (1.0f / (float)(1u << (16 + B)));
-    // a scale that is no longer a normal number (a tile that spans more than about 2^120)
-    // would lose bits: such a tile takes the element-wise form below
-    fast = FULL && !ERR && (scale16 == 0.0f || scale >= 1.17549435e-38f);
   }
   // TernGrad: one Philox call per pair of rows (see rnd16_counter); a tile that does
   // not start on a 2048-element boundary of its tensor cannot share calls
@@ -296,10 +274,6 @@ __device__ __forceinline__ void encode_tile_impl(float (&x)[kIter][4], int m, co
       half = paired ? (uint32_t)(j & 1) : rnd16_half(ge);
       if (!paired || !(j & 1))
         rnd = philox4x32(rnd16_counter(ge), tensor_id, P.step, salt, P.seed_lo, P.seed_hi);
-    }
-    if (ALG == kTernGrad && fast) {
-      frag[j] = tern_frag<B>(x[j], meta[0], scale, rnd, half);
-      continue;
     }
     uint32_t f = 0u;
 #pragma unroll
@@ -327,45 +301,67 @@ __device__ __forceinline__ void encode_tile_impl(float (&x)[kIter][4], int m, co
   }
 }
 
-template <int ALG, int B>
-__device__ __forceinline__ void encode_tile(float (&x)[kIter][4], int m, const DenseParams& P,
-                                            uint32_t tensor_id, uint64_t elem0, uint32_t salt,
-                                            TileSmem& s, float (&meta)[2],
-                                            uint32_t (&frag)[kIter], bool want_err = true) {
-  if (ALG == kTernGrad && !want_err) {
-    if (m == kTile) encode_tile_impl<ALG, B, true, false>(x, m, P, tensor_id, elem0, salt, s, meta, frag);
-    else encode_tile_impl<ALG, B, false, false>(x, m, P, tensor_id, elem0, salt, s, meta, frag);
+// The usual TernGrad tile: full, no residual, on a 2048-element boundary of its tensor.
+// The draws do not depend on the data, so they are made while its loads are in flight.
+template <int B>
+__device__ __forceinline__ void tern_encode_full(float (&x)[kIter][4], const DenseParams& P, uint32_t tensor_id,
+                                                 uint64_t elem0, uint32_t salt, TileSmem& s, int buf,
+                                                 float (&meta)[2], uint32_t (&frag)[kIter]) {
+  static_assert(kIter == 4, "one draw serves two rows");
+  Philox4 rnd[2];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+    rnd[p] = philox4x32(rnd16_counter(elem0 + 4u * (2 * p * kThreads + threadIdx.x)), tensor_id, P.step, salt,
+                        P.seed_lo, P.seed_hi);
+  float mn = fmin3(x[0][0], x[0][1], x[0][2]), mx = fmax3(x[0][0], x[0][1], x[0][2]);
+  mn = fminf(mn, x[0][3]);
+  mx = fmaxf(mx, x[0][3]);
+#pragma unroll
+  for (int j = 1; j < kIter; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+      mn = fmin3(mn, x[j][e], x[j][e + 1]);
+      mx = fmax3(mx, x[j][e], x[j][e + 1]);
+    }
+  if (mn != mn) { mn = INFINITY; mx = -INFINITY; }   // sixteen NaNs
+  block_minmax(mn, mx, s, buf);
+  meta[0] = mn;
+  meta[1] = mx;
+  const float scale16 = tern_scale16(tern_gap(mn, mx, B));
+  const float scale = B == 8 ? scale16 : scale16 * (1.0f / (float)(1u << (16 + B)));
+  if (scale16 == 0.0f || scale >= 1.17549435e-38f) {
+#pragma unroll
+    for (int j = 0; j < kIter; ++j) frag[j] = tern_frag<B>(x[j], mn, scale, rnd[j >> 1], j & 1);
   } else {
-    if (m == kTile) encode_tile_impl<ALG, B, true, true>(x, m, P, tensor_id, elem0, salt, s, meta, frag);
-    else encode_tile_impl<ALG, B, false, true>(x, m, P, tensor_id, elem0, salt, s, meta, frag);
+    // a scale that is no longer a normal number (the tile spans more than about 2^120)
+    // would lose bits: element by element
+#pragma unroll
+    for (int j = 0; j < kIter; ++j) {
+      uint32_t f = 0u;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        f |= tern_code(x[j][e], mn, scale16, rnd16(rnd[j >> 1].v[e], j & 1), B) << (e * B);
+      frag[j] = f;
+    }
   }
 }
 
-// Byte layout of one dense payload of `n_layout` elements (n_layout fixes where
-// the code region starts; fewer elements may actually be valid).
-struct PayloadView {
-  uint8_t* base;
-  float* meta;
-  uint8_t* codes;
-};
-__device__ __forceinline__ PayloadView payload_view(uint8_t* base, int alg, uint64_t n_layout) {
-  PayloadView v;
-  v.base = base;
-  v.meta = reinterpret_cast<float*>(base + 16);
-  v.codes = base + 16 + dense_meta_bytes(alg, n_layout);
-  return v;
-}
-
-__device__ __forceinline__ void write_header(uint8_t* base, uint32_t n, int alg, int bits,
-                                             float tau) {
-  WireHeader h;
-  h.n = n;
-  h.alg = (uint8_t)alg;
-  h.bitwidth = (uint8_t)bits;
-  h.flags = dense_meta_floats(alg) ? 1 : 0;
-  h.a = alg == kTbq ? tau : 0.0f;
-  h.b = kTile;
-  *reinterpret_cast<uint4*>(base) = *reinterpret_cast<const uint4*>(&h);
+template <int ALG, int B>
+__device__ __forceinline__ void encode_tile(float (&x)[kIter][4], int m, const DenseParams& P,
+                                            uint32_t tensor_id, uint64_t elem0, uint32_t salt,
+                                            TileSmem& s, int buf, float (&meta)[2],
+                                            uint32_t (&frag)[kIter], bool want_err = true) {
+  if (ALG == kTernGrad) {
+    if (!want_err && m == kTile && (elem0 & 2047u) == 0)
+      tern_encode_full<B>(x, P, tensor_id, elem0, salt, s, buf, meta, frag);
+    else if (!want_err)
+      encode_tile_impl<ALG, B, false, false>(x, m, P, tensor_id, elem0, salt, s, buf, meta, frag);
+    else
+      encode_tile_impl<ALG, B, false, true>(x, m, P, tensor_id, elem0, salt, s, buf, meta, frag);
+  } else {
+    if (m == kTile) encode_tile_impl<ALG, B, true, true>(x, m, P, tensor_id, elem0, salt, s, buf, meta, frag);
+    else encode_tile_impl<ALG, B, false, true>(x, m, P, tensor_id, elem0, salt, s, buf, meta, frag);
+  }
 }
 
 // read tile metadata that may have been written by a peer

@@ -508,7 +508,7 @@ __device__ __forceinline__ void encode_phases(const BucketDev& bk, const HpComm&
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[j][e] = rr[j][e] + x[j][e];
         }
-        encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt + (uint32_t)pass, sm.tile,
+        encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt + (uint32_t)pass, sm.tile, pass,
                             meta, frag, rp != nullptr);
         // after an expired wait the merged input is not a real partial sum: the error
         // feedback state keeps its last good contents
@@ -703,8 +703,9 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 // for onebit and TBQ: 102.8 M elements, TBQ ring 278 us (5.92 TB/s) in the persistent
 // kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us; TernGrad is bound by instruction
 // issue (ring 195 -> 146 us, PS 378 -> 214 us).
-template <int ALG, int B, int TOPO>
-__global__ void __launch_bounds__(kThreads, TOPO == HP_TOPO_PS && ALG != kTernGrad ? 3 : 4)
+// RES: some tensor of the bucket keeps error-feedback state.
+template <int ALG, int B, int TOPO, bool RES>
+__global__ void __launch_bounds__(kThreads, TOPO == HP_TOPO_PS && RES ? 3 : 4)
 local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   __shared__ TileSmem s;
   int seg = 0;
@@ -715,8 +716,8 @@ local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   const uint32_t left = sg.n - t * kTile;
   const int m = (int)(left < (uint32_t)kTile ? left : (uint32_t)kTile);
   const float* gp = sg.g + off;
-  float* rp = sg.r ? sg.r + off : nullptr;
-  float* sp = TOPO == HP_TOPO_PS && sg.sr ? sg.sr + off : nullptr;
+  float* rp = RES && sg.r ? sg.r + off : nullptr;
+  float* sp = RES && TOPO == HP_TOPO_PS && sg.sr ? sg.sr + off : nullptr;
   float* op = sg.out + off;
   const bool full = m == kTile && ((reinterpret_cast<uintptr_t>(gp) | reinterpret_cast<uintptr_t>(rp) |
                                     reinterpret_cast<uintptr_t>(sp) | reinterpret_cast<uintptr_t>(op)) & 15) == 0;
@@ -743,7 +744,7 @@ local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) x[j][e] = (pass == 0 ? rr[j][e] : ss[j][e]) + x[j][e];
     }
-    encode_tile<ALG, B>(x, m, fp.P, sg.id, off, fp.P.salt + (uint32_t)pass, s, meta, frag, state != nullptr);
+    encode_tile<ALG, B>(x, m, fp.P, sg.id, off, fp.P.salt + (uint32_t)pass, s, pass, meta, frag, state != nullptr);
     if (state) {
       if (full) store_tile_full(state, x);
       else store_tile(state, m, x);
@@ -806,8 +807,13 @@ template <int ALG, int B>
 static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const FusedParams& fp,
                         int ctas, cudaStream_t st) {
   if (cm.nranks == 1) {
-    if (topo == HP_TOPO_RING) local_dense_kernel<ALG, B, HP_TOPO_RING><<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
-    else local_dense_kernel<ALG, B, HP_TOPO_PS><<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
+    bool res = false;
+    for (int i = 0; i < bk.nseg; ++i) res = res || bk.seg[i].r || bk.seg[i].sr;
+    auto kern = topo == HP_TOPO_RING ? (res ? local_dense_kernel<ALG, B, HP_TOPO_RING, true>
+                                            : local_dense_kernel<ALG, B, HP_TOPO_RING, false>)
+                                     : (res ? local_dense_kernel<ALG, B, HP_TOPO_PS, true>
+                                            : local_dense_kernel<ALG, B, HP_TOPO_PS, false>);
+    kern<<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
     return (int)cudaGetLastError();
   }
   void (*kern)(const BucketDev, const HpComm, const FusedParams) =
