@@ -22,8 +22,11 @@ struct PayloadPtrs {
 // with a block per tile the hardware gives the next tile to whichever is free (TBQ
 // encode with an incoming payload, 16.8 M elements: 38.8 us with 1184 CTAs striding over
 // the tiles, 31.0 us = 6.75 TB/s with a CTA per tile).
+// TernGrad without state needs few registers and has a long chain between a tile's loads
+// and its stores: six CTAs per SM hide it better than four (67.1 M elements 66 -> 61 us);
+// the others are at HBM speed with four and slightly slower with more.
 template <int ALG, int B, bool IN, bool RES>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, ALG == kTernGrad && !RES ? 6 : 4)
 dense_encode_kernel(const float* __restrict__ g, float* __restrict__ r, const PayloadPtrs in,
                     const PayloadPtrs out, const WireHeader hdr, uint32_t n, uint32_t tiles, DenseParams P,
                     uint32_t tensor_id, uint64_t elem_offset) {

@@ -702,10 +702,11 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 // share per CTA and 6.7 TB/s with one block per tile).  Bound by HBM
 // for onebit and TBQ: 102.8 M elements, TBQ ring 278 us (5.92 TB/s) in the persistent
 // kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us; TernGrad is bound by instruction
-// issue (ring 195 -> 146 us, PS 378 -> 214 us).
+// issue and latency (ring 195 -> 124 us, PS 378 -> 173 us, with six CTAs per SM where
+// no state is kept).
 // RES: some tensor of the bucket keeps error-feedback state.
 template <int ALG, int B, int TOPO, bool RES>
-__global__ void __launch_bounds__(kThreads, TOPO == HP_TOPO_PS && RES ? 3 : 4)
+__global__ void __launch_bounds__(kThreads, RES ? (TOPO == HP_TOPO_PS ? 3 : 4) : 6)
 local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   __shared__ TileSmem s;
   int seg = 0;
