@@ -99,6 +99,20 @@ int hp_cuda_enable_peer(int dev, int peer) {
   return (int)e;
 }
 
+// Ordering between two streams: work launched on dst from here on runs behind what src
+// holds now.  One event serves any number of calls (a wait refers to the record that
+// preceded it).
+int hp_cuda_event_create(void** ev) {
+  return (int)cudaEventCreateWithFlags(reinterpret_cast<cudaEvent_t*>(ev), cudaEventDisableTiming);
+}
+int hp_cuda_event_destroy(void* ev) { return (int)cudaEventDestroy((cudaEvent_t)ev); }
+int hp_cuda_stream_order(void* ev, void* src, void* dst) {
+  if (src == dst) return 0;
+  cudaError_t e = cudaEventRecord((cudaEvent_t)ev, (cudaStream_t)src);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent((cudaStream_t)dst, (cudaEvent_t)ev, 0);
+  return (int)e;
+}
+
 int hp_cuda_peer_store(const void* src, void* dst, uint64_t bytes, int ctas, void* stream) {
   if (bytes % 16) return HP_ERR_BAD_ARG;
   if (ctas <= 0) ctas = 148 * 4;

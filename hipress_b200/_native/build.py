@@ -1,10 +1,11 @@
-"""Builds the two native libraries in-tree.
+"""Builds the native libraries in-tree.
 
 ``libhipress_cpu.so``  g++   CPU oracle, planner cost model, host runtime
 ``libhipress_cuda.so`` nvcc  sm_100a kernels (``-gencode arch=compute_100a,code=sm_100a``)
+``_fastcall.so``       g++   CPython extension for the calls made once per tensor or bucket
 
-Both expose a plain C ABI that :mod:`hipress_b200._native.lib` binds with ctypes,
-so neither needs the PyTorch headers and a full rebuild takes well under a minute.
+The first two expose a plain C ABI that :mod:`hipress_b200._native.lib` binds with
+ctypes; none needs the PyTorch headers and a full rebuild takes well under a minute.
 Run ``python -m hipress_b200._native.build`` (add ``--force`` to rebuild).
 """
 from __future__ import annotations
@@ -14,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -98,7 +100,8 @@ def build(force: bool = False, verbose: bool = False) -> dict:
     """Compile whatever is out of date; returns the paths of the libraries."""
     cpu_src, cuda_src = _sources()
     OBJ.mkdir(exist_ok=True)
-    out = {"cpu": HERE / "libhipress_cpu.so", "cuda": HERE / "libhipress_cuda.so"}
+    out = {"cpu": HERE / "libhipress_cpu.so", "fast": HERE / "_fastcall.so",
+           "cuda": HERE / "libhipress_cuda.so"}
     inc = ["-I", str(CSRC / "include")]
     with open(OBJ / "build.log", "a") as log:
         stamp = OBJ / "cpu.sha"
@@ -108,6 +111,15 @@ def build(force: bool = False, verbose: bool = False) -> dict:
             stamp.write_text(dg)
             if verbose:
                 print("built", out["cpu"])
+        fast_src = sorted((CSRC / "host").glob("*.cpp"))
+        stamp = OBJ / "fast.sha"
+        dg = _digest(fast_src) + sys.version
+        if force or not out["fast"].exists() or not stamp.exists() or stamp.read_text() != dg:
+            _run(["g++", *GXX_FLAGS, "-Wno-unknown-pragmas", *inc, "-I", sysconfig.get_path("include"), "-shared",
+                  "-o", str(out["fast"]), *map(str, fast_src)], log)
+            stamp.write_text(dg)
+            if verbose:
+                print("built", out["fast"])
         nv = nvcc_path()
         if nv is None:
             if not out["cuda"].exists():

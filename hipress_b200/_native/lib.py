@@ -11,6 +11,8 @@ import ctypes as C
 import os
 from pathlib import Path
 
+import torch
+
 HERE = Path(__file__).resolve().parent
 
 MAX_RANKS = 8
@@ -43,6 +45,8 @@ class HpComm(C.Structure):
 
 _cpu = None
 _cuda = None
+_fast = None
+_fast_cuda = None
 
 
 def _ensure_built():
@@ -125,10 +129,6 @@ def cuda():
     vp = C.c_void_p
     _sig(L.hp_cuda_device_count, C.c_int)
     _sig(L.hp_cuda_error_string, C.c_char_p, C.c_int)
-    _sig(L.hp_cuda_dense_encode, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, C.c_uint64, C.c_float,
-         C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint64, C.c_int, vp)
-    _sig(L.hp_cuda_dense_decode, C.c_int, C.c_int, C.c_int, vp, vp, C.c_uint64, C.c_float,
-         C.c_float, C.c_int, C.c_int, vp)
     _sig(L.hp_fused_dense_layout, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_uint64),
          C.c_int, C.c_int, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64), C.POINTER(C.c_uint32))
     _sig(L.hp_fused_chunk_elems, C.c_uint64, C.c_uint64, C.c_int)
@@ -137,10 +137,7 @@ def cuda():
     _sig(L.hp_cuda_fused_dense, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(HpSeg), C.c_int,
          C.POINTER(HpComm), C.c_float, C.c_uint64, C.c_uint32, C.c_uint32, C.c_int, vp)
     _sig(L.hp_sparse_workspace_bytes, C.c_uint64)
-    _sig(L.hp_cuda_sparse_encode, C.c_int, C.c_int, vp, vp, vp, C.c_uint64, C.c_uint64,
-         C.c_uint64, C.c_float, C.c_int, vp, vp, C.c_uint64, C.c_int, vp)
     _sig(L.hp_sparse_workspace_bytes_for, C.c_uint64, C.c_uint64)
-    _sig(L.hp_cuda_sparse_decode, C.c_int, vp, vp, C.c_uint64, C.c_uint64, C.c_float, C.c_int, vp)
     _sig(L.hp_cuda_arena_alloc, C.c_int, C.c_uint64, C.POINTER(C.c_void_p))
     _sig(L.hp_cuda_arena_free, C.c_int, vp)
     _sig(L.hp_cuda_ipc_handle_bytes, C.c_int)
@@ -148,6 +145,9 @@ def cuda():
     _sig(L.hp_cuda_ipc_open, C.c_int, vp, C.POINTER(C.c_void_p))
     _sig(L.hp_cuda_ipc_close, C.c_int, vp)
     _sig(L.hp_cuda_enable_peer, C.c_int, C.c_int, C.c_int)
+    _sig(L.hp_cuda_event_create, C.c_int, C.POINTER(C.c_void_p))
+    _sig(L.hp_cuda_event_destroy, C.c_int, vp)
+    _sig(L.hp_cuda_stream_order, C.c_int, vp, vp, vp)
     _sig(L.hp_cuda_peer_store, C.c_int, vp, vp, C.c_uint64, C.c_int, vp)
     _sig(L.hp_cuda_wait_probe, C.c_int, vp, C.c_uint32, C.c_uint64, vp, vp)
     _sig(L.hp_cuda_set_flag, C.c_int, vp, C.c_uint32, vp)
@@ -162,6 +162,46 @@ def cuda():
 
 
 _CUDA_OPTIONAL: dict = {}
+
+
+def fast():
+    """The extension module ``_fastcall`` (csrc/host/fastcall.cpp): sizes, and -- once
+    :func:`fast_cuda` has bound them -- the per-tensor and per-bucket CUDA calls."""
+    global _fast
+    if _fast is None:
+        path = HERE / "_fastcall.so"
+        err = None
+        if not path.exists() or os.environ.get("HIPRESS_REBUILD"):
+            err = _ensure_built()
+        if not path.exists():
+            raise NativeLibraryError(f"{path} missing and could not be built: {err}")
+        from . import _fastcall
+        _fast = _fastcall
+    return _fast
+
+
+def fast_cuda():
+    """:func:`fast`, calling the CUDA library that :func:`cuda` loads."""
+    global _fast_cuda
+    if _fast_cuda is None:
+        L, F = cuda(), fast()
+        F.bind({n: C.cast(getattr(L, n), C.c_void_p).value for n in F.symbols()})
+        _fast_cuda = F
+    return _fast_cuda
+
+
+class OrderEvent:
+    """An event that orders one stream behind another (``stream_order``)."""
+
+    def __init__(self):
+        e = C.c_void_p()
+        check(cuda().hp_cuda_event_create(C.byref(e)), "event create")
+        self.handle = e.value
+
+    def __del__(self):
+        h, self.handle = getattr(self, "handle", None), None
+        if h is not None and _cuda is not None:
+            _cuda.hp_cuda_event_destroy(h)
 
 
 def check(code: int, what: str = "native call", device_call: bool = True):
@@ -183,6 +223,7 @@ def ptr(t):
 
 
 def stream_ptr(stream=None):
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """Handle of ``stream``, or of the current stream of the current device."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

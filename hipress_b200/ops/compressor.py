@@ -35,13 +35,13 @@ class Compressor:
 
     # ------------------------------------------------------------------ sizes
     def kmax(self, n: int) -> int:
-        return int(_lib.cpu().hp_sparse_k(n, self.spec.ratio)) if self.spec.sparse else 0
+        return _lib.fast().sparse_k(n, self.spec.ratio) if self.spec.sparse else 0
 
     def payload_bytes(self, n: int) -> int:
-        L = _lib.cpu()
-        if self.spec.sparse:
-            return int(L.hp_sparse_payload_bytes(self.kmax(n)))
-        return int(L.hp_dense_payload_bytes(self.spec.alg, self.spec.bits, n))
+        F, sp = _lib.fast(), self.spec
+        if sp.sparse:
+            return F.sparse_payload_bytes(F.sparse_k(n, sp.ratio))
+        return F.dense_payload_bytes(sp.alg, sp.bits, n)
 
     def new_state(self, n: int, device) -> dict:
         return {k: torch.zeros(n, dtype=torch.float32, device=device) for k in self.spec.state_names()}
@@ -71,7 +71,7 @@ class Compressor:
         n = g.numel()
         state = state or {}
         if out is None:
-            nb = self.payload_bytes(n) if kmax is None else int(_lib.cpu().hp_sparse_payload_bytes(kmax))
+            nb = self.payload_bytes(n) if kmax is None else _lib.fast().sparse_payload_bytes(kmax)
             out = torch.empty(nb, dtype=torch.uint8, device=g.device)
         if n == 0:
             return out
@@ -80,15 +80,17 @@ class Compressor:
             return self._encode_sparse(g, state, incoming, out, update, workspace, kmax, stream, max_ctas)
         r = state.get("residual") if sp.error_feedback else None
         if g.is_cuda:
-            L = _lib.cuda()
-            rc = L.hp_cuda_dense_encode(sp.alg, sp.bits, _c(g), _c(r), _c(incoming), _c(out), n,
-                                        sp.threshold, sp.seed, step, salt, tensor_id, elem_offset,
-                                        max_ctas, _lib.stream_ptr(stream))
+            # straight into the native call: a small tensor's kernel is shorter than a
+            # ctypes call with these arguments
+            rc = _lib.fast_cuda().dense_encode(sp.alg, sp.bits, g.data_ptr(), _c(r), _c(incoming), out.data_ptr(), n,
+                                               sp.threshold, sp.seed, step, salt, tensor_id, elem_offset, max_ctas,
+                                               _lib.stream_ptr(stream))
         else:
             rc = _lib.cpu().hp_cpu_dense_encode(sp.alg, sp.bits, _c(g), _c(r), _c(incoming), _c(out),
                                                 n, sp.threshold, sp.seed, step, salt, tensor_id,
                                                 elem_offset)
-        _lib.check(rc, f"{sp.name} encode", device_call=g.is_cuda)
+        if rc:
+            _lib.check(rc, f"{sp.name} encode", device_call=g.is_cuda)
         return out
 
     def _encode_sparse(self, g, state, incoming, out, update, workspace, kmax, stream, max_ctas):
@@ -99,17 +101,16 @@ class Compressor:
         a = state["accum_v"] if "accum_v" in state else state["residual"]
         u = state.get("momentum_u")
         if g.is_cuda:
-            L = _lib.cuda()
-            sptr = _lib.stream_ptr(stream)
             ws = workspace if workspace is not None else self.new_workspace(g.device, n)
             if incoming is not None:
                 # the accumulator must hold the updated local value before the merge
                 raise ValueError("merge incoming sparse payloads with decode(accumulate=True) "
                                  "after update_state(); then call encode(update=False)")
-            rc = L.hp_cuda_sparse_encode(sp.alg, _c(g), _c(a), _c(u), n, k, kmax, sp.momentum,
-                                         1 if update else 0, _c(out), _c(ws), ws.numel() * 4, max_ctas,
-                                         sptr)
-            _lib.check(rc, f"{sp.name} encode")
+            rc = _lib.fast_cuda().sparse_encode(sp.alg, _c(g), _c(a), _c(u), n, k, kmax, sp.momentum,
+                                                1 if update else 0, _c(out), _c(ws), ws.numel() * 4, max_ctas,
+                                                _lib.stream_ptr(stream))
+            if rc:
+                _lib.check(rc, f"{sp.name} encode")
             return out
         L = _lib.cpu()
         if update:
@@ -155,22 +156,22 @@ class Compressor:
         if n == 0:
             return out
         assert out.dtype == torch.float32 and out.is_contiguous()
-        if sp.sparse:
-            kmax = self.kmax(n) if kmax is None else kmax
-            if out.is_cuda:
-                rc = _lib.cuda().hp_cuda_sparse_decode(_c(payload), _c(out), n, kmax, scale,
-                                                       1 if accumulate else 0, _lib.stream_ptr(stream))
+        acc = 1 if accumulate else 0
+        if sp.sparse and kmax is None:
+            kmax = self.kmax(n)
+        if out.is_cuda:
+            F, st = _lib.fast_cuda(), _lib.stream_ptr(stream)
+            if sp.sparse:
+                rc = F.sparse_decode(payload.data_ptr(), out.data_ptr(), n, kmax, scale, acc, st)
             else:
-                rc = _lib.cpu().hp_cpu_sparse_decode(_c(payload), _c(out), n, kmax, scale,
-                                                     1 if accumulate else 0)
-        elif out.is_cuda:
-            rc = _lib.cuda().hp_cuda_dense_decode(sp.alg, sp.bits, _c(payload), _c(out), n,
-                                                  sp.threshold, scale, 1 if accumulate else 0,
-                                                  max_ctas, _lib.stream_ptr(stream))
+                rc = F.dense_decode(sp.alg, sp.bits, payload.data_ptr(), out.data_ptr(), n, sp.threshold, scale, acc,
+                                    max_ctas, st)
+        elif sp.sparse:
+            rc = _lib.cpu().hp_cpu_sparse_decode(_c(payload), _c(out), n, kmax, scale, acc)
         else:
-            rc = _lib.cpu().hp_cpu_dense_decode(sp.alg, sp.bits, _c(payload), _c(out), n,
-                                                sp.threshold, scale, 1 if accumulate else 0)
-        _lib.check(rc, f"{sp.name} decode", device_call=out.is_cuda)
+            rc = _lib.cpu().hp_cpu_dense_decode(sp.alg, sp.bits, _c(payload), _c(out), n, sp.threshold, scale, acc)
+        if rc:
+            _lib.check(rc, f"{sp.name} decode", device_call=out.is_cuda)
         return out
 
     _PAYLOAD_FAULTS = {1: "buffer shorter than the format needs", 2: "algorithm id", 3: "bit width",
