@@ -128,7 +128,7 @@ __device__ __forceinline__ uint32_t ll_finish(const uint2* slot, uint2 v, const 
       // that run next to this kernel while a peer is late
       if (polls > 4) __nanosleep(polls > 64 ? 400 : 100);
       if ((++polls & 63u) == 0 && (*poisoned || global_timer_ns() - t0 > cm.timeout_ns)) {
-        atomicCAS(status, 0u, code);
+        record_status(status, code);
         *poisoned = 1;
         break;
       }
@@ -136,7 +136,7 @@ __device__ __forceinline__ uint32_t ll_finish(const uint2* slot, uint2 v, const 
     if (cm.trace && threadIdx.x == 0) ws.spin_ns += global_timer_ns() - t0;
   }
   if (v.y == (cm.epoch | kGaveUp) && !*poisoned) {
-    atomicCAS(status, 0u, code | HP_STATUS_UPSTREAM);
+    record_status(status, code | HP_STATUS_UPSTREAM);
     *poisoned = 1;
   }
   return v.x;
@@ -182,7 +182,7 @@ __device__ __forceinline__ bool dbg_tile_ok(const BucketDev& bk, const void* inb
   const uint64_t limit = bk.dbg_limit ? bk.dbg_limit : bk.inbox_bytes;
   const uint64_t end = (uint64_t)(payload - lo) + (uint64_t)(t + 1) * tile_slots<ALG, B>() * 8ull;
   if (payload < lo || end > limit) {
-    atomicCAS(status, 0u, HP_STATUS_BOUNDS | what);
+    record_status(status, HP_STATUS_BOUNDS | what);
     return false;
   }
 #endif

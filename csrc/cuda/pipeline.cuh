@@ -65,7 +65,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   uint32_t polls = 0;
   while (!mbar_try_wait(bar, parity)) {
     if ((++polls & 255u) == 0 && global_timer_ns() - t0 > timeout_ns) {
-      atomicCAS(status, 0u, code);
+      record_status(status, code);
       return false;
     }
   }

@@ -24,6 +24,15 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
+// The first status word recorded stays.  `status` is this GPU's memory or pinned host
+// memory the kernel sees (the training loop reads the latter without a copy), so plain
+// accesses instead of an atomic: of several waits that expire at the same moment any
+// one may be the word that remains.
+__device__ __forceinline__ void record_status(uint32_t* status, uint32_t code) {
+  volatile uint32_t* s = status;
+  if (*s == 0u) *s = code;
+}
+
 struct WaitState {
   int poisoned;
   unsigned long long spin_ns;  // time thread 0 spent polling (only kept when tracing)
@@ -58,7 +67,7 @@ __device__ __forceinline__ void wait_flag(const uint32_t* flag, uint32_t epoch, 
         ++polls;
         if ((polls & 63) == 0 &&
             (global_timer_ns() - t0 > timeout_ns || polls > max_polls)) {
-          atomicCAS(status, 0u, code);
+          record_status(status, code);
           ws.poisoned = 1;
           break;
         }
@@ -66,7 +75,7 @@ __device__ __forceinline__ void wait_flag(const uint32_t* flag, uint32_t epoch, 
       }
     }
     if (v == (epoch | kGaveUp) && !ws.poisoned) {
-      atomicCAS(status, 0u, code | 0x40000000u);  // HP_STATUS_UPSTREAM
+      record_status(status, code | 0x40000000u);  // HP_STATUS_UPSTREAM
       ws.poisoned = 1;
     }
   }
@@ -95,7 +104,7 @@ __device__ __forceinline__ void grid_barrier(uint32_t* count, uint32_t& gen, uin
       uint64_t polls = 0;
       while (*vc < target) {
         if ((++polls & 255) == 0 && global_timer_ns() - t0 > timeout_ns) {
-          atomicCAS(status, 0u, code);
+          record_status(status, code);
           ws.poisoned = 1;
           break;
         }

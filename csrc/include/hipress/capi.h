@@ -51,7 +51,8 @@ typedef struct {
   uint64_t timeout_ns;  // bound of every flag wait
   void* inbox[HP_MAX_RANKS];   // rank q's inbox, mapped into this process
   void* flags[HP_MAX_RANKS];   // rank q's flag words (uint32), mapped into this process
-  void* status;                // this rank's status words (emulate: nranks * 4 words)
+  void* status;                // this rank's status words (emulate: nranks * 4 words), in device
+                               // memory or in pinned host memory mapped into the device
   // emulation only: element strides between consecutive ranks' copies of g / r / out / sr
   int64_t emu_stride_g, emu_stride_r, emu_stride_out, emu_stride_sr;
   // optional device-side timing of the fused dense kernels: HP_TRACE_WORDS uint64 per rank

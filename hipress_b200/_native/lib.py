@@ -28,21 +28,6 @@ class NativeLibraryError(RuntimeError):
     pass
 
 
-class HpSeg(C.Structure):
-    _fields_ = [("g", C.c_void_p), ("r", C.c_void_p), ("out", C.c_void_p), ("sr", C.c_void_p),
-                ("n", C.c_uint64), ("id", C.c_uint32), ("pad", C.c_uint32)]
-
-
-class HpComm(C.Structure):
-    _fields_ = [("nranks", C.c_int32), ("rank", C.c_int32), ("emulate", C.c_int32),
-                ("epoch", C.c_uint32), ("timeout_ns", C.c_uint64),
-                ("inbox", C.c_void_p * MAX_RANKS), ("flags", C.c_void_p * MAX_RANKS),
-                ("status", C.c_void_p),
-                ("emu_stride_g", C.c_int64), ("emu_stride_r", C.c_int64),
-                ("emu_stride_out", C.c_int64), ("emu_stride_sr", C.c_int64),
-                ("trace", C.c_void_p)]
-
-
 _cpu = None
 _cuda = None
 _fast = None
@@ -134,8 +119,6 @@ def cuda():
     _sig(L.hp_fused_chunk_elems, C.c_uint64, C.c_uint64, C.c_int)
     _sig(L.hp_cuda_debug_build, C.c_int)
     _sig(L.hp_cuda_debug_set_inbox_limit, C.c_int, C.c_uint64)
-    _sig(L.hp_cuda_fused_dense, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(HpSeg), C.c_int,
-         C.POINTER(HpComm), C.c_float, C.c_uint64, C.c_uint32, C.c_uint32, C.c_int, vp)
     _sig(L.hp_sparse_workspace_bytes, C.c_uint64)
     _sig(L.hp_sparse_workspace_bytes_for, C.c_uint64, C.c_uint64)
     _sig(L.hp_cuda_arena_alloc, C.c_int, C.c_uint64, C.POINTER(C.c_void_p))

@@ -38,6 +38,7 @@ from dataclasses import dataclass, field
 import torch
 import torch.distributed as dist
 
+from .._native.lib import stream_ptr
 from ..config import HipressConfig
 from ..ops.algorithms import get_algorithm
 from ..ops.compressor import TILE, Compressor
@@ -91,6 +92,15 @@ class Bucket:
     flat: torch.Tensor | None = None
     work: object = None
     stream: object = None
+    # fused buckets: (entry, byte offset) of every segment, and the addresses and ids that
+    # stay the same from launch to launch (make_launch_args)
+    at: list = field(default_factory=list)
+    in_order: bool = False
+    r_ptrs: list = field(default_factory=list)
+    u_ptrs: list = field(default_factory=list)
+    sr_ptrs: list = field(default_factory=list)
+    scratch: list = field(default_factory=list)
+    ids: list = field(default_factory=list)
     # hierarchical mode: per segment (lo, hi, state, owner state) of this rank's shard,
     # and the staging buffers of the all-gather inside the machine
     outer: list = field(default_factory=list)
@@ -198,7 +208,10 @@ class GradSyncEngine:
         self.launch_count = 0
         self.bytes_sent = 0
         self.timeline = Timeline()
-        self._events = [torch.cuda.Event() for _ in self.buckets] if self.on_cuda else []
+        if self.on_cuda:
+            from .._native import lib as _lib
+            self._fast = _lib.fast_cuda()
+            self._order = [_lib.OrderEvent() for _ in range(len(self.buckets) + 1)]
 
     # ------------------------------------------------------------------ plan
     def _make_entries(self, named):
@@ -341,12 +354,11 @@ class GradSyncEngine:
                     ctas=cfg.partition_ctas if on_part else cfg.ctas, timeout_s=cfg.timeout_s))
             total = sum(i.region_bytes() + 512 for i in impls) + 4096
             self.arena = SymmetricArena(total, self.group)
-            self.status = torch.zeros(4, dtype=torch.int32, device=self.device)
+            self.make_status()
             for b, impl in zip(fused_buckets, impls):
                 impl.bind(self.arena.carve(impl.region_bytes()), self.status)
                 b.impl = impl
-            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
-            self._status_event = None
+                self.make_launch_args(b)
         elif fused_buckets and not use_fused_kernels:
             self._host = HostSchedule(self.comp, cfg.topology, self.group)
         for b in self.buckets:
@@ -355,6 +367,29 @@ class GradSyncEngine:
                                      device=self.device)
         if self.outer is not None:
             self._setup_outer(fused_buckets)
+
+    def make_status(self):
+        """Status words of the fused kernels.  They are written only when a wait expires,
+        so they live in pinned host memory the kernels see: the step reads them without
+        a copy on the stream or a synchronisation."""
+        self.status = torch.zeros(4, dtype=torch.int32).pin_memory()
+        self._status_words = self.status.numpy()
+
+    def make_launch_args(self, b: Bucket):
+        """What stays the same between two launches of a fused bucket."""
+        pos = {id(e): i for i, e in enumerate(b.entries)}
+        b.at = [(pos[id(s.entry)], 4 * s.lo) for s in b.segs]
+        b.in_order = b.at == [(i, 0) for i in range(len(b.entries))]
+
+        def address(t, s):
+            return None if t is None else t.data_ptr() + 4 * s.lo
+        states = [s.entry.state for s in b.segs]
+        b.r_ptrs = [address(st.get("accum_v", st.get("residual")), s) for st, s in zip(states, b.segs)]
+        b.u_ptrs = [address(st.get("momentum_u"), s) for st, s in zip(states, b.segs)]
+        own = [s.entry.server_state[s.part] if s.entry.server_state else {} for s in b.segs]
+        b.sr_ptrs = [o["residual"].data_ptr() if "residual" in o else None for o in own]
+        b.scratch = [o["residual"] for o in own if o.get("_scratch")]
+        b.ids = [s.seg_id for s in b.segs]
 
     def _make_partition_stream(self):
         """Stream bound to a green context of cfg.partition_sms SMs; falls back to
@@ -405,9 +440,11 @@ class GradSyncEngine:
 
     def _grad(self, e: Entry) -> torch.Tensor:
         p = e.param
-        if p.grad is None:
-            p.grad = torch.zeros_like(p, memory_format=torch.preserve_format)
         g = p.grad
+        if g is None:
+            p.grad = g = torch.zeros_like(p, memory_format=torch.preserve_format)
+        if g.dtype is torch.float32 and not g.is_sparse and g.is_contiguous():
+            return g
         if g.is_sparse:
             raise TypeError(f"gradient of {e.name} is a sparse tensor; use dense gradients "
                             "(e.g. nn.Embedding(sparse=False))")
@@ -419,13 +456,11 @@ class GradSyncEngine:
 
     def _launch(self, b: Bucket):
         b.launched = True
-        if self.on_cuda and b.fused and b.impl is not None:
+        if b.impl is not None:
             # fused kernels take the raw stream: no stream context switch on the
             # autograd thread, which is busy launching backward
             st = b.stream or self.comm_stream
-            ev = self._events[b.index]
-            ev.record()
-            st.wait_event(ev)
+            self._fast.stream_order(self._order[b.index].handle, stream_ptr(), st.cuda_stream)
             tok = self.timeline.begin(f"bucket{b.index}", st) if self.timeline.enabled else None
             self._launch_fused(b)
             if self.outer is not None:
@@ -438,6 +473,8 @@ class GradSyncEngine:
                 with torch.cuda.stream(st):
                     self.on_bucket_done(b)
             return
+        if not b.fused and self.world == 1 and self.on_bucket_done is None:
+            return              # nobody to average with, nothing to order behind the gradients
         if self.on_cuda:
             st = b.stream or self.comm_stream
             ev = torch.cuda.Event()
@@ -463,41 +500,22 @@ class GradSyncEngine:
                 self.on_bucket_done(b)
 
     def _launch_fused(self, b: Bucket):
-        grads = {id(e): self._grad(e) for e in b.entries}
-        if b.impl is not None and self.comp.spec.sparse:
-            g_ptrs, a_ptrs, u_ptrs, sr_ptrs = [], [], [], []
-            for s in b.segs:
-                e = s.entry
-                g_ptrs.append(grads[id(e)].data_ptr() + 4 * s.lo)
-                acc = e.state["accum_v"] if "accum_v" in e.state else e.state["residual"]
-                a_ptrs.append(acc.data_ptr() + 4 * s.lo)
-                u = e.state.get("momentum_u")
-                u_ptrs.append(None if u is None else u.data_ptr() + 4 * s.lo)
-                sst = e.server_state[s.part] if e.server_state else {}
-                if sst.get("_scratch"):  # on the launch stream, ordered before the kernels
-                    with torch.cuda.stream(b.stream or self.comm_stream):
-                        sst["residual"].zero_()
-                sr_ptrs.append(sst["residual"].data_ptr() if "residual" in sst else None)
-            b.impl.launch_ptrs(g_ptrs, a_ptrs, u_ptrs, g_ptrs, sr_ptrs,
-                               stream=b.stream or self.comm_stream)
-            self.launch_count += 1
-        elif b.impl is not None:
-            g_ptrs, r_ptrs, sr_ptrs, ids = [], [], [], []
-            rname = "residual"
-            for s in b.segs:
-                e = s.entry
-                base = grads[id(e)].data_ptr()
-                g_ptrs.append(base + 4 * s.lo)
-                r = e.state.get(rname)
-                r_ptrs.append(None if r is None else r.data_ptr() + 4 * s.lo)
-                sst = e.server_state[s.part] if e.server_state else {}
-                sr = sst.get("residual")
-                sr_ptrs.append(None if sr is None else sr.data_ptr())
-                ids.append(s.seg_id)
-            b.impl.launch_ptrs(g_ptrs, r_ptrs, g_ptrs, sr_ptrs, step=self.step_no, tensor_ids=ids,
-                               stream=b.stream or self.comm_stream)
+        if b.impl is not None:
+            g = [self._grad(e).data_ptr() for e in b.entries]
+            if not b.in_order:
+                g = [g[i] + off for i, off in b.at]
+            st = b.stream or self.comm_stream
+            if self.comp.spec.sparse:
+                if b.scratch:  # on the launch stream, ordered before the kernels
+                    with torch.cuda.stream(st):
+                        for t in b.scratch:
+                            t.zero_()
+                b.impl.launch_ptrs(g, b.r_ptrs, b.u_ptrs, g, b.sr_ptrs, stream=st)
+            else:
+                b.impl.launch_ptrs(g, b.r_ptrs, g, b.sr_ptrs, step=self.step_no, tensor_ids=b.ids, stream=st)
             self.launch_count += 1
         else:
+            grads = {id(e): self._grad(e) for e in b.entries}
             views = []
             for s in b.segs:
                 e = s.entry
@@ -594,20 +612,21 @@ class GradSyncEngine:
             part = getattr(self, "part_stream", None)
             if part is not None and part is not self.comm_stream:
                 self.comm_stream.wait_stream(part)
-            with torch.cuda.stream(self.comm_stream):
-                for b in self.buckets:
-                    if not b.fused:
-                        self._finish_plain(b)
-                        if self.on_bucket_done is not None:
-                            self.on_bucket_done(b)
-                if self.arena is not None:
-                    self._poll_status()
-            torch.cuda.current_stream().wait_stream(self.comm_stream)
-            if self.arena is not None and self.cfg.strict_status:
-                # the host waits for this step's kernels and raises before the
-                # optimizer can apply a gradient that a late peer left incomplete
-                self._status_event.synchronize()
-                self._raise_on_status([w & 0xFFFFFFFF for w in self._status_host.tolist()])
+            if self.world > 1 or self.on_bucket_done is not None:
+                with torch.cuda.stream(self.comm_stream):
+                    for b in self.buckets:
+                        if not b.fused:
+                            self._finish_plain(b)
+                            if self.on_bucket_done is not None:
+                                self.on_bucket_done(b)
+            self._fast.stream_order(self._order[-1].handle, self.comm_stream.cuda_stream, stream_ptr())
+            if self.arena is not None:
+                if self.cfg.strict_status:
+                    # the host waits for this step's kernels and raises before the
+                    # optimizer can apply a gradient that a late peer left incomplete
+                    self.comm_stream.synchronize()
+                if self._status_words[0]:
+                    self._raise_on_status()
         else:
             for b in self.buckets:
                 if not b.fused:
@@ -617,26 +636,17 @@ class GradSyncEngine:
         self.step_no += 1
         self._begin()
 
-    def _raise_on_status(self, words):
+    def _raise_on_status(self):
+        """Called when a status word is set.  A wait that expired in one step is raised at
+        the next synchronize, by check(), or -- with ``strict_status`` -- by the same
+        synchronize before the optimizer runs.  A CTA whose wait expired writes neither
+        error-feedback state nor gradient (csrc/cuda/fused_dense.cu), so the late report
+        costs one step whose affected tensors carry the local instead of the averaged
+        gradient, never corrupt state; checkpoints call check() first."""
         from .fused import HipressTimeoutError, decode_status
-        if any(words):
-            self.status.zero_()
-            self._status_host.zero_()
-            raise HipressTimeoutError(f"rank {self.R}: " + decode_status(next(w for w in words if w)))
-
-    def _poll_status(self):
-        """Asynchronous read of the kernels' status words: a wait that expired in one
-        step is raised at the next synchronize, by check(), or -- with
-        ``strict_status`` -- by the same synchronize before the optimizer runs.  A CTA
-        whose wait expired writes neither error-feedback state nor gradient
-        (csrc/cuda/fused_dense.cu), so the late report costs one step whose affected
-        tensors carry the local instead of the averaged gradient, never corrupt
-        state; checkpoints call check() first."""
-        if self._status_event is not None and self._status_event.query():
-            self._raise_on_status([w & 0xFFFFFFFF for w in self._status_host.tolist()])
-        self._status_host.copy_(self.status, non_blocking=True)
-        self._status_event = torch.cuda.Event()
-        self._status_event.record(self.comm_stream)
+        words = [w & 0xFFFFFFFF for w in self._status_words.tolist()]
+        self.status.zero_()
+        raise HipressTimeoutError(f"rank {self.R}: " + decode_status(next(w for w in words if w)))
 
     def check(self):
         """Blocking check of the device status words and of the guard words
@@ -645,7 +655,8 @@ class GradSyncEngine:
             return
         self.arena.check_guards()
         torch.cuda.synchronize()
-        self._raise_on_status([w & 0xFFFFFFFF for w in self.status.cpu().tolist()])
+        if self._status_words.any():
+            self._raise_on_status()
 
     # ------------------------------------------------------------ checkpoint
     def state_dict(self) -> dict:

@@ -67,8 +67,8 @@ class FusedDenseBucket:
         self.ctas = max(1, min(self.ctas, self.tiles_total * phases))   # never more CTAs than work items
         self.inbox_ptrs = None
         self.status = None
-        self._segs = (_lib.HpSeg * len(self.sizes))()
-        self._comm = _lib.HpComm()
+        self._plan = None       # native launch plan (csrc/host/fastcall.cpp), made by bind()
+        self._launch = _lib.fast_cuda().launch
 
     # -- memory -----------------------------------------------------------
     def region_bytes(self) -> int:
@@ -79,6 +79,11 @@ class FusedDenseBucket:
         """region_ptrs[q]: address of rank q's region for this bucket."""
         self.inbox_ptrs = [int(p) for p in region_ptrs]
         self.status = status
+        sp = self.spec
+        # no flags: the dense kernels signal inside the payload slots
+        self._plan = _lib.fast_cuda().plan(self.topo, sp.alg, sp.bits, self.ctas, sp.threshold, 0.0, sp.seed, None,
+                                           self.sizes, self.nranks, self.rank, 1 if self.emulate else 0,
+                                           self.timeout_ns, self.inbox_ptrs, None, status.data_ptr())
         if self.trace_enabled:
             nr = self.nranks if self.emulate else 1
             self.trace = torch.zeros(TRACE_WORDS * nr, dtype=torch.int64, device=status.device)
@@ -117,28 +122,8 @@ class FusedDenseBucket:
         """grads[i]: fp32 tensor of sizes[i] elements (emulation: shape [N, sizes[i]]
         with the same row stride for every tensor class).  The averaged result is
         written to outs[i] (default: in place)."""
-        L = _lib.cuda()
-        nseg = len(self.sizes)
         outs = outs if outs is not None else grads
-        cm = self._comm
-        for i in range(nseg):
-            s = self._segs[i]
-            g = grads[i]
-            s.g = g.data_ptr()
-            s.r = residuals[i].data_ptr() if residuals is not None and residuals[i] is not None else None
-            s.out = outs[i].data_ptr()
-            s.sr = (server_residuals[i].data_ptr()
-                    if server_residuals is not None and server_residuals[i] is not None else None)
-            s.n = self.sizes[i]
-            s.id = tensor_ids[i] if tensor_ids is not None else i
-        self.epoch = self.epoch % 0x7FFFFFFE + 1     # 31 bits: the top bit of the wire word is a mark
-        cm.nranks, cm.rank, cm.emulate = self.nranks, self.rank, 1 if self.emulate else 0
-        cm.epoch, cm.timeout_ns = self.epoch, self.timeout_ns
-        for q in range(self.nranks):
-            cm.inbox[q] = self.inbox_ptrs[q]
-            cm.flags[q] = None      # the dense kernels signal inside the payload slots
-        cm.status = self.status.data_ptr()
-        self._arm_trace(cm, stream)
+        strides = None
         if self.emulate:
             def stride(ts):
                 if ts is None or ts[0] is None:
@@ -146,51 +131,34 @@ class FusedDenseBucket:
                 st = ts[0].stride(0)
                 assert all(t.stride(0) == st for t in ts if t is not None)
                 return st
-            cm.emu_stride_g = stride(grads)
-            cm.emu_stride_r = stride(residuals)
-            cm.emu_stride_out = stride(outs)
-            cm.emu_stride_sr = stride(server_residuals)
-        sp = self.spec
-        rc = L.hp_cuda_fused_dense(self.topo, sp.alg, sp.bits, self._segs, nseg, C.byref(cm),
-                                   sp.threshold, sp.seed, step, salt, self.ctas,
-                                   _lib.stream_ptr(stream))
-        _lib.check(rc, "fused dense launch")
+            strides = (stride(grads), stride(residuals), stride(outs), stride(server_residuals))
+
+        def ptrs(ts):
+            return None if ts is None else [None if t is None else t.data_ptr() for t in ts]
+        self.launch_ptrs(ptrs(grads), ptrs(residuals), ptrs(outs), ptrs(server_residuals), step=step, salt=salt,
+                         tensor_ids=tensor_ids, stream=stream, strides=strides)
 
     def launch_ptrs(self, g_ptrs, r_ptrs, out_ptrs, sr_ptrs, *, step=0, salt=0, tensor_ids=None,
-                    stream=None):
-        """Same as :meth:`launch` from raw device addresses (one per tensor; None = absent)."""
-        L = _lib.cuda()
-        nseg = len(self.sizes)
-        cm = self._comm
-        for i in range(nseg):
-            s = self._segs[i]
-            s.g, s.r, s.out, s.sr = g_ptrs[i], r_ptrs[i], out_ptrs[i], sr_ptrs[i]
-            s.n = self.sizes[i]
-            s.id = tensor_ids[i] if tensor_ids is not None else i
+                    stream=None, strides=None):
+        """Same as :meth:`launch` from raw device addresses (one per tensor; None = absent).
+        ``strides``: element strides between emulated ranks of gradients, residuals,
+        results and owner residuals."""
+        trace = None
+        if self.trace is not None:
+            trace = self._arm_trace(stream)
         self.epoch = self.epoch % 0x7FFFFFFE + 1     # 31 bits: the top bit of the wire word is a mark
-        cm.nranks, cm.rank, cm.emulate = self.nranks, self.rank, 0
-        cm.epoch, cm.timeout_ns = self.epoch, self.timeout_ns
-        for q in range(self.nranks):
-            cm.inbox[q] = self.inbox_ptrs[q]
-            cm.flags[q] = None      # the dense kernels signal inside the payload slots
-        cm.status = self.status.data_ptr()
-        self._arm_trace(cm, stream)
-        sp = self.spec
-        rc = L.hp_cuda_fused_dense(self.topo, sp.alg, sp.bits, self._segs, nseg, C.byref(cm),
-                                   sp.threshold, sp.seed, step, salt, self.ctas,
-                                   _lib.stream_ptr(stream))
-        _lib.check(rc, "fused dense launch")
+        rc = self._launch(self._plan, g_ptrs, r_ptrs, out_ptrs, sr_ptrs, tensor_ids, step, salt, self.epoch, trace,
+                          strides, _lib.stream_ptr(stream))
+        if rc:
+            _lib.check(rc, "fused dense launch")
 
-    def _arm_trace(self, cm, stream):
-        if self.trace is None:
-            cm.trace = None
-            return
+    def _arm_trace(self, stream):
         if stream is not None:
             with torch.cuda.stream(stream):
                 self.trace.copy_(self._trace_init)
         else:
             self.trace.copy_(self._trace_init)
-        cm.trace = self.trace.data_ptr()
+        return self.trace.data_ptr()
 
     def last_trace(self):
         """Device-side timing of the last launch, per rank played by it:

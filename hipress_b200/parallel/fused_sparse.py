@@ -9,7 +9,7 @@ import ctypes as C
 import torch
 
 from .._native import lib as _lib
-from ..ops.algorithms import DGC, AlgSpec
+from ..ops.algorithms import AlgSpec
 from .simulate import chunk_elems
 
 _bound = False
@@ -23,12 +23,6 @@ def _bind():
         L.hp_fused_sparse_layout.argtypes = [C.c_float, C.POINTER(C.c_uint64), C.c_int, C.c_int,
                                              C.POINTER(C.c_uint64), C.POINTER(C.c_uint64),
                                              C.POINTER(C.c_uint64)]
-        L.hp_cuda_fused_sparse_ps.restype = C.c_int
-        sig = [C.c_int, C.c_float, C.c_float, C.POINTER(_lib.HpSeg), C.POINTER(C.c_void_p), C.c_int,
-               C.POINTER(_lib.HpComm), C.c_void_p, C.c_int, C.c_void_p]
-        L.hp_cuda_fused_sparse_ps.argtypes = sig
-        L.hp_cuda_fused_sparse_ring.restype = C.c_int
-        L.hp_cuda_fused_sparse_ring.argtypes = sig
         _bound = True
     return L
 
@@ -51,11 +45,10 @@ class FusedSparseBucket:
         _lib.check(L.hp_fused_sparse_layout(spec.ratio, arr, len(self.sizes), nranks, C.byref(ib),
                                             C.byref(fw), C.byref(wb)), "sparse layout")
         self.inbox_bytes, self.flag_words, self.ws_bytes = ib.value, fw.value, wb.value
-        self._segs = (_lib.HpSeg * len(self.sizes))()
-        self._us = (C.c_void_p * len(self.sizes))()
-        self._comm = _lib.HpComm()
         self.ws = None
         self.status = None
+        self._plan = None       # native launch plan (csrc/host/fastcall.cpp), made by bind()
+        self._launch = _lib.fast_cuda().launch
 
     def region_bytes(self) -> int:
         return (self.inbox_bytes + 255) // 256 * 256 + (self.flag_words * 4 + 255) // 256 * 256
@@ -67,6 +60,11 @@ class FusedSparseBucket:
         self.status = status
         nr = self.nranks if self.emulate else 1
         self.ws = torch.zeros(self.ws_bytes * nr // 4, dtype=torch.int32, device=device)
+        sp = self.spec
+        self._plan = _lib.fast_cuda().plan(_lib.TOPO_PS if self.topology == "ps" else _lib.TOPO_RING, sp.alg, 0,
+                                           self.ctas, sp.ratio, sp.momentum, 0, self.ws.data_ptr(), self.sizes,
+                                           self.nranks, self.rank, 1 if self.emulate else 0, self.timeout_ns,
+                                           self.inbox_ptrs, self.flag_ptrs, status.data_ptr())
         return self
 
     def bind_local(self, device):
@@ -85,29 +83,11 @@ class FusedSparseBucket:
         """Addresses per tensor: gradient, accumulator (DGC v / GradDrop residual),
         DGC momentum (or None), output, server accumulator of the owned chunk.
         strides (emulation): element strides between ranks of g, state, out, sr."""
-        L = _bind()
-        nseg = len(self.sizes)
-        for i in range(nseg):
-            s = self._segs[i]
-            s.g, s.r, s.out, s.sr, s.n, s.id = g_ptrs[i], acc_ptrs[i], out_ptrs[i], sr_ptrs[i], \
-                self.sizes[i], i
-            self._us[i] = u_ptrs[i] if u_ptrs is not None else None
-        cm = self._comm
         self.epoch = self.epoch % 0x7FFFFFFE + 1     # 31 bits: the top bit of a flag is a mark
-        cm.nranks, cm.rank, cm.emulate = self.nranks, self.rank, 1 if self.emulate else 0
-        cm.epoch, cm.timeout_ns = self.epoch, self.timeout_ns
-        for q in range(self.nranks):
-            cm.inbox[q] = self.inbox_ptrs[q]
-            cm.flags[q] = self.flag_ptrs[q]
-        cm.status = self.status.data_ptr()
-        cm.trace = None
-        cm.emu_stride_g, cm.emu_stride_r, cm.emu_stride_out, cm.emu_stride_sr = strides
-        sp = self.spec
-        us = self._us if sp.alg == DGC else None
-        fn = L.hp_cuda_fused_sparse_ps if self.topology == "ps" else L.hp_cuda_fused_sparse_ring
-        rc = fn(sp.alg, sp.ratio, sp.momentum, self._segs, us, nseg, C.byref(cm), self.ws.data_ptr(),
-                self.ctas, _lib.stream_ptr(stream))
-        _lib.check(rc, "fused sparse launch")
+        rc = self._launch(self._plan, g_ptrs, acc_ptrs, out_ptrs, sr_ptrs, u_ptrs, 0, 0, self.epoch, None, strides,
+                          _lib.stream_ptr(stream))
+        if rc:
+            _lib.check(rc, "fused sparse launch")
 
     def last_phase_times(self):
         """Device-side profile of the last launch (rank 0 of an emulated launch): the
@@ -143,7 +123,7 @@ def setup_engine_buckets(engine, fused_buckets) -> bool:
              for b in fused_buckets]
     total = sum(i.region_bytes() + 512 for i in impls) + 4096
     engine.arena = SymmetricArena(total, engine.group)
-    engine.status = torch.zeros(4, dtype=torch.int32, device=engine.device)
+    engine.make_status()
     for b, impl in zip(fused_buckets, impls):
         impl.bind(engine.arena.carve(impl.region_bytes()), engine.status, engine.device)
         b.impl = impl
@@ -154,6 +134,5 @@ def setup_engine_buckets(engine, fused_buckets) -> bool:
                 sst["residual"] = torch.zeros(chunk_elems(s.n, engine.N), dtype=torch.float32,
                                               device=engine.device)
                 sst["_scratch"] = True
-    engine._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
-    engine._status_event = None
+        engine.make_launch_args(b)
     return True

@@ -43,3 +43,21 @@ def test_terngrad_codes_at_extreme_ranges(bits, what):
     elif what == "overflow":
         g[0], g[1] = 3e38, -3e38
     _payloads_equal(Compressor("terngrad", bitwidth=bits), g)
+
+
+def test_status_words_in_pinned_host_memory():
+    """The training loop keeps the status words in pinned host memory: a wait that runs
+    out shows there without a copy."""
+    from hipress_b200.parallel.fused import FusedDenseBucket, HipressTimeoutError
+    c = Compressor("tbq")
+    n = 20000
+    b = FusedDenseBucket(c.spec, "ring", [n], 2, 0, ctas=16, timeout_s=0.3)
+    arena = torch.zeros(2 * b.region_bytes(), dtype=torch.uint8, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32).pin_memory()
+    b.bind([arena.data_ptr(), arena.data_ptr() + b.region_bytes()], status)
+    g = torch.randn(n, device="cuda") * 0.02
+    b.launch_ptrs([g.data_ptr()], [torch.zeros_like(g).data_ptr()], [g.data_ptr()], [None])
+    torch.cuda.synchronize()
+    assert int(status[0]) != 0
+    with pytest.raises(HipressTimeoutError):
+        b.check_status()
