@@ -4,10 +4,10 @@
 // over the launch's own CTAs between phases that depend on one another); waiting
 // across GPUs happens on release / acquire flags, as in the dense kernels.
 //
-//   push   : per (tensor, owner) unit: state update + radix select (3 histogram
-//            passes) + compaction whose (index, value) pairs are stored straight
-//            into the owner GPU's inbox; the CTA that finishes a unit releases
-//            the owner's flag.
+//   push   : per (tensor, owner) unit: state update and exact top-k selection in one
+//            pass over the arrays (sparse_core.cuh), the (index, value) pairs stored
+//            straight into the owner GPU's inbox; the CTA that finishes a unit
+//            releases the owner's flag.
 //   server : the owner waits (bounded) for the N flags of a tensor, adds the N
 //            sparse payloads into its accumulator (= server-side residual),
 //            re-selects the top-k of the sum and stores the result into every
@@ -15,8 +15,10 @@
 //   pull   : every rank zero-fills the gradient, waits for each owner's flag and
 //            scatters value / N.
 //
-// All units of a bucket are batched in every phase (the CTAs share out the units'
-// slices), which is the "bulk synchronisation" of many small tensors.  An earlier
+// All units of a bucket are batched in every phase, which is the "bulk
+// synchronisation" of many small tensors: the update pass hands out the bucket's tiles
+// in stretches to whichever CTA is free, whatever the tensors' sizes (equal shares of
+// CTAs per tensor left ResNet-50's largest tensors on 15 CTAs each).  An earlier
 // version ran every stage as a launch of its own: 19 launches per bucket for PS and
 // 9 per ring hop, with a floor of about 0.2 ms per bucket from launch latency alone.
 //
@@ -38,7 +40,11 @@ struct SpSeg {
   float* out;  // averaged gradient (may alias g)
   float* sr;   // server accumulator for the owned chunk [chunk]
   uint32_t n, chunk, kmax, pay_off;
-  uint32_t cap;         // candidate pairs per (tensor, chunk) unit
+  uint32_t tiles;       // tiles of one chunk
+  uint32_t tile_prefix; // tiles of one chunk of the tensors before this one
+  uint32_t sampled;     // tiles of one chunk that are sampled (set at launch: depends on the grid)
+  uint32_t sample_prefix;
+  uint32_t cap;         // candidate pairs per (tensor, chunk) unit, for both lists
   uint64_t cand_push;   // first push unit's candidate list, in pairs from the region start
   uint64_t cand_srv;    // the server unit's candidate list
 };
@@ -50,6 +56,8 @@ struct SpBucket {
   float ratio, momentum, inv_n;
   uint64_t slot_bytes;
   uint64_t cand_pairs;  // candidate pairs of all units of one rank
+  uint32_t tiles_total; // tiles of one chunk summed over the tensors
+  uint32_t samples_total;
 };
 
 __device__ __forceinline__ uint32_t sp_chunk_valid(uint32_t n, uint32_t chunk, int c) {
@@ -67,19 +75,22 @@ __device__ __forceinline__ void write_empty_header(uint8_t* out, int alg) {
 
 // ------------------------------------------------------ persistent-kernel plumbing
 struct SpSmem {
-  uint32_t sh[kBins];
+  union {
+    SelSmem sel;
+    uint32_t sh[kBins];   // whole-array passes
+    EmitSmem es;
+  };
   FindSmem fs;
-  EmitSmem es;
-  SplitSmem sp;
   WaitState wst;
-  uint32_t any;
+  uint32_t any, ticket;
 };
 
 // control words of one rank played by a launch, behind its histogram blocks; zero
 // when the kernel starts (cleared with the histograms)
-constexpr int kCtlBarrier = 0;
 constexpr int kCtlStamps = 8;    // low 32 bits of %globaltimer: kernel start, then after every barrier
-constexpr int kCtlWords = 128;
+constexpr int kCtlTickets = 96;  // one per handed-out phase: two for a selection, cleared with the rest
+constexpr int kCtlBarrier = 128;
+constexpr int kCtlWords = kCtlBarrier + kBarrierWords;
 
 struct SpCtx {
   int N, R, E;
@@ -100,20 +111,14 @@ __device__ __forceinline__ void sp_barrier(const HpComm& cm, SpCtx& cx, SpSmem& 
   // a peer may be late by up to one wait bound before a CTA reaches the barrier
   grid_barrier(cx.ctl + kCtlBarrier, cx.gen, cx.G, 2 * cm.timeout_ns + 1000000000ull, cx.status,
                HP_STATUS_TIMEOUT | (8u << 16) | (cx.gen & 255u), sm.wst);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && kCtlStamps + cx.gen < (uint32_t)kCtlWords)
+  if (blockIdx.x == 0 && threadIdx.x == 0 && kCtlStamps + cx.gen < 64u)
     cx.ctl[kCtlStamps + cx.gen] = (uint32_t)global_timer_ns();
 }
 
 // extra stamps of CTA 0 inside a phase (profile words 64..)
 __device__ __forceinline__ void sp_mark(const SpCtx& cx, int id) {
-  if (blockIdx.x == 0 && threadIdx.x == 0 && 64 + id < kCtlWords)
+  if (blockIdx.x == 0 && threadIdx.x == 0 && 64 + id < kCtlTickets)
     cx.ctl[64 + id] = (uint32_t)global_timer_ns();
-}
-
-// between two stages that one CTA runs back to back on the same unit
-__device__ __forceinline__ void cta_fence_sync() {
-  __threadfence();
-  __syncthreads();
 }
 
 // Phase driver: `units` work units, each cut into `per` slices; slice v of the phase
@@ -128,36 +133,6 @@ __device__ __forceinline__ void run_units(const SpCtx& cx, uint32_t units, uint3
   }
 }
 
-// did any of `units` units (histogram blocks from `ws`) overflow its candidate list?
-// Read after a barrier that follows every writer, so all CTAs agree.
-__device__ __forceinline__ bool any_overflow(const uint32_t* ws, uint32_t units, SpSmem& sm) {
-  if (threadIdx.x == 0) sm.any = 0;
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < units; i += kSpThreads)
-    if (__ldcg(ws + (size_t)i * kWsWords + kWsOverflow)) sm.any = 1;
-  __syncthreads();
-  const bool r = sm.any != 0;
-  __syncthreads();
-  return r;
-}
-
-// longest candidate list among `units` units; same conditions as any_overflow
-__device__ __forceinline__ uint32_t max_candidates(const uint32_t* ws, uint32_t units, SpSmem& sm) {
-  if (threadIdx.x == 0) sm.any = 0;
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < units; i += kSpThreads)
-    atomicMax(&sm.any, __ldcg(ws + (size_t)i * kWsWords + kWsCandCount));
-  __syncthreads();
-  const uint32_t r = sm.any;
-  __syncthreads();
-  return r;
-}
-// A unit whose candidate list has at most this many pairs goes through both digit
-// passes and the compaction on ONE CTA with no barrier in between; longer lists
-// (a steady-state accumulator is dense just below its threshold) are shared out
-// over several CTAs again, with a barrier after each pass.
-constexpr uint32_t kSmallCand = 8192;
-
 __device__ __forceinline__ uint32_t slices_heavy(const SpCtx& cx, uint32_t units) {
   const uint32_t p = cx.G / (units ? units : 1);
   return p < 1 ? 1 : (p > 592 ? 592 : p);
@@ -167,157 +142,250 @@ __device__ __forceinline__ uint32_t slices_cap(const SpCtx& cx, uint32_t units, 
   return p > cap ? cap : p;
 }
 
-// ---------------------------------------------------------------- push
-// unit y = seg * N + owner
-// STAGE 0: update + hist0   1: split (certain elements go to the owner at once)
-//       2,3: digit passes on the candidate list   4: candidate compaction + flag
-//       5,6,7: full-array passes and compaction, only after a candidate overflow
-template <int STAGE>
-__device__ __forceinline__ void push_stage(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
-                                           SpSmem& sm, int y, uint32_t x, uint32_t nx) {
-  const int N = cx.N, R = cx.R, E = cx.E;
-  const int si = y / N, c = y % N;
-  const SpSeg& sg = bk.seg[si];
-  const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, c);
-  uint32_t* ws = cx.ws + (size_t)y * kWsWords;
-  float* cand_val = reinterpret_cast<float*>(cx.cand + (sg.cand_push + (uint64_t)c * sg.cap) * 8);
-  uint32_t* cand_idx = reinterpret_cast<uint32_t*>(cand_val + sg.cap);
-  const size_t off = (size_t)c * sg.chunk;
-  const float* g = sg.g + E * cm.emu_stride_g + off;
-  float* a = sg.a + E * cm.emu_stride_r + off;
-  float* u = sg.u ? sg.u + E * cm.emu_stride_r + off : nullptr;
-  const uint32_t k = (uint32_t)sparse_k(len, bk.ratio);
-  uint8_t* dst = reinterpret_cast<uint8_t*>(cm.inbox[c]) + (size_t)R * bk.slot_bytes + sg.pay_off;
-  EmitDst d;
-  d.n = 1;
-  d.out[0] = dst;
-  bool last = false;
-  if (STAGE == 0) {
-    if (len == 0) return;
-    if (bk.alg == kDgc) pass0_body<2>(g, a, u, len, bk.momentum, ws, sm.sh, x, nx);
-    else pass0_body<1>(g, a, u, len, bk.momentum, ws, sm.sh, x, nx);
-    return;
-  } else if (STAGE == 1) {
-    if (len == 0) return;
-    split_body(a, u, len, k, sg.kmax, d, ws, cand_val, cand_idx, sg.cap, sm.fs, sm.sp, x, nx);
-    return;
-  } else if (STAGE == 2 || STAGE == 3) {
-    if (len == 0 || ws[kWsOverflow]) return;
-    if (STAGE == 2) pass_body<1>(cand_val, ws[kWsCandCount], k, ws, sm.sh, sm.fs, x, nx);
-    else pass_body<2>(cand_val, ws[kWsCandCount], k, ws, sm.sh, sm.fs, x, nx);
-    return;
-  } else if (STAGE == 4) {
-    if (len == 0) {
-      last = x == 0 && threadIdx.x == 0;
-      if (last) write_empty_header(dst, bk.alg);
-    } else {
-      if (ws[kWsOverflow]) return;
-      last = emit_body(bk.alg, cand_val, u, ws[kWsCandCount], k, sg.kmax, d, ws, sm.fs, sm.es, x, nx,
-                       cand_idx, a, len);
-    }
-  } else if (STAGE == 5 || STAGE == 6) {
-    if (len == 0 || !ws[kWsOverflow]) return;
-    if (STAGE == 5) pass_body<1>(a, len, k, ws, sm.sh, sm.fs, x, nx);
-    else pass_body<2>(a, len, k, ws, sm.sh, sm.fs, x, nx);
-    return;
-  } else {
-    if (len == 0 || !ws[kWsOverflow]) return;
-    last = emit_body(bk.alg, a, u, len, k, sg.kmax, d, ws, sm.fs, sm.es, x, nx);
-  }
-  if (last) {  // thread 0 of the slice that completed the unit
-    __threadfence_system();
-    st_release_sys(reinterpret_cast<uint32_t*>(cm.flags[c]) + (size_t)R * bk.nseg + si,
-                   flag_value(cm, sm));
-  }
+// ------------------------------------------------------------ units of a selection
+// push : every (tensor, owner) pair, unit y = tensor * N + owner
+// serve: the owned chunk of every tensor, y = tensor
+// hop  : the chunk of every tensor that hop `hop` of the ring works on, y = tensor
+enum SelKind { kSelPush, kSelServe, kSelHop };
+
+struct UnitRef {
+  int si, c;
+};
+template <int KIND>
+__device__ __forceinline__ UnitRef unit_ref(const SpCtx& cx, int y, int hop) {
+  if (KIND == kSelPush) return {y / cx.N, y % cx.N};
+  if (KIND == kSelServe) return {y, cx.R};
+  return {y, (cx.R - hop + cx.N) % cx.N};
 }
 
-// -------------------------------------------------------------- server
-// unit y = seg; the owned chunk is chunk R
-// STAGE 0: wait + scatter-add   1: hist0   2: split (to every rank)   3,4: candidate
-//       digit passes   5: candidate compaction + flags   6,7,8: overflow path
-template <int STAGE>
-__device__ __forceinline__ void server_stage(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
-                                             SpSmem& sm, int y, uint32_t x, uint32_t nx) {
-  const int N = cx.N, R = cx.R, E = cx.E;
-  const int si = y;
+// the array of a unit; n = 0 for a chunk past the tensor's end
+template <int KIND>
+__device__ __forceinline__ SelUnit unit_of(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, int y, int hop) {
+  const UnitRef r = unit_ref<KIND>(cx, y, hop);
+  const SpSeg& sg = bk.seg[r.si];
+  const int E = cx.E;
+  const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, r.c);
+  const uint32_t k = (uint32_t)sparse_k(len, bk.ratio);
+  const size_t off = (size_t)r.c * sg.chunk;
+  if (KIND == kSelServe)
+    return sel_unit(nullptr, sg.sr + E * cm.emu_stride_sr, nullptr, len, k, sg.kmax,
+                    cx.ws + ((size_t)bk.nseg * cx.N + y) * kWsWords, cx.cand + sg.cand_srv * 8, sg.cap,
+                    sg.tiles, sg.sampled);
+  const size_t block = KIND == kSelPush ? (size_t)y : (size_t)hop * bk.nseg + r.si;
+  return sel_unit(sg.g + E * cm.emu_stride_g + off, sg.a + E * cm.emu_stride_r + off,
+                  sg.u ? sg.u + E * cm.emu_stride_r + off : nullptr, len, k, sg.kmax, cx.ws + block * kWsWords,
+                  cx.cand + (sg.cand_push + (uint64_t)r.c * sg.cap) * 8, sg.cap, sg.tiles, sg.sampled);
+}
+
+// where a unit's pairs go, and the flags that announce them
+struct UnitDst {
+  EmitDst out;
+  uint32_t* flag[HP_MAX_RANKS];
+};
+template <int KIND>
+__device__ __forceinline__ void unit_dst(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, int y, int hop,
+                                         UnitDst& d) {
+  const int N = cx.N, R = cx.R;
+  const UnitRef r = unit_ref<KIND>(cx, y, hop);
+  const bool all = KIND == kSelServe || (KIND == kSelHop && hop == N - 1);
+  const int first = KIND == kSelPush ? r.c : (all ? R : (R + 1) % N);
+  const int slot = KIND == kSelPush ? R : (KIND == kSelServe ? N + R : (all ? N - 1 + R : hop));
+  d.out.n = all ? N : 1;
+  for (int q = 0; q < d.out.n; ++q) {
+    const int to = (first + q) % N;
+    d.out.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[to]) + (size_t)slot * bk.slot_bytes + bk.seg[r.si].pay_off;
+    d.flag[q] = reinterpret_cast<uint32_t*>(cm.flags[to]) + (size_t)slot * bk.nseg + r.si;
+  }
+}
+// thread 0 of the CTA that completed the unit
+__device__ __forceinline__ void unit_release(const HpComm& cm, const SpSmem& sm, const UnitDst& d) {
+  __threadfence_system();
+  const uint32_t v = flag_value(cm, sm);
+  for (int q = 0; q < d.out.n; ++q) st_release_sys(d.flag[q], v);
+}
+
+// The selection of all units of one kind: two barriers (three when some list is longer
+// than one CTA finishes, more only when a sample misled).  `idle` runs on every CTA
+// after the update pass, while few of them finish lists.
+template <int KIND, typename F>
+__device__ __forceinline__ void select_units(const SpBucket& bk, const HpComm& cm, SpCtx& cx, SpSmem& sm, int hop,
+                                             int ticket, F idle) {
+  const uint32_t M = KIND == kSelPush ? (uint32_t)cx.N : 1u;   // units per tensor
+  const uint32_t units = (uint32_t)bk.nseg * M;
+  const int mode = KIND == kSelServe ? 0 : (bk.alg == kDgc ? 2 : 1);
+  auto unit = [&](uint32_t y) { return unit_of<KIND>(bk, cm, cx, (int)y, hop); };
+  // sampled tiles: item i belongs to unit y as its tile number j
+  const uint32_t samples = bk.samples_total * M;
+  auto sampled = [&](auto f) {
+    for (uint32_t i = blockIdx.x, r = 0; i < samples; i += cx.G, ++r) {
+      int si = 0;
+      while (si + 1 < bk.nseg && i >= bk.seg[si + 1].sample_prefix * M) ++si;
+      const SpSeg& sg = bk.seg[si];
+      const uint32_t at = i - sg.sample_prefix * M;
+      const uint32_t y = KIND == kSelPush ? si * cx.N + at / sg.sampled : (uint32_t)si;
+      const SelUnit s = unit(y);
+      if (s.n) f(s, y, at % sg.sampled, r < (uint32_t)kStash ? (int)r : -1);
+    }
+  };
+  sampled([&](const SelUnit& s, uint32_t, uint32_t j, int slot) {
+    if (mode == 0) sample_body<0>(s, bk.momentum, sm.sel, j, slot);
+    else if (mode == 1) sample_body<1>(s, bk.momentum, sm.sel, j, slot);
+    else sample_body<2>(s, bk.momentum, sm.sel, j, slot);
+  });
+  sp_barrier(cm, cx, sm);
+  if (threadIdx.x == 0) sm.sel.count = 0;
+  __syncthreads();
+  sampled([&](const SelUnit& s, uint32_t y, uint32_t j, int slot) { collect_sampled(s, y, sm.sel, j, slot); });
+  hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * M, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
+    int si = 0;
+    while (t < end) {
+      while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * M) ++si;
+      const SpSeg& sg = bk.seg[si];
+      const uint32_t at = t - sg.tile_prefix * M, c = at / sg.tiles, tt = at % sg.tiles;
+      const uint32_t stop = min(sg.tiles, tt + (end - t));
+      const uint32_t y = KIND == kSelPush ? si * cx.N + c : (uint32_t)si;
+      const SelUnit s = unit(y);
+      const uint32_t t1 = min(stop, (s.n + kTile - 1) / kTile);
+      if (tt < t1) {
+        if (mode == 0) collect_body<0>(s, y, bk.momentum, sm.sel, tt, t1);
+        else if (mode == 1) collect_body<1>(s, y, bk.momentum, sm.sel, tt, t1);
+        else collect_body<2>(s, y, bk.momentum, sm.sel, tt, t1);
+      }
+      t += stop - tt;
+    }
+    if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, unit);
+  });
+  collect_flush(sm.sel, unit);
+  sp_barrier(cm, cx, sm);
+  // behind the barrier every CTA reads the same counters and decides the same
+  if (threadIdx.x == 0) sm.any = sm.ticket = 0;
+  __syncthreads();
+  for (uint32_t y = threadIdx.x; y < units; y += kSpThreads) {
+    const SelUnit s = unit_of<KIND>(bk, cm, cx, (int)y, hop);
+    if (s.n == 0) continue;
+    if (selection_failed(s)) sm.any = 1;
+    else atomicMax(&sm.ticket, __ldcg(s.ws + kWsCandCount));
+  }
+  __syncthreads();
+  const bool failed = sm.any != 0, refined = sm.ticket > kFinishList;
+  __syncthreads();
+  if (refined) {
+    run_units(cx, units, slices_cap(cx, units, 64), [&](int y, uint32_t x, uint32_t nx) {
+      const SelUnit s = unit_of<KIND>(bk, cm, cx, y, hop);
+      if (s.n == 0 || selection_failed(s)) return;
+      UnitDst d;
+      unit_dst<KIND>(bk, cm, cx, y, hop, d);
+      refine_body(s, d.out, sm.sel, x, nx);
+    });
+    sp_barrier(cm, cx, sm);
+  }
+  sp_mark(cx, KIND == kSelServe ? 4 : 0);
+  const uint32_t share = cx.G / units ? cx.G / units : 1u;
+  run_units(cx, units, share, [&](int y, uint32_t x, uint32_t) {
+    const SelUnit s = unit_of<KIND>(bk, cm, cx, y, hop);
+    uint32_t nx = 1;
+    if (s.n && !selection_failed(s))
+      nx = finish_slices(min(__ldcg(s.ws + (refined ? kWsCand2Count : kWsCandCount)), s.cap), share);
+    if (x >= nx) return;
+    UnitDst d;
+    unit_dst<KIND>(bk, cm, cx, y, hop, d);
+    bool done = false;
+    if (s.n == 0) {
+      done = threadIdx.x == 0;
+      if (done)
+        for (int q = 0; q < d.out.n; ++q) write_empty_header(d.out.out[q], bk.alg);
+    } else if (!selection_failed(s)) {
+      done = finish_body(bk.alg, s, d.out, sm.sel, refined, x, nx);
+    }
+    if (done) unit_release(cm, sm, d);
+  });
+  sp_mark(cx, KIND == kSelServe ? 5 : 1);
+  idle();
+  sp_mark(cx, KIND == kSelServe ? 6 : 2);
+  if (!failed) return;
+  // whole-array passes for the units whose sample misled
+  const uint32_t ph = slices_heavy(cx, units);
+  auto again = [&](auto f) {
+    run_units(cx, units, ph, [&](int y, uint32_t x, uint32_t nx) {
+      const SelUnit s = unit_of<KIND>(bk, cm, cx, y, hop);
+      if (s.n != 0 && selection_failed(s)) f(s, y, x, nx);
+    });
+  };
+  again([&](const SelUnit& s, int, uint32_t x, uint32_t nx) {
+    for (uint32_t i = x * kSpThreads + threadIdx.x; i < 3u * kBins; i += nx * kSpThreads) s.ws[i] = 0;
+  });
+  sp_barrier(cm, cx, sm);
+  again([&](const SelUnit& s, int, uint32_t x, uint32_t nx) {
+    pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.sh, x, nx);
+  });
+  sp_barrier(cm, cx, sm);
+#pragma unroll 1
+  for (int pass = 1; pass <= 2; ++pass) {
+    again([&](const SelUnit& s, int, uint32_t x, uint32_t nx) {
+      pass_body_rt(pass, s.a, s.n, s.k, s.ws, sm.sh, sm.fs, x, nx);
+    });
+    sp_barrier(cm, cx, sm);
+  }
+  again([&](const SelUnit& s, int y, uint32_t x, uint32_t nx) {
+    UnitDst d;
+    unit_dst<KIND>(bk, cm, cx, y, hop, d);
+    if (emit_body(bk.alg, s.a, s.u, s.n, s.k, s.kmax, d.out, s.ws, sm.fs, sm.es, x, nx)) unit_release(cm, sm, d);
+  });
+}
+
+// ---------------------------------------------------------------- incoming payloads
+// PS owner: wait for the N pushes of tensor si and add them into the accumulator
+__device__ __forceinline__ void serve_in(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm, int si,
+                                         uint32_t x, uint32_t nx) {
+  const int N = cx.N, R = cx.R;
   const SpSeg& sg = bk.seg[si];
   const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, R);
-  uint32_t* ws = cx.ws + ((size_t)bk.nseg * N + y) * kWsWords;
-  float* cand_val = reinterpret_cast<float*>(cx.cand + sg.cand_srv * 8);
-  uint32_t* cand_idx = reinterpret_cast<uint32_t*>(cand_val + sg.cap);
-  float* acc = sg.sr + E * cm.emu_stride_sr;
-  const uint32_t k = (uint32_t)sparse_k(len, bk.ratio);
-  EmitDst d;
-  d.n = N;
+  const uint32_t* my_flags = reinterpret_cast<const uint32_t*>(cm.flags[R]);
   for (int q = 0; q < N; ++q)
-    d.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[(R + q) % N]) + (size_t)(N + R) * bk.slot_bytes +
-               sg.pay_off;
-  bool last = false;
-  if (STAGE == 0) {
-    const uint32_t* my_flags = reinterpret_cast<const uint32_t*>(cm.flags[R]);
-    for (int q = 0; q < N; ++q)
-      wait_flag(my_flags + (size_t)q * bk.nseg + si, cm.epoch, cm.timeout_ns, cx.status,
-                HP_STATUS_TIMEOUT | (4u << 16) | ((uint32_t)q << 8) | (si & 255), sm.wst);
-    if (len == 0) return;
-    const uint8_t* inbox = reinterpret_cast<const uint8_t*>(cm.inbox[R]);
-    for (int q = 0; q < N; ++q)
-      scatter_body(inbox + (size_t)q * bk.slot_bytes + sg.pay_off, acc, len, sg.kmax, 1.0f, 2, x, nx);
-    return;
-  } else if (STAGE == 1) {
-    if (len == 0) return;
-    pass0_body<0>(nullptr, acc, nullptr, len, 0.0f, ws, sm.sh, x, nx);
-    return;
-  } else if (STAGE == 2) {
-    if (len == 0) return;
-    split_body(acc, nullptr, len, k, sg.kmax, d, ws, cand_val, cand_idx, sg.cap, sm.fs, sm.sp, x, nx);
-    return;
-  } else if (STAGE == 3 || STAGE == 4) {
-    if (len == 0 || ws[kWsOverflow]) return;
-    if (STAGE == 3) pass_body<1>(cand_val, ws[kWsCandCount], k, ws, sm.sh, sm.fs, x, nx);
-    else pass_body<2>(cand_val, ws[kWsCandCount], k, ws, sm.sh, sm.fs, x, nx);
-    return;
-  } else if (STAGE == 5) {
-    if (len == 0) {
-      last = x == 0 && threadIdx.x == 0;
-      if (last)
-        for (int q = 0; q < N; ++q) write_empty_header(d.out[q], bk.alg);
-    } else {
-      if (ws[kWsOverflow]) return;
-      last = emit_body(bk.alg, cand_val, nullptr, ws[kWsCandCount], k, sg.kmax, d, ws, sm.fs, sm.es, x,
-                       nx, cand_idx, acc, len);
-    }
-  } else if (STAGE == 6 || STAGE == 7) {
-    if (len == 0 || !ws[kWsOverflow]) return;
-    if (STAGE == 6) pass_body<1>(acc, len, k, ws, sm.sh, sm.fs, x, nx);
-    else pass_body<2>(acc, len, k, ws, sm.sh, sm.fs, x, nx);
-    return;
-  } else {
-    if (len == 0 || !ws[kWsOverflow]) return;
-    last = emit_body(bk.alg, acc, nullptr, len, k, sg.kmax, d, ws, sm.fs, sm.es, x, nx);
-  }
-  if (last) {
-    __threadfence_system();
-    const uint32_t fv = flag_value(cm, sm);
-    for (int q = 0; q < N; ++q)
-      st_release_sys(reinterpret_cast<uint32_t*>(cm.flags[(R + q) % N]) +
-                         (size_t)(N + R) * bk.nseg + si,
-                     fv);
-  }
+    wait_flag(my_flags + (size_t)q * bk.nseg + si, cm.epoch, cm.timeout_ns, cx.status,
+              HP_STATUS_TIMEOUT | (4u << 16) | ((uint32_t)q << 8) | (si & 255), sm.wst);
+  if (len == 0) return;
+  const uint8_t* inbox = reinterpret_cast<const uint8_t*>(cm.inbox[R]);
+  for (int q = 0; q < N; ++q)
+    scatter_body(inbox + (size_t)q * bk.slot_bytes + sg.pay_off, sg.sr + cx.E * cm.emu_stride_sr, len, sg.kmax, 1.0f,
+                 2, x, nx);
+}
+
+// ring: wait for the predecessor's pairs of tensor si and add them into the accumulator
+__device__ __forceinline__ void hop_in(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm, int hop,
+                                       int si, uint32_t x, uint32_t nx) {
+  const SpSeg& sg = bk.seg[si];
+  const int c = (cx.R - hop + cx.N) % cx.N;
+  const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, c);
+  wait_flag(reinterpret_cast<const uint32_t*>(cm.flags[cx.R]) + (size_t)(hop - 1) * bk.nseg + si, cm.epoch,
+            cm.timeout_ns, cx.status, HP_STATUS_TIMEOUT | (6u << 16) | ((uint32_t)(hop - 1) << 8) | (si & 255),
+            sm.wst);
+  if (len == 0) return;
+  scatter_body(reinterpret_cast<const uint8_t*>(cm.inbox[cx.R]) + (size_t)(hop - 1) * bk.slot_bytes + sg.pay_off,
+               sg.a + cx.E * cm.emu_stride_r + (size_t)c * sg.chunk, len, sg.kmax, 1.0f, 1, x, nx);
 }
 
 // ---------------------------------------------------------------- pull
-// zero-fill of the result (unit y = seg).  It runs one phase after the update pass has
-// read the gradient (which may be the same buffer): clearing each element right behind
-// its load in that pass made the pass five times slower when the buffers were the same
-// (a store to a line whose fill is still in flight).
-__device__ __forceinline__ void zero_stage(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
-                                           int y, uint32_t x, uint32_t nx) {
-  const SpSeg& sg = bk.seg[y];
-  float* out = sg.out + cx.E * cm.emu_stride_out;
-  const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-  const uint64_t stride = (uint64_t)nx * kSpThreads * 4;
-  for (uint64_t i = ((uint64_t)x * kSpThreads + threadIdx.x) * 4; i < sg.n; i += stride)
-    st4(out, i, sg.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
+// Zero-fill of the result, tile by tile.  It runs behind the barrier of the update pass,
+// which reads the gradient (it may be the same buffer), on the CTAs that have no list to
+// finish: clearing each element right behind its load in the update pass made that
+// pass five times slower (a store to a line whose fill is still in flight).
+__device__ __forceinline__ void zero_result(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm,
+                                            int ticket) {
+  const uint32_t N = (uint32_t)cx.N;
+  hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * N, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
+    int si = 0;
+    for (; t < end; ++t) {
+      while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * N) ++si;
+      const SpSeg& sg = bk.seg[si];
+      float* out = sg.out + cx.E * cm.emu_stride_out;
+      const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+      const uint64_t i0 = (uint64_t)(t - sg.tile_prefix * N) * kTile + threadIdx.x * 4;
+#pragma unroll
+      for (int j = 0; j < kTile / (4 * kSpThreads); ++j)
+        st4(out, i0 + j * kSpThreads * 4, sg.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+  });
 }
 
 // wait for the reduced chunk c that arrives in inbox slot `slot` and scatter value / N
@@ -336,99 +404,6 @@ __device__ __forceinline__ void gather_stage(const SpBucket& bk, const HpComm& c
                      sg.pay_off;
   scatter_body(p, sg.out + cx.E * cm.emu_stride_out + (size_t)c * sg.chunk, len, sg.kmax, bk.inv_n, 0,
                x, nx);
-}
-
-// ---------------------------------------------------------------- ring
-// One hop of the sparse ring for every tensor of the bucket (unit y = seg).  At hop
-// h rank R works on chunk (R - h) mod N: the predecessor's pairs are added into the
-// local accumulator, then the state update, the exact top-k selection and the
-// compaction run, and the pairs go into the successor's inbox -- or, at the last
-// hop, into every rank's inbox.
-// STAGE 0: wait + add incoming   1: update + hist0   2: split   3,4: candidate digit
-//       passes   5: candidate compaction + flag(s)   6,7,8: overflow path
-template <int STAGE>
-__device__ __forceinline__ void ring_stage(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
-                                           SpSmem& sm, int hop, int y, uint32_t x, uint32_t nx) {
-  const int N = cx.N, R = cx.R, E = cx.E;
-  const int si = y;
-  const int c = (R - hop + N) % N;
-  const bool last_hop = hop == N - 1;
-  const SpSeg& sg = bk.seg[si];
-  const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, c);
-  uint32_t* ws = cx.ws + ((size_t)hop * bk.nseg + si) * kWsWords;
-  float* cand_val = reinterpret_cast<float*>(cx.cand + (sg.cand_push + (uint64_t)c * sg.cap) * 8);
-  uint32_t* cand_idx = reinterpret_cast<uint32_t*>(cand_val + sg.cap);
-  const size_t off = (size_t)c * sg.chunk;
-  const float* g = sg.g + E * cm.emu_stride_g + off;
-  float* a = sg.a + E * cm.emu_stride_r + off;
-  float* u = sg.u ? sg.u + E * cm.emu_stride_r + off : nullptr;
-  const uint32_t k = (uint32_t)sparse_k(len, bk.ratio);
-  EmitDst d;
-  if (!last_hop) {
-    d.n = 1;
-    d.out[0] = reinterpret_cast<uint8_t*>(cm.inbox[(R + 1) % N]) + (size_t)hop * bk.slot_bytes + sg.pay_off;
-  } else {
-    d.n = N;
-    for (int q = 0; q < N; ++q)
-      d.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[(R + q) % N]) +
-                 (size_t)(N - 1 + R) * bk.slot_bytes + sg.pay_off;
-  }
-  bool last = false;
-  if (STAGE == 0) {
-    if (hop == 0) return;
-    wait_flag(reinterpret_cast<const uint32_t*>(cm.flags[R]) + (size_t)(hop - 1) * bk.nseg + si,
-              cm.epoch, cm.timeout_ns, cx.status,
-              HP_STATUS_TIMEOUT | (6u << 16) | ((uint32_t)(hop - 1) << 8) | (si & 255), sm.wst);
-    if (len == 0) return;
-    scatter_body(reinterpret_cast<const uint8_t*>(cm.inbox[R]) + (size_t)(hop - 1) * bk.slot_bytes +
-                     sg.pay_off,
-                 a, len, sg.kmax, 1.0f, 1, x, nx);
-    return;
-  } else if (STAGE == 1) {
-    if (len == 0) return;
-    if (bk.alg == kDgc) pass0_body<2>(g, a, u, len, bk.momentum, ws, sm.sh, x, nx);
-    else pass0_body<1>(g, a, u, len, bk.momentum, ws, sm.sh, x, nx);
-    return;
-  } else if (STAGE == 2) {
-    if (len == 0) return;
-    split_body(a, u, len, k, sg.kmax, d, ws, cand_val, cand_idx, sg.cap, sm.fs, sm.sp, x, nx);
-    return;
-  } else if (STAGE == 3 || STAGE == 4) {
-    if (len == 0 || ws[kWsOverflow]) return;
-    if (STAGE == 3) pass_body<1>(cand_val, ws[kWsCandCount], k, ws, sm.sh, sm.fs, x, nx);
-    else pass_body<2>(cand_val, ws[kWsCandCount], k, ws, sm.sh, sm.fs, x, nx);
-    return;
-  } else if (STAGE == 5) {
-    if (len == 0) {
-      last = x == 0 && threadIdx.x == 0;
-      if (last)
-        for (int q = 0; q < d.n; ++q) write_empty_header(d.out[q], bk.alg);
-    } else {
-      if (ws[kWsOverflow]) return;
-      last = emit_body(bk.alg, cand_val, u, ws[kWsCandCount], k, sg.kmax, d, ws, sm.fs, sm.es, x, nx,
-                       cand_idx, a, len);
-    }
-  } else if (STAGE == 6 || STAGE == 7) {
-    if (len == 0 || !ws[kWsOverflow]) return;
-    if (STAGE == 6) pass_body<1>(a, len, k, ws, sm.sh, sm.fs, x, nx);
-    else pass_body<2>(a, len, k, ws, sm.sh, sm.fs, x, nx);
-    return;
-  } else {
-    if (len == 0 || !ws[kWsOverflow]) return;
-    last = emit_body(bk.alg, a, u, len, k, sg.kmax, d, ws, sm.fs, sm.es, x, nx);
-  }
-  if (last) {
-    __threadfence_system();
-    const uint32_t fv = flag_value(cm, sm);
-    if (!last_hop) {
-      st_release_sys(reinterpret_cast<uint32_t*>(cm.flags[(R + 1) % N]) + (size_t)hop * bk.nseg + si, fv);
-    } else {
-      for (int q = 0; q < N; ++q)
-        st_release_sys(reinterpret_cast<uint32_t*>(cm.flags[(R + q) % N]) +
-                           (size_t)(N - 1 + R) * bk.nseg + si,
-                       fv);
-    }
-  }
 }
 
 // ------------------------------------------------------------- the two kernels
@@ -459,154 +434,60 @@ __device__ __forceinline__ void sp_prologue(const HpComm& cm, const SpLaunch& L,
 // be scattering: the stamps are a profile of the phases, not a completion signal)
 __device__ __forceinline__ void sp_epilogue(const SpCtx& cx) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (kCtlStamps + cx.gen + 1 < (uint32_t)kCtlWords)
+    if (kCtlStamps + cx.gen + 1 < 64u)
       cx.ctl[kCtlStamps + cx.gen + 1] = (uint32_t)global_timer_ns();
     cx.ctl[1] = cx.gen;
   }
 }
 
-// PS: push (every rank selects per owner and stores the pairs into the owner's
-// inbox), server (the owner adds the N payloads, re-selects, stores the result into
-// every inbox), pull (every rank scatters value / N).  Five barriers when the
-// candidate lists are short, nine otherwise (more only after an overflow).
+// PS: push (every rank selects per owner and stores the pairs into the owner's inbox),
+// serve (the owner adds the N payloads, re-selects, stores the result into every
+// inbox), pull (every rank scatters value / N).  Five barriers when the candidate lists
+// are short.  @PS_NOTE@
 __global__ void __launch_bounds__(kSpThreads, 3)
 sp_ps_kernel(const SpBucket bk, const HpComm cm, const SpLaunch L) {
-  __shared__ SpSmem sm;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
   SpCtx cx;
   sp_prologue(cm, L, cx, sm);
-  const uint32_t nseg = (uint32_t)bk.nseg, units = nseg * (uint32_t)cx.N;
-  const uint32_t ph = slices_heavy(cx, units), pc = slices_cap(cx, units, 32);
-  const uint32_t sh = slices_heavy(cx, nseg), sc = slices_cap(cx, nseg, 32);
-#define PUSH(S, P) run_units(cx, units, P, [&](int y, uint32_t x, uint32_t nx) { push_stage<S>(bk, cm, cx, sm, y, x, nx); })
-#define SRV(S, P) run_units(cx, nseg, P, [&](int y, uint32_t x, uint32_t nx) { server_stage<S>(bk, cm, cx, sm, y, x, nx); })
-  PUSH(0, ph);
-  sp_barrier(cm, cx, sm);
-  PUSH(1, ph);
-  sp_barrier(cm, cx, sm);
-  const bool ovf = any_overflow(cx.ws, units, sm);
-  // the candidate list of a unit is short (about as many pairs as are sent): one CTA
-  // takes a unit through both digit passes and the compaction, no barrier in between
-  if (max_candidates(cx.ws, units, sm) <= kSmallCand) {
-    run_units(cx, units, 1, [&](int y, uint32_t x, uint32_t nx) {
-      push_stage<2>(bk, cm, cx, sm, y, x, nx);
-      cta_fence_sync();
-      push_stage<3>(bk, cm, cx, sm, y, x, nx);
-      cta_fence_sync();
-      push_stage<4>(bk, cm, cx, sm, y, x, nx);
-    });
-  } else {
-    PUSH(2, pc);
-    sp_barrier(cm, cx, sm);
-    PUSH(3, pc);
-    sp_barrier(cm, cx, sm);
-    PUSH(4, pc);
-  }
-  if (ovf) {
-    PUSH(5, ph);
-    sp_barrier(cm, cx, sm);
-    PUSH(6, ph);
-    sp_barrier(cm, cx, sm);
-    PUSH(7, ph);
-  }
-  // The gradient was read two barriers ago (it may be the result buffer): clear the
-  // result here, where the CTAs would otherwise only wait for the peers' pushes.
-  run_units(cx, nseg, sh, [&](int y, uint32_t x, uint32_t nx) { zero_stage(bk, cm, cx, y, x, nx); });
-  SRV(0, sh);
-  sp_barrier(cm, cx, sm);
-  SRV(1, sh);
-  sp_barrier(cm, cx, sm);
-  SRV(2, sh);
-  sp_barrier(cm, cx, sm);
-  const bool ovf2 = any_overflow(cx.ws + (size_t)units * kWsWords, nseg, sm);
-  if (max_candidates(cx.ws + (size_t)units * kWsWords, nseg, sm) <= kSmallCand) {
-    run_units(cx, nseg, 1, [&](int y, uint32_t x, uint32_t nx) {
-      server_stage<3>(bk, cm, cx, sm, y, x, nx);
-      cta_fence_sync();
-      server_stage<4>(bk, cm, cx, sm, y, x, nx);
-      cta_fence_sync();
-      server_stage<5>(bk, cm, cx, sm, y, x, nx);
-    });
-  } else {
-    SRV(3, sc);
-    sp_barrier(cm, cx, sm);
-    SRV(4, sc);
-    sp_barrier(cm, cx, sm);
-    SRV(5, sc);
-  }
-  if (ovf2) {
-    SRV(6, sh);
-    sp_barrier(cm, cx, sm);
-    SRV(7, sh);
-    sp_barrier(cm, cx, sm);
-    SRV(8, sh);
-  }
   const int N = cx.N;
+  const uint32_t nseg = (uint32_t)bk.nseg, units = nseg * (uint32_t)N;
+  select_units<kSelPush>(bk, cm, cx, sm, 0, 0, [&] { zero_result(bk, cm, cx, sm, 1); });
+  run_units(cx, nseg, slices_cap(cx, nseg, 32),
+            [&](int y, uint32_t x, uint32_t nx) { serve_in(bk, cm, cx, sm, y, x, nx); });
+  sp_barrier(cm, cx, sm);
+  select_units<kSelServe>(bk, cm, cx, sm, 0, 2, [] {});
   run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
     const int j = y % N;
     gather_stage(bk, cm, cx, sm, y / N, N + j, j, 5u, x, nx);
   });
-#undef PUSH
-#undef SRV
   sp_epilogue(cx);
 }
 
-// Ring: N hops of (add the predecessor's pairs, update, select, store into the
+// Ring: N hops of (add the predecessor's pairs, update and select, store into the
 // successor's inbox), the last hop storing into every inbox; then every rank scatters
-// the N reduced chunks.  Three barriers per hop when the candidate lists are short,
-// five otherwise.
+// the N reduced chunks.  Three barriers per hop when the candidate lists are short.
 __global__ void __launch_bounds__(kSpThreads, 3)
 sp_ring_kernel(const SpBucket bk, const HpComm cm, const SpLaunch L) {
-  __shared__ SpSmem sm;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
   SpCtx cx;
   sp_prologue(cm, L, cx, sm);
   const int N = cx.N;
   const uint32_t nseg = (uint32_t)bk.nseg;
-  const uint32_t sh = slices_heavy(cx, nseg), sc = slices_cap(cx, nseg, 32);
-#define HOP(S, P) run_units(cx, nseg, P, [&](int y, uint32_t x, uint32_t nx) { ring_stage<S>(bk, cm, cx, sm, hop, y, x, nx); })
   for (int hop = 0; hop < N; ++hop) {
     if (hop > 0) {
-      HOP(0, sc);
+      run_units(cx, nseg, slices_cap(cx, nseg, 32),
+                [&](int y, uint32_t x, uint32_t nx) { hop_in(bk, cm, cx, sm, hop, y, x, nx); });
       sp_barrier(cm, cx, sm);
     }
-    HOP(1, sh);
-    sp_barrier(cm, cx, sm);
-    HOP(2, sh);
-    if (hop == N - 1)  // every chunk of the gradient has been read: clear the result
-      run_units(cx, nseg, sh, [&](int y, uint32_t x, uint32_t nx) { zero_stage(bk, cm, cx, y, x, nx); });
-    sp_barrier(cm, cx, sm);
-    const bool ovf = any_overflow(cx.ws + (size_t)hop * nseg * kWsWords, nseg, sm);
-    if (max_candidates(cx.ws + (size_t)hop * nseg * kWsWords, nseg, sm) <= kSmallCand) {
-      sp_mark(cx, 0);
-      run_units(cx, nseg, 1, [&](int y, uint32_t x, uint32_t nx) {
-        ring_stage<3>(bk, cm, cx, sm, hop, y, x, nx);
-        cta_fence_sync();
-        sp_mark(cx, 1);
-        ring_stage<4>(bk, cm, cx, sm, hop, y, x, nx);
-        cta_fence_sync();
-        sp_mark(cx, 2);
-        ring_stage<5>(bk, cm, cx, sm, hop, y, x, nx);
-        sp_mark(cx, 3);
-      });
-    } else {
-      HOP(3, sc);
-      sp_barrier(cm, cx, sm);
-      HOP(4, sc);
-      sp_barrier(cm, cx, sm);
-      sp_mark(cx, 2);
-      HOP(5, sc);
-      sp_mark(cx, 3);
-    }
-    if (ovf) {
-      HOP(6, sh);
-      sp_barrier(cm, cx, sm);
-      HOP(7, sh);
-      sp_barrier(cm, cx, sm);
-      HOP(8, sh);
-    }
+    // the last hop has read every chunk of the gradient when its update pass is done
+    select_units<kSelHop>(bk, cm, cx, sm, hop, 2 * hop, [&] {
+      if (hop == N - 1) zero_result(bk, cm, cx, sm, 2 * hop + 1);
+    });
   }
-#undef HOP
-  // gather: rank src finalised chunk src + 1
-  sp_mark(cx, 4);
+  // gather: rank src finalised chunk src + 1 (every CTA has cleared its share of the result)
+  sp_barrier(cm, cx, sm);
   const uint32_t units = nseg * (uint32_t)N;
   run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
     const int src = y % N;
@@ -619,7 +500,7 @@ static int build_sp_bucket(int alg, float ratio, float momentum, const HpSeg* se
                            void* const* accs, void* const* us, int nseg, int nranks, SpBucket& bk) {
   if (nseg < 1 || nseg > HP_MAX_SEGS || nranks < 1 || nranks > HP_MAX_RANKS) return HP_ERR_BAD_ARG;
   if (alg != kDgc && alg != kGradDrop) return HP_ERR_BAD_ARG;
-  uint64_t pay = 0, cand = 0;
+  uint64_t pay = 0, cand = 0, tiles = 0;
   for (int i = 0; i < nseg; ++i) {
     const uint64_t n = segs[i].n;
     if (n == 0 || n > 0xFFFFF000ull) return HP_ERR_BAD_ARG;
@@ -634,6 +515,9 @@ static int build_sp_bucket(int alg, float ratio, float momentum, const HpSeg* se
     d.chunk = (uint32_t)chunk;
     d.kmax = (uint32_t)sparse_k(chunk, ratio);
     d.pay_off = (uint32_t)pay;
+    d.tiles = (uint32_t)(chunk / kTile);
+    d.tile_prefix = (uint32_t)tiles;
+    tiles += d.tiles;
     d.cap = (uint32_t)align_up(8ull * d.kmax + 4096, 32);
     d.cand_push = cand;
     cand += (uint64_t)d.cap * nranks;
@@ -649,6 +533,8 @@ static int build_sp_bucket(int alg, float ratio, float momentum, const HpSeg* se
   bk.inv_n = 1.0f / (float)nranks;
   bk.slot_bytes = pay;
   bk.cand_pairs = cand;
+  if (tiles * (uint64_t)nranks > 0x7FFFFFFFull) return HP_ERR_TOO_LARGE;
+  bk.tiles_total = (uint32_t)tiles;
   return 0;
 }
 
@@ -657,7 +543,7 @@ static uint64_t sp_hist_words(int nseg, int nranks) {
   return (uint64_t)(nseg * nranks + nseg) * kWsWords;   // the ring uses nseg * nranks of them
 }
 
-static int launch_sparse(int topo, const SpBucket& bk, const HpComm& cm, void* ws, int ctas,
+static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int ctas,
                          cudaStream_t st) {
   const void* kern = topo == HP_TOPO_RING ? (const void*)sp_ring_kernel : (const void*)sp_ps_kernel;
   const int N = cm.nranks, nseg = bk.nseg;
@@ -666,10 +552,13 @@ static int launch_sparse(int topo, const SpBucket& bk, const HpComm& cm, void* w
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
   int cap = (dev >= 0 && dev < 64) ? resident[topo][dev] : 0;
+  const size_t smem = sizeof(SpSmem);
   if (cap == 0) {
     int sms = 0, per_sm = 0;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSpThreads, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSpThreads, smem);
     if (e != cudaSuccess) return (int)e;
     cap = per_sm * sms;
     if (cap < 1) return HP_ERR_RESIDENCY;
@@ -677,13 +566,18 @@ static int launch_sparse(int topo, const SpBucket& bk, const HpComm& cm, void* w
   }
   const int ranks_here = cm.emulate ? N : 1;
   int G = ctas;
-  if (G <= 0) {   // a quarter of the bucket's tiles, at least 32, at most what the GPU holds
-    uint64_t tiles = 0;
-    for (int i = 0; i < nseg; ++i) tiles += (bk.seg[i].n + kTile - 1) / kTile;
-    G = (int)(tiles / 4 < 32 ? 32 : (tiles / 4 > 592 ? 592 : tiles / 4));
+  if (G <= 0) {   // a CTA per tile of the bucket, at least 8, at most what the GPU holds
+    const uint64_t tiles = (uint64_t)bk.tiles_total * N;
+    G = tiles < 8 ? 8 : (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
     if (G > cap / ranks_here) G = cap / ranks_here;
   }
   if (G < 1 || (long long)G * ranks_here > (long long)cap) return HP_ERR_RESIDENCY;
+  bk.samples_total = 0;
+  for (int i = 0; i < nseg; ++i) {  // a sampled tile for every CTA, over the units of a push or of a hop
+    bk.seg[i].sampled = sampled_tiles(bk.seg[i].tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);
+    bk.seg[i].sample_prefix = bk.samples_total;
+    bk.samples_total += bk.seg[i].sampled;
+  }
   SpLaunch L;
   L.ws = static_cast<uint8_t*>(ws);
   L.hist_words = sp_hist_words(nseg, N);
@@ -695,7 +589,7 @@ static int launch_sparse(int topo, const SpBucket& bk, const HpComm& cm, void* w
   }
   void* args[] = {(void*)&bk, (void*)&cm, (void*)&L};
   // cooperative: the CTAs of a launch wait for one another at the phase barriers
-  e = cudaLaunchCooperativeKernel(kern, dim3(G, ranks_here), dim3(kSpThreads), args, 0, st);
+  e = cudaLaunchCooperativeKernel(kern, dim3(G, ranks_here), dim3(kSpThreads), args, smem, st);
   return (int)e;
 }
 

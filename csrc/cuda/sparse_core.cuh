@@ -18,8 +18,13 @@ constexpr int kBins = 4096;
 constexpr int kWsOutCount = 3 * kBins + 0;
 constexpr int kWsTieCount = 3 * kBins + 1;
 constexpr int kWsDone = 3 * kBins + 2;
-constexpr int kWsCandCount = 3 * kBins + 3;  // candidates appended by the split pass
-constexpr int kWsOverflow = 3 * kBins + 4;   // candidate list did not fit: use the full passes
+constexpr int kWsCandCount = 3 * kBins + 3;   // candidates collected by the update pass
+constexpr int kWsOverflow = 3 * kBins + 4;    // they did not fit: use the full passes
+constexpr int kWsLow = 3 * kBins + 5;         // magnitude key from which an element is a candidate
+constexpr int kWsSampled = 3 * kBins + 6;     // slices of the sample that are done
+constexpr int kWsCand2Count = 3 * kBins + 7;  // candidates left after the first digit
+constexpr int kWsTicket = 3 * kBins + 8;      // stand-alone kernel: tile ticket, status
+constexpr int kWsStatus = 3 * kBins + 9;
 constexpr int kWsWords = 3 * kBins + 16;
 
 __device__ __forceinline__ uint32_t digit_of(uint32_t key, int pass) {
@@ -27,25 +32,29 @@ __device__ __forceinline__ uint32_t digit_of(uint32_t key, int pass) {
 }
 
 struct FindSmem {
-  uint32_t sums[kSpThreads];
+  uint32_t sums[kSpThreads / 32];
   uint32_t res[2];
 };
 
-// Largest bin whose suffix count reaches k.  krem = how many of the k fall in
-// that bin or below the bins above it, i.e. k - count(bins > bin).
-static __device__ __noinline__ void find_bin(const uint32_t* __restrict__ hist, uint32_t k,
-                                         FindSmem& fs, uint32_t& bin, uint32_t& krem) {
+// Largest bin of a histogram of kBins bins whose suffix count reaches k, and krem = how
+// many of the k fall in that bin, i.e. k - count(bins > bin); (0, 0) when fewer than k are
+// counted.  `hist` is in shared or in global memory, where other CTAs' atomics wrote it.
+static __device__ __noinline__ void find_bin(const uint32_t* hist, uint32_t k, FindSmem& fs, uint32_t& bin,
+                                             uint32_t& krem) {
   constexpr int per = kBins / kSpThreads;  // 16
   uint32_t c[per];
   uint32_t sum = 0;
 #pragma unroll
-  for (int i = 0; i < per; ++i) {
-    c[i] = __ldcg(hist + threadIdx.x * per + i);  // written by other CTAs' atomics: read at L2
-    sum += c[i];
+  for (int i = 0; i < per; i += 4) {
+    asm volatile("ld.volatile.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(c[i]), "=r"(c[i + 1]), "=r"(c[i + 2]), "=r"(c[i + 3])
+                 : "l"(hist + threadIdx.x * per + i)
+                 : "memory");
+    sum += c[i] + c[i + 1] + c[i + 2] + c[i + 3];
   }
   // above = how many elements sit in the bins of higher threads: suffix sum by warp
   // shuffles plus the warps' totals (a serial walk over the 256 partial sums cost
-  // several microseconds per call, and a selection makes six calls)
+  // several microseconds per call)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t v = sum;
 #pragma unroll
@@ -201,18 +210,12 @@ struct EmitDst {
   int n;
 };
 
-// Compaction.  Tile = 4096 elements per CTA iteration, 16 per thread.  Returns
-// true in thread 0 of the CTA that finished last, after it wrote the headers.
-// With `remap` the scanned array `a` is a compacted candidate list: element i stands
-// for element remap[i] of the accumulator a_orig (and of u), which is what gets
-// reported and zeroed.
+// Compaction of the whole array.  Tile = 4096 elements per CTA iteration, 16 per thread.
+// Returns true in thread 0 of the CTA that finished last, after it wrote the headers.
 static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, float* __restrict__ u,
                                           uint64_t n, uint32_t k, uint32_t kmax, const EmitDst& dst,
                                           uint32_t* __restrict__ ws, FindSmem& fs, EmitSmem& es,
-                                          uint32_t cta, uint32_t nctas,
-                                          const uint32_t* __restrict__ remap = nullptr,
-                                          float* __restrict__ a_orig = nullptr,
-                                          uint32_t n_orig = 0) {
+                                          uint32_t cta, uint32_t nctas) {
   uint32_t bin0, k1, bin1, k2, bin2, need_eq;
   find_bin(ws, k, fs, bin0, k1);
   find_bin(ws + kBins, k1, fs, bin1, k2);
@@ -280,7 +283,6 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
     const uint32_t base = es.base_gt, acc_eq = es.base_eq;
     uint32_t pg = base + (excl & 0xFFFFu);             // next slot for a "greater" element
     uint32_t rank_eq = excl >> 16;                     // tie rank inside this tile
-    const bool rvec = (reinterpret_cast<uintptr_t>(remap) & 15) == 0;
 #pragma unroll 1
     for (int j = 0; j < 4; ++j) {
       const uint32_t fj = (flag >> (8 * j)) & 255u;
@@ -288,12 +290,6 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
       const uint64_t i = t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
       const float4 av = ld4(a, i, n, vec);
       const float e4[4] = {av.x, av.y, av.z, av.w};
-      uint32_t r4[4] = {0u, 0u, 0u, 0u};
-      if (remap) {  // original indices of a candidate list, fetched four at a time
-        const float4 rv = ld4(reinterpret_cast<const float*>(remap), i, n, rvec);
-        r4[0] = __float_as_uint(rv.x); r4[1] = __float_as_uint(rv.y);
-        r4[2] = __float_as_uint(rv.z); r4[3] = __float_as_uint(rv.w);
-      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const uint32_t f = (fj >> (2 * q)) & 3u;
@@ -304,15 +300,12 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
           ++rank_eq;
         }
         if (pos < kmax) {
-          uint32_t where = remap ? r4[q] : (uint32_t)(i + q);
-          if (remap && where >= n_orig) where = 0;  // never index outside the accumulator
           for (int d = 0; d < dst.n; ++d) {
-            reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = where;
+            reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = (uint32_t)(i + q);
             reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = e4[q];
           }
-          if (remap) a_orig[where] = 0.0f;
-          else a[i + q] = 0.0f;
-          if (u) u[where] = 0.0f;
+          a[i + q] = 0.0f;
+          if (u) u[i + q] = 0.0f;
         }
       }
     }
@@ -330,7 +323,7 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
       __threadfence();
       const uint32_t sent = atomicAdd(ws + kWsOutCount, 0u);
       WireHeader h;
-      h.n = remap ? n_orig : (uint32_t)n;  // always the length of the accumulator
+      h.n = (uint32_t)n;
       h.alg = (uint8_t)alg;
       h.bitwidth = 0;
       h.flags = 0;
@@ -344,109 +337,471 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
   return false;
 }
 
-// Split pass (after pass 0): everything above the threshold's 12-bit bin is
-// certainly among the k largest and is sent and zeroed at once; the elements of
-// that bin go to a compact candidate list (value + original index) on which the
-// remaining two digit passes and the final compaction run.  One pass over the
-// array instead of three.  A candidate list that does not fit raises the
-// overflow word and the full-array passes take over.
-constexpr int kSplitBuf = 1024;  // pairs a CTA collects in shared memory per list
+// ---------------------------------------------------------------------------
+// Exact top-k with ONE pass over the arrays.  A selection used to read the accumulator
+// again after the update to split it at a threshold bin, and every element went through
+// a shared-memory histogram; both are gone:
+//
+//   sample   some tiles of the array, spread evenly, are updated first; the histogram of
+//            their magnitudes gives a `low` below which an element is almost surely not
+//            among the k largest, and above which about 1.1 to 1.7 k are
+//   collect  the other tiles are updated; elements of at least `low` are appended to a
+//            candidate list with the histogram of their first digit (the sampled tiles'
+//            from shared memory).  The list holds the k largest exactly when it has k
+//            elements.
+//   finish   digit by digit on the list: the exact threshold, the pairs, the header.  A
+//            long list first goes through one distributed step (refine) that sends what
+//            lies above the first digit's bin and keeps what lies in it.
+//
+// State is read and written once: HBM bound at 20 bytes per element for DGC, 12 for
+// GradDrop.  A list that came out shorter than k or longer than its room (a sample that
+// misled, or massive ties) makes the launch fall back to histogram passes over the
+// whole array.
+constexpr uint32_t kFinishKeys = 8192;  // list length up to which a CTA keeps the keys in shared memory
+constexpr uint32_t kFinishList = 12288; // longest list one CTA finishes by itself
+constexpr uint32_t kMinSampled = 4;     // tiles of an array that are sampled at least
+constexpr int kSelTile = 4096;          // elements per tile: 16 per thread
 
-struct SplitSmem {
-  float sel_val[kSplitBuf];
-  uint32_t sel_idx[kSplitBuf];
-  float cnd_val[kSplitBuf];
-  uint32_t cnd_idx[kSplitBuf];
-  uint32_t nsel, ncnd, base_sel, base_cnd;
+// One array to select from.
+struct SelUnit {
+  const float* g;
+  float* a;
+  float* u;
+  uint32_t* ws;
+  float* cv;       // candidate list: `cap` values, then `cap` indices; a second list of the
+  uint32_t* ci;    // same size behind it
+  uint32_t n, k, kmax, cap;
+  uint32_t tiles, sampled;  // tiles of the array's layout (some may lie past n), and how many are sampled
 };
 
-// Selected elements are rare (about 0.1 % of the array), so a CTA collects its
-// finds in shared memory with plain shared atomics -- no block scan, no barrier
-// per tile -- and reserves its slice of the global lists once at the end.  Finds
-// beyond the shared buffer go to the global lists one by one.
-static __device__ __noinline__ void split_body(float* __restrict__ a, float* __restrict__ u, uint64_t n,
-                                           uint32_t k, uint32_t kmax, const EmitDst& dst,
-                                           uint32_t* __restrict__ ws, float* __restrict__ cand_val,
-                                           uint32_t* __restrict__ cand_idx, uint32_t cand_cap,
-                                           FindSmem& fs, SplitSmem& sp, uint32_t cta, uint32_t nctas) {
-  uint32_t bin0, k1;
-  if (threadIdx.x == 0) {
-    sp.nsel = 0;
-    sp.ncnd = 0;
-  }
-  find_bin(ws, k, fs, bin0, k1);  // contains the barriers that publish nsel / ncnd
-  const size_t val_off = 16 + align_up(4ull * kmax, 16);
-  const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(u)) & 15) == 0;
-  const uint64_t tiles = (n + 4095) / 4096;
-  for (uint64_t t = cta; t < tiles; t += nctas) {
-    float4 av[4];
+HP_HD SelUnit sel_unit(const float* g, float* a, float* u, uint32_t n, uint32_t k, uint32_t kmax, uint32_t* ws,
+                       void* cand, uint32_t pairs, uint32_t tiles, uint32_t sampled) {
+  SelUnit s;
+  s.g = g; s.a = a; s.u = u; s.ws = ws;
+  s.n = n; s.k = k; s.kmax = kmax;
+  s.tiles = tiles; s.sampled = sampled;
+  s.cap = pairs / 2 & ~3u;   // keeps every list on 16 bytes
+  s.cv = static_cast<float*>(cand);
+  s.ci = reinterpret_cast<uint32_t*>(s.cv + s.cap);
+  return s;
+}
+// how many of an array's tiles are sampled when ctas CTAs share `total` tiles: one each
+HP_HD uint32_t sampled_tiles(uint32_t tiles, uint64_t total, uint32_t ctas) {
+  const uint64_t share = ((uint64_t)tiles * ctas + total / 2) / (total ? total : 1);
+  const uint64_t f = share < kMinSampled ? kMinSampled : share;
+  return f < tiles ? (uint32_t)f : tiles;
+}
+// the i-th sampled tile, and the test for one
+__device__ __forceinline__ uint32_t sampled_tile(uint32_t i, uint32_t tiles, uint32_t sampled) {
+  return (uint32_t)((uint64_t)i * tiles / sampled);
+}
+__device__ __forceinline__ bool is_sampled(uint32_t t, uint32_t tiles, uint32_t sampled) {
+  const uint32_t i = (uint32_t)(((uint64_t)t * sampled + tiles - 1) / tiles);
+  return i < sampled && sampled_tile(i, tiles, sampled) == t;
+}
+__device__ __forceinline__ float* list2_values(const SelUnit& s) { return s.cv + 2 * (size_t)s.cap; }
+__device__ __forceinline__ uint32_t* list2_indices(const SelUnit& s) {
+  return reinterpret_cast<uint32_t*>(s.cv + 3 * (size_t)s.cap);
+}
+
+constexpr int kCollectBuf = 1024;  // candidates a CTA gathers before it reserves room in the lists
+constexpr int kStash = kFinishKeys / kSelTile;  // sampled tiles whose values stay in shared memory
+
+struct SelSmem {
+  union {
+    uint32_t hist[kBins];            // sample; finish: digit histograms
+    struct {
+      float val[kCollectBuf];
+      uint32_t idx[kCollectBuf];
+      uint16_t unit[kCollectBuf];
+    } buf;                           // collect
+  };
+  union {
+    uint32_t keys[kFinishKeys];      // finish
+    float stash[kStash][kSelTile];   // sample to collect
+  };
+  FindSmem fs;
+  uint32_t count, base, ticket, flag;
+  uint32_t sent, ties;
+};
+
+// Loads tile t and applies the update (MODE as in pass0_body), all loads before the first
+// store.  Elements past the end read as zero, and a zero is never sent.
+template <int MODE>
+__device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[4]) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
+                     (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
+  const uint64_t i0 = (uint64_t)t * kSelTile + threadIdx.x * 4;
+  float4 gv[4], uv[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      av[j] = ld4(a, t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4, n, vec);
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t i = i0 + j * kSpThreads * 4;
+    av[j] = ld4(s.a, i, s.n, vec);
+    if (MODE >= 1) gv[j] = ld4(s.g, i, s.n, vec);
+    if (MODE == 2) uv[j] = ld4(s.u, i, s.n, vec);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t i = i0 + j * kSpThreads * 4;
+    float4& v = av[j];
+    if (MODE == 1) {
+      v.x = v.x + gv[j].x; v.y = v.y + gv[j].y; v.z = v.z + gv[j].z; v.w = v.w + gv[j].w;
+      st4(s.a, i, s.n, vec, v);
+    } else if (MODE == 2) {
+      float4 w;
+      w.x = __fmaf_rn(momentum, uv[j].x, gv[j].x);
+      w.y = __fmaf_rn(momentum, uv[j].y, gv[j].y);
+      w.z = __fmaf_rn(momentum, uv[j].z, gv[j].z);
+      w.w = __fmaf_rn(momentum, uv[j].w, gv[j].w);
+      v.x = v.x + w.x; v.y = v.y + w.y; v.z = v.z + w.z; v.w = v.w + w.w;
+      st4(s.u, i, s.n, vec, w);
+      st4(s.a, i, s.n, vec, v);
+    }
+  }
+}
+
+// Sampled tile number i of an array: update, magnitudes into the array's sample histogram,
+// values into stash `slot` (-1: none).  The CTA that completes the sample turns it into
+// the candidates' lower bound.
+template <int MODE>
+static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum, SelSmem& sm, uint32_t i, int slot) {
+  const uint32_t t = sampled_tile(i, s.tiles, s.sampled);
+  if ((uint64_t)t * kSelTile < s.n) {
+    float4 av[4];
+    update_tile<MODE>(s, momentum, t, av);
+    for (int b = threadIdx.x; b < kBins / 4; b += kSpThreads)
+      reinterpret_cast<uint4*>(sm.hist)[b] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint64_t i = t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
+      if (slot >= 0) reinterpret_cast<float4*>(sm.stash[slot])[j * kSpThreads + threadIdx.x] = av[j];
       const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const uint32_t bin = abs_key(e[q]) >> 19;
-        if (i + q >= n || bin < bin0) continue;
-        if (bin > bin0) {  // certainly among the k largest: send and zero now
-          const uint32_t p = atomicAdd(&sp.nsel, 1u);
-          if (p < (uint32_t)kSplitBuf) {
-            sp.sel_val[p] = e[q];
-            sp.sel_idx[p] = (uint32_t)(i + q);
-          } else {
-            const uint32_t pos = atomicAdd(ws + kWsOutCount, 1u);
-            if (pos < kmax)
-              for (int d = 0; d < dst.n; ++d) {
-                reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = (uint32_t)(i + q);
-                reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = e[q];
-              }
-          }
-          a[i + q] = 0.0f;
-          if (u) u[i + q] = 0.0f;
-        } else {           // inside the threshold bin: decided on the candidate list
-          const uint32_t p = atomicAdd(&sp.ncnd, 1u);
-          if (p < (uint32_t)kSplitBuf) {
-            sp.cnd_val[p] = e[q];
-            sp.cnd_idx[p] = (uint32_t)(i + q);
-          } else {
-            const uint32_t pos = atomicAdd(ws + kWsCandCount, 1u);
-            if (pos < cand_cap) {
-              cand_val[pos] = e[q];
-              cand_idx[pos] = (uint32_t)(i + q);
-            } else {
-              ws[kWsOverflow] = 1u;
-            }
-          }
+        const uint32_t key = abs_key(e[q]);
+        if (key) atomicAdd(&sm.hist[key >> 19], 1u);
+      }
+    }
+    __syncthreads();
+    flush_hist(sm.hist, s.ws);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();   // cumulative over the CTA's counts, which the barrier ordered before it
+    sm.flag = atomicAdd(s.ws + kWsSampled, 1u) == s.sampled - 1;
+  }
+  __syncthreads();
+  if (!sm.flag) return;
+  __threadfence();
+  uint32_t rank = s.k;
+  if (s.sampled < s.tiles) {
+    // elements in the sample: what of the sampled tiles lies before n
+    uint32_t m = 0;
+    for (uint32_t q = threadIdx.x; q < s.sampled; q += kSpThreads) {
+      const uint64_t lo = (uint64_t)sampled_tile(q, s.tiles, s.sampled) * kSelTile;
+      if (lo < s.n) m += (uint32_t)min((uint64_t)kSelTile, s.n - lo);
+    }
+    if (threadIdx.x == 0) sm.base = 0;
+    __syncthreads();
+    if (m) atomicAdd(&sm.base, m);
+    __syncthreads();
+    // k scaled to the sample, plus five standard deviations, plus a tenth because
+    // neighbouring elements are not independent
+    const float hits = (float)((double)s.k * (double)sm.base / (double)s.n);
+    rank = (uint32_t)(1.1f * hits + 5.0f * sqrtf(hits) + 4.0f);
+  }
+  uint32_t bin, rem;
+  find_bin(s.ws, rank, sm.fs, bin, rem);   // bin 0 when fewer than rank are counted
+  if (threadIdx.x == 0) s.ws[kWsLow] = bin ? bin << 19 : 1u;   // zeros are never sent
+  __syncthreads();
+}
+
+// Items [0, total) in stretches, taken from *word by whichever of the ctas CTAs is free:
+// SMs do not run at one speed, and equal shares leave the fast ones waiting.  f(lo, hi)
+// runs with the whole CTA; `slot` is shared memory.  (Asking for the next stretch before
+// working on the current one split thread 0 from its warp, and the two halves then
+// counted twice at the barriers that follow.)
+template <typename F>
+__device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t ctas, uint32_t& slot, F f) {
+  const uint32_t stretch = total / (4u * ctas) + 1u;
+  for (;;) {
+    if (threadIdx.x == 0) slot = atomicAdd(word, stretch);
+    __syncthreads();
+    const uint32_t lo = slot;
+    __syncthreads();
+    if (lo >= total) break;
+    f(lo, min(lo + stretch, total));
+  }
+}
+
+// Put the elements of a tile that reach `low` into the CTA's buffer, for unit `uid`.
+__device__ __forceinline__ void collect_values(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, uint32_t t,
+                                               const float4 (&av)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
+    const uint32_t most = max(max(abs_key(e[0]), abs_key(e[1])), max(abs_key(e[2]), abs_key(e[3])));
+    if (most < low) continue;
+    const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t key = abs_key(e[q]);
+      if (key < low) continue;
+      const uint32_t p = atomicAdd(&sm.count, 1u);
+      if (p < (uint32_t)kCollectBuf) {
+        sm.buf.val[p] = e[q];
+        sm.buf.idx[p] = i + q;
+        sm.buf.unit[p] = (uint16_t)uid;
+      } else {   // more than the buffer holds: straight into the list
+        const uint32_t pos = atomicAdd(s.ws + kWsCandCount, 1u);
+        atomicAdd(s.ws + kBins + (key >> 19), 1u);
+        if (pos < s.cap) {
+          s.cv[pos] = e[q];
+          s.ci[pos] = i + q;
+        } else {
+          s.ws[kWsOverflow] = 1u;
         }
       }
     }
   }
-  __syncthreads();
-  const uint32_t nsel = min(sp.nsel, (uint32_t)kSplitBuf), ncnd = min(sp.ncnd, (uint32_t)kSplitBuf);
-  if (threadIdx.x == 0) {
-    sp.base_sel = nsel ? atomicAdd(ws + kWsOutCount, nsel) : 0u;
-    sp.base_cnd = ncnd ? atomicAdd(ws + kWsCandCount, ncnd) : 0u;
-    if (ncnd && sp.base_cnd + ncnd > cand_cap) ws[kWsOverflow] = 1u;
+}
+
+// Tiles [t0, t1) of one array without the sampled ones.
+template <int MODE>
+static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid, float momentum, SelSmem& sm,
+                                                 uint32_t t0, uint32_t t1) {
+  const uint32_t low = __ldcg(s.ws + kWsLow);
+  for (uint32_t t = t0; t < t1; ++t) {
+    if (is_sampled(t, s.tiles, s.sampled)) continue;
+    float4 av[4];
+    update_tile<MODE>(s, momentum, t, av);
+    collect_values(s, uid, sm, low, t, av);
   }
+}
+
+// Sampled tile number i again, updated before: from stash `slot`, or read again (-1).
+static __device__ __noinline__ void collect_sampled(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t i, int slot) {
+  const uint32_t t = sampled_tile(i, s.tiles, s.sampled);
+  if ((uint64_t)t * kSelTile >= s.n) return;
+  const uint32_t low = __ldcg(s.ws + kWsLow);
+  float4 av[4];
+  if (slot >= 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) av[j] = reinterpret_cast<const float4*>(sm.stash[slot])[j * kSpThreads + threadIdx.x];
+  } else {
+    update_tile<0>(s, 0.0f, t, av);
+  }
+  collect_values(s, uid, sm, low, t, av);
+}
+
+// Append the CTA's gathered candidates to their lists, and their first digits to the
+// lists' histograms.  A warp's entries mostly belong to one list: one reservation for each
+// group of lanes with the same list.  unit(uid) gives the array.
+template <typename F>
+__device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
   __syncthreads();
-  for (uint32_t p = threadIdx.x; p < nsel; p += kSpThreads) {
-    const uint32_t pos = sp.base_sel + p;
-    if (pos < kmax)
-      for (int d = 0; d < dst.n; ++d) {
-        reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = sp.sel_idx[p];
-        reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = sp.sel_val[p];
+  const uint32_t n = min(sm.count, (uint32_t)kCollectBuf);
+  for (uint32_t p0 = 0; p0 < n; p0 += kSpThreads) {
+    const uint32_t p = p0 + threadIdx.x;
+    const bool have = p < n;
+    const uint32_t mask = __ballot_sync(0xffffffffu, have);
+    if (have) {
+      const uint32_t uid = sm.buf.unit[p], lane = threadIdx.x & 31;
+      const float v = sm.buf.val[p];
+      const SelUnit s = unit(uid);
+      const uint32_t group = __match_any_sync(mask, uid);
+      const int lead = __ffs(group) - 1;
+      uint32_t pos = 0;
+      if ((int)lane == lead) pos = atomicAdd(s.ws + kWsCandCount, (uint32_t)__popc(group));
+      atomicAdd(s.ws + kBins + (abs_key(v) >> 19), 1u);
+      pos = __shfl_sync(group, pos, lead) + __popc(group & ((1u << lane) - 1u));
+      if (pos < s.cap) {
+        s.cv[pos] = v;
+        s.ci[pos] = sm.buf.idx[p];
+      } else {
+        s.ws[kWsOverflow] = 1u;
       }
-  }
-  for (uint32_t p = threadIdx.x; p < ncnd; p += kSpThreads) {
-    const uint32_t pos = sp.base_cnd + p;
-    if (pos < cand_cap) {
-      cand_val[pos] = sp.cnd_val[p];
-      cand_idx[pos] = sp.cnd_idx[p];
     }
   }
+  __syncthreads();
+  if (threadIdx.x == 0) sm.count = 0;
+  __syncthreads();
+}
+
+// store one pair at place `pos` of every destination's payload
+__device__ __forceinline__ void put_pair(const EmitDst& dst, size_t val_off, uint32_t kmax, uint32_t pos,
+                                         uint32_t idx, float val) {
+  if (pos >= kmax) return;
+  for (int d = 0; d < dst.n; ++d) {
+    reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = idx;
+    reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = val;
+  }
+}
+
+// Slice x of nx of a list too long for one CTA: pairs above the first digit's bin are
+// sent (and their state cleared), pairs in it move to the second list.  The finds of a
+// stretch are counted in shared memory so that the global counters are touched twice
+// per CTA and stretch.
+static __device__ __noinline__ void refine_body(const SelUnit& s, const EmitDst& dst, SelSmem& sm, uint32_t x,
+                                                uint32_t nx) {
+  const uint32_t L = min(__ldcg(s.ws + kWsCandCount), s.cap);
+  uint32_t bin0, rem;
+  find_bin(s.ws + kBins, min(s.k, L), sm.fs, bin0, rem);
+  const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
+  const uint32_t lo = (uint32_t)((uint64_t)L * x / nx), hi = (uint32_t)((uint64_t)L * (x + 1) / nx);
+  for (uint32_t p0 = lo; p0 < hi; p0 += 4 * kSpThreads) {
+    if (threadIdx.x == 0) sm.sent = sm.ties = 0;
+    __syncthreads();
+    float v[4];
+    uint32_t at[4], idx[4];
+    int what[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t p = p0 + j * kSpThreads + threadIdx.x;
+      v[j] = p < hi ? __ldcg(s.cv + p) : 0.0f;
+      idx[j] = p < hi ? __ldcg(s.ci + p) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t bin = abs_key(v[j]) >> 19;
+      const bool have = p0 + j * kSpThreads + threadIdx.x < hi;
+      what[j] = !have || bin < bin0 ? 0 : (bin > bin0 ? 1 : 2);
+      at[j] = what[j] == 1 ? atomicAdd(&sm.sent, 1u) : (what[j] == 2 ? atomicAdd(&sm.ties, 1u) : 0u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      sm.base = sm.sent ? atomicAdd(s.ws + kWsOutCount, sm.sent) : 0u;
+      sm.ticket = sm.ties ? atomicAdd(s.ws + kWsCand2Count, sm.ties) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (what[j] == 1 && idx[j] < s.n) {
+        put_pair(dst, val_off, s.kmax, sm.base + at[j], idx[j], v[j]);
+        s.a[idx[j]] = 0.0f;
+        if (s.u) s.u[idx[j]] = 0.0f;
+      } else if (what[j] == 2) {
+        const uint32_t pos = sm.ticket + at[j];   // never more than the first list holds
+        if (pos < s.cap) {
+          list2_values(s)[pos] = v[j];
+          list2_indices(s)[pos] = idx[j];
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Slice x of nx of the finish of one array.  The nx CTAs all work out the exact threshold
+// of the list (the second one after a refine step) -- its keys are a few kilobytes in L2,
+// and repeating the three digits costs less than a barrier after them -- and each sends
+// its share of the pairs.  True in thread 0 of the CTA that finished last, behind the
+// headers.  Every step runs once per launch, so its time is latency and instruction
+// fetch: one copy of the digit search, rolled loops.
+static __device__ __noinline__ bool finish_body(int alg, const SelUnit& s, const EmitDst& dst, SelSmem& sm,
+                                                bool refined, uint32_t x, uint32_t nx) {
+  const uint32_t all = min(__ldcg(s.ws + kWsCandCount), s.cap);
+  const uint32_t k = min(s.k, all);          // fewer than k non-zero elements: all of them
+  const uint32_t L = refined ? min(__ldcg(s.ws + kWsCand2Count), s.cap) : all;
+  const float* cv = refined ? list2_values(s) : s.cv;
+  const uint32_t* ci = refined ? list2_indices(s) : s.ci;
+  const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
+  // keys into shared memory, sixteen a thread in flight; past L whatever the list's room holds
+  for (uint32_t p0 = 0; p0 < L && p0 < kFinishKeys; p0 += 16 * kSpThreads) {
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t p = p0 + (j * kSpThreads + threadIdx.x) * 4;
+      v[j] = p < L ? __ldcg(reinterpret_cast<const uint4*>(cv + p)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t p = p0 + (j * kSpThreads + threadIdx.x) * 4;
+      *reinterpret_cast<uint4*>(sm.keys + p) =
+          make_uint4(v[j].x & 0x7FFFFFFFu, v[j].y & 0x7FFFFFFFu, v[j].z & 0x7FFFFFFFu, v[j].w & 0x7FFFFFFFu);
+    }
+  }
+  auto key_at = [&](uint32_t p) { return p < kFinishKeys ? sm.keys[p] : abs_key(__ldcg(cv + p)); };
+  uint32_t prefix, rem;
+  find_bin(s.ws + kBins, k, sm.fs, prefix, rem);
+  // the remaining digits: 11 bits, then 8
+#pragma unroll 1
+  for (int d = 0; d < 2; ++d) {
+    const int low = d == 0 ? 8 : 0, bits = d == 0 ? 11 : 8;
+    for (int b = threadIdx.x; b < kBins / 4; b += kSpThreads)
+      reinterpret_cast<uint4*>(sm.hist)[b] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < L; p += kSpThreads) {
+      const uint32_t key = key_at(p);
+      if ((key >> (low + bits)) == prefix) atomicAdd(&sm.hist[(key >> low) & ((1u << bits) - 1u)], 1u);
+    }
+    __syncthreads();
+    uint32_t bin, r;
+    find_bin(sm.hist, rem, sm.fs, bin, r);
+    prefix = (prefix << bits) | bin;
+    rem = r;
+  }
+  const uint32_t thr = prefix, need = rem;   // `need` of the elements equal to thr are sent
+  const uint32_t lo = (uint32_t)((uint64_t)L * x / nx), hi = (uint32_t)((uint64_t)L * (x + 1) / nx);
+  for (uint32_t p0 = lo; p0 < hi; p0 += kSpThreads) {
+    if (threadIdx.x == 0) sm.sent = sm.ties = 0;
+    __syncthreads();
+    const uint32_t p = p0 + threadIdx.x;
+    const uint32_t key = p < hi ? key_at(p) : 0u;
+    const bool more = p < hi && key > thr, tie = p < hi && key == thr;
+    uint32_t idx = 0, at = 0;
+    float val = 0.0f;
+    if (more || tie) {
+      idx = __ldcg(ci + p);
+      val = __ldcg(cv + p);
+      at = more ? atomicAdd(&sm.sent, 1u) : atomicAdd(&sm.ties, 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      // of this stretch's ties those that come early enough in the launch are sent
+      uint32_t ok = 0;
+      if (sm.ties && need) {
+        const uint32_t before = atomicAdd(s.ws + kWsTieCount, sm.ties);
+        ok = before < need ? min(sm.ties, need - before) : 0u;
+      }
+      sm.ties = ok;
+      sm.base = sm.sent + ok ? atomicAdd(s.ws + kWsOutCount, sm.sent + ok) : 0u;
+    }
+    __syncthreads();
+    const bool send = more || (tie && at < sm.ties);
+    if (send && idx < s.n) {
+      put_pair(dst, val_off, s.kmax, sm.base + (more ? at : sm.sent + at), idx, val);
+      s.a[idx] = 0.0f;
+      if (s.u) s.u[idx] = 0.0f;
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return false;
+  __threadfence();
+  if (atomicAdd(s.ws + kWsDone, 1u) != nx - 1) return false;
+  __threadfence();
+  const uint32_t sent = atomicAdd(s.ws + kWsOutCount, 0u);
+  WireHeader h;
+  h.n = s.n;
+  h.alg = (uint8_t)alg;
+  h.bitwidth = 0;
+  h.flags = 0;
+  h.a = all < s.k ? 0.0f : __uint_as_float(thr);
+  h.b = sent < s.kmax ? sent : s.kmax;
+  for (int d = 0; d < dst.n; ++d) *reinterpret_cast<uint4*>(dst.out[d]) = *reinterpret_cast<const uint4*>(&h);
+  return true;
+}
+// CTAs that share the finish of a list of L elements
+__device__ __forceinline__ uint32_t finish_slices(uint32_t L, uint32_t most) {
+  const uint32_t n = L / 256u + 1u;
+  return n < most ? n : most;
+}
+
+// The sample misled: the list lacks some of the k largest.
+__device__ __forceinline__ bool selection_failed(const SelUnit& s) {
+  const uint32_t c = __ldcg(s.ws + kWsCandCount);
+  return __ldcg(s.ws + kWsOverflow) != 0u || (c < s.k && __ldcg(s.ws + kWsLow) > 1u);
 }
 
 // out[idx] (+)= val * scale ; indices come from another rank: bounds-checked

@@ -1,15 +1,15 @@
 // Sparse (top-k) compression for DGC and GradDrop on sm_100a.
 //
+// With room for a candidate list (the usual call) an encode is ONE cooperative launch:
+// sample, update + collect, finish (sparse_core.cuh), with grid barriers in between.
+// It was a chain of eight launches; @OPS_NOTE@
+//
+// Without it (the allocation-free entry point) four launches read the array once each:
 //   pass 0   state update fused with the first radix histogram
 //              DGC      : u = m*u + g ; v += u        (momentum correction)
 //              GradDrop : r += g
-//            and a 4096-bin shared-memory histogram of bits 30..19 of |v|
-//   pass 1,2 histograms of bits 18..8 and 7..0 among elements matching the
-//            prefix chosen so far (every CTA re-derives the prefix from the global
-//            histograms, so no tiny "scan" launches sit between the passes)
-//   emit     exact threshold known: block-aggregated compaction of (index,value)
-//            pairs straight into the payload (which may live on a peer GPU), sent
-//            entries of v (and u) zeroed, header written by the last CTA.
+//   pass 1,2 histograms of bits 18..8 and 7..0 among elements matching the prefix so far
+//   emit     compaction of (index,value) pairs, sent entries of v (and u) zeroed
 //
 // The selection is exact: every |v_i| above the k-th largest magnitude is sent,
 // plus entries equal to it until k are sent (which of several equal entries is
@@ -21,6 +21,7 @@
 // sort/copy_if for them (src/CompLL/GCGen/unit.py:24-29) but has no translation
 // rule, so there is no reference kernel to compare with.
 #include "sparse_core.cuh"
+#include "sync.cuh"
 #include "hipress/noalloc.h"
 
 namespace hipress {
@@ -53,64 +54,78 @@ sparse_emit_kernel(int alg, float* __restrict__ a, float* __restrict__ u, uint64
   emit_body(alg, a, u, n, k, kmax, d, ws, fs, es, blockIdx.x, gridDim.x);
 }
 
-// ---- candidate path: split pass, then digit passes and compaction on the list
-__global__ void __launch_bounds__(kSpThreads)
-sparse_split_kernel(float* __restrict__ a, float* __restrict__ u, uint64_t n, uint32_t k,
-                    uint32_t kmax, uint8_t* __restrict__ out, uint32_t* __restrict__ ws,
-                    float* __restrict__ cand_val, uint32_t* __restrict__ cand_idx, uint32_t cap) {
+// ---- the whole encode in one cooperative launch
+struct SelArgs {
+  SelUnit unit;
+  int alg, mode;
+  float momentum;
+  uint8_t* out;
+};
+
+union SelOrPassSmem {
+  SelSmem sel;
+  uint32_t hist[kBins];   // whole-array passes
+  EmitSmem emit;
+};
+
+__global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const SelArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SelOrPassSmem& sm = *reinterpret_cast<SelOrPassSmem*>(smem_raw);
+  __shared__ WaitState wst;
   __shared__ FindSmem fs;
-  __shared__ SplitSmem sp;
+  const SelUnit& s = A.unit;
+  const uint32_t G = gridDim.x, c = blockIdx.x;
+  uint32_t gen = 0;
+  wait_init(wst);
+  auto barrier = [&]() {
+    grid_barrier(s.ws + kWsWords, gen, G, kGridBarrierNs, s.ws + kWsStatus, 1u, wst);
+  };
+  for (uint32_t i = c, r = 0; i < s.sampled; i += G, ++r) {
+    const int slot = r < (uint32_t)kStash ? (int)r : -1;
+    if (A.mode == 0) sample_body<0>(s, A.momentum, sm.sel, i, slot);
+    else if (A.mode == 1) sample_body<1>(s, A.momentum, sm.sel, i, slot);
+    else sample_body<2>(s, A.momentum, sm.sel, i, slot);
+  }
+  barrier();
+  if (threadIdx.x == 0) sm.sel.count = 0;
+  __syncthreads();
+  for (uint32_t i = c, r = 0; i < s.sampled; i += G, ++r)
+    collect_sampled(s, 0, sm.sel, i, r < (uint32_t)kStash ? (int)r : -1);
+  auto self = [&](uint32_t) { return s; };
+  if (s.sampled < s.tiles)
+    hand_out(s.ws + kWsTicket, s.tiles, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
+      if (A.mode == 0) collect_body<0>(s, 0, A.momentum, sm.sel, t0, t1);
+      else if (A.mode == 1) collect_body<1>(s, 0, A.momentum, sm.sel, t0, t1);
+      else collect_body<2>(s, 0, A.momentum, sm.sel, t0, t1);
+      if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, self);
+    });
+  collect_flush(sm.sel, self);
+  barrier();
   EmitDst d;
   d.n = 1;
-  d.out[0] = out;
-  split_body(a, u, n, k, kmax, d, ws, cand_val, cand_idx, cap, fs, sp, blockIdx.x, gridDim.x);
-}
-
-template <int PASS>
-__global__ void __launch_bounds__(kSpThreads)
-sparse_cand_pass_kernel(const float* __restrict__ cand_val, uint32_t k, uint32_t* __restrict__ ws) {
-  __shared__ uint32_t sh[kBins];
-  __shared__ FindSmem fs;
-  if (ws[kWsOverflow]) return;
-  pass_body<PASS>(cand_val, ws[kWsCandCount], k, ws, sh, fs, blockIdx.x, gridDim.x);
-}
-
-__global__ void __launch_bounds__(kSpThreads)
-sparse_cand_emit_kernel(int alg, float* __restrict__ cand_val, const uint32_t* __restrict__ cand_idx,
-                        float* __restrict__ a, float* __restrict__ u, uint32_t k, uint32_t kmax,
-                        uint8_t* __restrict__ out, uint32_t* __restrict__ ws, uint64_t n) {
-  __shared__ FindSmem fs;
-  __shared__ EmitSmem es;
-  if (ws[kWsOverflow]) return;
-  EmitDst d;
-  d.n = 1;
-  d.out[0] = out;
-  emit_body(alg, cand_val, u, ws[kWsCandCount], k, kmax, d, ws, fs, es, blockIdx.x, gridDim.x,
-            cand_idx, a, (uint32_t)n);
-}
-
-// ---- the full-array passes, run only when the candidate list overflowed
-template <int PASS>
-__global__ void __launch_bounds__(kSpThreads)
-sparse_fallback_pass_kernel(const float* __restrict__ a, uint64_t n, uint32_t k,
-                            uint32_t* __restrict__ ws) {
-  __shared__ uint32_t sh[kBins];
-  __shared__ FindSmem fs;
-  if (!ws[kWsOverflow]) return;
-  pass_body<PASS>(a, n, k, ws, sh, fs, blockIdx.x, gridDim.x);
-}
-
-__global__ void __launch_bounds__(kSpThreads)
-sparse_fallback_emit_kernel(int alg, float* __restrict__ a, float* __restrict__ u, uint64_t n,
-                            uint32_t k, uint32_t kmax, uint8_t* __restrict__ out,
-                            uint32_t* __restrict__ ws) {
-  __shared__ FindSmem fs;
-  __shared__ EmitSmem es;
-  if (!ws[kWsOverflow]) return;
-  EmitDst d;
-  d.n = 1;
-  d.out[0] = out;
-  emit_body(alg, a, u, n, k, kmax, d, ws, fs, es, blockIdx.x, gridDim.x);
+  d.out[0] = A.out;
+  if (!selection_failed(s)) {   // every CTA reads the same answer: its writers are behind the barrier
+    uint32_t L = min(__ldcg(s.ws + kWsCandCount), s.cap);
+    const bool longer = L > kFinishList;
+    if (longer) {
+      refine_body(s, d, sm.sel, c, G);
+      barrier();
+      L = min(__ldcg(s.ws + kWsCand2Count), s.cap);
+    }
+    const uint32_t nx = finish_slices(L, G);
+    if (c < nx) finish_body(A.alg, s, d, sm.sel, longer, c, nx);
+    return;
+  }
+  // whole-array passes
+  for (uint32_t i = c * kSpThreads + threadIdx.x; i < 3u * kBins; i += G * kSpThreads) s.ws[i] = 0;
+  barrier();
+  pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
+  barrier();
+  pass_body<1>(s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
+  barrier();
+  pass_body<2>(s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
+  barrier();
+  emit_body(A.alg, s.a, s.u, s.n, s.k, s.kmax, d, s.ws, fs, sm.emit, c, G);
 }
 
 __global__ void __launch_bounds__(kSpThreads)
@@ -119,21 +134,50 @@ sparse_scatter_kernel(const uint8_t* __restrict__ payload, float* __restrict__ o
   scatter_body(payload, out, n, kmax, scale, accumulate, blockIdx.x, gridDim.x);
 }
 
+// Decode of a short payload in one launch: every CTA clears its share of the result and
+// then looks through all pairs for those that fall into it (at most kScanPairs, read from
+// L2), instead of a memset, a wait and a scatter.
+constexpr uint32_t kScanPairs = 4096;
+__global__ void __launch_bounds__(kSpThreads)
+sparse_decode_kernel(const uint8_t* __restrict__ payload, float* __restrict__ out, uint64_t n, uint32_t kmax,
+                     float scale) {
+  const uint64_t per = ((n + gridDim.x - 1) / gridDim.x + 3) & ~3ull;
+  const uint64_t lo = min((uint64_t)blockIdx.x * per, n), hi = min(lo + per, n);
+  const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  for (uint64_t i = lo + threadIdx.x * 4; i < hi; i += kSpThreads * 4)
+    st4(out, i, hi, vec, make_float4(0.f, 0.f, 0.f, 0.f));
+  __syncthreads();
+  const WireHeader* h = reinterpret_cast<const WireHeader*>(payload);
+  const uint32_t k = min(__ldcg(&h->b), kmax);
+  const uint32_t* idx = reinterpret_cast<const uint32_t*>(payload + 16);
+  const float* val = reinterpret_cast<const float*>(payload + 16 + align_up(4ull * kmax, 16));
+  for (uint32_t p0 = 0; p0 < k; p0 += 4 * kSpThreads) {
+    uint32_t i[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t p = p0 + j * kSpThreads + threadIdx.x;
+      i[j] = p < k ? __ldcg(idx + p) : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i[j] >= lo && i[j] < hi) out[i[j]] = __ldcg(val + p0 + j * kSpThreads + threadIdx.x) * scale;
+  }
+}
+
 }  // namespace hipress
 
 using namespace hipress;
 
 extern "C" {
 
-// minimum scratch (histograms + counters); with room for a candidate list of
-// about 8 * kmax pairs on top, the encoder reads the array once instead of three
-// times after the state update
+// minimum scratch (histograms + counters); with room for two candidate lists of
+// 4 * kmax pairs each on top, the encoder reads the state once, in the update
 uint64_t hp_sparse_workspace_bytes() { return (uint64_t)kWsWords * 4; }
 uint64_t hp_sparse_workspace_bytes_for(uint64_t kmax) {
-  return (uint64_t)kWsWords * 4 + (8 * kmax + 4096) * 8;
+  return (uint64_t)(kWsWords + kBarrierWords) * 4 + (8 * kmax + 4096) * 8;
 }
 
-// ws_bytes beyond the histogram block is used as the candidate list; when there
+// ws_bytes beyond the histogram block is used for the candidate lists; when there
 // is none (the allocation-free entry point) the three full-array passes run.
 static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint64_t n, uint64_t k,
                               uint64_t kmax, float momentum, int update, uint8_t* out,
@@ -144,37 +188,54 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
   if (reinterpret_cast<uintptr_t>(out) & 15) return HP_ERR_BAD_ARG;
   if (update && !g) return HP_ERR_BAD_ARG;
   if (update && alg == kDgc && !u) return HP_ERR_BAD_ARG;
-  if (max_ctas <= 0) max_ctas = 148 * 4;
   const uint64_t tiles = (n + 4095) / 4096;
-  const int grid = (int)(tiles < (uint64_t)max_ctas ? tiles : (uint64_t)max_ctas);
-  cudaError_t e = cudaMemsetAsync(ws, 0, (size_t)kWsWords * 4, st);
-  if (e != cudaSuccess) return (int)e;
-  if (!update) sparse_pass0_kernel<0><<<grid, kSpThreads, 0, st>>>(g, a, u, n, momentum, ws);
-  else if (alg == kGradDrop) sparse_pass0_kernel<1><<<grid, kSpThreads, 0, st>>>(g, a, u, n, momentum, ws);
-  else sparse_pass0_kernel<2><<<grid, kSpThreads, 0, st>>>(g, a, u, n, momentum, ws);
   float* uu = alg == kDgc ? u : nullptr;
-  const uint64_t head = (uint64_t)kWsWords * 4;
-  const uint64_t cap = ws_bytes > head ? (ws_bytes - head) / 8 : 0;
-  if (cap >= 1024) {
-    float* cand_val = reinterpret_cast<float*>(ws + kWsWords);
-    uint32_t* cand_idx = reinterpret_cast<uint32_t*>(cand_val + cap);
-    const int cgrid = grid < 64 ? grid : 64;
-    sparse_split_kernel<<<grid, kSpThreads, 0, st>>>(a, uu, n, (uint32_t)k, (uint32_t)kmax, out, ws,
-                                                      cand_val, cand_idx, (uint32_t)cap);
-    sparse_cand_pass_kernel<1><<<cgrid, kSpThreads, 0, st>>>(cand_val, (uint32_t)k, ws);
-    sparse_cand_pass_kernel<2><<<cgrid, kSpThreads, 0, st>>>(cand_val, (uint32_t)k, ws);
-    sparse_cand_emit_kernel<<<cgrid, kSpThreads, 0, st>>>(alg, cand_val, cand_idx, a, uu, (uint32_t)k,
-                                                          (uint32_t)kmax, out, ws, n);
-    sparse_fallback_pass_kernel<1><<<grid, kSpThreads, 0, st>>>(a, n, (uint32_t)k, ws);
-    sparse_fallback_pass_kernel<2><<<grid, kSpThreads, 0, st>>>(a, n, (uint32_t)k, ws);
-    sparse_fallback_emit_kernel<<<grid, kSpThreads, 0, st>>>(alg, a, uu, n, (uint32_t)k,
-                                                              (uint32_t)kmax, out, ws);
-  } else {
-    sparse_pass_kernel<1><<<grid, kSpThreads, 0, st>>>(a, n, (uint32_t)k, ws);
-    sparse_pass_kernel<2><<<grid, kSpThreads, 0, st>>>(a, n, (uint32_t)k, ws);
-    sparse_emit_kernel<<<grid, kSpThreads, 0, st>>>(alg, a, uu, n, (uint32_t)k, (uint32_t)kmax, out,
-                                                     ws);
+  const int mode = !update ? 0 : (alg == kGradDrop ? 1 : 2);
+  // histograms and counters, then the barrier words and the candidate lists
+  const uint64_t head = (uint64_t)(kWsWords + kBarrierWords) * 4;
+  const uint64_t pairs = ws_bytes > head ? (ws_bytes - head) / 8 : 0;
+  const bool listed = pairs >= 1024;
+  cudaError_t e = cudaMemsetAsync(ws, 0, listed ? head : (size_t)kWsWords * 4, st);
+  if (e != cudaSuccess) return (int)e;
+  if (listed) {
+    const size_t smem = sizeof(SelOrPassSmem);
+    static int resident[64] = {};   // CTAs the GPU holds at once, per device
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    int cap = dev >= 0 && dev < 64 ? resident[dev] : 0;
+    if (cap == 0) {
+      int sms = 0, per = 0;
+      e = cudaFuncSetAttribute((const void*)sparse_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return (int)e;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sparse_encode_kernel, kSpThreads, smem);
+      if (e != cudaSuccess) return (int)e;
+      cap = per * sms;
+      if (cap < 1) return HP_ERR_RESIDENCY;
+      if (dev >= 0 && dev < 64) resident[dev] = cap;
+    }
+    if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
+    const int grid = (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
+    SelArgs A;
+    A.unit = sel_unit(g, a, uu, (uint32_t)n, (uint32_t)k, (uint32_t)kmax, ws, ws + kWsWords + kBarrierWords,
+                      (uint32_t)(pairs < 0xFFFFFFFEull ? pairs : 0xFFFFFFFEull), (uint32_t)tiles,
+                      sampled_tiles((uint32_t)tiles, tiles, (uint32_t)grid));
+    A.alg = alg;
+    A.mode = mode;
+    A.momentum = momentum;
+    A.out = out;
+    void* args[] = {(void*)&A};
+    return (int)cudaLaunchCooperativeKernel((const void*)sparse_encode_kernel, dim3(grid), dim3(kSpThreads), args, smem, st);
   }
+  if (max_ctas <= 0) max_ctas = 148 * 4;
+  const int grid = (int)(tiles < (uint64_t)max_ctas ? tiles : (uint64_t)max_ctas);
+  if (mode == 0) sparse_pass0_kernel<0><<<grid, kSpThreads, 0, st>>>(g, a, u, n, momentum, ws);
+  else if (mode == 1) sparse_pass0_kernel<1><<<grid, kSpThreads, 0, st>>>(g, a, u, n, momentum, ws);
+  else sparse_pass0_kernel<2><<<grid, kSpThreads, 0, st>>>(g, a, u, n, momentum, ws);
+  sparse_pass_kernel<1><<<grid, kSpThreads, 0, st>>>(a, n, (uint32_t)k, ws);
+  sparse_pass_kernel<2><<<grid, kSpThreads, 0, st>>>(a, n, (uint32_t)k, ws);
+  sparse_emit_kernel<<<grid, kSpThreads, 0, st>>>(alg, a, uu, n, (uint32_t)k, (uint32_t)kmax, out, ws);
   return (int)cudaGetLastError();
 }
 
@@ -225,6 +286,11 @@ int hp_cuda_sparse_decode(const uint8_t* payload, float* out, uint64_t n, uint64
   if (n == 0) return 0;
   if (reinterpret_cast<uintptr_t>(payload) & 15) return HP_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
+  if (!accumulate && kmax && kmax <= kScanPairs) {
+    const uint64_t tiles = (n + 4095) / 4096;
+    sparse_decode_kernel<<<(int)(tiles < 148 * 8 ? tiles : 148 * 8), kSpThreads, 0, st>>>(payload, out, n, (uint32_t)kmax, scale);
+    return (int)cudaGetLastError();
+  }
   if (!accumulate) {
     cudaError_t e = cudaMemsetAsync(out, 0, n * sizeof(float), st);
     if (e != cudaSuccess) return (int)e;
