@@ -42,8 +42,10 @@ struct SpSeg {
   uint32_t n, chunk, kmax, pay_off;
   uint32_t tiles;       // tiles of one chunk
   uint32_t tile_prefix; // tiles of one chunk of the tensors before this one
-  uint32_t sampled;     // tiles of one chunk that are sampled (set at launch: depends on the grid)
-  uint32_t sample_prefix;
+  uint32_t k_last;      // pairs of the last chunk, which may be shorter
+  // set at launch, they depend on the grid: every stride-th tile of a chunk is sampled,
+  // `sampled` of them
+  uint32_t stride, sampled, sample_prefix;
   uint32_t cap;         // candidate pairs per (tensor, chunk) unit, for both lists
   uint64_t cand_push;   // first push unit's candidate list, in pairs from the region start
   uint64_t cand_srv;    // the server unit's candidate list
@@ -142,39 +144,89 @@ __device__ __forceinline__ uint32_t slices_cap(const SpCtx& cx, uint32_t units, 
   return p > cap ? cap : p;
 }
 
+// Zero-fill of the result, tile by tile.  It runs behind the barrier of the update pass,
+// which reads the gradient (it may be the same buffer), on the CTAs that have no list to
+// finish: clearing each element right behind its load in the update pass made that
+// pass five times slower (a store to a line whose fill is still in flight).
+static __device__ __noinline__ void zero_result(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm,
+                                            int ticket) {
+  const uint32_t N = (uint32_t)cx.N;
+  hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * N, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
+    int si = 0;
+    for (; t < end; ++t) {
+      while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * N) ++si;
+      const SpSeg& sg = bk.seg[si];
+      float* out = sg.out + cx.E * cm.emu_stride_out;
+      const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+      const uint64_t i0 = (uint64_t)(t - sg.tile_prefix * N) * kTile + threadIdx.x * 4;
+#pragma unroll
+      for (int j = 0; j < kTile / (4 * kSpThreads); ++j)
+        st4(out, i0 + j * kSpThreads * 4, sg.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+  });
+}
+
 // ------------------------------------------------------------ units of a selection
 // push : every (tensor, owner) pair, unit y = tensor * N + owner
 // serve: the owned chunk of every tensor, y = tensor
 // hop  : the chunk of every tensor that hop `hop` of the ring works on, y = tensor
+// The kind is a run-time value: the two selections of a PS launch and the hops of a ring
+// run the same instructions, so all but the first find them in the instruction cache.
 enum SelKind { kSelPush, kSelServe, kSelHop };
+
+struct SelPhase {
+  int kind, hop;
+  uint32_t per_tensor;  // units per tensor
+  uint32_t units;
+  int mode;             // of the update: see pass0_body
+};
+__device__ __forceinline__ SelPhase sel_phase(const SpBucket& bk, const SpCtx& cx, int kind, int hop) {
+  SelPhase p;
+  p.kind = kind;
+  p.hop = hop;
+  p.per_tensor = kind == kSelPush ? (uint32_t)cx.N : 1u;
+  p.units = (uint32_t)bk.nseg * p.per_tensor;
+  p.mode = kind == kSelServe ? 0 : (bk.alg == kDgc ? 2 : 1);
+  return p;
+}
 
 struct UnitRef {
   int si, c;
 };
-template <int KIND>
-__device__ __forceinline__ UnitRef unit_ref(const SpCtx& cx, int y, int hop) {
-  if (KIND == kSelPush) return {y / cx.N, y % cx.N};
-  if (KIND == kSelServe) return {y, cx.R};
-  return {y, (cx.R - hop + cx.N) % cx.N};
+__device__ __forceinline__ UnitRef unit_ref(const SpCtx& cx, const SelPhase& ph, uint32_t y) {
+  if (ph.kind == kSelPush) return {(int)(y / (uint32_t)cx.N), (int)(y % (uint32_t)cx.N)};
+  if (ph.kind == kSelServe) return {(int)y, cx.R};
+  const int c = cx.R - ph.hop;
+  return {(int)y, c < 0 ? c + cx.N : c};
 }
 
 // the array of a unit; n = 0 for a chunk past the tensor's end
-template <int KIND>
-__device__ __forceinline__ SelUnit unit_of(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, int y, int hop) {
-  const UnitRef r = unit_ref<KIND>(cx, y, hop);
+static __device__ __noinline__ void unit_of(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, const SelPhase& ph,
+                                            uint32_t y, SelUnit& s) {
+  const UnitRef r = unit_ref(cx, ph, y);
   const SpSeg& sg = bk.seg[r.si];
-  const int E = cx.E;
-  const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, r.c);
-  const uint32_t k = (uint32_t)sparse_k(len, bk.ratio);
-  const size_t off = (size_t)r.c * sg.chunk;
-  if (KIND == kSelServe)
-    return sel_unit(nullptr, sg.sr + E * cm.emu_stride_sr, nullptr, len, k, sg.kmax,
-                    cx.ws + ((size_t)bk.nseg * cx.N + y) * kWsWords, cx.cand + sg.cand_srv * 8, sg.cap,
-                    sg.tiles, sg.sampled);
-  const size_t block = KIND == kSelPush ? (size_t)y : (size_t)hop * bk.nseg + r.si;
-  return sel_unit(sg.g + E * cm.emu_stride_g + off, sg.a + E * cm.emu_stride_r + off,
-                  sg.u ? sg.u + E * cm.emu_stride_r + off : nullptr, len, k, sg.kmax, cx.ws + block * kWsWords,
-                  cx.cand + (sg.cand_push + (uint64_t)r.c * sg.cap) * 8, sg.cap, sg.tiles, sg.sampled);
+  const size_t E = (size_t)cx.E, off = (size_t)r.c * sg.chunk;
+  s.n = sp_chunk_valid(sg.n, sg.chunk, r.c);
+  s.k = s.n == sg.chunk ? sg.kmax : sg.k_last;   // only the last chunk is shorter
+  s.kmax = sg.kmax;
+  s.cap = list_cap(sg.cap);
+  s.stride = sg.stride;
+  s.sampled = s.n == sg.chunk ? sg.sampled : ((s.n + kTile - 1) / kTile + sg.stride - 1) / sg.stride;
+  uint64_t list = sg.cand_srv;
+  uint32_t block = (uint32_t)(bk.nseg * cx.N) + y;
+  s.g = nullptr;
+  s.u = nullptr;
+  if (ph.kind == kSelServe) {
+    s.a = sg.sr + E * cm.emu_stride_sr;
+  } else {
+    s.g = sg.g + E * cm.emu_stride_g + off;
+    s.a = sg.a + E * cm.emu_stride_r + off;
+    if (sg.u) s.u = sg.u + E * cm.emu_stride_r + off;
+    list = sg.cand_push + (uint64_t)r.c * sg.cap;
+    block = ph.kind == kSelPush ? y : (uint32_t)(ph.hop * bk.nseg + r.si);
+  }
+  s.ws = cx.ws + (size_t)block * kWsWords;
+  s.cv = reinterpret_cast<float*>(cx.cand + list * 8);
 }
 
 // where a unit's pairs go, and the flags that announce them
@@ -182,86 +234,102 @@ struct UnitDst {
   EmitDst out;
   uint32_t* flag[HP_MAX_RANKS];
 };
-template <int KIND>
-__device__ __forceinline__ void unit_dst(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, int y, int hop,
-                                         UnitDst& d) {
+static __device__ __noinline__ void unit_dst(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, const SelPhase& ph,
+                                             uint32_t y, UnitDst& d) {
   const int N = cx.N, R = cx.R;
-  const UnitRef r = unit_ref<KIND>(cx, y, hop);
-  const bool all = KIND == kSelServe || (KIND == kSelHop && hop == N - 1);
-  const int first = KIND == kSelPush ? r.c : (all ? R : (R + 1) % N);
-  const int slot = KIND == kSelPush ? R : (KIND == kSelServe ? N + R : (all ? N - 1 + R : hop));
+  const UnitRef r = unit_ref(cx, ph, y);
+  const bool all = ph.kind == kSelServe || (ph.kind == kSelHop && ph.hop == N - 1);
+  int to = ph.kind == kSelPush ? r.c : (all ? R : R + 1);
+  const int slot = ph.kind == kSelPush ? R : (ph.kind == kSelServe ? N + R : (all ? N - 1 + R : ph.hop));
   d.out.n = all ? N : 1;
-  for (int q = 0; q < d.out.n; ++q) {
-    const int to = (first + q) % N;
+#pragma unroll 1
+  for (int q = 0; q < d.out.n; ++q, ++to) {
+    if (to >= N) to -= N;
     d.out.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[to]) + (size_t)slot * bk.slot_bytes + bk.seg[r.si].pay_off;
     d.flag[q] = reinterpret_cast<uint32_t*>(cm.flags[to]) + (size_t)slot * bk.nseg + r.si;
   }
 }
 // thread 0 of the CTA that completed the unit
-__device__ __forceinline__ void unit_release(const HpComm& cm, const SpSmem& sm, const UnitDst& d) {
+static __device__ __noinline__ void unit_release(const HpComm& cm, const SpSmem& sm, const UnitDst& d) {
   __threadfence_system();
   const uint32_t v = flag_value(cm, sm);
+#pragma unroll 1
   for (int q = 0; q < d.out.n; ++q) st_release_sys(d.flag[q], v);
 }
 
-// The selection of all units of one kind: two barriers (three when some list is longer
-// than one CTA finishes, more only when a sample misled).  `idle` runs on every CTA
-// after the update pass, while few of them finish lists.
-template <int KIND, typename F>
-__device__ __forceinline__ void select_units(const SpBucket& bk, const HpComm& cm, SpCtx& cx, SpSmem& sm, int hop,
-                                             int ticket, F idle) {
-  const uint32_t M = KIND == kSelPush ? (uint32_t)cx.N : 1u;   // units per tensor
-  const uint32_t units = (uint32_t)bk.nseg * M;
-  const int mode = KIND == kSelServe ? 0 : (bk.alg == kDgc ? 2 : 1);
-  auto unit = [&](uint32_t y) { return unit_of<KIND>(bk, cm, cx, (int)y, hop); };
-  // sampled tiles: item i belongs to unit y as its tile number j
-  const uint32_t samples = bk.samples_total * M;
-  auto sampled = [&](auto f) {
-    for (uint32_t i = blockIdx.x, r = 0; i < samples; i += cx.G, ++r) {
-      int si = 0;
-      while (si + 1 < bk.nseg && i >= bk.seg[si + 1].sample_prefix * M) ++si;
-      const SpSeg& sg = bk.seg[si];
-      const uint32_t at = i - sg.sample_prefix * M;
-      const uint32_t y = KIND == kSelPush ? si * cx.N + at / sg.sampled : (uint32_t)si;
-      const SelUnit s = unit(y);
-      if (s.n) f(s, y, at % sg.sampled, r < (uint32_t)kStash ? (int)r : -1);
-    }
-  };
-  sampled([&](const SelUnit& s, uint32_t, uint32_t j, int slot) {
-    if (mode == 0) sample_body<0>(s, bk.momentum, sm.sel, j, slot);
-    else if (mode == 1) sample_body<1>(s, bk.momentum, sm.sel, j, slot);
-    else sample_body<2>(s, bk.momentum, sm.sel, j, slot);
+static __device__ __noinline__ void flush_units(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
+                                                const SelPhase& ph, SpSmem& sm) {
+  collect_flush(sm.sel, [&](uint32_t y) {
+    SelUnit s;
+    unit_of(bk, cm, cx, ph, y, s);
+    return s;
   });
+}
+
+// The sampled tiles of this CTA, in the sample pass or (collect) after it: item i belongs
+// to one unit as its tile number j.  The first two stay in shared memory in between.
+static __device__ __noinline__ void sample_units(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
+                                                 const SelPhase& ph, SpSmem& sm, bool collect) {
+  const uint32_t M = ph.per_tensor, total = bk.samples_total * M;
+  const bool more = blockIdx.x + 2 * cx.G < total;   // the second stash is used again
+  int si = 0;
+#pragma unroll 1
+  for (uint32_t i = blockIdx.x, r = 0; i < total; i += cx.G, ++r) {
+    while (si + 1 < bk.nseg && i >= bk.seg[si + 1].sample_prefix * M) ++si;
+    const SpSeg& sg = bk.seg[si];
+    const uint32_t at = i - sg.sample_prefix * M, c = at / sg.sampled, j = at - c * sg.sampled;
+    const uint32_t y = (uint32_t)si * M + (M > 1 ? c : 0u);
+    SelUnit s;
+    unit_of(bk, cm, cx, ph, y, s);
+    if (j >= s.sampled) continue;
+    float* stash = sm.sel.stash[r < 1 ? 0 : 1];
+    if (collect) collect_sampled(s, y, sm.sel, j, stash, r >= 1 && more);
+    else sample_body(ph.mode, s, bk.momentum, sm.sel, j, stash);
+  }
+}
+
+// The selection of all units of one kind: two barriers (three when some list is long,
+// more only when a sample misled).  Tickets `ticket` and, when the result is to be
+// cleared behind the update pass, ticket + 1.
+static __device__ __noinline__ void select_units(const SpBucket& bk, const HpComm& cm, SpCtx& cx, SpSmem& sm, int kind,
+                                                 int hop, int ticket, bool zero) {
+  const SelPhase ph = sel_phase(bk, cx, kind, hop);
+  const uint32_t M = ph.per_tensor, units = ph.units;
+  sample_units(bk, cm, cx, ph, sm, false);
   sp_barrier(cm, cx, sm);
   if (threadIdx.x == 0) sm.sel.count = 0;
   __syncthreads();
-  sampled([&](const SelUnit& s, uint32_t y, uint32_t j, int slot) { collect_sampled(s, y, sm.sel, j, slot); });
+  sample_units(bk, cm, cx, ph, sm, true);
   hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * M, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
     int si = 0;
+#pragma unroll 1
     while (t < end) {
       while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * M) ++si;
       const SpSeg& sg = bk.seg[si];
-      const uint32_t at = t - sg.tile_prefix * M, c = at / sg.tiles, tt = at % sg.tiles;
+      const uint32_t at = t - sg.tile_prefix * M, c = at / sg.tiles, tt = at - c * sg.tiles;
       const uint32_t stop = min(sg.tiles, tt + (end - t));
-      const uint32_t y = KIND == kSelPush ? si * cx.N + c : (uint32_t)si;
-      const SelUnit s = unit(y);
-      const uint32_t t1 = min(stop, (s.n + kTile - 1) / kTile);
-      if (tt < t1) {
-        if (mode == 0) collect_body<0>(s, y, bk.momentum, sm.sel, tt, t1);
-        else if (mode == 1) collect_body<1>(s, y, bk.momentum, sm.sel, tt, t1);
+      const uint32_t y = (uint32_t)si * M + (M > 1 ? c : 0u);
+      if (sg.stride > 1) {
+        SelUnit s;
+        unit_of(bk, cm, cx, ph, y, s);
+        const uint32_t t1 = min(stop, (s.n + kTile - 1) / kTile);
+        if (ph.mode == 0) collect_body<0>(s, y, bk.momentum, sm.sel, tt, t1);
+        else if (ph.mode == 1) collect_body<1>(s, y, bk.momentum, sm.sel, tt, t1);
         else collect_body<2>(s, y, bk.momentum, sm.sel, tt, t1);
       }
       t += stop - tt;
     }
-    if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, unit);
+    if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) flush_units(bk, cm, cx, ph, sm);
   });
-  collect_flush(sm.sel, unit);
+  flush_units(bk, cm, cx, ph, sm);
   sp_barrier(cm, cx, sm);
   // behind the barrier every CTA reads the same counters and decides the same
   if (threadIdx.x == 0) sm.any = sm.ticket = 0;
   __syncthreads();
+#pragma unroll 1
   for (uint32_t y = threadIdx.x; y < units; y += kSpThreads) {
-    const SelUnit s = unit_of<KIND>(bk, cm, cx, (int)y, hop);
+    SelUnit s;
+    unit_of(bk, cm, cx, ph, y, s);
     if (s.n == 0) continue;
     if (selection_failed(s)) sm.any = 1;
     else atomicMax(&sm.ticket, __ldcg(s.ws + kWsCandCount));
@@ -271,66 +339,62 @@ __device__ __forceinline__ void select_units(const SpBucket& bk, const HpComm& c
   __syncthreads();
   if (refined) {
     run_units(cx, units, slices_cap(cx, units, 64), [&](int y, uint32_t x, uint32_t nx) {
-      const SelUnit s = unit_of<KIND>(bk, cm, cx, y, hop);
+      SelUnit s;
+      unit_of(bk, cm, cx, ph, (uint32_t)y, s);
       if (s.n == 0 || selection_failed(s)) return;
       UnitDst d;
-      unit_dst<KIND>(bk, cm, cx, y, hop, d);
+      unit_dst(bk, cm, cx, ph, (uint32_t)y, d);
       refine_body(s, d.out, sm.sel, x, nx);
     });
     sp_barrier(cm, cx, sm);
   }
-  sp_mark(cx, KIND == kSelServe ? 4 : 0);
-  const uint32_t share = cx.G / units ? cx.G / units : 1u;
+  const uint32_t share = slices_cap(cx, units, 64);
   run_units(cx, units, share, [&](int y, uint32_t x, uint32_t) {
-    const SelUnit s = unit_of<KIND>(bk, cm, cx, y, hop);
-    uint32_t nx = 1;
-    if (s.n && !selection_failed(s))
-      nx = finish_slices(min(__ldcg(s.ws + (refined ? kWsCand2Count : kWsCandCount)), s.cap), share);
-    if (x >= nx) return;
+    SelUnit s;
+    unit_of(bk, cm, cx, ph, (uint32_t)y, s);
+    const bool bad = s.n && selection_failed(s);
+    const uint32_t nx =
+        s.n && !bad ? finish_slices(min(__ldcg(s.ws + (refined ? kWsCand2Count : kWsCandCount)), s.cap), share) : 1u;
+    if (x >= nx || bad) return;
     UnitDst d;
-    unit_dst<KIND>(bk, cm, cx, y, hop, d);
+    unit_dst(bk, cm, cx, ph, (uint32_t)y, d);
     bool done = false;
     if (s.n == 0) {
       done = threadIdx.x == 0;
       if (done)
         for (int q = 0; q < d.out.n; ++q) write_empty_header(d.out.out[q], bk.alg);
-    } else if (!selection_failed(s)) {
+    } else {
       done = finish_body(bk.alg, s, d.out, sm.sel, refined, x, nx);
     }
     if (done) unit_release(cm, sm, d);
   });
-  sp_mark(cx, KIND == kSelServe ? 5 : 1);
-  idle();
-  sp_mark(cx, KIND == kSelServe ? 6 : 2);
+  sp_mark(cx, kind == kSelServe ? 2 : 0);
+  if (zero) zero_result(bk, cm, cx, sm, ticket + 1);
+  sp_mark(cx, kind == kSelServe ? 3 : 1);
   if (!failed) return;
-  // whole-array passes for the units whose sample misled
-  const uint32_t ph = slices_heavy(cx, units);
-  auto again = [&](auto f) {
-    run_units(cx, units, ph, [&](int y, uint32_t x, uint32_t nx) {
-      const SelUnit s = unit_of<KIND>(bk, cm, cx, y, hop);
-      if (s.n != 0 && selection_failed(s)) f(s, y, x, nx);
-    });
-  };
-  again([&](const SelUnit& s, int, uint32_t x, uint32_t nx) {
-    for (uint32_t i = x * kSpThreads + threadIdx.x; i < 3u * kBins; i += nx * kSpThreads) s.ws[i] = 0;
-  });
-  sp_barrier(cm, cx, sm);
-  again([&](const SelUnit& s, int, uint32_t x, uint32_t nx) {
-    pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.sh, x, nx);
-  });
-  sp_barrier(cm, cx, sm);
+  // whole-array passes for the units whose sample misled: clear the histograms, count the
+  // three digits, send
+  const uint32_t heavy = slices_heavy(cx, units);
 #pragma unroll 1
-  for (int pass = 1; pass <= 2; ++pass) {
-    again([&](const SelUnit& s, int, uint32_t x, uint32_t nx) {
-      pass_body_rt(pass, s.a, s.n, s.k, s.ws, sm.sh, sm.fs, x, nx);
+  for (int pass = -1; pass <= 3; ++pass) {
+    run_units(cx, units, heavy, [&](int y, uint32_t x, uint32_t nx) {
+      SelUnit s;
+      unit_of(bk, cm, cx, ph, (uint32_t)y, s);
+      if (s.n == 0 || !selection_failed(s)) return;
+      if (pass < 0) {
+        for (uint32_t i = x * kSpThreads + threadIdx.x; i < 3u * kBins; i += nx * kSpThreads) s.ws[i] = 0;
+      } else if (pass == 0) {
+        pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.sh, x, nx);
+      } else if (pass < 3) {
+        pass_body_rt(pass, s.a, s.n, s.k, s.ws, sm.sh, sm.fs, x, nx);
+      } else {
+        UnitDst d;
+        unit_dst(bk, cm, cx, ph, (uint32_t)y, d);
+        if (emit_body(bk.alg, s.a, s.u, s.n, s.k, s.kmax, d.out, s.ws, sm.fs, sm.es, x, nx)) unit_release(cm, sm, d);
+      }
     });
-    sp_barrier(cm, cx, sm);
+    if (pass < 3) sp_barrier(cm, cx, sm);
   }
-  again([&](const SelUnit& s, int y, uint32_t x, uint32_t nx) {
-    UnitDst d;
-    unit_dst<KIND>(bk, cm, cx, y, hop, d);
-    if (emit_body(bk.alg, s.a, s.u, s.n, s.k, s.kmax, d.out, s.ws, sm.fs, sm.es, x, nx)) unit_release(cm, sm, d);
-  });
 }
 
 // ---------------------------------------------------------------- incoming payloads
@@ -366,28 +430,6 @@ __device__ __forceinline__ void hop_in(const SpBucket& bk, const HpComm& cm, con
 }
 
 // ---------------------------------------------------------------- pull
-// Zero-fill of the result, tile by tile.  It runs behind the barrier of the update pass,
-// which reads the gradient (it may be the same buffer), on the CTAs that have no list to
-// finish: clearing each element right behind its load in the update pass made that
-// pass five times slower (a store to a line whose fill is still in flight).
-__device__ __forceinline__ void zero_result(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm,
-                                            int ticket) {
-  const uint32_t N = (uint32_t)cx.N;
-  hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * N, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
-    int si = 0;
-    for (; t < end; ++t) {
-      while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * N) ++si;
-      const SpSeg& sg = bk.seg[si];
-      float* out = sg.out + cx.E * cm.emu_stride_out;
-      const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-      const uint64_t i0 = (uint64_t)(t - sg.tile_prefix * N) * kTile + threadIdx.x * 4;
-#pragma unroll
-      for (int j = 0; j < kTile / (4 * kSpThreads); ++j)
-        st4(out, i0 + j * kSpThreads * 4, sg.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
-    }
-  });
-}
-
 // wait for the reduced chunk c that arrives in inbox slot `slot` and scatter value / N
 // into the (zero-filled) result; unit y = seg * N + j.  A CTA that has given up leaves
 // the result alone.
@@ -445,18 +487,18 @@ __device__ __forceinline__ void sp_epilogue(const SpCtx& cx) {
 // inbox), pull (every rank scatters value / N).  Five barriers when the candidate lists
 // are short.  @PS_NOTE@
 __global__ void __launch_bounds__(kSpThreads, 3)
-sp_ps_kernel(const SpBucket bk, const HpComm cm, const SpLaunch L) {
+sp_ps_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm cm, const __grid_constant__ SpLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
   SpCtx cx;
   sp_prologue(cm, L, cx, sm);
   const int N = cx.N;
   const uint32_t nseg = (uint32_t)bk.nseg, units = nseg * (uint32_t)N;
-  select_units<kSelPush>(bk, cm, cx, sm, 0, 0, [&] { zero_result(bk, cm, cx, sm, 1); });
+  select_units(bk, cm, cx, sm, kSelPush, 0, 0, true);
   run_units(cx, nseg, slices_cap(cx, nseg, 32),
             [&](int y, uint32_t x, uint32_t nx) { serve_in(bk, cm, cx, sm, y, x, nx); });
   sp_barrier(cm, cx, sm);
-  select_units<kSelServe>(bk, cm, cx, sm, 0, 2, [] {});
+  select_units(bk, cm, cx, sm, kSelServe, 0, 2, false);
   run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
     const int j = y % N;
     gather_stage(bk, cm, cx, sm, y / N, N + j, j, 5u, x, nx);
@@ -468,7 +510,7 @@ sp_ps_kernel(const SpBucket bk, const HpComm cm, const SpLaunch L) {
 // successor's inbox), the last hop storing into every inbox; then every rank scatters
 // the N reduced chunks.  Three barriers per hop when the candidate lists are short.
 __global__ void __launch_bounds__(kSpThreads, 3)
-sp_ring_kernel(const SpBucket bk, const HpComm cm, const SpLaunch L) {
+sp_ring_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm cm, const __grid_constant__ SpLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
   SpCtx cx;
@@ -482,9 +524,7 @@ sp_ring_kernel(const SpBucket bk, const HpComm cm, const SpLaunch L) {
       sp_barrier(cm, cx, sm);
     }
     // the last hop has read every chunk of the gradient when its update pass is done
-    select_units<kSelHop>(bk, cm, cx, sm, hop, 2 * hop, [&] {
-      if (hop == N - 1) zero_result(bk, cm, cx, sm, 2 * hop + 1);
-    });
+    select_units(bk, cm, cx, sm, kSelHop, hop, 2 * hop, hop == N - 1);
   }
   // gather: rank src finalised chunk src + 1 (every CTA has cleared its share of the result)
   sp_barrier(cm, cx, sm);
@@ -514,6 +554,7 @@ static int build_sp_bucket(int alg, float ratio, float momentum, const HpSeg* se
     d.n = (uint32_t)n;
     d.chunk = (uint32_t)chunk;
     d.kmax = (uint32_t)sparse_k(chunk, ratio);
+    d.k_last = (uint32_t)sparse_k(n % chunk, ratio);
     d.pay_off = (uint32_t)pay;
     d.tiles = (uint32_t)(chunk / kTile);
     d.tile_prefix = (uint32_t)tiles;
@@ -574,7 +615,9 @@ static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int
   if (G < 1 || (long long)G * ranks_here > (long long)cap) return HP_ERR_RESIDENCY;
   bk.samples_total = 0;
   for (int i = 0; i < nseg; ++i) {  // a sampled tile for every CTA, over the units of a push or of a hop
-    bk.seg[i].sampled = sampled_tiles(bk.seg[i].tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);
+    SpSeg& sg = bk.seg[i];
+    sg.stride = sample_stride(sg.tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);
+    sg.sampled = (sg.tiles + sg.stride - 1) / sg.stride;
     bk.seg[i].sample_prefix = bk.samples_total;
     bk.samples_total += bk.seg[i].sampled;
   }

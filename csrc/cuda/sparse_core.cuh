@@ -32,64 +32,69 @@ __device__ __forceinline__ uint32_t digit_of(uint32_t key, int pass) {
 }
 
 struct FindSmem {
+  alignas(16) uint32_t counts[kBins / kSpThreads];
   uint32_t sums[kSpThreads / 32];
-  uint32_t res[2];
+  uint32_t owner, above;
 };
 
 // Largest bin of a histogram of kBins bins whose suffix count reaches k, and krem = how
 // many of the k fall in that bin, i.e. k - count(bins > bin); (0, 0) when fewer than k are
 // counted.  `hist` is in shared or in global memory, where other CTAs' atomics wrote it.
+// Thread t sums bins 16t .. 16t+15; the thread in whose bins the k-th lies hands its
+// sixteen counts to everybody, and every warp finds the bin among them.
 static __device__ __noinline__ void find_bin(const uint32_t* hist, uint32_t k, FindSmem& fs, uint32_t& bin,
                                              uint32_t& krem) {
   constexpr int per = kBins / kSpThreads;  // 16
-  uint32_t c[per];
+  uint4 c[per / 4];
   uint32_t sum = 0;
 #pragma unroll
-  for (int i = 0; i < per; i += 4) {
+  for (int i = 0; i < per / 4; ++i) {
     asm volatile("ld.volatile.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(c[i]), "=r"(c[i + 1]), "=r"(c[i + 2]), "=r"(c[i + 3])
-                 : "l"(hist + threadIdx.x * per + i)
+                 : "=r"(c[i].x), "=r"(c[i].y), "=r"(c[i].z), "=r"(c[i].w)
+                 : "l"(hist + threadIdx.x * per + 4 * i)
                  : "memory");
-    sum += c[i] + c[i + 1] + c[i + 2] + c[i + 3];
+    sum += c[i].x + c[i].y + c[i].z + c[i].w;
   }
-  // above = how many elements sit in the bins of higher threads: suffix sum by warp
-  // shuffles plus the warps' totals (a serial walk over the 256 partial sums cost
-  // several microseconds per call)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t v = sum;
+  uint32_t v = sum;   // suffix sum over the warp
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_down_sync(0xffffffffu, v, o);
     if (lane + o < 32) v += y;
   }
   if (lane == 0) fs.sums[warp] = v;
-  if (threadIdx.x == 0) {
-    fs.res[0] = 0;
-    fs.res[1] = 0;
-  }
+  if (threadIdx.x == 0) fs.owner = 0xFFFFFFFFu;
   __syncthreads();
-  uint32_t above = v - sum;
-#pragma unroll
-  for (int w = 0; w < kSpThreads / 32; ++w)
-    if (w > warp) above += fs.sums[w];
+  const uint32_t higher = lane > warp && lane < kSpThreads / 32 ? fs.sums[lane] : 0u;
+  const uint32_t above = v - sum + __reduce_add_sync(0xffffffffu, higher);  // in the bins of higher threads
   if (above < k && k <= above + sum) {
-    uint32_t acc = above;
+    fs.owner = threadIdx.x;
+    fs.above = above;
 #pragma unroll
-    for (int i = per - 1; i >= 0; --i) {
-      if (acc < k && k <= acc + c[i]) {
-        fs.res[0] = threadIdx.x * per + i;
-        fs.res[1] = k - acc;
-      }
-      acc += c[i];
-    }
+    for (int i = 0; i < per / 4; ++i) *reinterpret_cast<uint4*>(fs.counts + 4 * i) = c[i];
   }
   __syncthreads();
-  bin = fs.res[0];
-  krem = fs.res[1];
+  const uint32_t owner = fs.owner;
+  bin = krem = 0;
+  if (owner != 0xFFFFFFFFu) {
+    const uint32_t mine = lane < per ? fs.counts[lane & (per - 1)] : 0u;
+    uint32_t w = mine;
+#pragma unroll
+    for (int o = 1; o < per; o <<= 1) {
+      const uint32_t y = __shfl_down_sync(0xffffffffu, w, o);
+      if (lane + o < per) w += y;
+    }
+    const uint32_t acc = fs.above + w - mine;
+    const uint32_t hit = __ballot_sync(0xffffffffu, lane < per && acc < k && k <= acc + mine);
+    const int at = __ffs(hit) - 1;
+    bin = owner * per + at;
+    krem = k - __shfl_sync(0xffffffffu, acc, at);
+  }
   __syncthreads();
 }
 
 __device__ __forceinline__ void flush_hist(const uint32_t* sh, uint32_t* __restrict__ gh) {
+#pragma unroll 1
   for (int i = threadIdx.x; i < kBins; i += kSpThreads) {
     const uint32_t c = sh[i];
     if (c) atomicAdd(gh + i, c);
@@ -342,9 +347,9 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 // again after the update to split it at a threshold bin, and every element went through
 // a shared-memory histogram; both are gone:
 //
-//   sample   some tiles of the array, spread evenly, are updated first; the histogram of
-//            their magnitudes gives a `low` below which an element is almost surely not
-//            among the k largest, and above which about 1.1 to 1.7 k are
+//   sample   every stride-th tile of the array is updated first; the histogram of its
+//            magnitudes gives a `low` below which an element is almost surely not among
+//            the k largest, and above which about 1.1 to 1.7 k are
 //   collect  the other tiles are updated; elements of at least `low` are appended to a
 //            candidate list with the histogram of their first digit (the sampled tiles'
 //            from shared memory).  The list holds the k largest exactly when it has k
@@ -357,10 +362,17 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 // GradDrop.  A list that came out shorter than k or longer than its room (a sample that
 // misled, or massive ties) makes the launch fall back to histogram passes over the
 // whole array.
+//
+// Up to a few million elements the time is not memory but instruction fetch: most of
+// this code runs once or twice per launch, and code that is not in the instruction cache
+// comes in at a few instructions per 0.1 us (one CTA on 4000 elements: 1900 instructions
+// per warp took 25 us, half of all warp-cycles waiting for one).  Hence one out-of-line
+// copy of every step, rolled loops where a step runs once, 32-bit arithmetic, and sizes
+// worked out on the host.
 constexpr uint32_t kFinishKeys = 8192;  // list length up to which a CTA keeps the keys in shared memory
-constexpr uint32_t kFinishList = 12288; // longest list one CTA finishes by itself
+constexpr uint32_t kFinishList = 12288; // longest list that is finished without a refine step
 constexpr uint32_t kMinSampled = 4;     // tiles of an array that are sampled at least
-constexpr int kSelTile = 4096;          // elements per tile: 16 per thread
+constexpr uint32_t kSelTile = 4096;     // elements per tile: 16 per thread
 
 // One array to select from.
 struct SelUnit {
@@ -369,43 +381,28 @@ struct SelUnit {
   float* u;
   uint32_t* ws;
   float* cv;       // candidate list: `cap` values, then `cap` indices; a second list of the
-  uint32_t* ci;    // same size behind it
+                   // same size behind it
   uint32_t n, k, kmax, cap;
-  uint32_t tiles, sampled;  // tiles of the array's layout (some may lie past n), and how many are sampled
+  uint32_t stride, sampled;  // every stride-th tile is sampled: how many that is
 };
-
-HP_HD SelUnit sel_unit(const float* g, float* a, float* u, uint32_t n, uint32_t k, uint32_t kmax, uint32_t* ws,
-                       void* cand, uint32_t pairs, uint32_t tiles, uint32_t sampled) {
-  SelUnit s;
-  s.g = g; s.a = a; s.u = u; s.ws = ws;
-  s.n = n; s.k = k; s.kmax = kmax;
-  s.tiles = tiles; s.sampled = sampled;
-  s.cap = pairs / 2 & ~3u;   // keeps every list on 16 bytes
-  s.cv = static_cast<float*>(cand);
-  s.ci = reinterpret_cast<uint32_t*>(s.cv + s.cap);
-  return s;
-}
-// how many of an array's tiles are sampled when ctas CTAs share `total` tiles: one each
-HP_HD uint32_t sampled_tiles(uint32_t tiles, uint64_t total, uint32_t ctas) {
-  const uint64_t share = ((uint64_t)tiles * ctas + total / 2) / (total ? total : 1);
-  const uint64_t f = share < kMinSampled ? kMinSampled : share;
-  return f < tiles ? (uint32_t)f : tiles;
-}
-// the i-th sampled tile, and the test for one
-__device__ __forceinline__ uint32_t sampled_tile(uint32_t i, uint32_t tiles, uint32_t sampled) {
-  return (uint32_t)((uint64_t)i * tiles / sampled);
-}
-__device__ __forceinline__ bool is_sampled(uint32_t t, uint32_t tiles, uint32_t sampled) {
-  const uint32_t i = (uint32_t)(((uint64_t)t * sampled + tiles - 1) / tiles);
-  return i < sampled && sampled_tile(i, tiles, sampled) == t;
-}
+__device__ __forceinline__ uint32_t* list_indices(const SelUnit& s) { return reinterpret_cast<uint32_t*>(s.cv + s.cap); }
 __device__ __forceinline__ float* list2_values(const SelUnit& s) { return s.cv + 2 * (size_t)s.cap; }
 __device__ __forceinline__ uint32_t* list2_indices(const SelUnit& s) {
   return reinterpret_cast<uint32_t*>(s.cv + 3 * (size_t)s.cap);
 }
+// room of each of the two lists in `pairs` pairs; keeps every list on 16 bytes
+HP_HD uint32_t list_cap(uint64_t pairs) {
+  return (uint32_t)(pairs / 2 < 0x7FFFFFFCull ? pairs / 2 : 0x7FFFFFFCull) & ~3u;
+}
+// stride of the sampled tiles of an array when ctas CTAs share `total` tiles: about a
+// sampled tile for every CTA
+HP_HD uint32_t sample_stride(uint32_t tiles, uint64_t total, uint32_t ctas) {
+  uint64_t share = ((uint64_t)tiles * ctas) / (total ? total : 1);
+  if (share < kMinSampled) share = kMinSampled;
+  return share >= tiles ? 1u : (uint32_t)((tiles + share - 1) / share);
+}
 
 constexpr int kCollectBuf = 1024;  // candidates a CTA gathers before it reserves room in the lists
-constexpr int kStash = kFinishKeys / kSelTile;  // sampled tiles whose values stay in shared memory
 
 struct SelSmem {
   union {
@@ -418,97 +415,120 @@ struct SelSmem {
   };
   union {
     uint32_t keys[kFinishKeys];      // finish
-    float stash[kStash][kSelTile];   // sample to collect
+    float stash[2][kSelTile];        // sample to collect
   };
   FindSmem fs;
   uint32_t count, base, ticket, flag;
   uint32_t sent, ties;
 };
 
-// Loads tile t and applies the update (MODE as in pass0_body), all loads before the first
-// store.  Elements past the end read as zero, and a zero is never sent.
+__device__ __forceinline__ void clear_hist(uint32_t* sh) {
+#pragma unroll 1
+  for (int b = threadIdx.x; b < kBins / 4; b += kSpThreads)
+    reinterpret_cast<uint4*>(sh)[b] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The update of one element.  MODE as in pass0_body.
 template <int MODE>
-__device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[4]) {
+__device__ __forceinline__ float update_value(float v, float g, float& u, float momentum) {
+  if (MODE == 1) v = v + g;
+  if (MODE == 2) {
+    u = __fmaf_rn(momentum, u, g);
+    v = v + u;
+  }
+  return v;
+}
+
+// Loads tile t and applies the update, all loads before the first store; put(j, v) gets
+// float4 number j * 256 + thread.  A tile that is not full or not on 16 bytes goes
+// element by element; what lies past the end reads as zero, and a zero is never sent.
+template <int MODE, typename F>
+__device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, F put) {
+  const size_t base = (size_t)t * kSelTile;
   const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
                      (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
-  const uint64_t i0 = (uint64_t)t * kSelTile + threadIdx.x * 4;
-  float4 gv[4], uv[4];
+  if (vec && base + kSelTile <= s.n) {
+    float4 av[4], gv[4], uv[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint64_t i = i0 + j * kSpThreads * 4;
-    av[j] = ld4(s.a, i, s.n, vec);
-    if (MODE >= 1) gv[j] = ld4(s.g, i, s.n, vec);
-    if (MODE == 2) uv[j] = ld4(s.u, i, s.n, vec);
-  }
+    for (int j = 0; j < 4; ++j) {
+      const size_t i = base + (j * kSpThreads + threadIdx.x) * 4;
+      av[j] = *reinterpret_cast<const float4*>(s.a + i);
+      if (MODE >= 1) gv[j] = *reinterpret_cast<const float4*>(s.g + i);
+      if (MODE == 2) uv[j] = *reinterpret_cast<const float4*>(s.u + i);
+    }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint64_t i = i0 + j * kSpThreads * 4;
-    float4& v = av[j];
-    if (MODE == 1) {
-      v.x = v.x + gv[j].x; v.y = v.y + gv[j].y; v.z = v.z + gv[j].z; v.w = v.w + gv[j].w;
-      st4(s.a, i, s.n, vec, v);
-    } else if (MODE == 2) {
-      float4 w;
-      w.x = __fmaf_rn(momentum, uv[j].x, gv[j].x);
-      w.y = __fmaf_rn(momentum, uv[j].y, gv[j].y);
-      w.z = __fmaf_rn(momentum, uv[j].z, gv[j].z);
-      w.w = __fmaf_rn(momentum, uv[j].w, gv[j].w);
-      v.x = v.x + w.x; v.y = v.y + w.y; v.z = v.z + w.z; v.w = v.w + w.w;
-      st4(s.u, i, s.n, vec, w);
-      st4(s.a, i, s.n, vec, v);
+    for (int j = 0; j < 4; ++j) {
+      const size_t i = base + (j * kSpThreads + threadIdx.x) * 4;
+      float4& v = av[j];
+      v.x = update_value<MODE>(v.x, gv[j].x, uv[j].x, momentum);
+      v.y = update_value<MODE>(v.y, gv[j].y, uv[j].y, momentum);
+      v.z = update_value<MODE>(v.z, gv[j].z, uv[j].z, momentum);
+      v.w = update_value<MODE>(v.w, gv[j].w, uv[j].w, momentum);
+      if (MODE == 2) *reinterpret_cast<float4*>(s.u + i) = uv[j];
+      if (MODE >= 1) *reinterpret_cast<float4*>(s.a + i) = v;
+      put(j, v);
+    }
+  } else {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      float e[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const size_t i = base + (j * kSpThreads + threadIdx.x) * 4 + q;
+        e[q] = 0.0f;
+        if (i < s.n) {
+          float w = MODE == 2 ? s.u[i] : 0.0f;
+          e[q] = update_value<MODE>(s.a[i], MODE >= 1 ? s.g[i] : 0.0f, w, momentum);
+          if (MODE == 2) s.u[i] = w;
+          if (MODE >= 1) s.a[i] = e[q];
+        }
+      }
+      put(j, make_float4(e[0], e[1], e[2], e[3]));
     }
   }
 }
 
-// Sampled tile number i of an array: update, magnitudes into the array's sample histogram,
-// values into stash `slot` (-1: none).  The CTA that completes the sample turns it into
-// the candidates' lower bound.
 template <int MODE>
-static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum, SelSmem& sm, uint32_t i, int slot) {
-  const uint32_t t = sampled_tile(i, s.tiles, s.sampled);
-  if ((uint64_t)t * kSelTile < s.n) {
-    float4 av[4];
-    update_tile<MODE>(s, momentum, t, av);
-    for (int b = threadIdx.x; b < kBins / 4; b += kSpThreads)
-      reinterpret_cast<uint4*>(sm.hist)[b] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (slot >= 0) reinterpret_cast<float4*>(sm.stash[slot])[j * kSpThreads + threadIdx.x] = av[j];
-      const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t key = abs_key(e[q]);
-        if (key) atomicAdd(&sm.hist[key >> 19], 1u);
-      }
-    }
-    __syncthreads();
-    flush_hist(sm.hist, s.ws);
+static __device__ __noinline__ void update_to_stash(const SelUnit& s, float momentum, uint32_t t, float* stash) {
+  update_tile<MODE>(s, momentum, t, [&](int j, const float4& v) {
+    reinterpret_cast<float4*>(stash)[j * kSpThreads + threadIdx.x] = v;
+  });
+}
+
+// Sampled tile number i of an array: update, values into `stash`, magnitudes into the
+// array's sample histogram.  The CTA that completes the sample turns it into the
+// candidates' lower bound.
+static __device__ __noinline__ void sample_body(int mode, const SelUnit& s, float momentum, SelSmem& sm, uint32_t i,
+                                                float* stash) {
+  const uint32_t t = i * s.stride;
+  if (mode == 0) update_to_stash<0>(s, momentum, t, stash);
+  else if (mode == 1) update_to_stash<1>(s, momentum, t, stash);
+  else update_to_stash<2>(s, momentum, t, stash);
+  clear_hist(sm.hist);
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t p = threadIdx.x; p < kSelTile; p += kSpThreads) {
+    const uint32_t key = abs_key(stash[p]);
+    if (key) atomicAdd(&sm.hist[key >> 19], 1u);
   }
   __syncthreads();
+  flush_hist(sm.hist, s.ws);
+  __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();   // cumulative over the CTA's counts, which the barrier ordered before it
-    sm.flag = atomicAdd(s.ws + kWsSampled, 1u) == s.sampled - 1;
+    uint32_t done;   // release the CTA's counts, acquire those of the CTAs before
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(done) : "l"(s.ws + kWsSampled) : "memory");
+    sm.flag = done == s.sampled - 1;
   }
   __syncthreads();
   if (!sm.flag) return;
-  __threadfence();
   uint32_t rank = s.k;
-  if (s.sampled < s.tiles) {
-    // elements in the sample: what of the sampled tiles lies before n
-    uint32_t m = 0;
-    for (uint32_t q = threadIdx.x; q < s.sampled; q += kSpThreads) {
-      const uint64_t lo = (uint64_t)sampled_tile(q, s.tiles, s.sampled) * kSelTile;
-      if (lo < s.n) m += (uint32_t)min((uint64_t)kSelTile, s.n - lo);
-    }
-    if (threadIdx.x == 0) sm.base = 0;
-    __syncthreads();
-    if (m) atomicAdd(&sm.base, m);
-    __syncthreads();
+  if (s.stride > 1) {
     // k scaled to the sample, plus five standard deviations, plus a tenth because
     // neighbouring elements are not independent
-    const float hits = (float)((double)s.k * (double)sm.base / (double)s.n);
-    rank = (uint32_t)(1.1f * hits + 5.0f * sqrtf(hits) + 4.0f);
+    const float hits = __fdividef((float)s.k * (float)(s.sampled * kSelTile), (float)s.n);
+    float dev;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(dev) : "f"(hits));
+    rank = (uint32_t)(1.1f * hits + 5.0f * dev + 4.0f);
   }
   uint32_t bin, rem;
   find_bin(s.ws, rank, sm.fs, bin, rem);   // bin 0 when fewer than rank are counted
@@ -524,6 +544,7 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
 template <typename F>
 __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t ctas, uint32_t& slot, F f) {
   const uint32_t stretch = total / (4u * ctas) + 1u;
+#pragma unroll 1
   for (;;) {
     if (threadIdx.x == 0) slot = atomicAdd(word, stretch);
     __syncthreads();
@@ -534,35 +555,22 @@ __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_
   }
 }
 
-// Put the elements of a tile that reach `low` into the CTA's buffer, for unit `uid`.
-__device__ __forceinline__ void collect_values(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, uint32_t t,
-                                               const float4 (&av)[4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
-    const uint32_t most = max(max(abs_key(e[0]), abs_key(e[1])), max(abs_key(e[2]), abs_key(e[3])));
-    if (most < low) continue;
-    const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t key = abs_key(e[q]);
-      if (key < low) continue;
-      const uint32_t p = atomicAdd(&sm.count, 1u);
-      if (p < (uint32_t)kCollectBuf) {
-        sm.buf.val[p] = e[q];
-        sm.buf.idx[p] = i + q;
-        sm.buf.unit[p] = (uint16_t)uid;
-      } else {   // more than the buffer holds: straight into the list
-        const uint32_t pos = atomicAdd(s.ws + kWsCandCount, 1u);
-        atomicAdd(s.ws + kBins + (key >> 19), 1u);
-        if (pos < s.cap) {
-          s.cv[pos] = e[q];
-          s.ci[pos] = i + q;
-        } else {
-          s.ws[kWsOverflow] = 1u;
-        }
-      }
-    }
+// one candidate into the CTA's buffer, or, when that is full, straight into its list
+static __device__ __noinline__ void collect_one(const SelUnit& s, uint32_t uid, SelSmem& sm, float v, uint32_t i) {
+  const uint32_t p = atomicAdd(&sm.count, 1u);
+  if (p < (uint32_t)kCollectBuf) {
+    sm.buf.val[p] = v;
+    sm.buf.idx[p] = i;
+    sm.buf.unit[p] = (uint16_t)uid;
+    return;
+  }
+  const uint32_t pos = atomicAdd(s.ws + kWsCandCount, 1u);
+  atomicAdd(s.ws + kBins + (abs_key(v) >> 19), 1u);
+  if (pos < s.cap) {
+    s.cv[pos] = v;
+    list_indices(s)[pos] = i;
+  } else {
+    s.ws[kWsOverflow] = 1u;
   }
 }
 
@@ -571,27 +579,36 @@ template <int MODE>
 static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid, float momentum, SelSmem& sm,
                                                  uint32_t t0, uint32_t t1) {
   const uint32_t low = __ldcg(s.ws + kWsLow);
+  uint32_t phase = t0 % s.stride;   // 0: a sampled tile
+#pragma unroll 1
   for (uint32_t t = t0; t < t1; ++t) {
-    if (is_sampled(t, s.tiles, s.sampled)) continue;
-    float4 av[4];
-    update_tile<MODE>(s, momentum, t, av);
-    collect_values(s, uid, sm, low, t, av);
+    const bool skip = phase == 0;
+    if (++phase == s.stride) phase = 0;
+    if (skip) continue;
+    update_tile<MODE>(s, momentum, t, [&](int j, const float4& v) {
+      const uint32_t most = max(max(abs_key(v.x), abs_key(v.y)), max(abs_key(v.z), abs_key(v.w)));
+      if (most < low) return;
+      const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
+      if (abs_key(v.x) >= low) collect_one(s, uid, sm, v.x, i);
+      if (abs_key(v.y) >= low) collect_one(s, uid, sm, v.y, i + 1);
+      if (abs_key(v.z) >= low) collect_one(s, uid, sm, v.z, i + 2);
+      if (abs_key(v.w) >= low) collect_one(s, uid, sm, v.w, i + 3);
+    });
   }
 }
 
-// Sampled tile number i again, updated before: from stash `slot`, or read again (-1).
-static __device__ __noinline__ void collect_sampled(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t i, int slot) {
-  const uint32_t t = sampled_tile(i, s.tiles, s.sampled);
-  if ((uint64_t)t * kSelTile >= s.n) return;
-  const uint32_t low = __ldcg(s.ws + kWsLow);
-  float4 av[4];
-  if (slot >= 0) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) av[j] = reinterpret_cast<const float4*>(sm.stash[slot])[j * kSpThreads + threadIdx.x];
-  } else {
-    update_tile<0>(s, 0.0f, t, av);
+// Sampled tile number i again, updated before: from its stash, or (again) read once more.
+static __device__ __noinline__ void collect_sampled(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t i,
+                                                    float* stash, bool again) {
+  const uint32_t t = i * s.stride, low = __ldcg(s.ws + kWsLow);
+  if (again) update_to_stash<0>(s, 0.0f, t, stash);
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t p = threadIdx.x; p < kSelTile; p += kSpThreads) {
+    const float v = stash[p];
+    if (abs_key(v) >= low) collect_one(s, uid, sm, v, t * kSelTile + p);
   }
-  collect_values(s, uid, sm, low, t, av);
+  __syncthreads();
 }
 
 // Append the CTA's gathered candidates to their lists, and their first digits to the
@@ -601,6 +618,7 @@ template <typename F>
 __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
   __syncthreads();
   const uint32_t n = min(sm.count, (uint32_t)kCollectBuf);
+#pragma unroll 1
   for (uint32_t p0 = 0; p0 < n; p0 += kSpThreads) {
     const uint32_t p = p0 + threadIdx.x;
     const bool have = p < n;
@@ -617,7 +635,7 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
       pos = __shfl_sync(group, pos, lead) + __popc(group & ((1u << lane) - 1u));
       if (pos < s.cap) {
         s.cv[pos] = v;
-        s.ci[pos] = sm.buf.idx[p];
+        list_indices(s)[pos] = sm.buf.idx[p];
       } else {
         s.ws[kWsOverflow] = 1u;
       }
@@ -632,6 +650,7 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
 __device__ __forceinline__ void put_pair(const EmitDst& dst, size_t val_off, uint32_t kmax, uint32_t pos,
                                          uint32_t idx, float val) {
   if (pos >= kmax) return;
+#pragma unroll 1
   for (int d = 0; d < dst.n; ++d) {
     reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = idx;
     reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = val;
@@ -648,7 +667,8 @@ static __device__ __noinline__ void refine_body(const SelUnit& s, const EmitDst&
   uint32_t bin0, rem;
   find_bin(s.ws + kBins, min(s.k, L), sm.fs, bin0, rem);
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
-  const uint32_t lo = (uint32_t)((uint64_t)L * x / nx), hi = (uint32_t)((uint64_t)L * (x + 1) / nx);
+  const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
+#pragma unroll 1
   for (uint32_t p0 = lo; p0 < hi; p0 += 4 * kSpThreads) {
     if (threadIdx.x == 0) sm.sent = sm.ties = 0;
     __syncthreads();
@@ -659,7 +679,7 @@ static __device__ __noinline__ void refine_body(const SelUnit& s, const EmitDst&
     for (int j = 0; j < 4; ++j) {
       const uint32_t p = p0 + j * kSpThreads + threadIdx.x;
       v[j] = p < hi ? __ldcg(s.cv + p) : 0.0f;
-      idx[j] = p < hi ? __ldcg(s.ci + p) : 0u;
+      idx[j] = p < hi ? __ldcg(list_indices(s) + p) : 0u;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -704,22 +724,19 @@ static __device__ __noinline__ bool finish_body(int alg, const SelUnit& s, const
   const uint32_t k = min(s.k, all);          // fewer than k non-zero elements: all of them
   const uint32_t L = refined ? min(__ldcg(s.ws + kWsCand2Count), s.cap) : all;
   const float* cv = refined ? list2_values(s) : s.cv;
-  const uint32_t* ci = refined ? list2_indices(s) : s.ci;
+  const uint32_t* ci = refined ? list2_indices(s) : list_indices(s);
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
-  // keys into shared memory, sixteen a thread in flight; past L whatever the list's room holds
-  for (uint32_t p0 = 0; p0 < L && p0 < kFinishKeys; p0 += 16 * kSpThreads) {
-    uint4 v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t p = p0 + (j * kSpThreads + threadIdx.x) * 4;
-      v[j] = p < L ? __ldcg(reinterpret_cast<const uint4*>(cv + p)) : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t p = p0 + (j * kSpThreads + threadIdx.x) * 4;
-      *reinterpret_cast<uint4*>(sm.keys + p) =
-          make_uint4(v[j].x & 0x7FFFFFFFu, v[j].y & 0x7FFFFFFFu, v[j].z & 0x7FFFFFFFu, v[j].w & 0x7FFFFFFFu);
-    }
+  // keys into shared memory, eight a thread in flight; past L whatever the list's room holds
+#pragma unroll 1
+  for (uint32_t p = threadIdx.x * 4; p < L && p < kFinishKeys; p += 8 * kSpThreads) {
+    const uint32_t q = p + 4 * kSpThreads;
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(cv + p));
+    uint4 w = v;
+    if (q < L) w = __ldcg(reinterpret_cast<const uint4*>(cv + q));
+    *reinterpret_cast<uint4*>(sm.keys + p) =
+        make_uint4(v.x & 0x7FFFFFFFu, v.y & 0x7FFFFFFFu, v.z & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu);
+    *reinterpret_cast<uint4*>(sm.keys + q) =
+        make_uint4(w.x & 0x7FFFFFFFu, w.y & 0x7FFFFFFFu, w.z & 0x7FFFFFFFu, w.w & 0x7FFFFFFFu);
   }
   auto key_at = [&](uint32_t p) { return p < kFinishKeys ? sm.keys[p] : abs_key(__ldcg(cv + p)); };
   uint32_t prefix, rem;
@@ -728,9 +745,9 @@ static __device__ __noinline__ bool finish_body(int alg, const SelUnit& s, const
 #pragma unroll 1
   for (int d = 0; d < 2; ++d) {
     const int low = d == 0 ? 8 : 0, bits = d == 0 ? 11 : 8;
-    for (int b = threadIdx.x; b < kBins / 4; b += kSpThreads)
-      reinterpret_cast<uint4*>(sm.hist)[b] = make_uint4(0u, 0u, 0u, 0u);
+    clear_hist(sm.hist);
     __syncthreads();
+#pragma unroll 1
     for (uint32_t p = threadIdx.x; p < L; p += kSpThreads) {
       const uint32_t key = key_at(p);
       if ((key >> (low + bits)) == prefix) atomicAdd(&sm.hist[(key >> low) & ((1u << bits) - 1u)], 1u);
@@ -742,7 +759,8 @@ static __device__ __noinline__ bool finish_body(int alg, const SelUnit& s, const
     rem = r;
   }
   const uint32_t thr = prefix, need = rem;   // `need` of the elements equal to thr are sent
-  const uint32_t lo = (uint32_t)((uint64_t)L * x / nx), hi = (uint32_t)((uint64_t)L * (x + 1) / nx);
+  const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
+#pragma unroll 1
   for (uint32_t p0 = lo; p0 < hi; p0 += kSpThreads) {
     if (threadIdx.x == 0) sm.sent = sm.ties = 0;
     __syncthreads();
@@ -789,6 +807,7 @@ static __device__ __noinline__ bool finish_body(int alg, const SelUnit& s, const
   h.flags = 0;
   h.a = all < s.k ? 0.0f : __uint_as_float(thr);
   h.b = sent < s.kmax ? sent : s.kmax;
+#pragma unroll 1
   for (int d = 0; d < dst.n; ++d) *reinterpret_cast<uint4*>(dst.out[d]) = *reinterpret_cast<const uint4*>(&h);
   return true;
 }

@@ -68,7 +68,7 @@ union SelOrPassSmem {
   EmitSmem emit;
 };
 
-__global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const SelArgs A) {
+__global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __grid_constant__ SelArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SelOrPassSmem& sm = *reinterpret_cast<SelOrPassSmem*>(smem_raw);
   __shared__ WaitState wst;
@@ -80,20 +80,20 @@ __global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const SelA
   auto barrier = [&]() {
     grid_barrier(s.ws + kWsWords, gen, G, kGridBarrierNs, s.ws + kWsStatus, 1u, wst);
   };
-  for (uint32_t i = c, r = 0; i < s.sampled; i += G, ++r) {
-    const int slot = r < (uint32_t)kStash ? (int)r : -1;
-    if (A.mode == 0) sample_body<0>(s, A.momentum, sm.sel, i, slot);
-    else if (A.mode == 1) sample_body<1>(s, A.momentum, sm.sel, i, slot);
-    else sample_body<2>(s, A.momentum, sm.sel, i, slot);
-  }
+  const uint32_t tiles = (s.n - 1) / kSelTile + 1;
+  uint32_t mine = 0;   // sampled tiles of this CTA: the first two stay in shared memory
+#pragma unroll 1
+  for (uint32_t i = c; i < s.sampled; i += G, ++mine)
+    sample_body(A.mode, s, A.momentum, sm.sel, i, sm.sel.stash[mine < 2 ? mine : 1]);
   barrier();
   if (threadIdx.x == 0) sm.sel.count = 0;
   __syncthreads();
-  for (uint32_t i = c, r = 0; i < s.sampled; i += G, ++r)
-    collect_sampled(s, 0, sm.sel, i, r < (uint32_t)kStash ? (int)r : -1);
+#pragma unroll 1
+  for (uint32_t i = c, r = 0; r < mine; i += G, ++r)   // the second stash holds the last one sampled
+    collect_sampled(s, 0, sm.sel, i, sm.sel.stash[r < 1 ? 0 : 1], r >= 1 && mine > 2);
   auto self = [&](uint32_t) { return s; };
-  if (s.sampled < s.tiles)
-    hand_out(s.ws + kWsTicket, s.tiles, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
+  if (s.stride > 1)
+    hand_out(s.ws + kWsTicket, tiles, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
       if (A.mode == 0) collect_body<0>(s, 0, A.momentum, sm.sel, t0, t1);
       else if (A.mode == 1) collect_body<1>(s, 0, A.momentum, sm.sel, t0, t1);
       else collect_body<2>(s, 0, A.momentum, sm.sel, t0, t1);
@@ -218,9 +218,18 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
     if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
     const int grid = (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
     SelArgs A;
-    A.unit = sel_unit(g, a, uu, (uint32_t)n, (uint32_t)k, (uint32_t)kmax, ws, ws + kWsWords + kBarrierWords,
-                      (uint32_t)(pairs < 0xFFFFFFFEull ? pairs : 0xFFFFFFFEull), (uint32_t)tiles,
-                      sampled_tiles((uint32_t)tiles, tiles, (uint32_t)grid));
+    SelUnit& U = A.unit;
+    U.g = g;
+    U.a = a;
+    U.u = uu;
+    U.ws = ws;
+    U.cv = reinterpret_cast<float*>(ws + kWsWords + kBarrierWords);
+    U.n = (uint32_t)n;
+    U.k = (uint32_t)k;
+    U.kmax = (uint32_t)kmax;
+    U.cap = list_cap(pairs);
+    U.stride = sample_stride((uint32_t)tiles, tiles, (uint32_t)grid);
+    U.sampled = ((uint32_t)tiles + U.stride - 1) / U.stride;
     A.alg = alg;
     A.mode = mode;
     A.momentum = momentum;
