@@ -43,9 +43,7 @@ struct SpSeg {
   uint32_t tiles;       // tiles of one chunk
   uint32_t tile_prefix; // tiles of one chunk of the tensors before this one
   uint32_t k_last;      // pairs of the last chunk, which may be shorter
-  // set at launch, they depend on the grid: every stride-th tile of a chunk is sampled,
-  // `sampled` of them
-  uint32_t stride, sampled, sample_prefix;
+  uint32_t stride;      // every stride-th tile is sampled (set at launch: depends on the grid)
   uint32_t cap;         // candidate pairs per (tensor, chunk) unit, for both lists
   uint64_t cand_push;   // first push unit's candidate list, in pairs from the region start
   uint64_t cand_srv;    // the server unit's candidate list
@@ -59,7 +57,6 @@ struct SpBucket {
   uint64_t slot_bytes;
   uint64_t cand_pairs;  // candidate pairs of all units of one rank
   uint32_t tiles_total; // tiles of one chunk summed over the tensors
-  uint32_t samples_total;
 };
 
 __device__ __forceinline__ uint32_t sp_chunk_valid(uint32_t n, uint32_t chunk, int c) {
@@ -76,6 +73,12 @@ __device__ __forceinline__ void write_empty_header(uint8_t* out, int alg) {
 }
 
 // ------------------------------------------------------ persistent-kernel plumbing
+struct UnitDst {
+  EmitDst out;
+  uint32_t* flag[HP_MAX_RANKS];
+};
+constexpr int kMaxUnits = HP_MAX_SEGS * HP_MAX_RANKS;
+
 struct SpSmem {
   union {
     SelSmem sel;
@@ -84,7 +87,10 @@ struct SpSmem {
   };
   FindSmem fs;
   WaitState wst;
-  uint32_t any, ticket;
+  uint32_t ticket;
+  UnitDst dst;
+  SelUnit unit[kMaxUnits];
+  uint32_t tile_at[kMaxUnits + 1], sample_at[kMaxUnits + 1];
 };
 
 // control words of one rank played by a launch, behind its histogram blocks; zero
@@ -152,7 +158,14 @@ static __device__ __noinline__ void zero_result(const SpBucket& bk, const HpComm
                                             int ticket) {
   const uint32_t N = (uint32_t)cx.N;
   hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * N, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
-    int si = 0;
+    int si = 0, hi = bk.nseg;
+#pragma unroll 1
+    while (hi - si > 1) {
+      const int mid = (si + hi) / 2;
+      if (bk.seg[mid].tile_prefix * N <= t) si = mid;
+      else hi = mid;
+    }
+#pragma unroll 1
     for (; t < end; ++t) {
       while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * N) ++si;
       const SpSeg& sg = bk.seg[si];
@@ -176,197 +189,197 @@ enum SelKind { kSelPush, kSelServe, kSelHop };
 
 struct SelPhase {
   int kind, hop;
-  uint32_t per_tensor;  // units per tensor
   uint32_t units;
-  int mode;             // of the update: see pass0_body
+  int mode;   // of the update: see pass0_body
 };
-__device__ __forceinline__ SelPhase sel_phase(const SpBucket& bk, const SpCtx& cx, int kind, int hop) {
-  SelPhase p;
-  p.kind = kind;
-  p.hop = hop;
-  p.per_tensor = kind == kSelPush ? (uint32_t)cx.N : 1u;
-  p.units = (uint32_t)bk.nseg * p.per_tensor;
-  p.mode = kind == kSelServe ? 0 : (bk.alg == kDgc ? 2 : 1);
-  return p;
-}
 
-struct UnitRef {
-  int si, c;
-};
-__device__ __forceinline__ UnitRef unit_ref(const SpCtx& cx, const SelPhase& ph, uint32_t y) {
-  if (ph.kind == kSelPush) return {(int)(y / (uint32_t)cx.N), (int)(y % (uint32_t)cx.N)};
-  if (ph.kind == kSelServe) return {(int)y, cx.R};
-  const int c = cx.R - ph.hop;
-  return {(int)y, c < 0 ? c + cx.N : c};
-}
-
-// the array of a unit; n = 0 for a chunk past the tensor's end
-static __device__ __noinline__ void unit_of(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, const SelPhase& ph,
-                                            uint32_t y, SelUnit& s) {
-  const UnitRef r = unit_ref(cx, ph, y);
-  const SpSeg& sg = bk.seg[r.si];
-  const size_t E = (size_t)cx.E, off = (size_t)r.c * sg.chunk;
-  s.n = sp_chunk_valid(sg.n, sg.chunk, r.c);
-  s.k = s.n == sg.chunk ? sg.kmax : sg.k_last;   // only the last chunk is shorter
-  s.kmax = sg.kmax;
-  s.cap = list_cap(sg.cap);
-  s.stride = sg.stride;
-  s.sampled = s.n == sg.chunk ? sg.sampled : ((s.n + kTile - 1) / kTile + sg.stride - 1) / sg.stride;
-  uint64_t list = sg.cand_srv;
-  uint32_t block = (uint32_t)(bk.nseg * cx.N) + y;
-  s.g = nullptr;
-  s.u = nullptr;
-  if (ph.kind == kSelServe) {
-    s.a = sg.sr + E * cm.emu_stride_sr;
-  } else {
-    s.g = sg.g + E * cm.emu_stride_g + off;
-    s.a = sg.a + E * cm.emu_stride_r + off;
-    if (sg.u) s.u = sg.u + E * cm.emu_stride_r + off;
-    list = sg.cand_push + (uint64_t)r.c * sg.cap;
-    block = ph.kind == kSelPush ? y : (uint32_t)(ph.hop * bk.nseg + r.si);
+__device__ __forceinline__ void unit_ref(const SpCtx& cx, const SelPhase& ph, uint32_t y, int& si, int& c) {
+  si = (int)y;
+  c = cx.R;
+  if (ph.kind == kSelPush) {
+    si = (int)(y / (uint32_t)cx.N);
+    c = (int)(y % (uint32_t)cx.N);
+  } else if (ph.kind == kSelHop) {
+    c = cx.R - ph.hop;
+    if (c < 0) c += cx.N;
   }
-  s.ws = cx.ws + (size_t)block * kWsWords;
-  s.cv = reinterpret_cast<float*>(cx.cand + list * 8);
 }
 
-// where a unit's pairs go, and the flags that announce them
-struct UnitDst {
-  EmitDst out;
-  uint32_t* flag[HP_MAX_RANKS];
-};
-static __device__ __noinline__ void unit_dst(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, const SelPhase& ph,
-                                             uint32_t y, UnitDst& d) {
-  const int N = cx.N, R = cx.R;
-  const UnitRef r = unit_ref(cx, ph, y);
-  const bool all = ph.kind == kSelServe || (ph.kind == kSelHop && ph.hop == N - 1);
-  int to = ph.kind == kSelPush ? r.c : (all ? R : R + 1);
-  const int slot = ph.kind == kSelPush ? R : (ph.kind == kSelServe ? N + R : (all ? N - 1 + R : ph.hop));
-  d.out.n = all ? N : 1;
+// Every unit's array, and prefix sums of the units' tiles and sampled tiles, in shared
+// memory: worked out once per phase by all threads, looked up at every stretch of tiles.
+static __device__ __noinline__ void set_units(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
+                                              const SelPhase& ph, SpSmem& sm) {
+  __syncthreads();
 #pragma unroll 1
-  for (int q = 0; q < d.out.n; ++q, ++to) {
-    if (to >= N) to -= N;
-    d.out.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[to]) + (size_t)slot * bk.slot_bytes + bk.seg[r.si].pay_off;
-    d.flag[q] = reinterpret_cast<uint32_t*>(cm.flags[to]) + (size_t)slot * bk.nseg + r.si;
+  for (uint32_t y = threadIdx.x; y < ph.units; y += kSpThreads) {
+    int si, c;
+    unit_ref(cx, ph, y, si, c);
+    const SpSeg& sg = bk.seg[si];
+    SelUnit& s = sm.unit[y];
+    const size_t E = (size_t)cx.E, off = (size_t)c * sg.chunk;
+    const uint32_t n = sp_chunk_valid(sg.n, sg.chunk, c), tiles = (n + kTile - 1) / kTile;
+    s.n = n;
+    s.k = n == sg.chunk ? sg.kmax : sg.k_last;   // only the last chunk is shorter
+    s.kmax = sg.kmax;
+    s.cap = list_cap(sg.cap);
+    s.stride = sg.stride;
+    s.sampled = (tiles + sg.stride - 1) / sg.stride;
+    uint64_t list = sg.cand_srv;
+    uint32_t block = (uint32_t)(bk.nseg * cx.N) + y;
+    s.g = nullptr;
+    s.u = nullptr;
+    if (ph.kind == kSelServe) {
+      s.a = sg.sr + E * cm.emu_stride_sr;
+    } else {
+      s.g = sg.g + E * cm.emu_stride_g + off;
+      s.a = sg.a + E * cm.emu_stride_r + off;
+      if (sg.u) s.u = sg.u + E * cm.emu_stride_r + off;
+      list = sg.cand_push + (uint64_t)c * sg.cap;
+      block = ph.kind == kSelPush ? y : (uint32_t)(ph.hop * bk.nseg + si);
+    }
+    s.ws = cx.ws + (size_t)block * kWsWords;
+    s.cv = reinterpret_cast<float*>(cx.cand + list * 8);
+    sm.tile_at[y + 1] = tiles;
+    sm.sample_at[y + 1] = s.sampled;
   }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    uint32_t t0 = 0, s0 = 0;
+#pragma unroll 1
+    for (uint32_t b = 0; b < ph.units; b += 32) {
+      const uint32_t y = b + threadIdx.x;
+      uint32_t t = y < ph.units ? sm.tile_at[y + 1] : 0u, q = y < ph.units ? sm.sample_at[y + 1] : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xffffffffu, t, o), c = __shfl_up_sync(0xffffffffu, q, o);
+        if ((int)threadIdx.x >= o) {
+          t += a;
+          q += c;
+        }
+      }
+      if (y < ph.units) {
+        sm.tile_at[y + 1] = t0 + t;
+        sm.sample_at[y + 1] = s0 + q;
+      }
+      t0 += __shfl_sync(0xffffffffu, t, 31);
+      s0 += __shfl_sync(0xffffffffu, q, 31);
+    }
+    if (threadIdx.x == 0) sm.tile_at[0] = sm.sample_at[0] = 0;
+  }
+  __syncthreads();
+}
+// the unit in whose stretch of the prefix sums item t lies
+__device__ __forceinline__ uint32_t unit_at(const uint32_t* at, uint32_t units, uint32_t t) {
+  uint32_t lo = 0, hi = units;
+#pragma unroll 1
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) / 2;
+    if (at[mid] <= t) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// where a unit's pairs go, and the flags that announce them: into sm.dst (whole CTA)
+__device__ __forceinline__ void unit_dst(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, const SelPhase& ph,
+                                         uint32_t y, SpSmem& sm) {
+  const int N = cx.N, R = cx.R, q = (int)threadIdx.x;
+  int si, c;
+  unit_ref(cx, ph, y, si, c);
+  const bool all = ph.kind == kSelServe || (ph.kind == kSelHop && ph.hop == N - 1);
+  const int slot = ph.kind == kSelPush ? R : (ph.kind == kSelServe ? N + R : (all ? N - 1 + R : ph.hop));
+  const int n = all ? N : 1;
+  __syncthreads();
+  if (q == 0) sm.dst.out.n = n;
+  if (q < n) {
+    int to = (ph.kind == kSelPush ? c : (all ? R : R + 1)) + q;
+    if (to >= N) to -= N;
+    sm.dst.out.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[to]) + (size_t)slot * bk.slot_bytes + bk.seg[si].pay_off;
+    sm.dst.flag[q] = reinterpret_cast<uint32_t*>(cm.flags[to]) + (size_t)slot * bk.nseg + si;
+  }
+  __syncthreads();
 }
 // thread 0 of the CTA that completed the unit
-static __device__ __noinline__ void unit_release(const HpComm& cm, const SpSmem& sm, const UnitDst& d) {
+__device__ __forceinline__ void unit_release(const HpComm& cm, const SpSmem& sm) {
   __threadfence_system();
   const uint32_t v = flag_value(cm, sm);
 #pragma unroll 1
-  for (int q = 0; q < d.out.n; ++q) st_release_sys(d.flag[q], v);
+  for (int q = 0; q < sm.dst.out.n; ++q) st_release_sys(sm.dst.flag[q], v);
 }
 
-static __device__ __noinline__ void flush_units(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
-                                                const SelPhase& ph, SpSmem& sm) {
-  collect_flush(sm.sel, [&](uint32_t y) {
-    SelUnit s;
-    unit_of(bk, cm, cx, ph, y, s);
-    return s;
-  });
-}
-
-// The sampled tiles of this CTA, in the sample pass or (collect) after it: item i belongs
-// to one unit as its tile number j.  The first two stay in shared memory in between.
-static __device__ __noinline__ void sample_units(const SpBucket& bk, const HpComm& cm, const SpCtx& cx,
-                                                 const SelPhase& ph, SpSmem& sm, bool collect) {
-  const uint32_t M = ph.per_tensor, total = bk.samples_total * M;
-  const bool more = blockIdx.x + 2 * cx.G < total;   // the second stash is used again
-  int si = 0;
-#pragma unroll 1
-  for (uint32_t i = blockIdx.x, r = 0; i < total; i += cx.G, ++r) {
-    while (si + 1 < bk.nseg && i >= bk.seg[si + 1].sample_prefix * M) ++si;
-    const SpSeg& sg = bk.seg[si];
-    const uint32_t at = i - sg.sample_prefix * M, c = at / sg.sampled, j = at - c * sg.sampled;
-    const uint32_t y = (uint32_t)si * M + (M > 1 ? c : 0u);
-    SelUnit s;
-    unit_of(bk, cm, cx, ph, y, s);
-    if (j >= s.sampled) continue;
-    float* stash = sm.sel.stash[r < 1 ? 0 : 1];
-    if (collect) collect_sampled(s, y, sm.sel, j, stash, r >= 1 && more);
-    else sample_body(ph.mode, s, bk.momentum, sm.sel, j, stash);
-  }
-}
-
-// The selection of all units of one kind: two barriers (three when some list is long,
-// more only when a sample misled).  Tickets `ticket` and, when the result is to be
-// cleared behind the update pass, ticket + 1.
+// The selection of all units of one kind: two barriers (more only when a sample misled).
+// Tickets `ticket` and, when the result is to be cleared behind the update pass, ticket + 1.
 static __device__ __noinline__ void select_units(const SpBucket& bk, const HpComm& cm, SpCtx& cx, SpSmem& sm, int kind,
                                                  int hop, int ticket, bool zero) {
-  const SelPhase ph = sel_phase(bk, cx, kind, hop);
-  const uint32_t M = ph.per_tensor, units = ph.units;
-  sample_units(bk, cm, cx, ph, sm, false);
+  SelPhase ph;
+  ph.kind = kind;
+  ph.hop = hop;
+  ph.units = (uint32_t)bk.nseg * (kind == kSelPush ? (uint32_t)cx.N : 1u);
+  ph.mode = kind == kSelServe ? 0 : (bk.alg == kDgc ? 2 : 1);
+  const uint32_t units = ph.units;
+  set_units(bk, cm, cx, ph, sm);
+  const uint32_t samples = sm.sample_at[units];
+  // sampled tiles of this CTA; the first two stay in shared memory until they are collected
+  uint32_t mine = 0;
+#pragma unroll 1
+  for (uint32_t i = blockIdx.x; i < samples; i += cx.G, ++mine) {
+    const uint32_t y = unit_at(sm.sample_at, units, i), j = i - sm.sample_at[y];
+    float* stash = sm.sel.stash[mine < 1 ? 0 : 1];
+    if (ph.mode == 0) sample_body<0>(sm.unit[y], bk.momentum, sm.sel, j, stash);
+    else if (ph.mode == 1) sample_body<1>(sm.unit[y], bk.momentum, sm.sel, j, stash);
+    else sample_body<2>(sm.unit[y], bk.momentum, sm.sel, j, stash);
+    __syncthreads();
+  }
   sp_barrier(cm, cx, sm);
   if (threadIdx.x == 0) sm.sel.count = 0;
   __syncthreads();
-  sample_units(bk, cm, cx, ph, sm, true);
-  hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * M, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
-    int si = 0;
 #pragma unroll 1
-    while (t < end) {
-      while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * M) ++si;
-      const SpSeg& sg = bk.seg[si];
-      const uint32_t at = t - sg.tile_prefix * M, c = at / sg.tiles, tt = at - c * sg.tiles;
-      const uint32_t stop = min(sg.tiles, tt + (end - t));
-      const uint32_t y = (uint32_t)si * M + (M > 1 ? c : 0u);
-      if (sg.stride > 1) {
-        SelUnit s;
-        unit_of(bk, cm, cx, ph, y, s);
-        const uint32_t t1 = min(stop, (s.n + kTile - 1) / kTile);
-        if (ph.mode == 0) collect_body<0>(s, y, bk.momentum, sm.sel, tt, t1);
-        else if (ph.mode == 1) collect_body<1>(s, y, bk.momentum, sm.sel, tt, t1);
-        else collect_body<2>(s, y, bk.momentum, sm.sel, tt, t1);
+  for (uint32_t i = blockIdx.x, r = 0; r < mine; i += cx.G, ++r) {
+    const uint32_t y = unit_at(sm.sample_at, units, i);
+    collect_sampled(sm.unit[y], y, sm.sel, i - sm.sample_at[y], sm.sel.stash[r < 1 ? 0 : 1], r >= 1 && mine > 2);
+  }
+  auto unit = [&](uint32_t y) -> const SelUnit& { return sm.unit[y]; };
+  hand_out(cx.ctl + kCtlTickets + ticket, sm.tile_at[units], cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
+    uint32_t y = unit_at(sm.tile_at, units, t);
+#pragma unroll 1
+    for (; t < end; ++y) {
+      const uint32_t base = sm.tile_at[y], t1 = min(sm.tile_at[y + 1], end);
+      if (t1 <= t) continue;   // an empty unit
+      const SelUnit& s = sm.unit[y];
+      if (s.stride > 1) {
+        if (ph.mode == 0) collect_body<0>(s, y, bk.momentum, sm.sel, t - base, t1 - base);
+        else if (ph.mode == 1) collect_body<1>(s, y, bk.momentum, sm.sel, t - base, t1 - base);
+        else collect_body<2>(s, y, bk.momentum, sm.sel, t - base, t1 - base);
       }
-      t += stop - tt;
+      t = t1;
     }
-    if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) flush_units(bk, cm, cx, ph, sm);
+    if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, unit);
   });
-  flush_units(bk, cm, cx, ph, sm);
+  collect_flush(sm.sel, unit);
   sp_barrier(cm, cx, sm);
   // behind the barrier every CTA reads the same counters and decides the same
-  if (threadIdx.x == 0) sm.any = sm.ticket = 0;
-  __syncthreads();
+  int bad = 0;
 #pragma unroll 1
-  for (uint32_t y = threadIdx.x; y < units; y += kSpThreads) {
-    SelUnit s;
-    unit_of(bk, cm, cx, ph, y, s);
-    if (s.n == 0) continue;
-    if (selection_failed(s)) sm.any = 1;
-    else atomicMax(&sm.ticket, __ldcg(s.ws + kWsCandCount));
-  }
-  __syncthreads();
-  const bool failed = sm.any != 0, refined = sm.ticket > kFinishList;
-  __syncthreads();
-  if (refined) {
-    run_units(cx, units, slices_cap(cx, units, 64), [&](int y, uint32_t x, uint32_t nx) {
-      SelUnit s;
-      unit_of(bk, cm, cx, ph, (uint32_t)y, s);
-      if (s.n == 0 || selection_failed(s)) return;
-      UnitDst d;
-      unit_dst(bk, cm, cx, ph, (uint32_t)y, d);
-      refine_body(s, d.out, sm.sel, x, nx);
-    });
-    sp_barrier(cm, cx, sm);
-  }
+  for (uint32_t y = threadIdx.x; y < units; y += kSpThreads)
+    bad |= sm.unit[y].n && selection_failed(sm.unit[y], list_state(sm.unit[y]));
+  const bool failed = __syncthreads_or(bad);
   const uint32_t share = slices_cap(cx, units, 64);
   run_units(cx, units, share, [&](int y, uint32_t x, uint32_t) {
-    SelUnit s;
-    unit_of(bk, cm, cx, ph, (uint32_t)y, s);
-    const bool bad = s.n && selection_failed(s);
-    const uint32_t nx =
-        s.n && !bad ? finish_slices(min(__ldcg(s.ws + (refined ? kWsCand2Count : kWsCandCount)), s.cap), share) : 1u;
-    if (x >= nx || bad) return;
-    UnitDst d;
-    unit_dst(bk, cm, cx, ph, (uint32_t)y, d);
+    const SelUnit& s = sm.unit[y];
+    const ListState ls = list_state(s);
+    if (s.n && selection_failed(s, ls)) return;
+    const uint32_t nx = s.n ? emit_slices(ls.count, share) : 1u;
+    if (x >= nx) return;
+    unit_dst(bk, cm, cx, ph, (uint32_t)y, sm);
     bool done = false;
     if (s.n == 0) {
       done = threadIdx.x == 0;
       if (done)
-        for (int q = 0; q < d.out.n; ++q) write_empty_header(d.out.out[q], bk.alg);
+        for (int q = 0; q < sm.dst.out.n; ++q) write_empty_header(sm.dst.out.out[q], bk.alg);
     } else {
-      done = finish_body(bk.alg, s, d.out, sm.sel, refined, x, nx);
+      done = emit_slice(bk.alg, s, ls, sm.dst.out, sm.sel, x, nx);
     }
-    if (done) unit_release(cm, sm, d);
+    if (done) unit_release(cm, sm);
   });
   sp_mark(cx, kind == kSelServe ? 2 : 0);
   if (zero) zero_result(bk, cm, cx, sm, ticket + 1);
@@ -378,9 +391,8 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
 #pragma unroll 1
   for (int pass = -1; pass <= 3; ++pass) {
     run_units(cx, units, heavy, [&](int y, uint32_t x, uint32_t nx) {
-      SelUnit s;
-      unit_of(bk, cm, cx, ph, (uint32_t)y, s);
-      if (s.n == 0 || !selection_failed(s)) return;
+      const SelUnit& s = sm.unit[y];
+      if (s.n == 0 || !selection_failed(s, list_state(s))) return;
       if (pass < 0) {
         for (uint32_t i = x * kSpThreads + threadIdx.x; i < 3u * kBins; i += nx * kSpThreads) s.ws[i] = 0;
       } else if (pass == 0) {
@@ -388,9 +400,8 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
       } else if (pass < 3) {
         pass_body_rt(pass, s.a, s.n, s.k, s.ws, sm.sh, sm.fs, x, nx);
       } else {
-        UnitDst d;
-        unit_dst(bk, cm, cx, ph, (uint32_t)y, d);
-        if (emit_body(bk.alg, s.a, s.u, s.n, s.k, s.kmax, d.out, s.ws, sm.fs, sm.es, x, nx)) unit_release(cm, sm, d);
+        unit_dst(bk, cm, cx, ph, (uint32_t)y, sm);
+        if (emit_body(bk.alg, s.a, s.u, s.n, s.k, s.kmax, sm.dst.out, s.ws, sm.fs, sm.es, x, nx)) unit_release(cm, sm);
       }
     });
     if (pass < 3) sp_barrier(cm, cx, sm);
@@ -613,14 +624,9 @@ static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int
     if (G > cap / ranks_here) G = cap / ranks_here;
   }
   if (G < 1 || (long long)G * ranks_here > (long long)cap) return HP_ERR_RESIDENCY;
-  bk.samples_total = 0;
-  for (int i = 0; i < nseg; ++i) {  // a sampled tile for every CTA, over the units of a push or of a hop
-    SpSeg& sg = bk.seg[i];
-    sg.stride = sample_stride(sg.tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);
-    sg.sampled = (sg.tiles + sg.stride - 1) / sg.stride;
-    bk.seg[i].sample_prefix = bk.samples_total;
-    bk.samples_total += bk.seg[i].sampled;
-  }
+  for (int i = 0; i < nseg; ++i)  // a sampled tile for every CTA, over the units of a push or of a hop
+    bk.seg[i].stride =
+        sample_stride(bk.seg[i].tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);
   SpLaunch L;
   L.ws = static_cast<uint8_t*>(ws);
   L.hist_words = sp_hist_words(nseg, N);

@@ -18,11 +18,11 @@ constexpr int kBins = 4096;
 constexpr int kWsOutCount = 3 * kBins + 0;
 constexpr int kWsTieCount = 3 * kBins + 1;
 constexpr int kWsDone = 3 * kBins + 2;
-constexpr int kWsCandCount = 3 * kBins + 3;   // candidates collected by the update pass
-constexpr int kWsOverflow = 3 * kBins + 4;    // they did not fit: use the full passes
-constexpr int kWsLow = 3 * kBins + 5;         // magnitude key from which an element is a candidate
-constexpr int kWsSampled = 3 * kBins + 6;     // slices of the sample that are done
-constexpr int kWsCand2Count = 3 * kBins + 7;  // candidates left after the first digit
+constexpr int kWsSampled = 3 * kBins + 3;     // sampled tiles that are done
+constexpr int kWsCandCount = 3 * kBins + 4;   // candidates collected by the update pass
+constexpr int kWsOverflow = 3 * kBins + 5;    // they did not fit: use the full passes
+constexpr int kWsLow = 3 * kBins + 6;         // magnitude key from which an element is a candidate
+constexpr int kWsCand2Count = 3 * kBins + 7;  // candidates in the bin of the k-th largest
 constexpr int kWsTicket = 3 * kBins + 8;      // stand-alone kernel: tile ticket, status
 constexpr int kWsStatus = 3 * kBins + 9;
 constexpr int kWsWords = 3 * kBins + 16;
@@ -32,72 +32,82 @@ __device__ __forceinline__ uint32_t digit_of(uint32_t key, int pass) {
 }
 
 struct FindSmem {
-  alignas(16) uint32_t counts[kBins / kSpThreads];
   uint32_t sums[kSpThreads / 32];
-  uint32_t owner, above;
+  uint2 res;
 };
 
 // Largest bin of a histogram of kBins bins whose suffix count reaches k, and krem = how
 // many of the k fall in that bin, i.e. k - count(bins > bin); (0, 0) when fewer than k are
 // counted.  `hist` is in shared or in global memory, where other CTAs' atomics wrote it.
-// Thread t sums bins 16t .. 16t+15; the thread in whose bins the k-th lies hands its
-// sixteen counts to everybody, and every warp finds the bin among them.
+// A warp sums 512 consecutive bins, read without bank conflicts; the warp in whose bins
+// the k-th lies narrows it down to a row of 128, a lane and a bin.  (With 16 bins in a row
+// per thread, every read of a histogram in shared memory was a 16-way conflict and a
+// call took 0.9 us.)
 static __device__ __noinline__ void find_bin(const uint32_t* hist, uint32_t k, FindSmem& fs, uint32_t& bin,
                                              uint32_t& krem) {
-  constexpr int per = kBins / kSpThreads;  // 16
-  uint4 c[per / 4];
-  uint32_t sum = 0;
+  constexpr int kRows = kBins / (kSpThreads * 4);  // rows of 128 bins per warp
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint4 c[kRows];
+  uint32_t rows[kRows], all = 0;
 #pragma unroll
-  for (int i = 0; i < per / 4; ++i) {
+  for (int j = 0; j < kRows; ++j)
     asm volatile("ld.volatile.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(c[i].x), "=r"(c[i].y), "=r"(c[i].z), "=r"(c[i].w)
-                 : "l"(hist + threadIdx.x * per + 4 * i)
+                 : "=r"(c[j].x), "=r"(c[j].y), "=r"(c[j].z), "=r"(c[j].w)
+                 : "l"(hist + warp * (kRows * 128) + j * 128 + lane * 4)
                  : "memory");
-    sum += c[i].x + c[i].y + c[i].z + c[i].w;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t v = sum;   // suffix sum over the warp
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_down_sync(0xffffffffu, v, o);
-    if (lane + o < 32) v += y;
+  for (int j = 0; j < kRows; ++j) {
+    rows[j] = __reduce_add_sync(0xffffffffu, c[j].x + c[j].y + c[j].z + c[j].w);
+    all += rows[j];
   }
-  if (lane == 0) fs.sums[warp] = v;
-  if (threadIdx.x == 0) fs.owner = 0xFFFFFFFFu;
+  if (lane == 0) fs.sums[warp] = all;
+  if (threadIdx.x == 0) fs.res = make_uint2(0u, 0u);
   __syncthreads();
-  const uint32_t higher = lane > warp && lane < kSpThreads / 32 ? fs.sums[lane] : 0u;
-  const uint32_t above = v - sum + __reduce_add_sync(0xffffffffu, higher);  // in the bins of higher threads
-  if (above < k && k <= above + sum) {
-    fs.owner = threadIdx.x;
-    fs.above = above;
+  // elements in the bins of higher warps
+  uint32_t above =
+      __reduce_add_sync(0xffffffffu, lane > warp && lane < kSpThreads / 32 ? fs.sums[lane & (kSpThreads / 32 - 1)] : 0u);
+  if (above < k && k <= above + all) {
+    int row = kRows - 1;
+    uint4 v = c[kRows - 1];
 #pragma unroll
-    for (int i = 0; i < per / 4; ++i) *reinterpret_cast<uint4*>(fs.counts + 4 * i) = c[i];
-  }
-  __syncthreads();
-  const uint32_t owner = fs.owner;
-  bin = krem = 0;
-  if (owner != 0xFFFFFFFFu) {
-    const uint32_t mine = lane < per ? fs.counts[lane & (per - 1)] : 0u;
-    uint32_t w = mine;
+    for (int j = kRows - 1; j > 0; --j)
+      if (row == j && above + rows[j] < k) {
+        above += rows[j];
+        row = j - 1;
+        v = c[j - 1];
+      }
+    const uint32_t mine = v.x + v.y + v.z + v.w;
+    uint32_t suffix = mine;
 #pragma unroll
-    for (int o = 1; o < per; o <<= 1) {
-      const uint32_t y = __shfl_down_sync(0xffffffffu, w, o);
-      if (lane + o < per) w += y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_down_sync(0xffffffffu, suffix, o);
+      if (lane + o < 32) suffix += y;
     }
-    const uint32_t acc = fs.above + w - mine;
-    const uint32_t hit = __ballot_sync(0xffffffffu, lane < per && acc < k && k <= acc + mine);
-    const int at = __ffs(hit) - 1;
-    bin = owner * per + at;
-    krem = k - __shfl_sync(0xffffffffu, acc, at);
+    above += suffix - mine;   // in the bins of higher lanes too
+    if (above < k && k <= above + mine) {
+      uint32_t b = 3;
+      if (above + v.w < k) { above += v.w; b = 2;
+        if (above + v.z < k) { above += v.z; b = 1;
+          if (above + v.y < k) { above += v.y; b = 0; } } }
+      fs.res = make_uint2(warp * (kRows * 128) + row * 128 + lane * 4 + b, k - above);
+    }
   }
+  __syncthreads();
+  const uint2 r = fs.res;
+  bin = r.x;
+  krem = r.y;
   __syncthreads();
 }
 
 __device__ __forceinline__ void flush_hist(const uint32_t* sh, uint32_t* __restrict__ gh) {
-#pragma unroll 1
-  for (int i = threadIdx.x; i < kBins; i += kSpThreads) {
-    const uint32_t c = sh[i];
-    if (c) atomicAdd(gh + i, c);
+#pragma unroll
+  for (int i = 0; i < kBins / 4; i += kSpThreads) {
+    const uint4 c = reinterpret_cast<const uint4*>(sh)[i + threadIdx.x];
+    uint32_t* to = gh + 4 * (i + threadIdx.x);
+    if (c.x) atomicAdd(to, c.x);
+    if (c.y) atomicAdd(to + 1, c.y);
+    if (c.z) atomicAdd(to + 2, c.z);
+    if (c.w) atomicAdd(to + 3, c.w);
   }
 }
 
@@ -349,28 +359,26 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 //
 //   sample   every stride-th tile of the array is updated first; the histogram of its
 //            magnitudes gives a `low` below which an element is almost surely not among
-//            the k largest, and above which about 1.1 to 1.7 k are
+//            the k largest
 //   collect  the other tiles are updated; elements of at least `low` are appended to a
-//            candidate list with the histogram of their first digit (the sampled tiles'
-//            from shared memory).  The list holds the k largest exactly when it has k
-//            elements.
-//   finish   digit by digit on the list: the exact threshold, the pairs, the header.  A
-//            long list first goes through one distributed step (refine) that sends what
-//            lies above the first digit's bin and keeps what lies in it.
+//            candidate list with a histogram of their distance from `low` (the sampled
+//            tiles' from shared memory).  The list holds the k largest exactly when it
+//            has k elements.
+//   emit     every CTA takes a slice of the list, sends what lies above the histogram bin
+//            of the k-th largest and moves what lies in that bin to a second list, a few
+//            dozen elements; the CTA that comes last selects exactly among those and
+//            writes the header.
 //
 // State is read and written once: HBM bound at 20 bytes per element for DGC, 12 for
 // GradDrop.  A list that came out shorter than k or longer than its room (a sample that
 // misled, or massive ties) makes the launch fall back to histogram passes over the
 // whole array.
 //
-// Up to a few million elements the time is not memory but instruction fetch: most of
-// this code runs once or twice per launch, and code that is not in the instruction cache
-// comes in at a few instructions per 0.1 us (one CTA on 4000 elements: 1900 instructions
-// per warp took 25 us, half of all warp-cycles waiting for one).  Hence one out-of-line
-// copy of every step, rolled loops where a step runs once, 32-bit arithmetic, and sizes
-// worked out on the host.
-constexpr uint32_t kFinishKeys = 8192;  // list length up to which a CTA keeps the keys in shared memory
-constexpr uint32_t kFinishList = 12288; // longest list that is finished without a refine step
+// Up to a few million elements the time is a chain of latencies instead: two grid
+// barriers, and steps of a few dependent L2 accesses each (about 0.7 us an atomic).  So
+// bins are fine where the k-th largest is to be expected, which leaves one digit to
+// resolve; counters that are read together lie together; and slices send without a
+// barrier behind the histogram.
 constexpr uint32_t kMinSampled = 4;     // tiles of an array that are sampled at least
 constexpr uint32_t kSelTile = 4096;     // elements per tile: 16 per thread
 
@@ -390,10 +398,8 @@ __device__ __forceinline__ float* list2_values(const SelUnit& s) { return s.cv +
 __device__ __forceinline__ uint32_t* list2_indices(const SelUnit& s) {
   return reinterpret_cast<uint32_t*>(s.cv + 3 * (size_t)s.cap);
 }
-// room of each of the two lists in `pairs` pairs; keeps every list on 16 bytes
-HP_HD uint32_t list_cap(uint64_t pairs) {
-  return (uint32_t)(pairs / 2 < 0x7FFFFFFCull ? pairs / 2 : 0x7FFFFFFCull) & ~3u;
-}
+// room of each of the two lists in `pairs` pairs
+HP_HD uint32_t list_cap(uint64_t pairs) { return (uint32_t)(pairs / 2 < 0x7FFFFFFFull ? pairs / 2 : 0x7FFFFFFFull); }
 // stride of the sampled tiles of an array when ctas CTAs share `total` tiles: about a
 // sampled tile for every CTA
 HP_HD uint32_t sample_stride(uint32_t tiles, uint64_t total, uint32_t ctas) {
@@ -402,114 +408,104 @@ HP_HD uint32_t sample_stride(uint32_t tiles, uint64_t total, uint32_t ctas) {
   return share >= tiles ? 1u : (uint32_t)((tiles + share - 1) / share);
 }
 
+// First digit of a candidate.  Its distance from `low` in steps of 2^12 keys (1/2048 of
+// the magnitude), the last bin for everything more than two octaves above, where the
+// k-th largest is not to be expected.  When all non-zero elements are candidates
+// (low == 1) they may span any range: the leading 12 bits then.
+__device__ __forceinline__ uint32_t cand_digit(uint32_t key, uint32_t low) {
+  return low <= 1u ? key >> 19 : min((key - low) >> 12, (uint32_t)kBins - 1u);
+}
+
+// counters that are read together behind the update pass
+struct ListState {
+  uint32_t count, overflow, low;
+};
+__device__ __forceinline__ ListState list_state(const SelUnit& s) {
+  const uint4 v = __ldcg(reinterpret_cast<const uint4*>(s.ws + kWsCandCount));
+  return {v.x, v.y, v.z};
+}
+// the list lacks some of the k largest
+__device__ __forceinline__ bool selection_failed(const SelUnit& s, const ListState& l) {
+  return l.overflow != 0u || (l.count < s.k && l.low > 1u);
+}
+
 constexpr int kCollectBuf = 1024;  // candidates a CTA gathers before it reserves room in the lists
 
 struct SelSmem {
   union {
-    uint32_t hist[kBins];            // sample; finish: digit histograms
+    uint32_t hist[kBins];            // sample; emit: the last digits
     struct {
       float val[kCollectBuf];
       uint32_t idx[kCollectBuf];
       uint16_t unit[kCollectBuf];
     } buf;                           // collect
   };
-  union {
-    uint32_t keys[kFinishKeys];      // finish
-    float stash[2][kSelTile];        // sample to collect
-  };
+  float stash[2][kSelTile];          // sample to collect
   FindSmem fs;
-  uint32_t count, base, ticket, flag;
+  uint32_t count, base, base2, ticket, flag;
   uint32_t sent, ties;
 };
 
 __device__ __forceinline__ void clear_hist(uint32_t* sh) {
-#pragma unroll 1
-  for (int b = threadIdx.x; b < kBins / 4; b += kSpThreads)
-    reinterpret_cast<uint4*>(sh)[b] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int b = 0; b < kBins / 4; b += kSpThreads)
+    reinterpret_cast<uint4*>(sh)[b + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// The update of one element.  MODE as in pass0_body.
+// Loads tile t and applies the update (MODE as in pass0_body), all loads before the first
+// store.  Elements past the end read as zero, and a zero is never sent.
 template <int MODE>
-__device__ __forceinline__ float update_value(float v, float g, float& u, float momentum) {
-  if (MODE == 1) v = v + g;
-  if (MODE == 2) {
-    u = __fmaf_rn(momentum, u, g);
-    v = v + u;
-  }
-  return v;
-}
-
-// Loads tile t and applies the update, all loads before the first store; put(j, v) gets
-// float4 number j * 256 + thread.  A tile that is not full or not on 16 bytes goes
-// element by element; what lies past the end reads as zero, and a zero is never sent.
-template <int MODE, typename F>
-__device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, F put) {
-  const size_t base = (size_t)t * kSelTile;
+__device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[4]) {
   const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
                      (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
-  if (vec && base + kSelTile <= s.n) {
-    float4 av[4], gv[4], uv[4];
+  const uint64_t i0 = (uint64_t)t * kSelTile + threadIdx.x * 4;
+  float4 gv[4], uv[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const size_t i = base + (j * kSpThreads + threadIdx.x) * 4;
-      av[j] = *reinterpret_cast<const float4*>(s.a + i);
-      if (MODE >= 1) gv[j] = *reinterpret_cast<const float4*>(s.g + i);
-      if (MODE == 2) uv[j] = *reinterpret_cast<const float4*>(s.u + i);
-    }
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t i = i0 + j * kSpThreads * 4;
+    av[j] = ld4(s.a, i, s.n, vec);
+    if (MODE >= 1) gv[j] = ld4(s.g, i, s.n, vec);
+    if (MODE == 2) uv[j] = ld4(s.u, i, s.n, vec);
+  }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const size_t i = base + (j * kSpThreads + threadIdx.x) * 4;
-      float4& v = av[j];
-      v.x = update_value<MODE>(v.x, gv[j].x, uv[j].x, momentum);
-      v.y = update_value<MODE>(v.y, gv[j].y, uv[j].y, momentum);
-      v.z = update_value<MODE>(v.z, gv[j].z, uv[j].z, momentum);
-      v.w = update_value<MODE>(v.w, gv[j].w, uv[j].w, momentum);
-      if (MODE == 2) *reinterpret_cast<float4*>(s.u + i) = uv[j];
-      if (MODE >= 1) *reinterpret_cast<float4*>(s.a + i) = v;
-      put(j, v);
-    }
-  } else {
-#pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
-      float e[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const size_t i = base + (j * kSpThreads + threadIdx.x) * 4 + q;
-        e[q] = 0.0f;
-        if (i < s.n) {
-          float w = MODE == 2 ? s.u[i] : 0.0f;
-          e[q] = update_value<MODE>(s.a[i], MODE >= 1 ? s.g[i] : 0.0f, w, momentum);
-          if (MODE == 2) s.u[i] = w;
-          if (MODE >= 1) s.a[i] = e[q];
-        }
-      }
-      put(j, make_float4(e[0], e[1], e[2], e[3]));
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t i = i0 + j * kSpThreads * 4;
+    float4& v = av[j];
+    if (MODE == 1) {
+      v.x = v.x + gv[j].x; v.y = v.y + gv[j].y; v.z = v.z + gv[j].z; v.w = v.w + gv[j].w;
+      st4(s.a, i, s.n, vec, v);
+    } else if (MODE == 2) {
+      float4 w;
+      w.x = __fmaf_rn(momentum, uv[j].x, gv[j].x);
+      w.y = __fmaf_rn(momentum, uv[j].y, gv[j].y);
+      w.z = __fmaf_rn(momentum, uv[j].z, gv[j].z);
+      w.w = __fmaf_rn(momentum, uv[j].w, gv[j].w);
+      v.x = v.x + w.x; v.y = v.y + w.y; v.z = v.z + w.z; v.w = v.w + w.w;
+      st4(s.u, i, s.n, vec, w);
+      st4(s.a, i, s.n, vec, v);
     }
   }
-}
-
-template <int MODE>
-static __device__ __noinline__ void update_to_stash(const SelUnit& s, float momentum, uint32_t t, float* stash) {
-  update_tile<MODE>(s, momentum, t, [&](int j, const float4& v) {
-    reinterpret_cast<float4*>(stash)[j * kSpThreads + threadIdx.x] = v;
-  });
 }
 
 // Sampled tile number i of an array: update, values into `stash`, magnitudes into the
 // array's sample histogram.  The CTA that completes the sample turns it into the
 // candidates' lower bound.
-static __device__ __noinline__ void sample_body(int mode, const SelUnit& s, float momentum, SelSmem& sm, uint32_t i,
+template <int MODE>
+static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum, SelSmem& sm, uint32_t i,
                                                 float* stash) {
-  const uint32_t t = i * s.stride;
-  if (mode == 0) update_to_stash<0>(s, momentum, t, stash);
-  else if (mode == 1) update_to_stash<1>(s, momentum, t, stash);
-  else update_to_stash<2>(s, momentum, t, stash);
   clear_hist(sm.hist);
+  float4 av[4];
+  update_tile<MODE>(s, momentum, i * s.stride, av);
   __syncthreads();
-#pragma unroll 1
-  for (uint32_t p = threadIdx.x; p < kSelTile; p += kSpThreads) {
-    const uint32_t key = abs_key(stash[p]);
-    if (key) atomicAdd(&sm.hist[key >> 19], 1u);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    reinterpret_cast<float4*>(stash)[j * kSpThreads + threadIdx.x] = av[j];
+    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t key = abs_key(e[q]);
+      if (key) atomicAdd(&sm.hist[key >> 19], 1u);
+    }
   }
   __syncthreads();
   flush_hist(sm.hist, s.ws);
@@ -533,30 +529,40 @@ static __device__ __noinline__ void sample_body(int mode, const SelUnit& s, floa
   uint32_t bin, rem;
   find_bin(s.ws, rank, sm.fs, bin, rem);   // bin 0 when fewer than rank are counted
   if (threadIdx.x == 0) s.ws[kWsLow] = bin ? bin << 19 : 1u;   // zeros are never sent
-  __syncthreads();
 }
 
 // Items [0, total) in stretches, taken from *word by whichever of the ctas CTAs is free:
-// SMs do not run at one speed, and equal shares leave the fast ones waiting.  f(lo, hi)
-// runs with the whole CTA; `slot` is shared memory.  (Asking for the next stretch before
-// working on the current one split thread 0 from its warp, and the two halves then
-// counted twice at the barriers that follow.)
+// SMs do not run at one speed, and equal shares leave the fast ones waiting.  The next
+// stretch is asked for before the current one is worked on, by predicated instructions
+// (an `if` around them split thread 0 from its warp, and the two halves then counted
+// twice at the barriers that follow).  f(lo, hi) runs with the whole CTA; `slot` is
+// shared memory.
 template <typename F>
 __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t ctas, uint32_t& slot, F f) {
   const uint32_t stretch = total / (4u * ctas) + 1u;
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(&slot);
+  uint32_t next = 0;
+  auto take = [&] {
+    asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %1, 0;\n@p atom.add.relaxed.gpu.global.u32 %0, [%2], %3;\n}"
+                 : "+r"(next) : "r"(threadIdx.x), "l"(word), "r"(stretch) : "memory");
+  };
+  take();
 #pragma unroll 1
   for (;;) {
-    if (threadIdx.x == 0) slot = atomicAdd(word, stretch);
+    asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %1, 0;\n@p st.shared.u32 [%2], %0;\n}" ::"r"(next),
+                 "r"(threadIdx.x), "r"(at) : "memory");
     __syncthreads();
-    const uint32_t lo = slot;
+    const uint32_t lo = *(volatile uint32_t*)&slot;
     __syncthreads();
     if (lo >= total) break;
+    take();
     f(lo, min(lo + stretch, total));
   }
 }
 
 // one candidate into the CTA's buffer, or, when that is full, straight into its list
-static __device__ __noinline__ void collect_one(const SelUnit& s, uint32_t uid, SelSmem& sm, float v, uint32_t i) {
+__device__ __forceinline__ void collect_one(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, float v,
+                                            uint32_t i) {
   const uint32_t p = atomicAdd(&sm.count, 1u);
   if (p < (uint32_t)kCollectBuf) {
     sm.buf.val[p] = v;
@@ -565,12 +571,26 @@ static __device__ __noinline__ void collect_one(const SelUnit& s, uint32_t uid, 
     return;
   }
   const uint32_t pos = atomicAdd(s.ws + kWsCandCount, 1u);
-  atomicAdd(s.ws + kBins + (abs_key(v) >> 19), 1u);
+  atomicAdd(s.ws + kBins + cand_digit(abs_key(v), low), 1u);
   if (pos < s.cap) {
     s.cv[pos] = v;
     list_indices(s)[pos] = i;
   } else {
     s.ws[kWsOverflow] = 1u;
+  }
+}
+// the elements of a tile that reach `low`
+__device__ __forceinline__ void collect_tile(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, uint32_t t,
+                                             const float4 (&av)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
+    const uint32_t most = max(max(abs_key(e[0]), abs_key(e[1])), max(abs_key(e[2]), abs_key(e[3])));
+    if (most < low) continue;
+    const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (abs_key(e[q]) >= low) collect_one(s, uid, sm, low, e[q], i + q);
   }
 }
 
@@ -585,30 +605,34 @@ static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid,
     const bool skip = phase == 0;
     if (++phase == s.stride) phase = 0;
     if (skip) continue;
-    update_tile<MODE>(s, momentum, t, [&](int j, const float4& v) {
-      const uint32_t most = max(max(abs_key(v.x), abs_key(v.y)), max(abs_key(v.z), abs_key(v.w)));
-      if (most < low) return;
-      const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
-      if (abs_key(v.x) >= low) collect_one(s, uid, sm, v.x, i);
-      if (abs_key(v.y) >= low) collect_one(s, uid, sm, v.y, i + 1);
-      if (abs_key(v.z) >= low) collect_one(s, uid, sm, v.z, i + 2);
-      if (abs_key(v.w) >= low) collect_one(s, uid, sm, v.w, i + 3);
-    });
+    float4 av[4];
+    update_tile<MODE>(s, momentum, t, av);
+    if (MODE == 0 && phase != 0 && t + 1 < t1) {
+      // one array only: a second tile's loads in flight keep the memory busy
+      float4 bv[4];
+      update_tile<0>(s, momentum, t + 1, bv);
+      collect_tile(s, uid, sm, low, t, av);
+      collect_tile(s, uid, sm, low, t + 1, bv);
+      ++t;
+      if (++phase == s.stride) phase = 0;
+    } else {
+      collect_tile(s, uid, sm, low, t, av);
+    }
   }
 }
 
 // Sampled tile number i again, updated before: from its stash, or (again) read once more.
 static __device__ __noinline__ void collect_sampled(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t i,
-                                                    float* stash, bool again) {
+                                                    const float* stash, bool again) {
   const uint32_t t = i * s.stride, low = __ldcg(s.ws + kWsLow);
-  if (again) update_to_stash<0>(s, 0.0f, t, stash);
-  __syncthreads();
-#pragma unroll 1
-  for (uint32_t p = threadIdx.x; p < kSelTile; p += kSpThreads) {
-    const float v = stash[p];
-    if (abs_key(v) >= low) collect_one(s, uid, sm, v, t * kSelTile + p);
+  float4 av[4];
+  if (again) {
+    update_tile<0>(s, 0.0f, t, av);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) av[j] = reinterpret_cast<const float4*>(stash)[j * kSpThreads + threadIdx.x];
   }
-  __syncthreads();
+  collect_tile(s, uid, sm, low, t, av);
 }
 
 // Append the CTA's gathered candidates to their lists, and their first digits to the
@@ -626,12 +650,13 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
     if (have) {
       const uint32_t uid = sm.buf.unit[p], lane = threadIdx.x & 31;
       const float v = sm.buf.val[p];
-      const SelUnit s = unit(uid);
+      const SelUnit& s = unit(uid);
+      const uint32_t low = __ldcg(s.ws + kWsLow);
       const uint32_t group = __match_any_sync(mask, uid);
       const int lead = __ffs(group) - 1;
       uint32_t pos = 0;
       if ((int)lane == lead) pos = atomicAdd(s.ws + kWsCandCount, (uint32_t)__popc(group));
-      atomicAdd(s.ws + kBins + (abs_key(v) >> 19), 1u);
+      atomicAdd(s.ws + kBins + cand_digit(abs_key(v), low), 1u);
       pos = __shfl_sync(group, pos, lead) + __popc(group & ((1u << lane) - 1u));
       if (pos < s.cap) {
         s.cv[pos] = v;
@@ -657,170 +682,114 @@ __device__ __forceinline__ void put_pair(const EmitDst& dst, size_t val_off, uin
   }
 }
 
-// Slice x of nx of a list too long for one CTA: pairs above the first digit's bin are
-// sent (and their state cleared), pairs in it move to the second list.  The finds of a
-// stretch are counted in shared memory so that the global counters are touched twice
-// per CTA and stretch.
-static __device__ __noinline__ void refine_body(const SelUnit& s, const EmitDst& dst, SelSmem& sm, uint32_t x,
-                                                uint32_t nx) {
-  const uint32_t L = min(__ldcg(s.ws + kWsCandCount), s.cap);
-  uint32_t bin0, rem;
-  find_bin(s.ws + kBins, min(s.k, L), sm.fs, bin0, rem);
-  const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
-  const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
-#pragma unroll 1
-  for (uint32_t p0 = lo; p0 < hi; p0 += 4 * kSpThreads) {
-    if (threadIdx.x == 0) sm.sent = sm.ties = 0;
-    __syncthreads();
-    float v[4];
-    uint32_t at[4], idx[4];
-    int what[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t p = p0 + j * kSpThreads + threadIdx.x;
-      v[j] = p < hi ? __ldcg(s.cv + p) : 0.0f;
-      idx[j] = p < hi ? __ldcg(list_indices(s) + p) : 0u;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t bin = abs_key(v[j]) >> 19;
-      const bool have = p0 + j * kSpThreads + threadIdx.x < hi;
-      what[j] = !have || bin < bin0 ? 0 : (bin > bin0 ? 1 : 2);
-      at[j] = what[j] == 1 ? atomicAdd(&sm.sent, 1u) : (what[j] == 2 ? atomicAdd(&sm.ties, 1u) : 0u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      sm.base = sm.sent ? atomicAdd(s.ws + kWsOutCount, sm.sent) : 0u;
-      sm.ticket = sm.ties ? atomicAdd(s.ws + kWsCand2Count, sm.ties) : 0u;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (what[j] == 1 && idx[j] < s.n) {
-        put_pair(dst, val_off, s.kmax, sm.base + at[j], idx[j], v[j]);
-        s.a[idx[j]] = 0.0f;
-        if (s.u) s.u[idx[j]] = 0.0f;
-      } else if (what[j] == 2) {
-        const uint32_t pos = sm.ticket + at[j];   // never more than the first list holds
-        if (pos < s.cap) {
-          list2_values(s)[pos] = v[j];
-          list2_indices(s)[pos] = idx[j];
-        }
-      }
-    }
-    __syncthreads();
-  }
+// CTAs that share a list of L elements
+__device__ __forceinline__ uint32_t emit_slices(uint32_t L, uint32_t most) {
+  const uint32_t n = L / kSpThreads + 1u;
+  return n < most ? n : most;
 }
 
-// Slice x of nx of the finish of one array.  The nx CTAs all work out the exact threshold
-// of the list (the second one after a refine step) -- its keys are a few kilobytes in L2,
-// and repeating the three digits costs less than a barrier after them -- and each sends
-// its share of the pairs.  True in thread 0 of the CTA that finished last, behind the
-// headers.  Every step runs once per launch, so its time is latency and instruction
-// fetch: one copy of the digit search, rolled loops.
-static __device__ __noinline__ bool finish_body(int alg, const SelUnit& s, const EmitDst& dst, SelSmem& sm,
-                                                bool refined, uint32_t x, uint32_t nx) {
-  const uint32_t all = min(__ldcg(s.ws + kWsCandCount), s.cap);
-  const uint32_t k = min(s.k, all);          // fewer than k non-zero elements: all of them
-  const uint32_t L = refined ? min(__ldcg(s.ws + kWsCand2Count), s.cap) : all;
-  const float* cv = refined ? list2_values(s) : s.cv;
-  const uint32_t* ci = refined ? list2_indices(s) : list_indices(s);
+// Slice x of nx of one array's candidates.  True in thread 0 of the CTA that finished
+// last, behind the headers.
+static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const ListState& ls, const EmitDst& dst,
+                                               SelSmem& sm, uint32_t x, uint32_t nx) {
+  const uint32_t L = ls.count, low = ls.low;   // no overflow: the list holds all of them
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
-  // keys into shared memory, eight a thread in flight; past L whatever the list's room holds
-#pragma unroll 1
-  for (uint32_t p = threadIdx.x * 4; p < L && p < kFinishKeys; p += 8 * kSpThreads) {
-    const uint32_t q = p + 4 * kSpThreads;
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(cv + p));
-    uint4 w = v;
-    if (q < L) w = __ldcg(reinterpret_cast<const uint4*>(cv + q));
-    *reinterpret_cast<uint4*>(sm.keys + p) =
-        make_uint4(v.x & 0x7FFFFFFFu, v.y & 0x7FFFFFFFu, v.z & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu);
-    *reinterpret_cast<uint4*>(sm.keys + q) =
-        make_uint4(w.x & 0x7FFFFFFFu, w.y & 0x7FFFFFFFu, w.z & 0x7FFFFFFFu, w.w & 0x7FFFFFFFu);
-  }
-  auto key_at = [&](uint32_t p) { return p < kFinishKeys ? sm.keys[p] : abs_key(__ldcg(cv + p)); };
-  uint32_t prefix, rem;
-  find_bin(s.ws + kBins, k, sm.fs, prefix, rem);
-  // the remaining digits: 11 bits, then 8
-#pragma unroll 1
-  for (int d = 0; d < 2; ++d) {
-    const int low = d == 0 ? 8 : 0, bits = d == 0 ? 11 : 8;
-    clear_hist(sm.hist);
-    __syncthreads();
-#pragma unroll 1
-    for (uint32_t p = threadIdx.x; p < L; p += kSpThreads) {
-      const uint32_t key = key_at(p);
-      if ((key >> (low + bits)) == prefix) atomicAdd(&sm.hist[(key >> low) & ((1u << bits) - 1u)], 1u);
-    }
-    __syncthreads();
-    uint32_t bin, r;
-    find_bin(sm.hist, rem, sm.fs, bin, r);
-    prefix = (prefix << bits) | bin;
-    rem = r;
-  }
-  const uint32_t thr = prefix, need = rem;   // `need` of the elements equal to thr are sent
+  const bool every = L < s.k;                  // fewer than k are not zero: all are sent
+  uint32_t bin0 = 0, rem = 0;
+  if (!every) find_bin(s.ws + kBins, s.k, sm.fs, bin0, rem);
   const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
 #pragma unroll 1
   for (uint32_t p0 = lo; p0 < hi; p0 += kSpThreads) {
     if (threadIdx.x == 0) sm.sent = sm.ties = 0;
     __syncthreads();
     const uint32_t p = p0 + threadIdx.x;
-    const uint32_t key = p < hi ? key_at(p) : 0u;
-    const bool more = p < hi && key > thr, tie = p < hi && key == thr;
+    float v = 0.0f;
     uint32_t idx = 0, at = 0;
-    float val = 0.0f;
-    if (more || tie) {
-      idx = __ldcg(ci + p);
-      val = __ldcg(cv + p);
-      at = more ? atomicAdd(&sm.sent, 1u) : atomicAdd(&sm.ties, 1u);
+    bool send = false, keep = false;
+    if (p < hi) {
+      v = __ldcg(s.cv + p);
+      idx = __ldcg(list_indices(s) + p);
+      const uint32_t d = cand_digit(abs_key(v), low);
+      send = every || d > bin0;
+      keep = !every && d == bin0;
+      if (send) at = atomicAdd(&sm.sent, 1u);
+      if (keep) at = atomicAdd(&sm.ties, 1u);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      // of this stretch's ties those that come early enough in the launch are sent
-      uint32_t ok = 0;
-      if (sm.ties && need) {
-        const uint32_t before = atomicAdd(s.ws + kWsTieCount, sm.ties);
-        ok = before < need ? min(sm.ties, need - before) : 0u;
-      }
-      sm.ties = ok;
-      sm.base = sm.sent + ok ? atomicAdd(s.ws + kWsOutCount, sm.sent + ok) : 0u;
-    }
+    if (threadIdx.x == 0 && sm.sent) sm.base = atomicAdd(s.ws + kWsOutCount, sm.sent);
+    if (threadIdx.x == 32 && sm.ties) sm.base2 = atomicAdd(s.ws + kWsCand2Count, sm.ties);
     __syncthreads();
-    const bool send = more || (tie && at < sm.ties);
     if (send && idx < s.n) {
-      put_pair(dst, val_off, s.kmax, sm.base + (more ? at : sm.sent + at), idx, val);
+      put_pair(dst, val_off, s.kmax, sm.base + at, idx, v);
       s.a[idx] = 0.0f;
       if (s.u) s.u[idx] = 0.0f;
     }
-    __syncthreads();
+    if (keep) {   // never more than the first list holds
+      list2_values(s)[sm.base2 + at] = v;
+      list2_indices(s)[sm.base2 + at] = idx;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t done;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(done) : "l"(s.ws + kWsDone) : "memory");
+    sm.flag = done == nx - 1;
+  }
+  __syncthreads();
+  if (!sm.flag) return false;
+  // The last CTA: among the elements of the k-th's bin, `rem` are sent.  What is left of
+  // their keys is 12 bits in a fine bin, 19 in a bin of the leading bits, and up to 31 in
+  // the last fine bin.
+  const uint32_t L2 = every ? 0u : __ldcg(s.ws + kWsCand2Count);
+  if (threadIdx.x == 0) sm.sent = __ldcg(s.ws + kWsOutCount), sm.ties = 0;
+  const uint32_t start = low <= 1u ? bin0 << 19 : low + (bin0 << 12);
+  int shift = low <= 1u ? 7 : (bin0 == (uint32_t)kBins - 1u ? 19 : 0), bits = 12;
+  uint32_t prefix = 0;
+  const bool pick = L2 != 0u;
+  if (pick) {
+#pragma unroll 1
+    for (;;) {
+      clear_hist(sm.hist);
+      __syncthreads();
+#pragma unroll 1
+      for (uint32_t p = threadIdx.x; p < L2; p += kSpThreads) {
+        const uint32_t rest = abs_key(__ldcg(list2_values(s) + p)) - start;
+        if ((rest >> shift >> bits) == prefix) atomicAdd(&sm.hist[(rest >> shift) & ((1u << bits) - 1u)], 1u);
+      }
+      __syncthreads();
+      uint32_t b;
+      find_bin(sm.hist, rem, sm.fs, b, rem);
+      prefix = (prefix << bits) | b;
+      if (shift == 0) break;
+      bits = shift == 19 ? 12 : 7;
+      shift = shift == 19 ? 7 : 0;
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t p = threadIdx.x; p < L2; p += kSpThreads) {
+    const float v = __ldcg(list2_values(s) + p);
+    const uint32_t idx = __ldcg(list2_indices(s) + p), rest = abs_key(v) - start;
+    bool send = rest > prefix;
+    if (rest == prefix) send = atomicAdd(&sm.ties, 1u) < rem;
+    if (send && idx < s.n) {
+      put_pair(dst, val_off, s.kmax, atomicAdd(&sm.sent, 1u), idx, v);
+      s.a[idx] = 0.0f;
+      if (s.u) s.u[idx] = 0.0f;
+    }
   }
   __syncthreads();
   if (threadIdx.x != 0) return false;
-  __threadfence();
-  if (atomicAdd(s.ws + kWsDone, 1u) != nx - 1) return false;
-  __threadfence();
-  const uint32_t sent = atomicAdd(s.ws + kWsOutCount, 0u);
   WireHeader h;
   h.n = s.n;
   h.alg = (uint8_t)alg;
   h.bitwidth = 0;
   h.flags = 0;
-  h.a = all < s.k ? 0.0f : __uint_as_float(thr);
-  h.b = sent < s.kmax ? sent : s.kmax;
+  h.a = every ? 0.0f : __uint_as_float(start + prefix);
+  h.b = sm.sent < s.kmax ? sm.sent : s.kmax;
 #pragma unroll 1
   for (int d = 0; d < dst.n; ++d) *reinterpret_cast<uint4*>(dst.out[d]) = *reinterpret_cast<const uint4*>(&h);
   return true;
-}
-// CTAs that share the finish of a list of L elements
-__device__ __forceinline__ uint32_t finish_slices(uint32_t L, uint32_t most) {
-  const uint32_t n = L / 256u + 1u;
-  return n < most ? n : most;
-}
-
-// The sample misled: the list lacks some of the k largest.
-__device__ __forceinline__ bool selection_failed(const SelUnit& s) {
-  const uint32_t c = __ldcg(s.ws + kWsCandCount);
-  return __ldcg(s.ws + kWsOverflow) != 0u || (c < s.k && __ldcg(s.ws + kWsLow) > 1u);
 }
 
 // out[idx] (+)= val * scale ; indices come from another rank: bounds-checked

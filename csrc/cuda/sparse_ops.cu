@@ -83,15 +83,20 @@ __global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __gr
   const uint32_t tiles = (s.n - 1) / kSelTile + 1;
   uint32_t mine = 0;   // sampled tiles of this CTA: the first two stay in shared memory
 #pragma unroll 1
-  for (uint32_t i = c; i < s.sampled; i += G, ++mine)
-    sample_body(A.mode, s, A.momentum, sm.sel, i, sm.sel.stash[mine < 2 ? mine : 1]);
+  for (uint32_t i = c; i < s.sampled; i += G, ++mine) {
+    float* stash = sm.sel.stash[mine < 1 ? 0 : 1];
+    if (A.mode == 0) sample_body<0>(s, A.momentum, sm.sel, i, stash);
+    else if (A.mode == 1) sample_body<1>(s, A.momentum, sm.sel, i, stash);
+    else sample_body<2>(s, A.momentum, sm.sel, i, stash);
+    __syncthreads();
+  }
   barrier();
   if (threadIdx.x == 0) sm.sel.count = 0;
   __syncthreads();
 #pragma unroll 1
-  for (uint32_t i = c, r = 0; r < mine; i += G, ++r)   // the second stash holds the last one sampled
+  for (uint32_t i = c, r = 0; r < mine; i += G, ++r)
     collect_sampled(s, 0, sm.sel, i, sm.sel.stash[r < 1 ? 0 : 1], r >= 1 && mine > 2);
-  auto self = [&](uint32_t) { return s; };
+  auto self = [&](uint32_t) -> const SelUnit& { return s; };
   if (s.stride > 1)
     hand_out(s.ws + kWsTicket, tiles, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
       if (A.mode == 0) collect_body<0>(s, 0, A.momentum, sm.sel, t0, t1);
@@ -104,16 +109,10 @@ __global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __gr
   EmitDst d;
   d.n = 1;
   d.out[0] = A.out;
-  if (!selection_failed(s)) {   // every CTA reads the same answer: its writers are behind the barrier
-    uint32_t L = min(__ldcg(s.ws + kWsCandCount), s.cap);
-    const bool longer = L > kFinishList;
-    if (longer) {
-      refine_body(s, d, sm.sel, c, G);
-      barrier();
-      L = min(__ldcg(s.ws + kWsCand2Count), s.cap);
-    }
-    const uint32_t nx = finish_slices(L, G);
-    if (c < nx) finish_body(A.alg, s, d, sm.sel, longer, c, nx);
+  const ListState ls = list_state(s);   // the same in every CTA: its writers are behind the barrier
+  if (!selection_failed(s, ls)) {
+    const uint32_t nx = emit_slices(ls.count, G);
+    if (c < nx) emit_slice(A.alg, s, ls, d, sm.sel, c, nx);
     return;
   }
   // whole-array passes
