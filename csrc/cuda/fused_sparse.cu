@@ -12,8 +12,8 @@
 //            sparse payloads into its accumulator (= server-side residual),
 //            re-selects the top-k of the sum and stores the result into every
 //            rank's inbox, releasing their flags.
-//   pull   : every rank zero-fills the gradient, waits for each owner's flag and
-//            scatters value / N.
+//   pull   : every rank waits for each owner's flag and scatters value / N into the
+//            result, which the update pass cleared.
 //
 // All units of a bucket are batched in every phase, which is the "bulk
 // synchronisation" of many small tensors: the update pass hands out the bucket's tiles
@@ -41,7 +41,6 @@ struct SpSeg {
   float* sr;   // server accumulator for the owned chunk [chunk]
   uint32_t n, chunk, kmax, pay_off;
   uint32_t tiles;       // tiles of one chunk
-  uint32_t tile_prefix; // tiles of one chunk of the tensors before this one
   uint32_t k_last;      // pairs of the last chunk, which may be shorter
   uint32_t stride;      // every stride-th tile is sampled (set at launch: depends on the grid)
   uint32_t cap;         // candidate pairs per (tensor, chunk) unit, for both lists
@@ -96,7 +95,7 @@ struct SpSmem {
 // control words of one rank played by a launch, behind its histogram blocks; zero
 // when the kernel starts (cleared with the histograms)
 constexpr int kCtlStamps = 8;    // low 32 bits of %globaltimer: kernel start, then after every barrier
-constexpr int kCtlTickets = 96;  // one per handed-out phase: two for a selection, cleared with the rest
+constexpr int kCtlTickets = 96;  // one per selection, cleared with the rest
 constexpr int kCtlBarrier = 128;
 constexpr int kCtlWords = kCtlBarrier + kBarrierWords;
 
@@ -150,39 +149,12 @@ __device__ __forceinline__ uint32_t slices_cap(const SpCtx& cx, uint32_t units, 
   return p > cap ? cap : p;
 }
 
-// Zero-fill of the result, tile by tile.  It runs behind the barrier of the update pass,
-// which reads the gradient (it may be the same buffer), on the CTAs that have no list to
-// finish: clearing each element right behind its load in the update pass made that
-// pass five times slower (a store to a line whose fill is still in flight).
-static __device__ __noinline__ void zero_result(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm,
-                                            int ticket) {
-  const uint32_t N = (uint32_t)cx.N;
-  hand_out(cx.ctl + kCtlTickets + ticket, bk.tiles_total * N, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
-    int si = 0, hi = bk.nseg;
-#pragma unroll 1
-    while (hi - si > 1) {
-      const int mid = (si + hi) / 2;
-      if (bk.seg[mid].tile_prefix * N <= t) si = mid;
-      else hi = mid;
-    }
-#pragma unroll 1
-    for (; t < end; ++t) {
-      while (si + 1 < bk.nseg && t >= bk.seg[si + 1].tile_prefix * N) ++si;
-      const SpSeg& sg = bk.seg[si];
-      float* out = sg.out + cx.E * cm.emu_stride_out;
-      const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-      const uint64_t i0 = (uint64_t)(t - sg.tile_prefix * N) * kTile + threadIdx.x * 4;
-#pragma unroll
-      for (int j = 0; j < kTile / (4 * kSpThreads); ++j)
-        st4(out, i0 + j * kSpThreads * 4, sg.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
-    }
-  });
-}
-
 // ------------------------------------------------------------ units of a selection
 // push : every (tensor, owner) pair, unit y = tensor * N + owner
 // serve: the owned chunk of every tensor, y = tensor
 // hop  : the chunk of every tensor that hop `hop` of the ring works on, y = tensor
+// Every element of the gradient is read by exactly one push or hop, and the update clears
+// the result behind that read (it may be the same buffer).
 // The kind is a run-time value: the two selections of a PS launch and the hops of a ring
 // run the same instructions, so all but the first find them in the instruction cache.
 enum SelKind { kSelPush, kSelServe, kSelHop };
@@ -217,7 +189,7 @@ static __device__ __noinline__ void set_units(const SpBucket& bk, const HpComm& 
     const SpSeg& sg = bk.seg[si];
     SelUnit& s = sm.unit[y];
     const size_t E = (size_t)cx.E, off = (size_t)c * sg.chunk;
-    const uint32_t n = sp_chunk_valid(sg.n, sg.chunk, c), tiles = (n + kTile - 1) / kTile;
+    const uint32_t n = sp_chunk_valid(sg.n, sg.chunk, c), tiles = (n + kSpTile - 1) / kSpTile;
     s.n = n;
     s.k = n == sg.chunk ? sg.kmax : sg.k_last;   // only the last chunk is shorter
     s.kmax = sg.kmax;
@@ -228,12 +200,14 @@ static __device__ __noinline__ void set_units(const SpBucket& bk, const HpComm& 
     uint32_t block = (uint32_t)(bk.nseg * cx.N) + y;
     s.g = nullptr;
     s.u = nullptr;
+    s.clear = nullptr;
     if (ph.kind == kSelServe) {
       s.a = sg.sr + E * cm.emu_stride_sr;
     } else {
       s.g = sg.g + E * cm.emu_stride_g + off;
       s.a = sg.a + E * cm.emu_stride_r + off;
       if (sg.u) s.u = sg.u + E * cm.emu_stride_r + off;
+      s.clear = sg.out + E * cm.emu_stride_out + off;
       list = sg.cand_push + (uint64_t)c * sg.cap;
       block = ph.kind == kSelPush ? y : (uint32_t)(ph.hop * bk.nseg + si);
     }
@@ -280,37 +254,48 @@ __device__ __forceinline__ uint32_t unit_at(const uint32_t* at, uint32_t units, 
   return lo;
 }
 
-// where a unit's pairs go, and the flags that announce them: into sm.dst (whole CTA)
+// Where a unit's pairs go, and the flags that announce them: into sm.dst (whole CTA).
+// What stays on this rank does not pass through its inbox: the push of the own chunk is
+// added to the owner's accumulator, and a final chunk goes into the result.
 __device__ __forceinline__ void unit_dst(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, const SelPhase& ph,
                                          uint32_t y, SpSmem& sm) {
   const int N = cx.N, R = cx.R, q = (int)threadIdx.x;
   int si, c;
   unit_ref(cx, ph, y, si, c);
-  const bool all = ph.kind == kSelServe || (ph.kind == kSelHop && ph.hop == N - 1);
-  const int slot = ph.kind == kSelPush ? R : (ph.kind == kSelServe ? N + R : (all ? N - 1 + R : ph.hop));
-  const int n = all ? N : 1;
+  const SpSeg& sg = bk.seg[si];
+  const bool final_chunk = ph.kind == kSelServe || (ph.kind == kSelHop && ph.hop == N - 1);
+  const bool own_push = ph.kind == kSelPush && c == R;
+  const int slot = ph.kind == kSelPush ? R : (ph.kind == kSelServe ? N + R : (final_chunk ? N - 1 + R : ph.hop));
+  const int n = final_chunk ? N - 1 : (own_push ? 0 : 1);
   __syncthreads();
-  if (q == 0) sm.dst.out.n = n;
+  if (q == 0) {
+    sm.dst.out.n = n;
+    sm.dst.out.add = own_push ? sg.sr + cx.E * cm.emu_stride_sr : nullptr;
+    // a CTA that has given up leaves the result alone
+    sm.dst.out.set = final_chunk && !*(volatile int*)&sm.wst.poisoned ? sg.out + cx.E * cm.emu_stride_out + (size_t)c * sg.chunk : nullptr;
+    sm.dst.out.scale = bk.inv_n;
+  }
   if (q < n) {
-    int to = (ph.kind == kSelPush ? c : (all ? R : R + 1)) + q;
+    int to = (ph.kind == kSelPush ? c : R + 1) + q;
     if (to >= N) to -= N;
-    sm.dst.out.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[to]) + (size_t)slot * bk.slot_bytes + bk.seg[si].pay_off;
+    sm.dst.out.out[q] = reinterpret_cast<uint8_t*>(cm.inbox[to]) + (size_t)slot * bk.slot_bytes + sg.pay_off;
     sm.dst.flag[q] = reinterpret_cast<uint32_t*>(cm.flags[to]) + (size_t)slot * bk.nseg + si;
   }
   __syncthreads();
 }
 // thread 0 of the CTA that completed the unit
 __device__ __forceinline__ void unit_release(const HpComm& cm, const SpSmem& sm) {
+  if (sm.dst.out.n == 0) return;
   __threadfence_system();
   const uint32_t v = flag_value(cm, sm);
 #pragma unroll 1
   for (int q = 0; q < sm.dst.out.n; ++q) st_release_sys(sm.dst.flag[q], v);
 }
 
-// The selection of all units of one kind: two barriers (more only when a sample misled).
-// Tickets `ticket` and, when the result is to be cleared behind the update pass, ticket + 1.
+// The selection of all units of one kind, the ticket-th of the launch: two barriers (more
+// only when a sample misled).
 static __device__ __noinline__ void select_units(const SpBucket& bk, const HpComm& cm, SpCtx& cx, SpSmem& sm, int kind,
-                                                 int hop, int ticket, bool zero) {
+                                                 int hop, int ticket) {
   SelPhase ph;
   ph.kind = kind;
   ph.hop = hop;
@@ -339,7 +324,7 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
     collect_sampled(sm.unit[y], y, sm.sel, i - sm.sample_at[y], sm.sel.stash[r < 1 ? 0 : 1], r >= 1 && mine > 2);
   }
   auto unit = [&](uint32_t y) -> const SelUnit& { return sm.unit[y]; };
-  hand_out(cx.ctl + kCtlTickets + ticket, sm.tile_at[units], cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
+  hand_out(cx.ctl + kCtlTickets + ticket, sm.tile_at[units], blockIdx.x, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
     uint32_t y = unit_at(sm.tile_at, units, t);
 #pragma unroll 1
     for (; t < end; ++y) {
@@ -381,9 +366,7 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
     }
     if (done) unit_release(cm, sm);
   });
-  sp_mark(cx, kind == kSelServe ? 2 : 0);
-  if (zero) zero_result(bk, cm, cx, sm, ticket + 1);
-  sp_mark(cx, kind == kSelServe ? 3 : 1);
+  sp_mark(cx, ticket);
   if (!failed) return;
   // whole-array passes for the units whose sample misled: clear the histograms, count the
   // three digits, send
@@ -409,7 +392,7 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
 }
 
 // ---------------------------------------------------------------- incoming payloads
-// PS owner: wait for the N pushes of tensor si and add them into the accumulator
+// PS owner: wait for the other ranks' pushes of tensor si and add them into the accumulator
 __device__ __forceinline__ void serve_in(const SpBucket& bk, const HpComm& cm, const SpCtx& cx, SpSmem& sm, int si,
                                          uint32_t x, uint32_t nx) {
   const int N = cx.N, R = cx.R;
@@ -417,13 +400,15 @@ __device__ __forceinline__ void serve_in(const SpBucket& bk, const HpComm& cm, c
   const uint32_t len = sp_chunk_valid(sg.n, sg.chunk, R);
   const uint32_t* my_flags = reinterpret_cast<const uint32_t*>(cm.flags[R]);
   for (int q = 0; q < N; ++q)
-    wait_flag(my_flags + (size_t)q * bk.nseg + si, cm.epoch, cm.timeout_ns, cx.status,
-              HP_STATUS_TIMEOUT | (4u << 16) | ((uint32_t)q << 8) | (si & 255), sm.wst);
+    if (q != R)
+      wait_flag(my_flags + (size_t)q * bk.nseg + si, cm.epoch, cm.timeout_ns, cx.status,
+                HP_STATUS_TIMEOUT | (4u << 16) | ((uint32_t)q << 8) | (si & 255), sm.wst);
   if (len == 0) return;
   const uint8_t* inbox = reinterpret_cast<const uint8_t*>(cm.inbox[R]);
   for (int q = 0; q < N; ++q)
-    scatter_body(inbox + (size_t)q * bk.slot_bytes + sg.pay_off, sg.sr + cx.E * cm.emu_stride_sr, len, sg.kmax, 1.0f,
-                 2, x, nx);
+    if (q != R)
+      scatter_body(inbox + (size_t)q * bk.slot_bytes + sg.pay_off, sg.sr + cx.E * cm.emu_stride_sr, len, sg.kmax,
+                   1.0f, 2, x, nx);
 }
 
 // ring: wait for the predecessor's pairs of tensor si and add them into the accumulator
@@ -494,33 +479,34 @@ __device__ __forceinline__ void sp_epilogue(const SpCtx& cx) {
 }
 
 // PS: push (every rank selects per owner and stores the pairs into the owner's inbox),
-// serve (the owner adds the N payloads, re-selects, stores the result into every
-// inbox), pull (every rank scatters value / N).  Five barriers when the candidate lists
-// are short.  @PS_NOTE@
-__global__ void __launch_bounds__(kSpThreads, 3)
+// serve (the owner adds the payloads, re-selects, stores the result into every inbox),
+// pull (every rank scatters value / N).  Five barriers.
+__global__ void __launch_bounds__(kSpThreads, 1)
 sp_ps_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm cm, const __grid_constant__ SpLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
   SpCtx cx;
   sp_prologue(cm, L, cx, sm);
   const int N = cx.N;
-  const uint32_t nseg = (uint32_t)bk.nseg, units = nseg * (uint32_t)N;
-  select_units(bk, cm, cx, sm, kSelPush, 0, 0, true);
-  run_units(cx, nseg, slices_cap(cx, nseg, 32),
-            [&](int y, uint32_t x, uint32_t nx) { serve_in(bk, cm, cx, sm, y, x, nx); });
+  const uint32_t nseg = (uint32_t)bk.nseg, units = nseg * (uint32_t)(N - 1);
+  select_units(bk, cm, cx, sm, kSelPush, 0, 0);
+  if (N > 1)
+    run_units(cx, nseg, slices_cap(cx, nseg, 32),
+              [&](int y, uint32_t x, uint32_t nx) { serve_in(bk, cm, cx, sm, y, x, nx); });
   sp_barrier(cm, cx, sm);
-  select_units(bk, cm, cx, sm, kSelServe, 0, 2, false);
-  run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
-    const int j = y % N;
-    gather_stage(bk, cm, cx, sm, y / N, N + j, j, 5u, x, nx);
-  });
+  select_units(bk, cm, cx, sm, kSelServe, 0, 1);
+  if (N > 1)
+    run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
+      const int j = (cx.R + 1 + y % (N - 1)) % N;
+      gather_stage(bk, cm, cx, sm, y / (N - 1), N + j, j, 5u, x, nx);
+    });
   sp_epilogue(cx);
 }
 
 // Ring: N hops of (add the predecessor's pairs, update and select, store into the
 // successor's inbox), the last hop storing into every inbox; then every rank scatters
-// the N reduced chunks.  Three barriers per hop when the candidate lists are short.
-__global__ void __launch_bounds__(kSpThreads, 3)
+// the reduced chunks of the others.  Three barriers per hop.
+__global__ void __launch_bounds__(kSpThreads, 1)
 sp_ring_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm cm, const __grid_constant__ SpLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
@@ -528,22 +514,22 @@ sp_ring_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpCo
   sp_prologue(cm, L, cx, sm);
   const int N = cx.N;
   const uint32_t nseg = (uint32_t)bk.nseg;
+#pragma unroll 1
   for (int hop = 0; hop < N; ++hop) {
     if (hop > 0) {
       run_units(cx, nseg, slices_cap(cx, nseg, 32),
                 [&](int y, uint32_t x, uint32_t nx) { hop_in(bk, cm, cx, sm, hop, y, x, nx); });
       sp_barrier(cm, cx, sm);
     }
-    // the last hop has read every chunk of the gradient when its update pass is done
-    select_units(bk, cm, cx, sm, kSelHop, hop, 2 * hop, hop == N - 1);
+    select_units(bk, cm, cx, sm, kSelHop, hop, hop);
   }
-  // gather: rank src finalised chunk src + 1 (every CTA has cleared its share of the result)
-  sp_barrier(cm, cx, sm);
-  const uint32_t units = nseg * (uint32_t)N;
-  run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
-    const int src = y % N;
-    gather_stage(bk, cm, cx, sm, y / N, N - 1 + src, (src + 1) % N, 7u, x, nx);
-  });
+  // gather: rank src finalised chunk src + 1
+  const uint32_t units = nseg * (uint32_t)(N - 1);
+  if (N > 1)
+    run_units(cx, units, slices_cap(cx, units, 16), [&](int y, uint32_t x, uint32_t nx) {
+      const int src = (cx.R + 1 + y % (N - 1)) % N;
+      gather_stage(bk, cm, cx, sm, y / (N - 1), N - 1 + src, (src + 1) % N, 7u, x, nx);
+    });
   sp_epilogue(cx);
 }
 
@@ -567,8 +553,7 @@ static int build_sp_bucket(int alg, float ratio, float momentum, const HpSeg* se
     d.kmax = (uint32_t)sparse_k(chunk, ratio);
     d.k_last = (uint32_t)sparse_k(n % chunk, ratio);
     d.pay_off = (uint32_t)pay;
-    d.tiles = (uint32_t)(chunk / kTile);
-    d.tile_prefix = (uint32_t)tiles;
+    d.tiles = (uint32_t)((chunk + kSpTile - 1) / kSpTile);
     tiles += d.tiles;
     d.cap = (uint32_t)align_up(8ull * d.kmax + 4096, 32);
     d.cand_push = cand;
@@ -618,12 +603,12 @@ static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int
   }
   const int ranks_here = cm.emulate ? N : 1;
   int G = ctas;
-  if (G <= 0) {   // a CTA per tile of the bucket, at least 8, at most what the GPU holds
+  if (G <= 0) {   // a CTA per tile of the bucket
     const uint64_t tiles = (uint64_t)bk.tiles_total * N;
-    G = tiles < 8 ? 8 : (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
-    if (G > cap / ranks_here) G = cap / ranks_here;
+    G = (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
   }
-  if (G < 1 || (long long)G * ranks_here > (long long)cap) return HP_ERR_RESIDENCY;
+  if (G > cap / ranks_here) G = cap / ranks_here;   // what the GPU holds at once
+  if (G < 1) return HP_ERR_RESIDENCY;
   for (int i = 0; i < nseg; ++i)  // a sampled tile for every CTA, over the units of a push or of a hop
     bk.seg[i].stride =
         sample_stride(bk.seg[i].tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);

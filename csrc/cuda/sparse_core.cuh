@@ -12,7 +12,12 @@
 
 namespace hipress {
 
-constexpr int kSpThreads = 256;
+// One CTA of 512 threads per SM in the grid-wide kernels: every CTA arrives at the same
+// barrier counter, adds to the same histograms and reserves room in the same lists, and
+// such an access to one address takes 10 to 25 ns of its own, so 444 CTAs of 256 threads
+// spent 4.5 us per barrier and 11 us on the sample histogram of one tensor.
+constexpr int kSpThreads = 512;
+constexpr uint32_t kSpTile = 16 * kSpThreads;   // elements per tile: 16 per thread
 constexpr int kBins = 4096;
 // workspace words: 3 histograms, then counters
 constexpr int kWsOutCount = 3 * kBins + 0;
@@ -183,16 +188,16 @@ static __device__ __noinline__ void pass_body_rt(int PASS, const float* __restri
   const uint32_t prefix = PASS == 1 ? bin0 : ((bin0 << 11) | bin1);
   const int shift = PASS == 1 ? 19 : 8;
   const bool vec = (reinterpret_cast<uintptr_t>(a) & 15) == 0;
-  // 4096-element tiles, four independent 16-byte loads per thread in flight
-  const uint64_t tiles = (n + 4095) / 4096;
+  // four independent 16-byte loads per thread in flight
+  const uint64_t tiles = (n + kSpTile - 1) / kSpTile;
   for (uint64_t t = cta; t < tiles; t += nctas) {
     float4 av[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      av[j] = ld4(a, t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4, n, vec);
+      av[j] = ld4(a, t * kSpTile + (uint64_t)(j * kSpThreads + threadIdx.x) * 4, n, vec);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint64_t i = t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
+      const uint64_t i = t * kSpTile + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
       const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -218,14 +223,30 @@ struct EmitSmem {
   uint32_t tot;
 };
 
-// where the pairs go: one payload per destination (several for a broadcast);
-// destinations may be peer GPUs' memory
+// Where the pairs go: one payload per destination (several for a broadcast), which may be
+// peer GPUs' memory, and on this GPU straight into an accumulator (`add`) or into the
+// cleared result (`set`, scaled), with no payload in between.
 struct EmitDst {
   uint8_t* out[HP_MAX_RANKS];
   int n;
+  float* add;
+  float* set;
+  float scale;
 };
+// store one pair at place `pos` of every destination
+__device__ __forceinline__ void put_pair(const EmitDst& dst, size_t val_off, uint32_t kmax, uint32_t pos,
+                                         uint32_t idx, float val) {
+  if (pos >= kmax) return;
+#pragma unroll 1
+  for (int d = 0; d < dst.n; ++d) {
+    reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = idx;
+    reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = val;
+  }
+  if (dst.add) atomicAdd(dst.add + idx, val);
+  if (dst.set) dst.set[idx] = val * dst.scale;
+}
 
-// Compaction of the whole array.  Tile = 4096 elements per CTA iteration, 16 per thread.
+// Compaction of the whole array, a tile per CTA iteration, 16 elements per thread.
 // Returns true in thread 0 of the CTA that finished last, after it wrote the headers.
 static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, float* __restrict__ u,
                                           uint64_t n, uint32_t k, uint32_t kmax, const EmitDst& dst,
@@ -241,7 +262,7 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
   const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(u)) & 15) == 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-  const uint64_t tiles = (n + 4095) / 4096;
+  const uint64_t tiles = (n + kSpTile - 1) / kSpTile;
   for (uint64_t t = cta; t < tiles; t += nctas) {
     // The loops over a thread's 16 elements stay rolled (and the second one loads the
     // values again, from cache) on purpose: this body runs once or a few times per
@@ -251,7 +272,7 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
     uint32_t cnt = 0;   // low 16: greater, high 16: equal
 #pragma unroll 1
     for (int j = 0; j < 4; ++j) {
-      const uint64_t i = t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
+      const uint64_t i = t * kSpTile + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
       const float4 av = ld4(a, i, n, vec);
       const float e4[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
@@ -302,7 +323,7 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
     for (int j = 0; j < 4; ++j) {
       const uint32_t fj = (flag >> (8 * j)) & 255u;
       if (fj == 0) continue;
-      const uint64_t i = t * 4096 + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
+      const uint64_t i = t * kSpTile + (uint64_t)(j * kSpThreads + threadIdx.x) * 4;
       const float4 av = ld4(a, i, n, vec);
       const float e4[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
@@ -315,10 +336,7 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
           ++rank_eq;
         }
         if (pos < kmax) {
-          for (int d = 0; d < dst.n; ++d) {
-            reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = (uint32_t)(i + q);
-            reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = e4[q];
-          }
+          put_pair(dst, val_off, kmax, pos, (uint32_t)(i + q), e4[q]);
           a[i + q] = 0.0f;
           if (u) u[i + q] = 0.0f;
         }
@@ -380,13 +398,14 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 // resolve; counters that are read together lie together; and slices send without a
 // barrier behind the histogram.
 constexpr uint32_t kMinSampled = 4;     // tiles of an array that are sampled at least
-constexpr uint32_t kSelTile = 4096;     // elements per tile: 16 per thread
+constexpr uint32_t kMaxSampled = 64;    // and at most: 0.5 M elements
 
 // One array to select from.
 struct SelUnit {
   const float* g;
   float* a;
   float* u;
+  float* clear;    // result that the update clears behind its reads (it may be g), or null
   uint32_t* ws;
   float* cv;       // candidate list: `cap` values, then `cap` indices; a second list of the
                    // same size behind it
@@ -405,6 +424,7 @@ HP_HD uint32_t list_cap(uint64_t pairs) { return (uint32_t)(pairs / 2 < 0x7FFFFF
 HP_HD uint32_t sample_stride(uint32_t tiles, uint64_t total, uint32_t ctas) {
   uint64_t share = ((uint64_t)tiles * ctas) / (total ? total : 1);
   if (share < kMinSampled) share = kMinSampled;
+  if (share > kMaxSampled) share = kMaxSampled;
   return share >= tiles ? 1u : (uint32_t)((tiles + share - 1) / share);
 }
 
@@ -440,7 +460,7 @@ struct SelSmem {
       uint16_t unit[kCollectBuf];
     } buf;                           // collect
   };
-  float stash[2][kSelTile];          // sample to collect
+  float stash[2][kSpTile];          // sample to collect
   FindSmem fs;
   uint32_t count, base, base2, ticket, flag;
   uint32_t sent, ties;
@@ -458,7 +478,7 @@ template <int MODE>
 __device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[4]) {
   const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
                      (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
-  const uint64_t i0 = (uint64_t)t * kSelTile + threadIdx.x * 4;
+  const uint64_t i0 = (uint64_t)t * kSpTile + threadIdx.x * 4;
   float4 gv[4], uv[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -484,6 +504,11 @@ __device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, ui
       st4(s.u, i, s.n, vec, w);
       st4(s.a, i, s.n, vec, v);
     }
+  }
+  if (MODE >= 1 && s.clear) {
+    const bool cvec = (reinterpret_cast<uintptr_t>(s.clear) & 15) == 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) st4(s.clear, i0 + j * kSpThreads * 4, s.n, cvec, make_float4(0.f, 0.f, 0.f, 0.f));
   }
 }
 
@@ -521,7 +546,7 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
   if (s.stride > 1) {
     // k scaled to the sample, plus five standard deviations, plus a tenth because
     // neighbouring elements are not independent
-    const float hits = __fdividef((float)s.k * (float)(s.sampled * kSelTile), (float)s.n);
+    const float hits = __fdividef((float)s.k * (float)(s.sampled * kSpTile), (float)s.n);
     float dev;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(dev) : "f"(hits));
     rank = (uint32_t)(1.1f * hits + 5.0f * dev + 4.0f);
@@ -531,15 +556,18 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
   if (threadIdx.x == 0) s.ws[kWsLow] = bin ? bin << 19 : 1u;   // zeros are never sent
 }
 
-// Items [0, total) in stretches, taken from *word by whichever of the ctas CTAs is free:
-// SMs do not run at one speed, and equal shares leave the fast ones waiting.  The next
-// stretch is asked for before the current one is worked on, by predicated instructions
-// (an `if` around them split thread 0 from its warp, and the two halves then counted
-// twice at the barriers that follow).  f(lo, hi) runs with the whole CTA; `slot` is
-// shared memory.
+// Items [0, total): three quarters in equal shares, the rest in short stretches taken from
+// *word by whichever of the ctas CTAs is free -- SMs do not run at one speed, and equal
+// shares alone leave the fast ones waiting, while handing out everything made the ticket
+// word the bottleneck.  The next stretch is asked for before the current one is worked
+// on, by predicated instructions (an `if` around them split thread 0 from its warp, and
+// the two halves then counted twice at the barriers that follow).  f(lo, hi) runs with
+// the whole CTA; `slot` is shared memory.
 template <typename F>
-__device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t ctas, uint32_t& slot, F f) {
-  const uint32_t stretch = total / (4u * ctas) + 1u;
+__device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t cta, uint32_t ctas, uint32_t& slot,
+                                         F f) {
+  const uint32_t share = total / ctas * 3u / 4u, dealt = share * ctas;
+  const uint32_t stretch = (total - dealt) / (4u * ctas) + 1u;
   const uint32_t at = (uint32_t)__cvta_generic_to_shared(&slot);
   uint32_t next = 0;
   auto take = [&] {
@@ -547,16 +575,18 @@ __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_
                  : "+r"(next) : "r"(threadIdx.x), "l"(word), "r"(stretch) : "memory");
   };
   take();
+  uint32_t lo = cta * share, hi = lo + share;
 #pragma unroll 1
   for (;;) {
+    if (lo < hi) f(lo, hi);
     asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %1, 0;\n@p st.shared.u32 [%2], %0;\n}" ::"r"(next),
                  "r"(threadIdx.x), "r"(at) : "memory");
     __syncthreads();
-    const uint32_t lo = *(volatile uint32_t*)&slot;
+    lo = dealt + *(volatile uint32_t*)&slot;
     __syncthreads();
     if (lo >= total) break;
+    hi = min(lo + stretch, total);
     take();
-    f(lo, min(lo + stretch, total));
   }
 }
 
@@ -587,7 +617,7 @@ __device__ __forceinline__ void collect_tile(const SelUnit& s, uint32_t uid, Sel
     const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
     const uint32_t most = max(max(abs_key(e[0]), abs_key(e[1])), max(abs_key(e[2]), abs_key(e[3])));
     if (most < low) continue;
-    const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
+    const uint32_t i = t * kSpTile + (j * kSpThreads + threadIdx.x) * 4;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (abs_key(e[q]) >= low) collect_one(s, uid, sm, low, e[q], i + q);
@@ -642,6 +672,31 @@ template <typename F>
 __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
   __syncthreads();
   const uint32_t n = min(sm.count, (uint32_t)kCollectBuf);
+  bool same = true;
+#pragma unroll
+  for (uint32_t p = threadIdx.x; p < (uint32_t)kCollectBuf; p += kSpThreads) same &= p >= n || sm.buf.unit[p] == sm.buf.unit[0];
+  if (__syncthreads_and(same)) {   // one reservation for the CTA
+    if (threadIdx.x == 0 && n) sm.base = atomicAdd(unit(sm.buf.unit[0]).ws + kWsCandCount, n);
+    const SelUnit& s = unit(n ? sm.buf.unit[0] : 0u);
+    const uint32_t low = n ? __ldcg(s.ws + kWsLow) : 0u;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t p = threadIdx.x; p < n; p += kSpThreads) {
+      const float v = sm.buf.val[p];
+      const uint32_t pos = sm.base + p;
+      atomicAdd(s.ws + kBins + cand_digit(abs_key(v), low), 1u);
+      if (pos < s.cap) {
+        s.cv[pos] = v;
+        list_indices(s)[pos] = sm.buf.idx[p];
+      } else {
+        s.ws[kWsOverflow] = 1u;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sm.count = 0;
+    __syncthreads();
+    return;
+  }
 #pragma unroll 1
   for (uint32_t p0 = 0; p0 < n; p0 += kSpThreads) {
     const uint32_t p = p0 + threadIdx.x;
@@ -669,17 +724,6 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
   __syncthreads();
   if (threadIdx.x == 0) sm.count = 0;
   __syncthreads();
-}
-
-// store one pair at place `pos` of every destination's payload
-__device__ __forceinline__ void put_pair(const EmitDst& dst, size_t val_off, uint32_t kmax, uint32_t pos,
-                                         uint32_t idx, float val) {
-  if (pos >= kmax) return;
-#pragma unroll 1
-  for (int d = 0; d < dst.n; ++d) {
-    reinterpret_cast<uint32_t*>(dst.out[d] + 16)[pos] = idx;
-    reinterpret_cast<float*>(dst.out[d] + val_off)[pos] = val;
-  }
 }
 
 // CTAs that share a list of L elements

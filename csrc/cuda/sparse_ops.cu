@@ -48,7 +48,7 @@ sparse_emit_kernel(int alg, float* __restrict__ a, float* __restrict__ u, uint64
                    uint32_t kmax, uint8_t* __restrict__ out, uint32_t* __restrict__ ws) {
   __shared__ FindSmem fs;
   __shared__ EmitSmem es;
-  EmitDst d;
+  EmitDst d = {};
   d.n = 1;
   d.out[0] = out;
   emit_body(alg, a, u, n, k, kmax, d, ws, fs, es, blockIdx.x, gridDim.x);
@@ -68,7 +68,7 @@ union SelOrPassSmem {
   EmitSmem emit;
 };
 
-__global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __grid_constant__ SelArgs A) {
+__global__ void __launch_bounds__(kSpThreads, 1) sparse_encode_kernel(const __grid_constant__ SelArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SelOrPassSmem& sm = *reinterpret_cast<SelOrPassSmem*>(smem_raw);
   __shared__ WaitState wst;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __gr
   auto barrier = [&]() {
     grid_barrier(s.ws + kWsWords, gen, G, kGridBarrierNs, s.ws + kWsStatus, 1u, wst);
   };
-  const uint32_t tiles = (s.n - 1) / kSelTile + 1;
+  const uint32_t tiles = (s.n - 1) / kSpTile + 1;
   uint32_t mine = 0;   // sampled tiles of this CTA: the first two stay in shared memory
 #pragma unroll 1
   for (uint32_t i = c; i < s.sampled; i += G, ++mine) {
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __gr
     collect_sampled(s, 0, sm.sel, i, sm.sel.stash[r < 1 ? 0 : 1], r >= 1 && mine > 2);
   auto self = [&](uint32_t) -> const SelUnit& { return s; };
   if (s.stride > 1)
-    hand_out(s.ws + kWsTicket, tiles, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
+    hand_out(s.ws + kWsTicket, tiles, c, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
       if (A.mode == 0) collect_body<0>(s, 0, A.momentum, sm.sel, t0, t1);
       else if (A.mode == 1) collect_body<1>(s, 0, A.momentum, sm.sel, t0, t1);
       else collect_body<2>(s, 0, A.momentum, sm.sel, t0, t1);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kSpThreads, 3) sparse_encode_kernel(const __gr
     });
   collect_flush(sm.sel, self);
   barrier();
-  EmitDst d;
+  EmitDst d = {};
   d.n = 1;
   d.out[0] = A.out;
   const ListState ls = list_state(s);   // the same in every CTA: its writers are behind the barrier
@@ -187,7 +187,7 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
   if (reinterpret_cast<uintptr_t>(out) & 15) return HP_ERR_BAD_ARG;
   if (update && !g) return HP_ERR_BAD_ARG;
   if (update && alg == kDgc && !u) return HP_ERR_BAD_ARG;
-  const uint64_t tiles = (n + 4095) / 4096;
+  const uint64_t tiles = (n + kSpTile - 1) / kSpTile;
   float* uu = alg == kDgc ? u : nullptr;
   const int mode = !update ? 0 : (alg == kGradDrop ? 1 : 2);
   // histograms and counters, then the barrier words and the candidate lists
@@ -221,6 +221,7 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
     U.g = g;
     U.a = a;
     U.u = uu;
+    U.clear = nullptr;
     U.ws = ws;
     U.cv = reinterpret_cast<float*>(ws + kWsWords + kBarrierWords);
     U.n = (uint32_t)n;
