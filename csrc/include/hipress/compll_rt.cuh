@@ -51,6 +51,11 @@ COMPLL_FN float compll_rand01(uint64_t seed, uint64_t elem, uint32_t site) {
 
 #if defined(__CUDACC__)
 // ---- support of the fused (one launch per function) target --------------------
+// a bit width known when the code is compiled
+template <uint32_t W>
+struct CompllWidth {
+  __device__ constexpr operator uint32_t() const { return W; }
+};
 // four consecutive floats starting at element i0 (a multiple of 4) of a vector of n
 __device__ __forceinline__ void compll_load4(const float* p, uint64_t i0, uint64_t n, float (&v)[4]) {
   if (i0 + 3 < n && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
@@ -94,6 +99,9 @@ __device__ __forceinline__ uint32_t compll_load_frag(const uint8_t* v, uint64_t 
   uint32_t w;
   if (width == 32 && off + 4 <= nbytes && (reinterpret_cast<uintptr_t>(v + off) & 3) == 0) {
     w = *reinterpret_cast<const uint32_t*>(v + off);
+  } else if (width >= 16 && off + width / 8 <= nbytes && (reinterpret_cast<uintptr_t>(v + off) & 1) == 0) {
+    w = *reinterpret_cast<const uint16_t*>(v + off);
+    if (width == 32) w |= (uint32_t)*reinterpret_cast<const uint16_t*>(v + off + 2) << 16;
   } else {
     const uint32_t nb = width <= 8 ? 1u : width / 8u;
     w = 0u;
@@ -109,6 +117,19 @@ __device__ __forceinline__ uint32_t compll_load_frag(const uint8_t* v, uint64_t 
 // `dst` is the vector's first byte, `nbytes` its length: nothing past it is written.
 __device__ __forceinline__ void compll_pack_store(uint8_t* dst, uint64_t nbytes, uint64_t q,
                                                   uint32_t frag, uint32_t bits) {
+  if ((reinterpret_cast<uintptr_t>(dst) & 3) != 0 && bits >= 2) {
+    // behind a header of an odd length: every lane stores its own one, two or four bytes
+    const uint64_t off = q * bits / 2;
+    const uint32_t nb = bits / 2;
+    uint8_t* p = dst + off;
+    if (nb >= 2 && (reinterpret_cast<uintptr_t>(p) & 1) == 0 && off + nb <= nbytes) {
+      *reinterpret_cast<uint16_t*>(p) = (uint16_t)frag;
+      if (nb == 4) *reinterpret_cast<uint16_t*>(p + 2) = (uint16_t)(frag >> 16);
+    } else {
+      for (uint32_t b = 0; b < nb && off + b < nbytes; ++b) p[b] = (uint8_t)(frag >> (8 * b));
+    }
+    return;
+  }
   const uint32_t lanes = 8u / bits;            // lanes per 32-bit word: 8, 4, 2, 1
   uint32_t w = frag;
   for (uint32_t s = 1, sh = 4u * bits; s < lanes; s <<= 1, sh <<= 1) {
@@ -126,26 +147,32 @@ __device__ __forceinline__ void compll_pack_store(uint8_t* dst, uint64_t nbytes,
   }
 }
 
-// Barrier over the blocks of a cooperative launch.  `word` counts arrivals (zero when
-// the kernel starts), `gen` is the caller's running barrier number.  Bounded: after
+// Barrier over the blocks of a cooperative launch.  `word` counts arrivals, word[32] is
+// the number of the last complete barrier (both zero when the kernel starts), `gen` is
+// the caller's running barrier number.  Bounded: after
 // about a second of polling a block gives up, raises `*err` and goes on.
 __device__ __forceinline__ void compll_grid_sync(unsigned int* word, unsigned int& gen,
                                                  unsigned int* err) {
   __syncthreads();
   ++gen;
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(word, 1u);
-    const unsigned int target = gen * gridDim.x;
-    volatile unsigned int* vw = word;
-    unsigned long long spins = 0;
-    while (*vw < target) {
-      if (++spins > (1ull << 26)) {
-        *err = 1u;
-        break;
+    unsigned int before, v;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(word) : "memory");
+    unsigned int* flag = word + 32;   // polled apart from the word everybody adds to
+    if (before == gen * gridDim.x - 1) {
+      __threadfence();
+      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(gen) : "memory");
+    } else {
+      unsigned long long spins = 0;
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+        if (v >= gen) break;
+        if (++spins > (1ull << 23)) {
+          *err = 1u;
+          break;
+        }
       }
     }
-    __threadfence();
   }
   __syncthreads();
 }

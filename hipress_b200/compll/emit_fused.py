@@ -344,12 +344,8 @@ class FusedGen:
             em._return_to = None
         # U groups of four elements per thread and trip, every load of a trip issued before
         # the first result is computed (a map only reads its own elements of the vectors
-        # it also writes, so hoisting the loads over the stores is safe).  Measured at
-        # 256 MB: a phase whose only inputs are packed fragments (the decodes, bound by
-        # their stores) gains from four groups in flight (TbqDecode 0.075 -> 0.061 ms,
-        # OnebitDecode 0.069 -> 0.057 ms); a phase that also streams a float vector in
-        # (decode-accumulate, the encoders) lost up to 25 % and keeps one.
-        U = 4 if not need_in else 1
+        # it also writes, so hoisting the loads over the stores is safe).
+        U = 4 if not need_in else (4 if not stores else 2)
         larr = [f"      {C_TYPES[em.syms[v].type.name]} in_{v}[{U}][4];" for v in need_in] + \
                [f"      uint32_t fr_{v}[{U}];" for v in need_frag]
         loads = [f"        compll_load4(c.v_{v}, i0, count, in_{v}[u]);" for v in need_in]
@@ -371,12 +367,7 @@ class FusedGen:
                                 f"(p_{tname}) + {off}, c.v_{fname});")
             if rows:
                 header = "    if (blockIdx.x == 0 && threadIdx.x == 0) {\n" + nl.join(rows) + "\n    }\n"
-        out = f"""  {{  // ---- phase {pi}: {', '.join((it.target if it.kind == 'map' else 'reduce ' + it.sym.name) for it in ph.items)}
-{header}    const uint64_t count = {ph.count};
-    const uint64_t groups = (count + 3) / 4;
-{nl.join(acc_init)}
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t qb0 = (uint64_t)blockIdx.x * blockDim.x; qb0 < groups; qb0 += stride * {U}) {{
+        main = f"""    for (uint64_t qb0 = (uint64_t)blockIdx.x * blockDim.x; qb0 < groups; qb0 += stride * {U}) {{
 {nl.join(larr)}
 #pragma unroll
       for (int u = 0; u < {U}; ++u) {{   // past the end the loads return zeros and touch nothing
@@ -391,20 +382,50 @@ class FusedGen:
       if (qb >= groups) break;
       const uint64_t q = qb + threadIdx.x;
       const uint64_t i0 = q * 4;
+      const bool full = i0 + 3 < count;   // one test for the four elements of nearly every group
+      (void)full;
 {nl.join(rngs)}
 {nl.join(decls)}
 #pragma unroll
       for (int e = 0; e < 4; ++e) {{
         const uint64_t i = i0 + e;
-        if (i >= count) continue;
+        if (!full && i >= count) continue;
 {nl.join(body)}
       }}
 {nl.join(stores)}
       }}
     }}
-{self._block_reduce(reds)}  }}
+"""
+        main = self._per_width(main, need_frag, ph)
+        out = f"""  {{  // ---- phase {pi}: {', '.join((it.target if it.kind == 'map' else 'reduce ' + it.sym.name) for it in ph.items)}
+{header}    const uint64_t count = {ph.count};
+    const uint64_t groups = (count + 3) / 4;
+{nl.join(acc_init)}
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+{main}{self._block_reduce(reds)}  }}
 """
         return out
+
+    def _per_width(self, main: str, need_frag, ph: Phase) -> str:
+        """A width that is a scalar of the function (a parameter, a header field) makes every
+        shift and mask of the packing a run-time one: the loop is compiled for the widths
+        1, 2, 4 and 8 as well, and the kernel takes the one that applies."""
+        em = self.em
+        names = set()
+        for v in list(need_frag) + [it.target for it in ph.items if it.kind == "map"]:
+            bits = em.syms[v].bits
+            if isinstance(bits, F.Name) and em.syms[bits.id].kind in ("param_scalar", "extracted"):
+                names.add(bits.id)
+        if len(names) != 1:
+            return main
+        name = f"c.v_{names.pop()}"
+        body = main.replace(name, "width")
+        cases = " ".join(f"case {w}: loop(CompllWidth<{w}>()); break;" for w in (1, 2, 4, 8))
+        return f"""    auto loop = [&](auto width_) {{
+      const uint32_t width = width_;
+{body}    }};
+    switch ({name}) {{ {cases} default: loop((uint32_t){name}); }}
+"""
 
     def _block_reduce(self, reds) -> str:
         if not reds:
@@ -436,15 +457,18 @@ class FusedGen:
             init = self.em.expr(s.expr.init, set())
             rows.append(f"""  {{
     {ty} a = ({ty})({init});
-    if (threadIdx.x < 32) {{
-      for (unsigned w = threadIdx.x; w < gridDim.x; w += 32)
-        a = {self._apply(s.expr, 'a', '(' + ty + ')__ldcg(&partials[' + str(s.slot) + ' * gridDim.x + w])')};
-      for (int off = 16; off > 0; off >>= 1) {{
-        {ty} o = __shfl_xor_sync(0xffffffffu, a, off);
-        a = {self._apply(s.expr, 'a', 'o')};
-      }}
-      if (threadIdx.x == 0) sh[{s.slot}][0] = (float)a;
+    for (unsigned w = threadIdx.x; w < gridDim.x; w += blockDim.x)
+      a = {self._apply(s.expr, 'a', '(' + ty + ')__ldcg(&partials[' + str(s.slot) + ' * gridDim.x + w])')};
+    for (int off = 16; off > 0; off >>= 1) {{
+      {ty} o = __shfl_xor_sync(0xffffffffu, a, off);
+      a = {self._apply(s.expr, 'a', 'o')};
     }}
+    if ((threadIdx.x & 31) == 0) sh[{s.slot}][threadIdx.x >> 5] = (float)a;
+    __syncthreads();
+    a = ({ty})sh[{s.slot}][0];
+    for (int w = 1; w < 8; ++w) a = {self._apply(s.expr, 'a', '(' + ty + ')sh[' + str(s.slot) + '][w]')};
+    __syncthreads();
+    if (threadIdx.x == 0) sh[{s.slot}][0] = (float)a;
     __syncthreads();
     red[{s.slot}] = sh[{s.slot}][0];
     __syncthreads();
@@ -471,6 +495,7 @@ class FusedGen:
   if (threadIdx.x == 0 && atomicAdd(sync + 1, 1u) == gridDim.x - 1) {
     sync[0] = 0;
     sync[1] = 0;
+    sync[32] = 0;
   }
 """
         return f"""
@@ -492,6 +517,16 @@ __global__ void __launch_bounds__(256) {name}_{self.tag}_kernel({em.kernel_param
         """Body of the launcher: grid sizing and the (cooperative) launch."""
         name = self.name
         coop = len(self.plan.phases) > 1
+        if coop:
+            # all blocks resident; four per SM, because every one of them arrives at the same
+            # barrier word (1184 blocks took 12 us per barrier)
+            rows = ("    if (blocks > (uint64_t)cap[dev]) blocks = cap[dev];\n"
+                    "    if (blocks > kMaxBlocks / 2) blocks = kMaxBlocks / 2;")
+        else:
+            # nothing waits: a few thousand blocks, which the hardware gives to whichever SM is
+            # free (a fixed share for every resident block costs about a tenth of the bandwidth)
+            rows = ("    blocks = (blocks + 3) / 4;\n"
+                    "    if (blocks > 0x7FFFFFFFull) blocks = 0x7FFFFFFFull;")
         most_rows = "\n".join(f"    if (n_{pname} > most) most = n_{pname};"
                               for ty, pname in self.em.fn.params if ty.vector)
         return f"""  {{
@@ -507,10 +542,9 @@ __global__ void __launch_bounds__(256) {name}_{self.tag}_kernel({em.kernel_param
     }}
     uint64_t most = work;
 {most_rows}
-    int fgrid = (int)((most / 4 + 255) / 256);
-    if (fgrid < 1) fgrid = 1;
-    if (fgrid > cap[dev]) fgrid = cap[dev];
-    if (fgrid > kMaxBlocks) fgrid = kMaxBlocks;
+    uint64_t blocks = (most / 4 + 255) / 256;
+{rows}
+    const int fgrid = blocks < 1 ? 1 : (int)blocks;
     unsigned int* sync = ticket;
     void* args[] = {{{', '.join('(void*)&' + a for a in self._arg_names())}, (void*)&partials, (void*)&sync}};
     cudaError_t e = {'cudaLaunchCooperativeKernel' if coop else 'cudaLaunchKernel'}(

@@ -41,7 +41,7 @@ def _have_nvcc() -> bool:
 
 def _digest(name: str, target: str) -> str:
     h = hashlib.sha256()
-    for p in [PSE / f"{name}.pse", HERE / "frontend.py", HERE / "emit_cuda.py", HERE / "emit_host.py",
+    for p in [PSE / f"{name}.pse", HERE / "frontend.py", HERE / "emit_cuda.py", HERE / "emit_fused.py", HERE / "emit_host.py",
               HERE / "generator.py", INCLUDE / "hipress" / "compll_rt.cuh", INCLUDE / "hipress" / "common.h"]:
         h.update(p.read_bytes())
     h.update(target.encode())
