@@ -117,8 +117,14 @@ __device__ __forceinline__ uint32_t compll_load_frag(const uint8_t* v, uint64_t 
 // `dst` is the vector's first byte, `nbytes` its length: nothing past it is written.
 __device__ __forceinline__ void compll_pack_store(uint8_t* dst, uint64_t nbytes, uint64_t q,
                                                   uint32_t frag, uint32_t bits) {
-  if ((reinterpret_cast<uintptr_t>(dst) & 3) != 0 && bits >= 2) {
-    // behind a header of an odd length: every lane stores its own one, two or four bytes
+  if ((reinterpret_cast<uintptr_t>(dst) & 3) != 0) {
+    // behind a header of an odd length: every lane stores its own one, two or four bytes,
+    // or with one bit every second lane a byte
+    if (bits == 1) {
+      const uint32_t hi = __shfl_down_sync(0xffffffffu, frag, 1);
+      if (!(q & 1) && q / 2 < nbytes) dst[q / 2] = (uint8_t)(frag | (hi << 4));
+      return;
+    }
     const uint64_t off = q * bits / 2;
     const uint32_t nb = bits / 2;
     uint8_t* p = dst + off;

@@ -345,7 +345,15 @@ class FusedGen:
         # U groups of four elements per thread and trip, every load of a trip issued before
         # the first result is computed (a map only reads its own elements of the vectors
         # it also writes, so hoisting the loads over the stores is safe).
-        U = 4 if not need_in else (4 if not stores else 2)
+        # Four groups where nothing but packed fragments comes in or nothing goes out.  A phase
+        # that streams floats in and out has enough loads with one group, but behind a header
+        # (whose fields every block has to read first) or a barrier two pay.
+        headed = bool(em.extracts) or len(self.plan.phases) > 1
+        U = 4 if not need_in or not stores else (2 if headed else 1)
+        # groups of a block in a grid that is not limited: a block that reads a header is
+        # worth more of them (TernGradDecodeAccumulate of 16.8 M elements 28.8 us with one
+        # group per thread and block, 25.4 with four)
+        self.unroll = 4 if headed else U
         larr = [f"      {C_TYPES[em.syms[v].type.name]} in_{v}[{U}][4];" for v in need_in] + \
                [f"      uint32_t fr_{v}[{U}];" for v in need_frag]
         loads = [f"        compll_load4(c.v_{v}, i0, count, in_{v}[u]);" for v in need_in]
@@ -499,6 +507,8 @@ class FusedGen:
   }
 """
         return f"""
+constexpr uint64_t {name}_{self.tag}_groups = {self.unroll};  // of four elements, per thread of a block
+
 // One launch for the whole function: {len(phases)} phase(s){', grid barriers in between' if len(phases) > 1 else ''}.
 __global__ void __launch_bounds__(256) {name}_{self.tag}_kernel({em.kernel_params()}, float* partials,
                                                        unsigned int* sync) {{
@@ -518,14 +528,16 @@ __global__ void __launch_bounds__(256) {name}_{self.tag}_kernel({em.kernel_param
         name = self.name
         coop = len(self.plan.phases) > 1
         if coop:
-            # all blocks resident; four per SM, because every one of them arrives at the same
-            # barrier word (1184 blocks took 12 us per barrier)
+            # all blocks resident; no more per SM than keep it busy, because every one of them
+            # arrives at the same barrier word, 10 ns each (TernGradEncode of 1 M elements 16.4 us
+            # with six blocks per SM, 12.4 with four; 17.2 with eight and one polled word)
             rows = ("    if (blocks > (uint64_t)cap[dev]) blocks = cap[dev];\n"
                     "    if (blocks > kMaxBlocks / 2) blocks = kMaxBlocks / 2;")
         else:
             # nothing waits: a few thousand blocks, which the hardware gives to whichever SM is
             # free (a fixed share for every resident block costs about a tenth of the bandwidth)
-            rows = ("    blocks = (blocks + 3) / 4;\n"
+            unroll = f"compll_gen_{name}::{name}_{self.tag}_groups"
+            rows = (f"    blocks = (blocks + {unroll} - 1) / {unroll};\n"
                     "    if (blocks > 0x7FFFFFFFull) blocks = 0x7FFFFFFFull;")
         most_rows = "\n".join(f"    if (n_{pname} > most) most = n_{pname};"
                               for ty, pname in self.em.fn.params if ty.vector)
