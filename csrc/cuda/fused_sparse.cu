@@ -189,7 +189,7 @@ static __device__ __noinline__ void set_units(const SpBucket& bk, const HpComm& 
     const SpSeg& sg = bk.seg[si];
     SelUnit& s = sm.unit[y];
     const size_t E = (size_t)cx.E, off = (size_t)c * sg.chunk;
-    const uint32_t n = sp_chunk_valid(sg.n, sg.chunk, c), tiles = (n + kSpTile - 1) / kSpTile;
+    const uint32_t n = sp_chunk_valid(sg.n, sg.chunk, c), tiles = (n + kSelTile - 1) / kSelTile;
     s.n = n;
     s.k = n == sg.chunk ? sg.kmax : sg.k_last;   // only the last chunk is shorter
     s.kmax = sg.kmax;
@@ -553,7 +553,7 @@ static int build_sp_bucket(int alg, float ratio, float momentum, const HpSeg* se
     d.kmax = (uint32_t)sparse_k(chunk, ratio);
     d.k_last = (uint32_t)sparse_k(n % chunk, ratio);
     d.pay_off = (uint32_t)pay;
-    d.tiles = (uint32_t)((chunk + kSpTile - 1) / kSpTile);
+    d.tiles = (uint32_t)((chunk + kSelTile - 1) / kSelTile);
     tiles += d.tiles;
     d.cap = (uint32_t)align_up(8ull * d.kmax + 4096, 32);
     d.cand_push = cand;

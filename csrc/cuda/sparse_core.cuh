@@ -17,7 +17,7 @@ namespace hipress {
 // such an access to one address takes 10 to 25 ns of its own, so 444 CTAs of 256 threads
 // spent 4.5 us per barrier and 11 us on the sample histogram of one tensor.
 constexpr int kSpThreads = 512;
-constexpr uint32_t kSpTile = 16 * kSpThreads;   // elements per tile: 16 per thread
+constexpr uint32_t kSpTile = 16 * kSpThreads;   // elements per tile of the whole-array passes
 constexpr int kBins = 4096;
 // workspace words: 3 histograms, then counters
 constexpr int kWsOutCount = 3 * kBins + 0;
@@ -398,7 +398,8 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 // resolve; counters that are read together lie together; and slices send without a
 // barrier behind the histogram.
 constexpr uint32_t kMinSampled = 4;     // tiles of an array that are sampled at least
-constexpr uint32_t kMaxSampled = 64;    // and at most: 0.5 M elements
+constexpr uint32_t kMaxSampled = 128;   // and at most: 0.5 M elements
+constexpr uint32_t kSelTile = 8 * kSpThreads;  // elements per tile: two float4 of each array per thread
 
 // One array to select from.
 struct SelUnit {
@@ -460,7 +461,7 @@ struct SelSmem {
       uint16_t unit[kCollectBuf];
     } buf;                           // collect
   };
-  float stash[2][kSpTile];          // sample to collect
+  float stash[2][kSelTile];          // sample to collect
   FindSmem fs;
   uint32_t count, base, base2, ticket, flag;
   uint32_t sent, ties;
@@ -472,23 +473,29 @@ __device__ __forceinline__ void clear_hist(uint32_t* sh) {
     reinterpret_cast<uint4*>(sh)[b + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Loads tile t and applies the update (MODE as in pass0_body), all loads before the first
-// store.  Elements past the end read as zero, and a zero is never sent.
-template <int MODE>
-__device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[4]) {
-  const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
-                     (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
-  const uint64_t i0 = (uint64_t)t * kSpTile + threadIdx.x * 4;
-  float4 gv[4], uv[4];
+// Loads T consecutive tiles from t and applies the update (MODE as in pass0_body), all
+// loads before the first store.  Elements past the end read as zero, and a zero is never
+// sent.
+template <int MODE, int T, bool FULL>
+__device__ __forceinline__ void update_tiles_impl(const SelUnit& s, float momentum, uint64_t i0, bool vec,
+                                                  float4 (&av)[2 * T]) {
+  auto ld4 = [&](const float* p, uint64_t i, uint32_t n, bool v) {
+    return FULL ? *reinterpret_cast<const float4*>(p + i) : hipress::ld4(p, i, n, v);
+  };
+  auto st4 = [&](float* p, uint64_t i, uint32_t n, bool v, const float4& x) {
+    if (FULL) *reinterpret_cast<float4*>(p + i) = x;
+    else hipress::st4(p, i, n, v, x);
+  };
+  float4 gv[2 * T], uv[2 * T];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 2 * T; ++j) {
     const uint64_t i = i0 + j * kSpThreads * 4;
     av[j] = ld4(s.a, i, s.n, vec);
     if (MODE >= 1) gv[j] = ld4(s.g, i, s.n, vec);
     if (MODE == 2) uv[j] = ld4(s.u, i, s.n, vec);
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 2 * T; ++j) {
     const uint64_t i = i0 + j * kSpThreads * 4;
     float4& v = av[j];
     if (MODE == 1) {
@@ -506,10 +513,19 @@ __device__ __forceinline__ void update_tile(const SelUnit& s, float momentum, ui
     }
   }
   if (MODE >= 1 && s.clear) {
-    const bool cvec = (reinterpret_cast<uintptr_t>(s.clear) & 15) == 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) st4(s.clear, i0 + j * kSpThreads * 4, s.n, cvec, make_float4(0.f, 0.f, 0.f, 0.f));
+    for (int j = 0; j < 2 * T; ++j) st4(s.clear, i0 + j * kSpThreads * 4, s.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
   }
+}
+template <int MODE, int T>
+__device__ __forceinline__ void update_tiles(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[2 * T]) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
+                     (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.clear) : 0) |
+                     (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
+  const uint64_t i0 = (uint64_t)t * kSelTile + threadIdx.x * 4;
+  // one test for the tiles: with one per load the loads did not overlap as they should
+  if (vec && (uint64_t)(t + T) * kSelTile <= s.n) update_tiles_impl<MODE, T, true>(s, momentum, i0, vec, av);
+  else update_tiles_impl<MODE, T, false>(s, momentum, i0, vec, av);
 }
 
 // Sampled tile number i of an array: update, values into `stash`, magnitudes into the
@@ -519,11 +535,11 @@ template <int MODE>
 static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum, SelSmem& sm, uint32_t i,
                                                 float* stash) {
   clear_hist(sm.hist);
-  float4 av[4];
-  update_tile<MODE>(s, momentum, i * s.stride, av);
+  float4 av[2];
+  update_tiles<MODE, 1>(s, momentum, i * s.stride, av);
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 2; ++j) {
     reinterpret_cast<float4*>(stash)[j * kSpThreads + threadIdx.x] = av[j];
     const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
 #pragma unroll
@@ -546,7 +562,7 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
   if (s.stride > 1) {
     // k scaled to the sample, plus five standard deviations, plus a tenth because
     // neighbouring elements are not independent
-    const float hits = __fdividef((float)s.k * (float)(s.sampled * kSpTile), (float)s.n);
+    const float hits = __fdividef((float)s.k * (float)(s.sampled * kSelTile), (float)s.n);
     float dev;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(dev) : "f"(hits));
     rank = (uint32_t)(1.1f * hits + 5.0f * dev + 4.0f);
@@ -609,45 +625,51 @@ __device__ __forceinline__ void collect_one(const SelUnit& s, uint32_t uid, SelS
     s.ws[kWsOverflow] = 1u;
   }
 }
-// the elements of a tile that reach `low`
-__device__ __forceinline__ void collect_tile(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, uint32_t t,
-                                             const float4 (&av)[4]) {
+// the elements of T tiles that reach `low`
+template <int T>
+__device__ __forceinline__ void collect_tiles(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, uint32_t t,
+                                              const float4 (&av)[2 * T]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 2 * T; ++j) {
     const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
     const uint32_t most = max(max(abs_key(e[0]), abs_key(e[1])), max(abs_key(e[2]), abs_key(e[3])));
     if (most < low) continue;
-    const uint32_t i = t * kSpTile + (j * kSpThreads + threadIdx.x) * 4;
+    const uint32_t i = t * kSelTile + (j * kSpThreads + threadIdx.x) * 4;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (abs_key(e[q]) >= low) collect_one(s, uid, sm, low, e[q], i + q);
   }
 }
 
-// Tiles [t0, t1) of one array without the sampled ones.
+// Tiles [t0, t1) of one array without the sampled ones, several at a time: 8 to 12 loads
+// of 16 bytes per thread are what keeps HBM busy with 16 warps per SM.
 template <int MODE>
 static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid, float momentum, SelSmem& sm,
                                                  uint32_t t0, uint32_t t1) {
+  constexpr int T = MODE == 0 ? 4 : 2;
   const uint32_t low = __ldcg(s.ws + kWsLow);
   uint32_t phase = t0 % s.stride;   // 0: a sampled tile
 #pragma unroll 1
-  for (uint32_t t = t0; t < t1; ++t) {
-    const bool skip = phase == 0;
-    if (++phase == s.stride) phase = 0;
-    if (skip) continue;
-    float4 av[4];
-    update_tile<MODE>(s, momentum, t, av);
-    if (MODE == 0 && phase != 0 && t + 1 < t1) {
-      // one array only: a second tile's loads in flight keep the memory busy
-      float4 bv[4];
-      update_tile<0>(s, momentum, t + 1, bv);
-      collect_tile(s, uid, sm, low, t, av);
-      collect_tile(s, uid, sm, low, t + 1, bv);
+  for (uint32_t t = t0; t < t1;) {
+    if (phase == 0) {
       ++t;
-      if (++phase == s.stride) phase = 0;
-    } else {
-      collect_tile(s, uid, sm, low, t, av);
+      phase = 1;
+      continue;
     }
+    if (t + T <= t1 && phase + T <= s.stride) {
+      float4 av[2 * T];
+      update_tiles<MODE, T>(s, momentum, t, av);
+      collect_tiles<T>(s, uid, sm, low, t, av);
+      t += T;
+      phase += T;
+    } else {
+      float4 av[2];
+      update_tiles<MODE, 1>(s, momentum, t, av);
+      collect_tiles<1>(s, uid, sm, low, t, av);
+      ++t;
+      ++phase;
+    }
+    if (phase == s.stride) phase = 0;
   }
 }
 
@@ -655,14 +677,14 @@ static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid,
 static __device__ __noinline__ void collect_sampled(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t i,
                                                     const float* stash, bool again) {
   const uint32_t t = i * s.stride, low = __ldcg(s.ws + kWsLow);
-  float4 av[4];
+  float4 av[2];
   if (again) {
-    update_tile<0>(s, 0.0f, t, av);
+    update_tiles<0, 1>(s, 0.0f, t, av);
   } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) av[j] = reinterpret_cast<const float4*>(stash)[j * kSpThreads + threadIdx.x];
+    for (int j = 0; j < 2; ++j) av[j] = reinterpret_cast<const float4*>(stash)[j * kSpThreads + threadIdx.x];
   }
-  collect_tile(s, uid, sm, low, t, av);
+  collect_tiles<1>(s, uid, sm, low, t, av);
 }
 
 // Append the CTA's gathered candidates to their lists, and their first digits to the
@@ -738,8 +760,8 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
                                                SelSmem& sm, uint32_t x, uint32_t nx) {
   const uint32_t L = ls.count, low = ls.low;   // no overflow: the list holds all of them
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
-  const bool every = L < s.k;                  // fewer than k are not zero: all are sent
-  uint32_t bin0 = 0, rem = 0;
+  const bool every = L <= s.k;                 // all candidates are sent
+  uint32_t bin0 = 0, rem = 0, least = 0xFFFFFFFFu;
   if (!every) find_bin(s.ws + kBins, s.k, sm.fs, bin0, rem);
   const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
 #pragma unroll 1
@@ -755,6 +777,7 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
       idx = __ldcg(list_indices(s) + p);
       const uint32_t d = cand_digit(abs_key(v), low);
       send = every || d > bin0;
+      least = min(least, abs_key(v));
       keep = !every && d == bin0;
       if (send) at = atomicAdd(&sm.sent, 1u);
       if (keep) at = atomicAdd(&sm.ties, 1u);
@@ -772,6 +795,10 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
       list2_values(s)[sm.base2 + at] = v;
       list2_indices(s)[sm.base2 + at] = idx;
     }
+  }
+  if (every) {   // the least key sent is the threshold: kept as the largest complement
+    least = __reduce_min_sync(0xffffffffu, least);
+    if ((threadIdx.x & 31) == 0) atomicMax(s.ws + kWsTieCount, ~least);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -829,7 +856,8 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
   h.alg = (uint8_t)alg;
   h.bitwidth = 0;
   h.flags = 0;
-  h.a = every ? 0.0f : __uint_as_float(start + prefix);
+  // zero when fewer than k are not zero
+  h.a = __uint_as_float(!every ? start + prefix : (L < s.k ? 0u : ~__ldcg(s.ws + kWsTieCount)));
   h.b = sm.sent < s.kmax ? sm.sent : s.kmax;
 #pragma unroll 1
   for (int d = 0; d < dst.n; ++d) *reinterpret_cast<uint4*>(dst.out[d]) = *reinterpret_cast<const uint4*>(&h);

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) sparse_encode_kernel(const __gr
   auto barrier = [&]() {
     grid_barrier(s.ws + kWsWords, gen, G, kGridBarrierNs, s.ws + kWsStatus, 1u, wst);
   };
-  const uint32_t tiles = (s.n - 1) / kSpTile + 1;
+  const uint32_t tiles = (s.n - 1) / kSelTile + 1;
   uint32_t mine = 0;   // sampled tiles of this CTA: the first two stay in shared memory
 #pragma unroll 1
   for (uint32_t i = c; i < s.sampled; i += G, ++mine) {
@@ -187,7 +187,7 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
   if (reinterpret_cast<uintptr_t>(out) & 15) return HP_ERR_BAD_ARG;
   if (update && !g) return HP_ERR_BAD_ARG;
   if (update && alg == kDgc && !u) return HP_ERR_BAD_ARG;
-  const uint64_t tiles = (n + kSpTile - 1) / kSpTile;
+  const uint64_t tiles = (n + kSelTile - 1) / kSelTile;
   float* uu = alg == kDgc ? u : nullptr;
   const int mode = !update ? 0 : (alg == kGradDrop ? 1 : 2);
   // histograms and counters, then the barrier words and the candidate lists
