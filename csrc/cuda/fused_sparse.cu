@@ -317,6 +317,7 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
   }
   sp_barrier(cm, cx, sm);
   if (threadIdx.x == 0) sm.sel.count = 0;
+  for (uint32_t y = threadIdx.x; y < units; y += kSpThreads) sm.unit[y].low = __ldcg(sm.unit[y].ws + kWsLow);
   __syncthreads();
 #pragma unroll 1
   for (uint32_t i = blockIdx.x, r = 0; r < mine; i += cx.G, ++r) {

@@ -412,6 +412,7 @@ struct SelUnit {
                    // same size behind it
   uint32_t n, k, kmax, cap;
   uint32_t stride, sampled;  // every stride-th tile is sampled: how many that is
+  uint32_t low;              // the candidates' lower bound, once the sample is complete
 };
 __device__ __forceinline__ uint32_t* list_indices(const SelUnit& s) { return reinterpret_cast<uint32_t*>(s.cv + s.cap); }
 __device__ __forceinline__ float* list2_values(const SelUnit& s) { return s.cv + 2 * (size_t)s.cap; }
@@ -474,11 +475,12 @@ __device__ __forceinline__ void clear_hist(uint32_t* sh) {
 }
 
 // Loads T consecutive tiles from t and applies the update (MODE as in pass0_body), all
-// loads before the first store.  Elements past the end read as zero, and a zero is never
-// sent.
+// loads before the first store.  Tiles not in `mask` are left out; what lies past the end
+// reads as zero, and a zero is never sent.
 template <int MODE, int T, bool FULL>
 __device__ __forceinline__ void update_tiles_impl(const SelUnit& s, float momentum, uint64_t i0, bool vec,
-                                                  float4 (&av)[2 * T]) {
+                                                  uint32_t mask, float4 (&av)[2 * T]) {
+  auto on = [&](int j) { return FULL || (mask >> (j / 2) & 1u); };
   auto ld4 = [&](const float* p, uint64_t i, uint32_t n, bool v) {
     return FULL ? *reinterpret_cast<const float4*>(p + i) : hipress::ld4(p, i, n, v);
   };
@@ -490,6 +492,8 @@ __device__ __forceinline__ void update_tiles_impl(const SelUnit& s, float moment
 #pragma unroll
   for (int j = 0; j < 2 * T; ++j) {
     const uint64_t i = i0 + j * kSpThreads * 4;
+    av[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!on(j)) continue;
     av[j] = ld4(s.a, i, s.n, vec);
     if (MODE >= 1) gv[j] = ld4(s.g, i, s.n, vec);
     if (MODE == 2) uv[j] = ld4(s.u, i, s.n, vec);
@@ -498,6 +502,7 @@ __device__ __forceinline__ void update_tiles_impl(const SelUnit& s, float moment
   for (int j = 0; j < 2 * T; ++j) {
     const uint64_t i = i0 + j * kSpThreads * 4;
     float4& v = av[j];
+    if (!on(j)) continue;
     if (MODE == 1) {
       v.x = v.x + gv[j].x; v.y = v.y + gv[j].y; v.z = v.z + gv[j].z; v.w = v.w + gv[j].w;
       st4(s.a, i, s.n, vec, v);
@@ -514,18 +519,22 @@ __device__ __forceinline__ void update_tiles_impl(const SelUnit& s, float moment
   }
   if (MODE >= 1 && s.clear) {
 #pragma unroll
-    for (int j = 0; j < 2 * T; ++j) st4(s.clear, i0 + j * kSpThreads * 4, s.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
+    for (int j = 0; j < 2 * T; ++j)
+      if (on(j)) st4(s.clear, i0 + j * kSpThreads * 4, s.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
   }
 }
 template <int MODE, int T>
-__device__ __forceinline__ void update_tiles(const SelUnit& s, float momentum, uint32_t t, float4 (&av)[2 * T]) {
+__device__ __forceinline__ void update_tiles(const SelUnit& s, float momentum, uint32_t t, uint32_t mask,
+                                             float4 (&av)[2 * T]) {
   const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
                      (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.clear) : 0) |
                      (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
   const uint64_t i0 = (uint64_t)t * kSelTile + threadIdx.x * 4;
   // one test for the tiles: with one per load the loads did not overlap as they should
-  if (vec && (uint64_t)(t + T) * kSelTile <= s.n) update_tiles_impl<MODE, T, true>(s, momentum, i0, vec, av);
-  else update_tiles_impl<MODE, T, false>(s, momentum, i0, vec, av);
+  if (vec && mask == (1u << T) - 1u && (uint64_t)(t + T) * kSelTile <= s.n)
+    update_tiles_impl<MODE, T, true>(s, momentum, i0, vec, mask, av);
+  else
+    update_tiles_impl<MODE, T, false>(s, momentum, i0, vec, mask, av);
 }
 
 // Sampled tile number i of an array: update, values into `stash`, magnitudes into the
@@ -536,7 +545,7 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
                                                 float* stash) {
   clear_hist(sm.hist);
   float4 av[2];
-  update_tiles<MODE, 1>(s, momentum, i * s.stride, av);
+  update_tiles<MODE, 1>(s, momentum, i * s.stride, 1u, av);
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
@@ -583,7 +592,8 @@ template <typename F>
 __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t cta, uint32_t ctas, uint32_t& slot,
                                          F f) {
   const uint32_t share = total / ctas * 3u / 4u, dealt = share * ctas;
-  const uint32_t stretch = (total - dealt) / (4u * ctas) + 1u;
+  uint32_t stretch = (total - dealt) / (2u * ctas) + 1u;
+  if (stretch > 2u) stretch = (stretch + 2u) & ~3u;   // whole groups of tiles
   const uint32_t at = (uint32_t)__cvta_generic_to_shared(&slot);
   uint32_t next = 0;
   auto take = [&] {
@@ -627,8 +637,9 @@ __device__ __forceinline__ void collect_one(const SelUnit& s, uint32_t uid, SelS
 }
 // the elements of T tiles that reach `low`
 template <int T>
-__device__ __forceinline__ void collect_tiles(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t low, uint32_t t,
+__device__ __forceinline__ void collect_tiles(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t t,
                                               const float4 (&av)[2 * T]) {
+  const uint32_t low = s.low;
 #pragma unroll
   for (int j = 0; j < 2 * T; ++j) {
     const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
@@ -646,45 +657,34 @@ __device__ __forceinline__ void collect_tiles(const SelUnit& s, uint32_t uid, Se
 template <int MODE>
 static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid, float momentum, SelSmem& sm,
                                                  uint32_t t0, uint32_t t1) {
-  constexpr int T = MODE == 0 ? 4 : 2;
-  const uint32_t low = __ldcg(s.ws + kWsLow);
+  constexpr uint32_t T = MODE == 0 ? 4 : 2;
   uint32_t phase = t0 % s.stride;   // 0: a sampled tile
 #pragma unroll 1
-  for (uint32_t t = t0; t < t1;) {
-    if (phase == 0) {
-      ++t;
-      phase = 1;
-      continue;
+  for (uint32_t t = t0; t < t1; t += T) {
+    uint32_t mask = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < T; ++q) {
+      if (phase != 0 && t + q < t1) mask |= 1u << q;
+      if (++phase == s.stride) phase = 0;
     }
-    if (t + T <= t1 && phase + T <= s.stride) {
-      float4 av[2 * T];
-      update_tiles<MODE, T>(s, momentum, t, av);
-      collect_tiles<T>(s, uid, sm, low, t, av);
-      t += T;
-      phase += T;
-    } else {
-      float4 av[2];
-      update_tiles<MODE, 1>(s, momentum, t, av);
-      collect_tiles<1>(s, uid, sm, low, t, av);
-      ++t;
-      ++phase;
-    }
-    if (phase == s.stride) phase = 0;
+    float4 av[2 * T];
+    update_tiles<MODE, T>(s, momentum, t, mask, av);
+    collect_tiles<T>(s, uid, sm, t, av);
   }
 }
 
 // Sampled tile number i again, updated before: from its stash, or (again) read once more.
 static __device__ __noinline__ void collect_sampled(const SelUnit& s, uint32_t uid, SelSmem& sm, uint32_t i,
                                                     const float* stash, bool again) {
-  const uint32_t t = i * s.stride, low = __ldcg(s.ws + kWsLow);
+  const uint32_t t = i * s.stride;
   float4 av[2];
   if (again) {
-    update_tiles<0, 1>(s, 0.0f, t, av);
+    update_tiles<0, 1>(s, 0.0f, t, 1u, av);
   } else {
 #pragma unroll
     for (int j = 0; j < 2; ++j) av[j] = reinterpret_cast<const float4*>(stash)[j * kSpThreads + threadIdx.x];
   }
-  collect_tiles<1>(s, uid, sm, low, t, av);
+  collect_tiles<1>(s, uid, sm, t, av);
 }
 
 // Append the CTA's gathered candidates to their lists, and their first digits to the
@@ -700,7 +700,7 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
   if (__syncthreads_and(same)) {   // one reservation for the CTA
     if (threadIdx.x == 0 && n) sm.base = atomicAdd(unit(sm.buf.unit[0]).ws + kWsCandCount, n);
     const SelUnit& s = unit(n ? sm.buf.unit[0] : 0u);
-    const uint32_t low = n ? __ldcg(s.ws + kWsLow) : 0u;
+    const uint32_t low = s.low;
     __syncthreads();
 #pragma unroll 1
     for (uint32_t p = threadIdx.x; p < n; p += kSpThreads) {
@@ -728,7 +728,7 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
       const uint32_t uid = sm.buf.unit[p], lane = threadIdx.x & 31;
       const float v = sm.buf.val[p];
       const SelUnit& s = unit(uid);
-      const uint32_t low = __ldcg(s.ws + kWsLow);
+      const uint32_t low = s.low;
       const uint32_t group = __match_any_sync(mask, uid);
       const int lead = __ffs(group) - 1;
       uint32_t pos = 0;

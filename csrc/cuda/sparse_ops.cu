@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(kSpThreads, 1) sparse_encode_kernel(const __gr
   SelOrPassSmem& sm = *reinterpret_cast<SelOrPassSmem*>(smem_raw);
   __shared__ WaitState wst;
   __shared__ FindSmem fs;
-  const SelUnit& s = A.unit;
+  __shared__ SelUnit s;
+  if (threadIdx.x == 0) s = A.unit;
   const uint32_t G = gridDim.x, c = blockIdx.x;
   uint32_t gen = 0;
   wait_init(wst);
@@ -91,7 +92,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) sparse_encode_kernel(const __gr
     __syncthreads();
   }
   barrier();
-  if (threadIdx.x == 0) sm.sel.count = 0;
+  if (threadIdx.x == 0) {
+    sm.sel.count = 0;
+    s.low = __ldcg(s.ws + kWsLow);
+  }
   __syncthreads();
 #pragma unroll 1
   for (uint32_t i = c, r = 0; r < mine; i += G, ++r)

@@ -225,6 +225,13 @@ def fused_segments(em: Emitter) -> list:
     return out
 
 
+def _ordered(r: F.Reduce) -> bool:
+    """Whether the result of a reduction depends on the order of its steps (a sum of floats
+    does, a minimum does not): such a function keeps its split over threads and blocks, so
+    that the same input gives the same bits from one version to the next."""
+    return not (isinstance(r.fn, F.Name) and r.fn.id in ("smaller", "greater"))
+
+
 class FusedGen:
     """Emits the fused kernel and its launch for a plan that is ``ok``."""
 
@@ -463,10 +470,23 @@ class FusedGen:
         for s in reds:
             ty = C_TYPES[s.type.name]
             init = self.em.expr(s.expr.init, set())
-            rows.append(f"""  {{
-    {ty} a = ({ty})({init});
-    for (unsigned w = threadIdx.x; w < gridDim.x; w += blockDim.x)
-      a = {self._apply(s.expr, 'a', '(' + ty + ')__ldcg(&partials[' + str(s.slot) + ' * gridDim.x + w])')};
+            load = '(' + ty + ')__ldcg(&partials[' + str(s.slot) + ' * gridDim.x + w])'
+            if _ordered(s.expr):
+                # one warp, every lane in a fixed order; eight loads in flight
+                fold = f"""    if (threadIdx.x < 32) {{
+#pragma unroll 8
+      for (unsigned w = threadIdx.x; w < gridDim.x; w += 32)
+        a = {self._apply(s.expr, 'a', load)};
+      for (int off = 16; off > 0; off >>= 1) {{
+        {ty} o = __shfl_xor_sync(0xffffffffu, a, off);
+        a = {self._apply(s.expr, 'a', 'o')};
+      }}
+      if (threadIdx.x == 0) sh[{s.slot}][0] = (float)a;
+    }}
+    __syncthreads();"""
+            else:
+                fold = f"""    for (unsigned w = threadIdx.x; w < gridDim.x; w += blockDim.x)
+      a = {self._apply(s.expr, 'a', load)};
     for (int off = 16; off > 0; off >>= 1) {{
       {ty} o = __shfl_xor_sync(0xffffffffu, a, off);
       a = {self._apply(s.expr, 'a', 'o')};
@@ -477,7 +497,10 @@ class FusedGen:
     for (int w = 1; w < 8; ++w) a = {self._apply(s.expr, 'a', '(' + ty + ')sh[' + str(s.slot) + '][w]')};
     __syncthreads();
     if (threadIdx.x == 0) sh[{s.slot}][0] = (float)a;
-    __syncthreads();
+    __syncthreads();"""
+            rows.append(f"""  {{
+    {ty} a = ({ty})({init});
+{fold}
     red[{s.slot}] = sh[{s.slot}][0];
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) scalars[{s.slot}] = red[{s.slot}];
@@ -506,11 +529,12 @@ class FusedGen:
     sync[32] = 0;
   }
 """
+        bound = ", 8" if any(_ordered(s.expr) for s in em.reduces) else ""   # kMaxBlocks resident
         return f"""
 constexpr uint64_t {name}_{self.tag}_groups = {self.unroll};  // of four elements, per thread of a block
 
 // One launch for the whole function: {len(phases)} phase(s){', grid barriers in between' if len(phases) > 1 else ''}.
-__global__ void __launch_bounds__(256) {name}_{self.tag}_kernel({em.kernel_params()}, float* partials,
+__global__ void __launch_bounds__(256{bound}) {name}_{self.tag}_kernel({em.kernel_params()}, float* partials,
                                                        unsigned int* sync) {{
   __shared__ float sh[{nred}][8];
   float red[{nred}];
@@ -531,8 +555,9 @@ __global__ void __launch_bounds__(256) {name}_{self.tag}_kernel({em.kernel_param
             # all blocks resident; no more per SM than keep it busy, because every one of them
             # arrives at the same barrier word, 10 ns each (TernGradEncode of 1 M elements 16.4 us
             # with six blocks per SM, 12.4 with four; 17.2 with eight and one polled word)
+            most = "kMaxBlocks" if any(_ordered(s.expr) for s in self.em.reduces) else "kMaxBlocks / 2"
             rows = ("    if (blocks > (uint64_t)cap[dev]) blocks = cap[dev];\n"
-                    "    if (blocks > kMaxBlocks / 2) blocks = kMaxBlocks / 2;")
+                    f"    if (blocks > {most}) blocks = {most};")
         else:
             # nothing waits: a few thousand blocks, which the hardware gives to whichever SM is
             # free (a fixed share for every resident block costs about a tenth of the bandwidth)
