@@ -42,7 +42,7 @@ struct SpSeg {
   uint32_t n, chunk, kmax, pay_off;
   uint32_t tiles;       // tiles of one chunk
   uint32_t k_last;      // pairs of the last chunk, which may be shorter
-  uint32_t stride;      // every stride-th tile is sampled (set at launch: depends on the grid)
+  Sampling sample;      // set at launch: depends on the grid
   uint32_t cap;         // candidate pairs per (tensor, chunk) unit, for both lists
   uint64_t cand_push;   // first push unit's candidate list, in pairs from the region start
   uint64_t cand_srv;    // the server unit's candidate list
@@ -194,8 +194,10 @@ static __device__ __noinline__ void set_units(const SpBucket& bk, const HpComm& 
     s.k = n == sg.chunk ? sg.kmax : sg.k_last;   // only the last chunk is shorter
     s.kmax = sg.kmax;
     s.cap = list_cap(sg.cap);
-    s.stride = sg.stride;
-    s.sampled = (tiles + sg.stride - 1) / sg.stride;
+    s.stride = sg.sample.stride;
+    s.top = sg.sample.top;
+    s.run = sg.sample.run;
+    s.sampled = (tiles + s.stride - 1) / s.stride;
     uint64_t list = sg.cand_srv;
     uint32_t block = (uint32_t)(bk.nseg * cx.N) + y;
     s.g = nullptr;
@@ -328,9 +330,9 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
   hand_out(cx.ctl + kCtlTickets + ticket, sm.tile_at[units], blockIdx.x, cx.G, sm.ticket, [&](uint32_t t, uint32_t end) {
     uint32_t y = unit_at(sm.tile_at, units, t);
 #pragma unroll 1
-    for (; t < end; ++y) {
-      const uint32_t base = sm.tile_at[y], t1 = min(sm.tile_at[y + 1], end);
-      if (t1 <= t) continue;   // an empty unit
+    while (t < end) {
+      while (sm.tile_at[y + 1] <= t) ++y;   // empty units
+      const uint32_t base = sm.tile_at[y], t1 = min(min(sm.tile_at[y + 1], end), t + sm.unit[y].run);
       const SelUnit& s = sm.unit[y];
       if (s.stride > 1) {
         if (ph.mode == 0) collect_body<0>(s, y, bk.momentum, sm.sel, t - base, t1 - base);
@@ -338,8 +340,8 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
         else collect_body<2>(s, y, bk.momentum, sm.sel, t - base, t1 - base);
       }
       t = t1;
+      if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, unit);
     }
-    if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, unit);
   });
   collect_flush(sm.sel, unit);
   sp_barrier(cm, cx, sm);
@@ -482,7 +484,7 @@ __device__ __forceinline__ void sp_epilogue(const SpCtx& cx) {
 // PS: push (every rank selects per owner and stores the pairs into the owner's inbox),
 // serve (the owner adds the payloads, re-selects, stores the result into every inbox),
 // pull (every rank scatters value / N).  Five barriers.
-__global__ void __launch_bounds__(kSpThreads, 1)
+__global__ void __launch_bounds__(kSpThreads, 2)
 sp_ps_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm cm, const __grid_constant__ SpLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
@@ -507,7 +509,7 @@ sp_ps_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm
 // Ring: N hops of (add the predecessor's pairs, update and select, store into the
 // successor's inbox), the last hop storing into every inbox; then every rank scatters
 // the reduced chunks of the others.  Three barriers per hop.
-__global__ void __launch_bounds__(kSpThreads, 1)
+__global__ void __launch_bounds__(kSpThreads, 2)
 sp_ring_kernel(const __grid_constant__ SpBucket bk, const __grid_constant__ HpComm cm, const __grid_constant__ SpLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpSmem& sm = *reinterpret_cast<SpSmem*>(smem_raw);
@@ -611,8 +613,8 @@ static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int
   if (G > cap / ranks_here) G = cap / ranks_here;   // what the GPU holds at once
   if (G < 1) return HP_ERR_RESIDENCY;
   for (int i = 0; i < nseg; ++i)  // a sampled tile for every CTA, over the units of a push or of a hop
-    bk.seg[i].stride =
-        sample_stride(bk.seg[i].tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G);
+    bk.seg[i].sample = sampling(bk.seg[i].tiles, (uint64_t)bk.tiles_total * (topo == HP_TOPO_PS ? N : 1), (uint32_t)G,
+                                bk.seg[i].chunk, bk.seg[i].kmax);
   SpLaunch L;
   L.ws = static_cast<uint8_t*>(ws);
   L.hist_words = sp_hist_words(nseg, N);

@@ -12,10 +12,11 @@
 
 namespace hipress {
 
-// One CTA of 512 threads per SM in the grid-wide kernels: every CTA arrives at the same
+// Two CTAs of 512 threads per SM in the grid-wide kernels: every CTA arrives at the same
 // barrier counter, adds to the same histograms and reserves room in the same lists, and
 // such an access to one address takes 10 to 25 ns of its own, so 444 CTAs of 256 threads
-// spent 4.5 us per barrier and 11 us on the sample histogram of one tensor.
+// spent 4.5 us per barrier.  One CTA per SM leaves HBM idle while it waits at its tile's
+// end: ResNet-50's bucket took 184 us instead of 173.
 constexpr int kSpThreads = 512;
 constexpr uint32_t kSpTile = 16 * kSpThreads;   // elements per tile of the whole-array passes
 constexpr int kBins = 4096;
@@ -24,6 +25,7 @@ constexpr int kWsOutCount = 3 * kBins + 0;
 constexpr int kWsTieCount = 3 * kBins + 1;
 constexpr int kWsDone = 3 * kBins + 2;
 constexpr int kWsSampled = 3 * kBins + 3;     // sampled tiles that are done
+constexpr int kWsKeyCount = 3 * kBins + 10;   // keys the sampled tiles contributed
 constexpr int kWsCandCount = 3 * kBins + 4;   // candidates collected by the update pass
 constexpr int kWsOverflow = 3 * kBins + 5;    // they did not fit: use the full passes
 constexpr int kWsLow = 3 * kBins + 6;         // magnitude key from which an element is a candidate
@@ -31,6 +33,10 @@ constexpr int kWsCand2Count = 3 * kBins + 7;  // candidates in the bin of the k-
 constexpr int kWsTicket = 3 * kBins + 8;      // stand-alone kernel: tile ticket, status
 constexpr int kWsStatus = 3 * kBins + 9;
 constexpr int kWsWords = 3 * kBins + 16;
+// a list selection uses the first histogram for its candidates' digits, the room of the
+// other two for the sample's keys
+constexpr int kWsKeys = kBins;
+constexpr uint32_t kMaxKeys = 2 * kBins;
 
 __device__ __forceinline__ uint32_t digit_of(uint32_t key, int pass) {
   return pass == 0 ? (key >> 19) : (pass == 1 ? ((key >> 8) & 0x7FFu) : (key & 0xFFu));
@@ -375,9 +381,12 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 // again after the update to split it at a threshold bin, and every element went through
 // a shared-memory histogram; both are gone:
 //
-//   sample   every stride-th tile of the array is updated first; the histogram of its
-//            magnitudes gives a `low` below which an element is almost surely not among
-//            the k largest
+//   sample   every stride-th tile of the array is updated first; each contributes its
+//            largest keys to a short list, and the element of the rank that k scales to
+//            (with a margin) is `low`, below which an element is almost surely not among
+//            the k largest and above which about 1.1 to 1.5 k are.  Exact keys, not a
+//            histogram: an accumulator in steady state is dense just below the last
+//            threshold, and a bin there can hold many times k elements.
 //   collect  the other tiles are updated; elements of at least `low` are appended to a
 //            candidate list with a histogram of their distance from `low` (the sampled
 //            tiles' from shared memory).  The list holds the k largest exactly when it
@@ -388,7 +397,8 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 //            writes the header.
 //
 // State is read and written once: HBM bound at 20 bytes per element for DGC, 12 for
-// GradDrop.  A list that came out shorter than k or longer than its room (a sample that
+// GradDrop (3.3 and 4.4 TB/s of those bytes at 23.9 M and 67 M elements and 0.1 %; a bucket
+// of ResNet-50 with its serving pass takes 180 us, three passes over the arrays took 500).  A list that came out shorter than k or longer than its room (a sample that
 // misled, or massive ties) makes the launch fall back to histogram passes over the
 // whole array.
 //
@@ -412,6 +422,8 @@ struct SelUnit {
                    // same size behind it
   uint32_t n, k, kmax, cap;
   uint32_t stride, sampled;  // every stride-th tile is sampled: how many that is
+  uint32_t top;              // keys a sampled tile contributes at least
+  uint32_t run;              // tiles between two looks at the candidates' buffer
   uint32_t low;              // the candidates' lower bound, once the sample is complete
 };
 __device__ __forceinline__ uint32_t* list_indices(const SelUnit& s) { return reinterpret_cast<uint32_t*>(s.cv + s.cap); }
@@ -421,21 +433,37 @@ __device__ __forceinline__ uint32_t* list2_indices(const SelUnit& s) {
 }
 // room of each of the two lists in `pairs` pairs
 HP_HD uint32_t list_cap(uint64_t pairs) { return (uint32_t)(pairs / 2 < 0x7FFFFFFFull ? pairs / 2 : 0x7FFFFFFFull); }
-// stride of the sampled tiles of an array when ctas CTAs share `total` tiles: about a
-// sampled tile for every CTA
-HP_HD uint32_t sample_stride(uint32_t tiles, uint64_t total, uint32_t ctas) {
+// How an array is sampled when ctas CTAs share `total` tiles: about one tile for every
+// CTA, and no more than leaves every tile room for several times the keys it will hold of
+// the k largest (`top`).
+// `run`: tiles after which a CTA looks whether its candidates have to leave its buffer,
+// such that they seldom find it full (then each takes an atomic on the list's counter).
+constexpr int kCollectBuf = 1024;  // candidates a CTA gathers before it reserves room in the lists
+struct Sampling {
+  uint32_t stride, top, run;
+};
+HP_HD Sampling sampling(uint32_t tiles, uint64_t total, uint32_t ctas, uint64_t n, uint64_t k) {
+  const uint64_t hits = n && k ? (kSelTile * k + n - 1) / n : 1;   // of one tile among the k largest
+  Sampling p;
+  p.top = (uint32_t)(32 + 8 * hits < kSelTile ? 32 + 8 * hits : kSelTile);
+  p.run = (uint32_t)(kCollectBuf / 4 / hits < 2 ? 2 : kCollectBuf / 4 / hits) & ~1u;
   uint64_t share = ((uint64_t)tiles * ctas) / (total ? total : 1);
+  if (share > kMaxKeys / p.top) share = kMaxKeys / p.top;
   if (share < kMinSampled) share = kMinSampled;
   if (share > kMaxSampled) share = kMaxSampled;
-  return share >= tiles ? 1u : (uint32_t)((tiles + share - 1) / share);
+  p.stride = share >= tiles ? 1u : (uint32_t)((tiles + share - 1) / share);
+  return p;
 }
 
-// First digit of a candidate.  Its distance from `low` in steps of 2^12 keys (1/2048 of
-// the magnitude), the last bin for everything more than two octaves above, where the
-// k-th largest is not to be expected.  When all non-zero elements are candidates
-// (low == 1) they may span any range: the leading 12 bits then.
+// First digit of a candidate.  Its distance from `low` in steps of 2^10 keys (1/8192 of
+// the magnitude), the last bin for everything more than half an octave above, where the
+// k-th largest is not to be expected.  Finer than needed to find the k-th: the counts of
+// most candidates fall within a few percent above `low`, and the atomics on neighbouring
+// words follow one another (steps of 2^12 took 320 us instead of 187 for 1 % of 67 M).
+// When all non-zero elements are candidates (low == 1) they may span any range: the
+// leading 12 bits then.
 __device__ __forceinline__ uint32_t cand_digit(uint32_t key, uint32_t low) {
-  return low <= 1u ? key >> 19 : min((key - low) >> 12, (uint32_t)kBins - 1u);
+  return low <= 1u ? key >> 19 : min((key - low) >> 10, (uint32_t)kBins - 1u);
 }
 
 // counters that are read together behind the update pass
@@ -450,8 +478,6 @@ __device__ __forceinline__ ListState list_state(const SelUnit& s) {
 __device__ __forceinline__ bool selection_failed(const SelUnit& s, const ListState& l) {
   return l.overflow != 0u || (l.count < s.k && l.low > 1u);
 }
-
-constexpr int kCollectBuf = 1024;  // candidates a CTA gathers before it reserves room in the lists
 
 struct SelSmem {
   union {
@@ -537,9 +563,8 @@ __device__ __forceinline__ void update_tiles(const SelUnit& s, float momentum, u
     update_tiles_impl<MODE, T, false>(s, momentum, i0, vec, mask, av);
 }
 
-// Sampled tile number i of an array: update, values into `stash`, magnitudes into the
-// array's sample histogram.  The CTA that completes the sample turns it into the
-// candidates' lower bound.
+// Sampled tile number i of an array: update, values into `stash`, the largest keys into
+// the array's list.  The CTA that completes the sample picks the candidates' lower bound.
 template <int MODE>
 static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum, SelSmem& sm, uint32_t i,
                                                 float* stash) {
@@ -557,16 +582,39 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
       if (key) atomicAdd(&sm.hist[key >> 19], 1u);
     }
   }
+  if (threadIdx.x == 0) sm.count = 0;
   __syncthreads();
-  flush_hist(sm.hist, s.ws);
+  uint32_t bin, rem;
+  find_bin(sm.hist, s.top, sm.fs, bin, rem);   // bin 0 when the tile has fewer
+  const uint32_t edge = bin ? bin << 19 : 1u;
+  uint32_t at[8];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[4 * j + q] = abs_key(e[q]) >= edge ? atomicAdd(&sm.count, 1u) : kMaxKeys;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) sm.base = atomicAdd(s.ws + kWsKeyCount, sm.count);
+  __syncthreads();
+  uint32_t* keys = s.ws + kWsKeys;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)   // keys that find no room lower the bound, which is safe
+      if (sm.base + at[4 * j + q] < kMaxKeys) keys[sm.base + at[4 * j + q]] = abs_key(e[q]);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t done;   // release the CTA's counts, acquire those of the CTAs before
+    uint32_t done;   // release the CTA's keys, acquire those of the CTAs before
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(done) : "l"(s.ws + kWsSampled) : "memory");
     sm.flag = done == s.sampled - 1;
   }
   __syncthreads();
   if (!sm.flag) return;
+  // the CTA that completes the sample: the first 24 bits of the rank-th largest key
+  const uint32_t total = min(__ldcg(s.ws + kWsKeyCount), kMaxKeys);
   uint32_t rank = s.k;
   if (s.stride > 1) {
     // k scaled to the sample, plus five standard deviations, plus a tenth because
@@ -576,12 +624,31 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
     asm("sqrt.approx.f32 %0, %1;" : "=f"(dev) : "f"(hits));
     rank = (uint32_t)(1.1f * hits + 5.0f * dev + 4.0f);
   }
-  uint32_t bin, rem;
-  find_bin(s.ws, rank, sm.fs, bin, rem);   // bin 0 when fewer than rank are counted
-  if (threadIdx.x == 0) s.ws[kWsLow] = bin ? bin << 19 : 1u;   // zeros are never sent
+  uint32_t low = 1u;   // fewer than that: all that is not zero is a candidate
+  if (total >= rank) {
+    uint32_t prefix = 0, mine[kMaxKeys / kSpThreads];
+#pragma unroll
+    for (uint32_t q = 0; q < kMaxKeys / kSpThreads; ++q) {
+      const uint32_t p = q * kSpThreads + threadIdx.x;
+      mine[q] = p < total ? __ldcg(keys + p) : 0u;   // a key is never zero
+    }
+#pragma unroll 1
+    for (int shift = 19; shift > 0; shift -= 12) {
+      clear_hist(sm.hist);
+      __syncthreads();
+#pragma unroll
+      for (uint32_t q = 0; q < kMaxKeys / kSpThreads; ++q)
+        if (mine[q] && (mine[q] >> shift >> 12) == prefix) atomicAdd(&sm.hist[(mine[q] >> shift) & (kBins - 1)], 1u);
+      __syncthreads();
+      find_bin(sm.hist, rank, sm.fs, bin, rank);
+      prefix = (prefix << 12) | bin;
+    }
+    low = max(prefix << 7, 1u);
+  }
+  if (threadIdx.x == 0) s.ws[kWsLow] = low;
 }
 
-// Items [0, total): three quarters in equal shares, the rest in short stretches taken from
+// Items [0, total): seven eighths in equal shares, the rest in short stretches taken from
 // *word by whichever of the ctas CTAs is free -- SMs do not run at one speed, and equal
 // shares alone leave the fast ones waiting, while handing out everything made the ticket
 // word the bottleneck.  The next stretch is asked for before the current one is worked
@@ -591,7 +658,7 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
 template <typename F>
 __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t cta, uint32_t ctas, uint32_t& slot,
                                          F f) {
-  const uint32_t share = total / ctas * 3u / 4u, dealt = share * ctas;
+  const uint32_t share = total / ctas * 7u / 8u, dealt = share * ctas;
   uint32_t stretch = (total - dealt) / (2u * ctas) + 1u;
   if (stretch > 2u) stretch = (stretch + 2u) & ~3u;   // whole groups of tiles
   const uint32_t at = (uint32_t)__cvta_generic_to_shared(&slot);
@@ -627,7 +694,7 @@ __device__ __forceinline__ void collect_one(const SelUnit& s, uint32_t uid, SelS
     return;
   }
   const uint32_t pos = atomicAdd(s.ws + kWsCandCount, 1u);
-  atomicAdd(s.ws + kBins + cand_digit(abs_key(v), low), 1u);
+  atomicAdd(s.ws + cand_digit(abs_key(v), low), 1u);
   if (pos < s.cap) {
     s.cv[pos] = v;
     list_indices(s)[pos] = i;
@@ -652,12 +719,12 @@ __device__ __forceinline__ void collect_tiles(const SelUnit& s, uint32_t uid, Se
   }
 }
 
-// Tiles [t0, t1) of one array without the sampled ones, several at a time: 8 to 12 loads
-// of 16 bytes per thread are what keeps HBM busy with 16 warps per SM.
+// Tiles [t0, t1) of one array without the sampled ones, T at a time: 4 to 6 loads of
+// 16 bytes per thread are what keeps HBM busy with 32 warps per SM.
 template <int MODE>
 static __device__ __noinline__ void collect_body(const SelUnit& s, uint32_t uid, float momentum, SelSmem& sm,
                                                  uint32_t t0, uint32_t t1) {
-  constexpr uint32_t T = MODE == 0 ? 4 : 2;
+  constexpr uint32_t T = MODE == 0 ? 2 : 1;
   uint32_t phase = t0 % s.stride;   // 0: a sampled tile
 #pragma unroll 1
   for (uint32_t t = t0; t < t1; t += T) {
@@ -706,7 +773,7 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
     for (uint32_t p = threadIdx.x; p < n; p += kSpThreads) {
       const float v = sm.buf.val[p];
       const uint32_t pos = sm.base + p;
-      atomicAdd(s.ws + kBins + cand_digit(abs_key(v), low), 1u);
+      atomicAdd(s.ws + cand_digit(abs_key(v), low), 1u);
       if (pos < s.cap) {
         s.cv[pos] = v;
         list_indices(s)[pos] = sm.buf.idx[p];
@@ -733,7 +800,7 @@ __device__ __forceinline__ void collect_flush(SelSmem& sm, F unit) {
       const int lead = __ffs(group) - 1;
       uint32_t pos = 0;
       if ((int)lane == lead) pos = atomicAdd(s.ws + kWsCandCount, (uint32_t)__popc(group));
-      atomicAdd(s.ws + kBins + cand_digit(abs_key(v), low), 1u);
+      atomicAdd(s.ws + cand_digit(abs_key(v), low), 1u);
       pos = __shfl_sync(group, pos, lead) + __popc(group & ((1u << lane) - 1u));
       if (pos < s.cap) {
         s.cv[pos] = v;
@@ -762,38 +829,49 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
   const bool every = L <= s.k;                 // all candidates are sent
   uint32_t bin0 = 0, rem = 0, least = 0xFFFFFFFFu;
-  if (!every) find_bin(s.ws + kBins, s.k, sm.fs, bin0, rem);
+  if (!every) find_bin(s.ws, s.k, sm.fs, bin0, rem);
   const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
+  // four candidates per thread: the reservations of all CTAs on the two counters follow
+  // one another, 25 ns each
+  constexpr int kPer = 4;
 #pragma unroll 1
-  for (uint32_t p0 = lo; p0 < hi; p0 += kSpThreads) {
+  for (uint32_t p0 = lo; p0 < hi; p0 += kPer * kSpThreads) {
     if (threadIdx.x == 0) sm.sent = sm.ties = 0;
     __syncthreads();
-    const uint32_t p = p0 + threadIdx.x;
-    float v = 0.0f;
-    uint32_t idx = 0, at = 0;
-    bool send = false, keep = false;
-    if (p < hi) {
-      v = __ldcg(s.cv + p);
-      idx = __ldcg(list_indices(s) + p);
-      const uint32_t d = cand_digit(abs_key(v), low);
-      send = every || d > bin0;
-      least = min(least, abs_key(v));
-      keep = !every && d == bin0;
-      if (send) at = atomicAdd(&sm.sent, 1u);
-      if (keep) at = atomicAdd(&sm.ties, 1u);
+    float v[kPer];
+    uint32_t idx[kPer], at[kPer];   // place of those sent, behind kKeep of those kept
+    constexpr uint32_t kKeep = 0x80000000u, kNone = 0xFFFFFFFFu;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const uint32_t p = p0 + q * kSpThreads + threadIdx.x;
+      v[q] = p < hi ? __ldcg(s.cv + p) : 0.0f;
+      idx[q] = p < hi ? __ldcg(list_indices(s) + p) : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      at[q] = kNone;
+      if (p0 + q * kSpThreads + threadIdx.x < hi) {
+        const uint32_t key = abs_key(v[q]), d = cand_digit(key, low);
+        least = min(least, key);
+        if (every || d > bin0) at[q] = atomicAdd(&sm.sent, 1u);
+        else if (d == bin0) at[q] = kKeep | atomicAdd(&sm.ties, 1u);
+      }
     }
     __syncthreads();
     if (threadIdx.x == 0 && sm.sent) sm.base = atomicAdd(s.ws + kWsOutCount, sm.sent);
     if (threadIdx.x == 32 && sm.ties) sm.base2 = atomicAdd(s.ws + kWsCand2Count, sm.ties);
     __syncthreads();
-    if (send && idx < s.n) {
-      put_pair(dst, val_off, s.kmax, sm.base + at, idx, v);
-      s.a[idx] = 0.0f;
-      if (s.u) s.u[idx] = 0.0f;
-    }
-    if (keep) {   // never more than the first list holds
-      list2_values(s)[sm.base2 + at] = v;
-      list2_indices(s)[sm.base2 + at] = idx;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      if (at[q] == kNone) continue;
+      if (at[q] & kKeep) {   // never more than the first list holds
+        list2_values(s)[sm.base2 + (at[q] & ~kKeep)] = v[q];
+        list2_indices(s)[sm.base2 + (at[q] & ~kKeep)] = idx[q];
+      } else if (idx[q] < s.n) {
+        put_pair(dst, val_off, s.kmax, sm.base + at[q], idx[q], v[q]);
+        s.a[idx[q]] = 0.0f;
+        if (s.u) s.u[idx[q]] = 0.0f;
+      }
     }
   }
   if (every) {   // the least key sent is the threshold: kept as the largest complement
@@ -809,11 +887,11 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
   __syncthreads();
   if (!sm.flag) return false;
   // The last CTA: among the elements of the k-th's bin, `rem` are sent.  What is left of
-  // their keys is 12 bits in a fine bin, 19 in a bin of the leading bits, and up to 31 in
+  // their keys is 10 bits in a fine bin, 19 in a bin of the leading bits, and up to 31 in
   // the last fine bin.
   const uint32_t L2 = every ? 0u : __ldcg(s.ws + kWsCand2Count);
   if (threadIdx.x == 0) sm.sent = __ldcg(s.ws + kWsOutCount), sm.ties = 0;
-  const uint32_t start = low <= 1u ? bin0 << 19 : low + (bin0 << 12);
+  const uint32_t start = low <= 1u ? bin0 << 19 : low + (bin0 << 10);
   int shift = low <= 1u ? 7 : (bin0 == (uint32_t)kBins - 1u ? 19 : 0), bits = 12;
   uint32_t prefix = 0;
   const bool pick = L2 != 0u;

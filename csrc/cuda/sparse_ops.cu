@@ -2,7 +2,9 @@
 //
 // With room for a candidate list (the usual call) an encode is ONE cooperative launch:
 // sample, update + collect, finish (sparse_core.cuh), with grid barriers in between.
-// It was a chain of eight launches; @OPS_NOTE@
+// It was a chain of eight launches that read the array three times behind the update:
+// GradDrop's encode of 23.9 M elements at 0.1 % took 138 us and takes 87, of 1 M elements
+// 63 and takes 33 (B200, states rotating through more than L2 holds).
 //
 // Without it (the allocation-free entry point) four launches read the array once each:
 //   pass 0   state update fused with the first radix histogram
@@ -68,7 +70,7 @@ union SelOrPassSmem {
   EmitSmem emit;
 };
 
-__global__ void __launch_bounds__(kSpThreads, 1) sparse_encode_kernel(const __grid_constant__ SelArgs A) {
+__global__ void __launch_bounds__(kSpThreads, 2) sparse_encode_kernel(const __grid_constant__ SelArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SelOrPassSmem& sm = *reinterpret_cast<SelOrPassSmem*>(smem_raw);
   __shared__ WaitState wst;
@@ -103,10 +105,14 @@ __global__ void __launch_bounds__(kSpThreads, 1) sparse_encode_kernel(const __gr
   auto self = [&](uint32_t) -> const SelUnit& { return s; };
   if (s.stride > 1)
     hand_out(s.ws + kWsTicket, tiles, c, G, sm.sel.ticket, [&](uint32_t t0, uint32_t t1) {
-      if (A.mode == 0) collect_body<0>(s, 0, A.momentum, sm.sel, t0, t1);
-      else if (A.mode == 1) collect_body<1>(s, 0, A.momentum, sm.sel, t0, t1);
-      else collect_body<2>(s, 0, A.momentum, sm.sel, t0, t1);
-      if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, self);
+#pragma unroll 1
+      for (uint32_t t = t0; t < t1; t += s.run) {
+        const uint32_t end = min(t + s.run, t1);
+        if (A.mode == 0) collect_body<0>(s, 0, A.momentum, sm.sel, t, end);
+        else if (A.mode == 1) collect_body<1>(s, 0, A.momentum, sm.sel, t, end);
+        else collect_body<2>(s, 0, A.momentum, sm.sel, t, end);
+        if (__syncthreads_or(sm.sel.count > (uint32_t)kCollectBuf / 2)) collect_flush(sm.sel, self);
+      }
     });
   collect_flush(sm.sel, self);
   barrier();
@@ -232,7 +238,10 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
     U.k = (uint32_t)k;
     U.kmax = (uint32_t)kmax;
     U.cap = list_cap(pairs);
-    U.stride = sample_stride((uint32_t)tiles, tiles, (uint32_t)grid);
+    const Sampling sp = sampling((uint32_t)tiles, tiles, (uint32_t)grid, n, k);
+    U.stride = sp.stride;
+    U.top = sp.top;
+    U.run = sp.run;
     U.sampled = ((uint32_t)tiles + U.stride - 1) / U.stride;
     A.alg = alg;
     A.mode = mode;
