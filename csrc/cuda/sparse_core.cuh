@@ -25,7 +25,6 @@ constexpr int kWsOutCount = 3 * kBins + 0;
 constexpr int kWsTieCount = 3 * kBins + 1;
 constexpr int kWsDone = 3 * kBins + 2;
 constexpr int kWsSampled = 3 * kBins + 3;     // sampled tiles that are done
-constexpr int kWsKeyCount = 3 * kBins + 10;   // keys the sampled tiles contributed
 constexpr int kWsCandCount = 3 * kBins + 4;   // candidates collected by the update pass
 constexpr int kWsOverflow = 3 * kBins + 5;    // they did not fit: use the full passes
 constexpr int kWsLow = 3 * kBins + 6;         // magnitude key from which an element is a candidate
@@ -435,7 +434,7 @@ __device__ __forceinline__ uint32_t* list2_indices(const SelUnit& s) {
 HP_HD uint32_t list_cap(uint64_t pairs) { return (uint32_t)(pairs / 2 < 0x7FFFFFFFull ? pairs / 2 : 0x7FFFFFFFull); }
 // How an array is sampled when ctas CTAs share `total` tiles: about one tile for every
 // CTA, and no more than leaves every tile room for several times the keys it will hold of
-// the k largest (`top`).
+// the k largest (`top`), and half as many again.
 // `run`: tiles after which a CTA looks whether its candidates have to leave its buffer,
 // such that they seldom find it full (then each takes an atomic on the list's counter).
 constexpr int kCollectBuf = 1024;  // candidates a CTA gathers before it reserves room in the lists
@@ -445,10 +444,10 @@ struct Sampling {
 HP_HD Sampling sampling(uint32_t tiles, uint64_t total, uint32_t ctas, uint64_t n, uint64_t k) {
   const uint64_t hits = n && k ? (kSelTile * k + n - 1) / n : 1;   // of one tile among the k largest
   Sampling p;
-  p.top = (uint32_t)(32 + 8 * hits < kSelTile ? 32 + 8 * hits : kSelTile);
+  p.top = (uint32_t)(24 + 4 * hits < kSelTile / 2 ? 24 + 4 * hits : kSelTile / 2);
   p.run = (uint32_t)(kCollectBuf / 4 / hits < 2 ? 2 : kCollectBuf / 4 / hits) & ~1u;
   uint64_t share = ((uint64_t)tiles * ctas) / (total ? total : 1);
-  if (share > kMaxKeys / p.top) share = kMaxKeys / p.top;
+  if (share > kMaxKeys * 2 / 3 / p.top) share = kMaxKeys * 2 / 3 / p.top;   // `top` rounded up to whole bins
   if (share < kMinSampled) share = kMinSampled;
   if (share > kMaxSampled) share = kMaxSampled;
   p.stride = share >= tiles ? 1u : (uint32_t)((tiles + share - 1) / share);
@@ -594,16 +593,16 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
 #pragma unroll
     for (int q = 0; q < 4; ++q) at[4 * j + q] = abs_key(e[q]) >= edge ? atomicAdd(&sm.count, 1u) : kMaxKeys;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) sm.base = atomicAdd(s.ws + kWsKeyCount, sm.count);
-  __syncthreads();
+  // places of its own: a reservation behind 100 others took 2 us.  Keys that find no room
+  // are left out, which lowers the bound: safe.
+  const uint32_t room = kMaxKeys / s.sampled;
   uint32_t* keys = s.ws + kWsKeys;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
 #pragma unroll
-    for (int q = 0; q < 4; ++q)   // keys that find no room lower the bound, which is safe
-      if (sm.base + at[4 * j + q] < kMaxKeys) keys[sm.base + at[4 * j + q]] = abs_key(e[q]);
+    for (int q = 0; q < 4; ++q)
+      if (at[4 * j + q] < room) keys[i * room + at[4 * j + q]] = abs_key(e[q]);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -614,7 +613,6 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
   __syncthreads();
   if (!sm.flag) return;
   // the CTA that completes the sample: the first 24 bits of the rank-th largest key
-  const uint32_t total = min(__ldcg(s.ws + kWsKeyCount), kMaxKeys);
   uint32_t rank = s.k;
   if (s.stride > 1) {
     // k scaled to the sample, plus five standard deviations, plus a tenth because
@@ -624,33 +622,30 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
     asm("sqrt.approx.f32 %0, %1;" : "=f"(dev) : "f"(hits));
     rank = (uint32_t)(1.1f * hits + 5.0f * dev + 4.0f);
   }
-  uint32_t low = 1u;   // fewer than that: all that is not zero is a candidate
-  if (total >= rank) {
-    uint32_t prefix = 0, mine[kMaxKeys / kSpThreads];
+  uint32_t prefix = 0, mine[kMaxKeys / kSpThreads];
 #pragma unroll
-    for (uint32_t q = 0; q < kMaxKeys / kSpThreads; ++q) {
-      const uint32_t p = q * kSpThreads + threadIdx.x;
-      mine[q] = p < total ? __ldcg(keys + p) : 0u;   // a key is never zero
-    }
+  for (uint32_t q = 0; q < kMaxKeys / kSpThreads; ++q) mine[q] = __ldcg(keys + q * kSpThreads + threadIdx.x);
 #pragma unroll 1
-    for (int shift = 19; shift > 0; shift -= 12) {
-      clear_hist(sm.hist);
-      __syncthreads();
+  for (int shift = 19; shift > 0; shift -= 12) {
+    clear_hist(sm.hist);
+    __syncthreads();
 #pragma unroll
-      for (uint32_t q = 0; q < kMaxKeys / kSpThreads; ++q)
-        if (mine[q] && (mine[q] >> shift >> 12) == prefix) atomicAdd(&sm.hist[(mine[q] >> shift) & (kBins - 1)], 1u);
-      __syncthreads();
-      find_bin(sm.hist, rank, sm.fs, bin, rank);
-      prefix = (prefix << 12) | bin;
-    }
-    low = max(prefix << 7, 1u);
+    for (uint32_t q = 0; q < kMaxKeys / kSpThreads; ++q)   // a place not taken holds zero
+      if (mine[q] && (mine[q] >> shift >> 12) == prefix) atomicAdd(&sm.hist[(mine[q] >> shift) & (kBins - 1)], 1u);
+    __syncthreads();
+    find_bin(sm.hist, rank, sm.fs, bin, rem);
+    if (rem == 0) break;   // fewer keys than that: all that is not zero is a candidate
+    rank = rem;
+    prefix = (prefix << 12) | bin;
   }
+  const uint32_t low = rem ? max(prefix << 7, 1u) : 1u;
   if (threadIdx.x == 0) s.ws[kWsLow] = low;
 }
 
 // Items [0, total).  Below 32 per CTA in equal shares: the tickets of all CTAs follow one
-// another, 25 ns each, and took longer than the SMs' unequal speed costs (24 us instead of
-// 23 for 1600 tiles, 33 instead of 30 for 5844).  Above, seven eighths in equal shares, the rest in short stretches taken from
+// another, 25 ns each, and took longer than the SMs' unequal speed costs (24 us instead
+// of 23 for 1600 tiles, 33 instead of 30 for 5844).  Above, seven eighths in equal
+// shares, the rest in short stretches taken from
 // *word by whichever of the ctas CTAs is free -- SMs do not run at one speed, and equal
 // shares alone leave the fast ones waiting, while handing out everything made the ticket
 // word the bottleneck.  The next stretch is asked for before the current one is worked
