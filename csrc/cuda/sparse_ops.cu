@@ -203,7 +203,7 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
   // histograms and counters, then the barrier words and the candidate lists
   const uint64_t head = (uint64_t)(kWsWords + kBarrierWords) * 4;
   const uint64_t pairs = ws_bytes > head ? (ws_bytes - head) / 8 : 0;
-  const bool listed = pairs >= 1024;
+  const bool listed = pairs >= 1024 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0;   // counters are read as uint4
   cudaError_t e = cudaMemsetAsync(ws, 0, listed ? head : (size_t)kWsWords * 4, st);
   if (e != cudaSuccess) return (int)e;
   if (listed) {

@@ -71,3 +71,14 @@ def test_selection_with_massive_ties_sends_exactly_k():
     assert idx.numel() == k and idx.unique().numel() == k
     assert torch.equal(g.cpu()[idx], val) and bool((val != 0).all())
     assert int((st["residual"] != 0).sum()) == int((g != 0).sum()) - k
+
+
+def test_selection_with_a_workspace_off_alignment():
+    """Four bytes off: the launch that reads its counters 16 bytes at a time is not taken."""
+    n = 100003
+    torch.manual_seed(2)
+    g, c = torch.randn(n), Compressor("graddrop", ratio=0.01)
+    ws = torch.cat([c.new_workspace("cuda", n), torch.zeros(1, dtype=torch.int32, device="cuda")])[1:]
+    ic, vc = sparse_pairs(c.encode(g, c.new_state(n, "cpu")), c.kmax(n))
+    ig, vg = sparse_pairs(c.encode(g.cuda(), c.new_state(n, "cuda"), workspace=ws), c.kmax(n))
+    assert torch.equal(ic, ig) and torch.equal(vc, vg)
