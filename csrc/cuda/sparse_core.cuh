@@ -59,12 +59,24 @@ static __device__ __noinline__ void find_bin(const uint32_t* hist, uint32_t k, F
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint4 c[kRows];
   uint32_t rows[kRows], all = 0;
+  const uint32_t* from = hist + warp * (kRows * 128) + lane * 4;
+  if ((reinterpret_cast<uintptr_t>(hist) & 15) == 0) {
 #pragma unroll
-  for (int j = 0; j < kRows; ++j)
-    asm volatile("ld.volatile.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(c[j].x), "=r"(c[j].y), "=r"(c[j].z), "=r"(c[j].w)
-                 : "l"(hist + warp * (kRows * 128) + j * 128 + lane * 4)
-                 : "memory");
+    for (int j = 0; j < kRows; ++j)
+      asm volatile("ld.volatile.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(c[j].x), "=r"(c[j].y), "=r"(c[j].z), "=r"(c[j].w)
+                   : "l"(from + j * 128)
+                   : "memory");
+  } else {   // a caller's workspace may lie on any word
+#pragma unroll 1
+    for (int j = 0; j < kRows; ++j) {
+      const volatile uint32_t* w = from + j * 128;
+      const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+      for (int q = 0; q < kRows; ++q)
+        if (q == j) c[q] = v;
+    }
+  }
 #pragma unroll
   for (int j = 0; j < kRows; ++j) {
     rows[j] = __reduce_add_sync(0xffffffffu, c[j].x + c[j].y + c[j].z + c[j].w);

@@ -32,7 +32,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kSpThreads)
 sparse_pass0_kernel(const float* __restrict__ g, float* __restrict__ a, float* __restrict__ u,
                     uint64_t n, float momentum, uint32_t* __restrict__ ws) {
-  __shared__ uint32_t sh[kBins];
+  __shared__ __align__(16) uint32_t sh[kBins];
   pass0_body<MODE>(g, a, u, n, momentum, ws, sh, blockIdx.x, gridDim.x);
 }
 
@@ -40,7 +40,7 @@ template <int PASS>
 __global__ void __launch_bounds__(kSpThreads)
 sparse_pass_kernel(const float* __restrict__ a, uint64_t n, uint32_t k,
                    uint32_t* __restrict__ ws) {
-  __shared__ uint32_t sh[kBins];
+  __shared__ __align__(16) uint32_t sh[kBins];
   __shared__ FindSmem fs;
   pass_body<PASS>(a, n, k, ws, sh, fs, blockIdx.x, gridDim.x);
 }
