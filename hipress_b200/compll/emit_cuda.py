@@ -748,7 +748,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _lib = None
 _cpu = None
-_scratch = {{}}
+_ready = {{}}     # device -> (launcher, address of its scratch, scratch)
 _SIG = [{", ".join(ctypes_sig)}]
 
 
@@ -762,6 +762,13 @@ def _load():
     return _lib
 
 
+def _prepare(dev):
+    """First call on a device, which is the current one."""
+    lib = _load()
+    scratch = torch.zeros(int(lib.compll_{name}_scratch_bytes()), dtype=torch.uint8, device="cuda")
+    return _ready.setdefault(dev, (lib.compll_{name}, scratch.data_ptr(), scratch))
+
+
 def _load_cpu():
     global _cpu
     if _cpu is None:
@@ -771,27 +778,31 @@ def _load_cpu():
     return _cpu
 
 
+def _launch({", ".join(args)}, seed, stream, dev):
+    call, scratch, _ = _ready.get(dev) or _prepare(dev)
+    st = torch._C._cuda_getCurrentRawStream(dev) if stream is None else stream.cuda_stream
+    return call({", ".join(conv)}, scratch, seed, st)
+
+
 def {name}({", ".join(args)}, seed=0, stream=None):
     """In-place op: vectors are contiguous torch tensors allocated by the caller,
     all on one device."""
-    vectors = ({", ".join(vecs)},)
-    if any(not t.is_contiguous() for t in vectors):
+    if not ({" and ".join(f"{v}.is_contiguous()" for v in vecs)}):
         raise ValueError("{name}: tensors must be contiguous")
-    if len({{t.device for t in vectors}}) != 1:
+    device = {vecs[0]}.device
+    if {" or ".join(f"{v}.device != device" for v in vecs[1:]) or "False"}:
         raise ValueError("{name}: tensors must share one device")
-    if not vectors[0].is_cuda:
+    if not {vecs[0]}.is_cuda:
         rc = _load_cpu().compll_{name}_cpu({", ".join(conv)}, seed)
         if rc != 0:
             raise RuntimeError(f"{name}: error {{rc}}")
         return
-    lib = _load()
-    dev = vectors[0].device.index
-    with torch.cuda.device(dev):
-        if dev not in _scratch:
-            _scratch[dev] = torch.zeros(int(lib.compll_{name}_scratch_bytes()), dtype=torch.uint8,
-                                        device="cuda")
-        st = (stream or torch.cuda.current_stream()).cuda_stream
-        rc = lib.compll_{name}({", ".join(conv)}, _scratch[dev].data_ptr(), seed, st)
+    dev = device.index
+    if dev == torch._C._cuda_getDevice():   # a device guard takes as long as a small kernel
+        rc = _launch({", ".join(args)}, seed, stream, dev)
+    else:
+        with torch.cuda.device(dev):
+            rc = _launch({", ".join(args)}, seed, stream, dev)
     if rc != 0:
         raise RuntimeError(f"{name}: CUDA error {{rc}}")
 '''
