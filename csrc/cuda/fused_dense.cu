@@ -13,17 +13,16 @@
 //          server residual, store the result into every peer's inbox and decode it;
 //          every rank decodes the other N-1 chunks.
 //
-// What a rank owns never goes through its own inbox: the tile is still in registers
+// What a rank owns does not go through its own inbox: the tile is still in registers
 // when its final codes exist, so the 8-byte slots, the poll and a second visit of the
-// tile are saved for 1/N of the gradient (for all of it on one rank, where VGG-19's
-// gradients took 416 us instead of 443 through TBQ + ring and a base Transformer's
-// 278 us instead of 321 through TernGrad + PS).
+// tile are saved for 1/N of the gradient.  The exception are small PS buckets of many
+// ranks (ps_own_here).
 //
 // There is no NCCL call and no separate encode or decode launch.  Payloads are
 // plain 8-byte stores {codes, epoch} to peer-mapped memory; the receiver polls its
 // own memory until the epoch of this launch shows up (see "transport" below).  A
-// CTA only ever waits for data produced by other GPUs, never for another CTA of
-// its own GPU.  Every wait is bounded: on expiry the thread records a status
+// CTA waits for data produced by other GPUs, and for another CTA of its own GPU only
+// where the own push takes the inbox.  Every wait is bounded: on expiry the thread records a status
 // word, the CTA stops waiting and still runs to completion inside its own
 // buffers.  g and r tiles are prefetched with bulk copies (pipeline.cuh).
 //
@@ -297,14 +296,10 @@ __device__ __forceinline__ PhaseSpec phase_spec(int ph, int N, int R) {
       p.ndst = N - 1; p.dst0 = (R + 1) % N; p.dst_slot = N - 1 + R;
     }
     p.salt = (uint32_t)(R * 256 + ph);
-  } else {  // PS: push to the remote owners first, own chunk (push and serve) last
+  } else {  // PS push: remote owners first, own chunk last
     p.chunk = (R + 1 + ph) % N;
     p.in_slot = -1;
-    if (ph < N - 1) {
-      p.ndst = 1; p.dst0 = p.chunk; p.dst_slot = R;
-    } else {
-      p.ndst = N - 1; p.dst0 = (R + 1) % N; p.dst_slot = N + R;
-    }
+    p.ndst = 1; p.dst0 = p.chunk; p.dst_slot = R;
     p.salt = (uint32_t)(R * 256);
   }
   return p;
@@ -318,7 +313,8 @@ struct TileRef {
 };
 
 // Work distribution.  A launch is a sequence of phases (N encode phases, the last of
-// which finishes the rank's own chunk, then N-1 gathers); every phase visits the
+// which finishes the rank's own chunk, then N-1 gathers; a PS launch whose own chunk
+// takes the inbox has N pushes, the serving phase and N pulls); every phase visits the
 // T = tiles_total tiles of one chunk of every tensor.  Tile i of phase ph is
 // work item ph * T + i, and item w belongs to CTA w % G: the assignment keeps
 // rotating across phases, so a bucket whose chunk has fewer tiles than there are
@@ -326,8 +322,8 @@ struct TileRef {
 // for their input while the earlier hops run elsewhere), and a chunk that is not
 // a multiple of G tiles leaves no CTA idle for a whole phase.  Every CTA takes its
 // items in increasing order, and an item only ever depends on a lower-numbered
-// item of another GPU, so the lowest unfinished item can always run: the grid must
-// fit the GPU (the launcher clamps it), nothing else is needed for progress.
+// item, so the lowest unfinished item can always run: the grid must fit the GPU (the
+// launcher clamps it), nothing else is needed for progress.
 struct Cursor {
   int phase, seg, chunk;
   uint32_t rot;          // (phase * T) % G
@@ -407,57 +403,121 @@ __device__ __forceinline__ void trace_phase(const HpComm& cm, int E, int ph, Wai
   }
 }
 
+// The prefetcher of one CTA: it runs ahead of the consumer over the same tile sequence,
+// across phases.
+struct Feed {
+  Cursor prod;
+  bool more;
+  uint32_t issued, consumed;  // tiles prefetched / used through the bulk pipeline
+};
+
+template <int TOPO>
+__device__ __forceinline__ void feed_begin(const BucketDev& bk, int N, int R, Feed& f) {
+  cursor_begin(bk, (int)gridDim.x, (int)blockIdx.x, 0, phase_spec<TOPO>(0, N, R).chunk, f.prod);
+  f.more = true;
+  f.issued = f.consumed = 0;
+}
+
+// top up the prefetch pipeline (stages of finished tiles are free: the previous tile
+// ended with a CTA barrier)
+template <int TOPO>
+__device__ __forceinline__ void feed_top_up(const BucketDev& bk, const HpComm& cm, FusedSmem& sm, int R, int E,
+                                            Feed& f, int N, int G, int b) {
+  while (f.more && f.issued - f.consumed < kStages) {
+    TileRef pr;
+    bool got = cursor_next(bk, G, b, f.prod, pr);
+    while (!got && f.prod.phase + 1 < N) {  // run ahead across phases
+      cursor_begin(bk, G, b, f.prod.phase + 1, phase_spec<TOPO>(f.prod.phase + 1, N, R).chunk, f.prod);
+      got = cursor_next(bk, G, b, f.prod, pr);
+    }
+    if (!got) {
+      f.more = false;
+      break;
+    }
+    const SegDev& psg = bk.seg[pr.seg];
+    const float* pg = psg.g + E * cm.emu_stride_g + pr.off;
+    const float* prr = psg.r ? psg.r + E * cm.emu_stride_r + pr.off : nullptr;
+    if (bulk_ok(pg, prr, pr.m)) {
+      if (threadIdx.x == 0) {
+        const int st = f.issued % kStages;
+        mbar_expect_tx(&sm.full[st], (prr ? 2u : 1u) * kTile * 4u);
+        bulk_load(sm.g[st], pg, kTile * 4u, &sm.full[st]);
+        if (prr) bulk_load(sm.r[st], prr, kTile * 4u, &sm.full[st]);
+      }
+      ++f.issued;
+    }
+  }
+}
+
+// the next tile's gradient into x; returns its stage, or -1 when it was not prefetched
+__device__ __forceinline__ int feed_take(const HpComm& cm, FusedSmem& sm, const float* gp, const float* rp, int m,
+                                         uint32_t* status, Feed& f, float (&x)[kIter][4]) {
+  if (!bulk_ok(gp, rp, m)) {
+    load_tile(gp, m, x);
+    return -1;
+  }
+  const int st = f.consumed % kStages;
+  if (!sm.ws.poisoned && !mbar_wait_bounded(&sm.full[st], (f.consumed / kStages) & 1, cm.timeout_ns, status,
+                                            HP_STATUS_TIMEOUT | (3u << 16) | (blockIdx.x & 255)))
+    sm.ws.poisoned = 1;
+  ++f.consumed;
+  load_tile_smem(sm.g[st], x);
+  return st;
+}
+
+// x = state + x, from the stage the tile was prefetched into or from memory
+__device__ __forceinline__ void add_state(const float* rp, const FusedSmem& sm, int st, int m, float (&x)[kIter][4]) {
+  float rr[kIter][4];
+  if (st >= 0) load_tile_smem(sm.r[st], rr);
+  else load_tile(rp, m, rr);
+#pragma unroll
+  for (int j = 0; j < kIter; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[j][e] = rr[j][e] + x[j][e];
+}
+
+__device__ __forceinline__ void store_checked(float* p, int m, const float (&x)[kIter][4]) {
+  if (tile_is_full_aligned(p, m)) store_tile_full(p, x);
+  else store_tile(p, m, x);
+}
+
+// one tile's codes to `ndst` ranks from dst0 on (a rolled loop: the broadcast is one
+// phase in N)
+template <int ALG, int B>
+__device__ __forceinline__ void send_to(const BucketDev& bk, const HpComm& cm, const PhaseSpec& ps, const SegDev& sg,
+                                        uint32_t t, const uint32_t (&frag)[kIter], const float (&meta)[2], bool bad,
+                                        uint32_t* status) {
+  uint32_t words[LL<B>::W];
+  pack_words<B>(frag, words);
+  const uint32_t ep = cm.epoch | (bad ? kGaveUp : 0u);
+#pragma unroll 1
+  for (int q = 0; q < ps.ndst; ++q) {
+    int d = ps.dst0 + q;
+    if (d >= cm.nranks) d -= cm.nranks;
+    uint8_t* dst = reinterpret_cast<uint8_t*>(cm.inbox[d]) + (size_t)ps.dst_slot * bk.slot_bytes + sg.pay_off;
+    if (dbg_tile_ok<ALG, B>(bk, cm.inbox[d], dst, t, status, 2u)) send_tile<ALG, B>(dst, t, words, meta, ep);
+  }
+}
+
+// ring: all N hops; PS: the pushes, `phases` of them
 template <int ALG, int B, int TOPO>
 __device__ __forceinline__ void encode_phases(const BucketDev& bk, const HpComm& cm,
                                               const FusedParams& fp, FusedSmem& sm, int R, int E,
-                                              uint32_t* status) {
+                                              uint32_t* status, Feed& feed, int phases) {
   const int N = cm.nranks;
   const int G = (int)gridDim.x;
   const int b = (int)blockIdx.x;
   uint8_t* my_inbox = reinterpret_cast<uint8_t*>(cm.inbox[R]);
-  // prefetcher state: runs ahead of the consumer over the same tile sequence
-  Cursor prod;
-  cursor_begin(bk, G, b, 0, phase_spec<TOPO>(0, N, R).chunk, prod);
-  bool prod_more = true;
-  uint32_t issued = 0, consumed = 0;  // tiles prefetched / used through the bulk pipeline
-
-  for (int ph = 0; ph < N; ++ph) {
+  for (int ph = 0; ph < phases; ++ph) {
     const PhaseSpec ps = phase_spec<TOPO>(ph, N, R);
     Cursor cons;
     cursor_begin(bk, G, b, ph, ps.chunk, cons);
-    const size_t dst_off = (size_t)ps.dst_slot * bk.slot_bytes;
     const uint8_t* in_base =
         ps.in_slot >= 0 ? my_inbox + (size_t)ps.in_slot * bk.slot_bytes : nullptr;
     TileRef tr;
     while (cursor_next(bk, G, b, cons, tr)) {
       const SegDev& sg = bk.seg[tr.seg];
-      // top up the prefetch pipeline (stages of finished tiles are free: the
-      // previous tile ended with a CTA barrier)
-      while (prod_more && issued - consumed < kStages) {
-        TileRef pr;
-        bool got = cursor_next(bk, G, b, prod, pr);
-        while (!got && prod.phase + 1 < N) {  // run ahead across phases
-          cursor_begin(bk, G, b, prod.phase + 1, phase_spec<TOPO>(prod.phase + 1, N, R).chunk,
-                       prod);
-          got = cursor_next(bk, G, b, prod, pr);
-        }
-        if (!got) {
-          prod_more = false;
-          break;
-        }
-        const SegDev& psg = bk.seg[pr.seg];
-        const float* pg = psg.g + E * cm.emu_stride_g + pr.off;
-        const float* prr = psg.r ? psg.r + E * cm.emu_stride_r + pr.off : nullptr;
-        if (bulk_ok(pg, prr, pr.m)) {
-          if (threadIdx.x == 0) {
-            const int st = issued % kStages;
-            mbar_expect_tx(&sm.full[st], (prr ? 2u : 1u) * kTile * 4u);
-            bulk_load(sm.g[st], pg, kTile * 4u, &sm.full[st]);
-            if (prr) bulk_load(sm.r[st], prr, kTile * 4u, &sm.full[st]);
-          }
-          ++issued;
-        }
-      }
+      feed_top_up<TOPO>(bk, cm, sm, R, E, feed, N, G, b);
       const int m = tr.m;
       const uint32_t t = tr.t;
       const float* gp = sg.g + E * cm.emu_stride_g + tr.off;
@@ -468,19 +528,7 @@ __device__ __forceinline__ void encode_phases(const BucketDev& bk, const HpComm&
       const bool has_in = in_base && dbg_tile_ok<ALG, B>(bk, my_inbox, in_base + sg.pay_off, t, status, 1u);
       if (in_base && !has_in) sm.ws.poisoned = 1;
       if (has_in) recv_issue<ALG, B>(in_base + sg.pay_off, t, rx);
-      const bool bulk = bulk_ok(gp, rp, m);
-      int st = 0;
-      if (bulk) {
-        st = consumed % kStages;
-        if (!sm.ws.poisoned &&
-            !mbar_wait_bounded(&sm.full[st], (consumed / kStages) & 1, cm.timeout_ns, status,
-                               HP_STATUS_TIMEOUT | (3u << 16) | (b & 255)))
-          sm.ws.poisoned = 1;
-        ++consumed;
-        load_tile_smem(sm.g[st], x);
-      } else {
-        load_tile(gp, m, x);
-      }
+      const int st = feed_take(cm, sm, gp, rp, m, status, feed, x);
       if (has_in) {
         float d[kIter][4];
         recv_finish<ALG, B>(in_base + sg.pay_off, t, rx, cm, status,
@@ -491,87 +539,106 @@ __device__ __forceinline__ void encode_phases(const BucketDev& bk, const HpComm&
 #pragma unroll
           for (int e = 0; e < 4; ++e) x[j][e] = x[j][e] + d[j][e];
       }
+      if (rp) add_state(rp, sm, st, m, x);
       float meta[2];
       uint32_t frag[kIter];
-      bool bad = false;
-      const bool final_tile = ph == N - 1;  // this rank's own chunk gets its final codes here
-      // PS encodes a tile of the own chunk twice: what this rank pushes, and the sum of
-      // the N pushes (a rolled loop: one copy of the encoder's code)
-#pragma unroll 1
-      for (int pass = 0;; ++pass) {
-        if (rp) {
-          float rr[kIter][4];
-          if (bulk && pass == 0) load_tile_smem(sm.r[st], rr);
-          else load_tile(rp, m, rr);
-#pragma unroll
-          for (int j = 0; j < kIter; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) x[j][e] = rr[j][e] + x[j][e];
-        }
-        encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt + (uint32_t)pass, sm.tile, pass,
-                            meta, frag, rp != nullptr);
-        // after an expired wait the merged input is not a real partial sum: the error
-        // feedback state keeps its last good contents
-        bad = *(volatile int*)&sm.ws.poisoned != 0;
-        if (rp && !bad) {
-          if (tile_is_full_aligned(rp, m)) store_tile_full(rp, x);
-          else store_tile(rp, m, x);
-        }
-        if (TOPO == HP_TOPO_RING || !final_tile || pass == 1) break;
-        // sum the N pushes of this tile in rank order.  The remote ones are polled one
-        // ahead: the loads of the next are in flight while the current one is decoded
-        TileRx<ALG, B> in[2];
-        if (N > 1 && !dbg_tile_ok<ALG, B>(bk, my_inbox, my_inbox + (size_t)(N - 1) * bk.slot_bytes + sg.pay_off,
-                                          t, status, 4u)) {
-          sm.ws.poisoned = 1;   // ll_finish returns at once, nothing is stored
-        } else if (R != 0) {
-          recv_issue<ALG, B>(my_inbox + sg.pay_off, t, in[0]);
-        }
-        for (int q = 0; q < N; ++q) {
-          if (q + 1 < N && q + 1 != R && !sm.ws.poisoned)
-            recv_issue<ALG, B>(my_inbox + (size_t)(q + 1) * bk.slot_bytes + sg.pay_off, t, in[(q + 1) & 1]);
-          float d[kIter][4];
-          if (q == R) {
-#pragma unroll
-            for (int j = 0; j < kIter; ++j) decode_frag<ALG, B>(frag[j], meta, fp.P.tau, d[j]);
-          } else {
-            recv_finish<ALG, B>(my_inbox + (size_t)q * bk.slot_bytes + sg.pay_off, t, in[q & 1], cm,
-                                status, HP_STATUS_TIMEOUT | (1u << 16) | ((uint32_t)q << 8) | (b & 255),
-                                sm.ws, fp.P.tau, d);
-          }
-#pragma unroll
-          for (int j = 0; j < kIter; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) x[j][e] = q > 0 ? x[j][e] + d[j][e] : d[j][e];
-        }
-        rp = sg.sr ? sg.sr + E * cm.emu_stride_sr + (size_t)t * kTile : nullptr;
-      }
-      uint32_t words[LL<B>::W];
-      pack_words<B>(frag, words);
-      const uint32_t ep = cm.epoch | (bad ? kGaveUp : 0u);
-      // one destination on a hop or push, every peer in the last phase (a rolled loop:
-      // the broadcast is one phase in N)
-#pragma unroll 1
-      for (int q = 0; q < ps.ndst; ++q) {
-        int d = ps.dst0 + q;
-        if (d >= N) d -= N;
-        uint8_t* dst = reinterpret_cast<uint8_t*>(cm.inbox[d]) + dst_off + sg.pay_off;
-        if (dbg_tile_ok<ALG, B>(bk, cm.inbox[d], dst, t, status, 2u))
-          send_tile<ALG, B>(dst, t, words, meta, ep);
-      }
-      // the own chunk is decoded from registers (a tile whose input never arrived is
-      // left as it was: the local gradient)
-      if (final_tile && !bad) {
-        float d[kIter][4];
-        decode_average<ALG, B>(frag, meta, fp, d);
-        float* op = sg.out + E * cm.emu_stride_out + tr.off;
-        if (tile_is_full_aligned(op, m)) store_tile_full(op, d);
-        else store_tile(op, m, d);
+      encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt, sm.tile, 0, meta, frag, rp != nullptr);
+      // after an expired wait the merged input is not a real partial sum: the error
+      // feedback state keeps its last good contents
+      const bool bad = *(volatile int*)&sm.ws.poisoned != 0;
+      if (rp && !bad) store_checked(rp, m, x);
+      send_to<ALG, B>(bk, cm, ps, sg, t, frag, meta, bad, status);
+      // the own chunk gets its final codes in the last hop and is decoded from registers
+      // (a tile whose input never arrived is left as it was: the local gradient)
+      if (TOPO == HP_TOPO_RING && ph == N - 1 && !bad) {
+        decode_average<ALG, B>(frag, meta, fp, x);
+        store_checked(sg.out + E * cm.emu_stride_out + tr.off, m, x);
       }
       __syncthreads();  // the prefetch stage of this tile may be refilled from here on
     }
     trace_phase(cm, E, ph, sm.ws);
   }
+}
+
+// PS, the phase behind the pushes: the N pushes of a tile of the own chunk are summed in
+// rank order, the sum is encoded and sent.  OWN_HERE: this rank's push of the tile is
+// made here and its result decoded here, both from registers; else both take the way
+// through the inbox that they take on the other ranks (see ps_own_here).
+//
+// A function of its own, and a kernel for each OWN_HERE: at 80 registers a thread, the
+// sum inside the push loop made every push spill.  N ranks emulated on one GPU, 64 M
+// elements in all, 2-bit TernGrad, us per launch for 2 / 4 / 8 ranks: everything through
+// the inbox 254 / 244 / 246, the sum inside the push loop 240 / 256 / 272, this 222 /
+// 228 / 240 (8 bits: 342 / 336 / 340, 275 / 318 / 350, 253 / 291 / 315; onebit 297 / 270 /
+// 263, 247 / 243 / 245, 250 / 248 / 252; TBQ 272 / 250 / 242, 240 / 234 / 238, 241 / 234 / 238).
+template <int ALG, int B, bool OWN_HERE>
+__device__ __forceinline__ void serve_phase(const BucketDev& bk, const HpComm& cm, const FusedParams& fp,
+                                            FusedSmem& sm, int R, int E, uint32_t* status, Feed& feed) {
+  const int N = cm.nranks;
+  const int G = (int)gridDim.x;
+  const int b = (int)blockIdx.x;
+  const int pushes = OWN_HERE ? N - 1 : N;
+  uint8_t* my_inbox = reinterpret_cast<uint8_t*>(cm.inbox[R]);
+  PhaseSpec ps = phase_spec<HP_TOPO_PS>(N - 1, N, R);
+  ps.ndst = pushes;
+  ps.dst0 = OWN_HERE ? (R + 1) % N : R;
+  ps.dst_slot = N + R;
+  Cursor cons;
+  cursor_begin(bk, G, b, pushes, R, cons);
+  TileRef tr;
+  while (cursor_next(bk, G, b, cons, tr)) {
+    const SegDev& sg = bk.seg[tr.seg];
+    const int m = tr.m;
+    const uint32_t t = tr.t;
+    // the remote pushes are polled one ahead: the loads of the next are in flight while
+    // the current one is decoded
+    TileRx<ALG, B> in[2];
+    if (!dbg_tile_ok<ALG, B>(bk, my_inbox, my_inbox + (size_t)(N - 1) * bk.slot_bytes + sg.pay_off, t, status, 4u))
+      sm.ws.poisoned = 1;   // ll_finish returns at once, nothing is stored
+    float x[kIter][4], own[2];
+    uint32_t frag[kIter];
+    if (OWN_HERE) {
+      feed_top_up<HP_TOPO_PS>(bk, cm, sm, R, E, feed, N, G, b);
+      const float* gp = sg.g + E * cm.emu_stride_g + tr.off;
+      float* rp = sg.r ? sg.r + E * cm.emu_stride_r + tr.off : nullptr;
+      const int st = feed_take(cm, sm, gp, rp, m, status, feed, x);
+      if (rp) add_state(rp, sm, st, m, x);
+      encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt, sm.tile, 0, own, frag, rp != nullptr);
+      if (rp && !*(volatile int*)&sm.ws.poisoned) store_checked(rp, m, x);
+    }
+    auto polled = [&](int q) { return !(OWN_HERE && q == R) && !sm.ws.poisoned; };
+    if (polled(0)) recv_issue<ALG, B>(my_inbox + sg.pay_off, t, in[0]);
+    for (int q = 0; q < N; ++q) {
+      if (q + 1 < N && polled(q + 1))
+        recv_issue<ALG, B>(my_inbox + (size_t)(q + 1) * bk.slot_bytes + sg.pay_off, t, in[(q + 1) & 1]);
+      float d[kIter][4];
+      if (OWN_HERE && q == R) {
+#pragma unroll
+        for (int j = 0; j < kIter; ++j) decode_frag<ALG, B>(frag[j], own, fp.P.tau, d[j]);
+      } else {
+        recv_finish<ALG, B>(my_inbox + (size_t)q * bk.slot_bytes + sg.pay_off, t, in[q & 1], cm,
+                            status, HP_STATUS_TIMEOUT | (1u << 16) | ((uint32_t)q << 8) | (b & 255),
+                            sm.ws, fp.P.tau, d);
+      }
+#pragma unroll
+      for (int j = 0; j < kIter; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[j][e] = q > 0 ? x[j][e] + d[j][e] : d[j][e];
+    }
+    float* sp = sg.sr ? sg.sr + E * cm.emu_stride_sr + (size_t)t * kTile : nullptr;
+    if (sp) add_state(sp, sm, -1, m, x);
+    float meta[2];
+    encode_tile<ALG, B>(x, m, fp.P, sg.id, tr.off, fp.P.salt + ps.salt + 1u, sm.tile, 1, meta, frag, sp != nullptr);
+    const bool bad = *(volatile int*)&sm.ws.poisoned != 0;
+    if (sp && !bad) store_checked(sp, m, x);
+    send_to<ALG, B>(bk, cm, ps, sg, t, frag, meta, bad, status);
+    if (OWN_HERE && !bad) {
+      decode_average<ALG, B>(frag, meta, fp, x);
+      store_checked(sg.out + E * cm.emu_stride_out + tr.off, m, x);
+    }
+    if (OWN_HERE) __syncthreads();  // the prefetch stage of this tile may be refilled from here on
+  }
+  trace_phase(cm, E, pushes, sm.ws);
 }
 
 // decode the reduced chunk `c` that arrives in inbox slot `slot` into the gradient;
@@ -655,7 +722,9 @@ ring_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   uint32_t* status = reinterpret_cast<uint32_t*>(cm.status) + 4 * E;
   fused_prologue(sm);
   trace_mark(cm, E, 0);
-  encode_phases<ALG, B, HP_TOPO_RING>(bk, cm, fp, sm, R, E, status);
+  Feed feed;
+  feed_begin<HP_TOPO_RING>(bk, N, R, feed);
+  encode_phases<ALG, B, HP_TOPO_RING>(bk, cm, fp, sm, R, E, status, feed, N);
   trace_mark(cm, E, 1);
   // gather: rank src finalised chunk src+1 (the own one is done)
   trace_phase(cm, E, N, sm.ws);
@@ -668,7 +737,7 @@ ring_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 }
 
 // -------------------------------------------------------------------------- PS
-template <int ALG, int B>
+template <int ALG, int B, bool OWN_HERE>
 __global__ void __launch_bounds__(kThreads, 3)
 ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -680,14 +749,17 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   fused_prologue(sm);
   trace_mark(cm, E, 0);
 
-  // phases 0 .. N-2: push; phase N-1: push and serve the own chunk
-  encode_phases<ALG, B, HP_TOPO_PS>(bk, cm, fp, sm, R, E, status);
+  constexpr int kOwn = OWN_HERE ? 1 : 0;
+  Feed feed;
+  feed_begin<HP_TOPO_PS>(bk, N, R, feed);
+  encode_phases<ALG, B, HP_TOPO_PS>(bk, cm, fp, sm, R, E, status, feed, N - kOwn);
+  serve_phase<ALG, B, OWN_HERE>(bk, cm, fp, sm, R, E, status, feed);
   trace_mark(cm, E, 1);
-  trace_phase(cm, E, N, sm.ws);
-  // pull: decode every other owner's reduced chunk
-  for (int i = 1; i < N; ++i) {
+  if (OWN_HERE) trace_phase(cm, E, N, sm.ws);
+  // pull: decode the reduced chunks that arrive in the inbox
+  for (int i = kOwn; i < N; ++i) {
     const int j = (R + i) % N;
-    decode_phase<ALG, B>(bk, cm, fp, sm, R, E, N + i - 1, N + j, j, status);
+    decode_phase<ALG, B>(bk, cm, fp, sm, R, E, N + 1 - 2 * kOwn + i, N + j, j, status);
     trace_phase(cm, E, N + i, sm.ws);
   }
   trace_mark(cm, E, 2);
@@ -804,6 +876,18 @@ static int num_slots(int topo, int nranks) {
 // phases of one launch that visit tiles (see Cursor)
 static int num_phases(int nranks) { return 2 * nranks - 1; }
 
+// PS: whether the owner makes its own push, and decodes its own result, in the serving
+// phase, or through its inbox like everybody else's.  That saves work for 1/N of the
+// gradient, but puts an encode and a decode on the serving CTA.  When a phase has fewer
+// tiles than the grid CTAs, a launch is a chain of latencies on which both lie, while idle
+// CTAs could do them; with two ranks the saved polls weigh more.  Emulated ranks, TBQ, us
+// through the inbox / here: 8 ranks, 1.5 M elements in all 23.6 / 26.5, 4 M 31.0 / 33.9,
+// 8 M (32 tiles a phase, 55 CTAs) 39.8 / 40.0; 4 ranks, 2 M 16.6 / 18.0, 8 M (128 tiles,
+// 111 CTAs) 33.5 / 33.4; 2 ranks, 1.5 M 11.1 / 9.5, 4 M 16.4 / 15.0.
+static bool ps_own_here(const BucketDev& bk, int nranks, int ctas) {
+  return nranks < 4 || bk.tiles_total >= (uint32_t)ctas;
+}
+
 template <int ALG, int B>
 static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const FusedParams& fp,
                         int ctas, cudaStream_t st) {
@@ -817,16 +901,18 @@ static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const F
     kern<<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
     return (int)cudaGetLastError();
   }
-  void (*kern)(const BucketDev, const HpComm, const FusedParams) =
-      topo == HP_TOPO_RING ? ring_dense_kernel<ALG, B> : ps_dense_kernel<ALG, B>;
+  void (*const kerns[3])(const BucketDev, const HpComm, const FusedParams) = {
+      ring_dense_kernel<ALG, B>, ps_dense_kernel<ALG, B, true>, ps_dense_kernel<ALG, B, false>};
+  const int which = topo == HP_TOPO_RING ? 0 : (ps_own_here(bk, cm.nranks, ctas) ? 1 : 2);
+  auto kern = kerns[which];
   const size_t smem = sizeof(FusedSmem);
-  // per (topology, device): the shared-memory attribute is sticky, and the number of
+  // per (kernel, device): the shared-memory attribute is sticky, and the number of
   // CTAs the GPU can hold at once does not change
-  static int resident[2][64] = {};
+  static int resident[3][64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
-  int cap = (dev >= 0 && dev < 64) ? resident[topo][dev] : 0;
+  int cap = (dev >= 0 && dev < 64) ? resident[which][dev] : 0;
   if (cap == 0) {
     e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
@@ -837,7 +923,7 @@ static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const F
     if (e != cudaSuccess) return (int)e;
     cap = per_sm * sms;
     if (cap < 1) return HP_ERR_RESIDENCY;
-    if (dev >= 0 && dev < 64) resident[topo][dev] = cap;
+    if (dev >= 0 && dev < 64) resident[which][dev] = cap;
   }
   if (cm.emulate) {
     if ((long long)ctas * cm.nranks > (long long)cap) return HP_ERR_RESIDENCY;

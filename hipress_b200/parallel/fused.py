@@ -171,9 +171,10 @@ class FusedDenseBucket:
     def last_trace_phases(self):
         """Per rank played by the last launch: for every phase (N hops or pushes, the
         last of which finishes the rank's own chunk, then N gathers or pulls, the first
-        of which is that own chunk and does nothing) the time, in ms from the first
-        CTA's start, at which the last CTA finished it, and the mean time a CTA spent
-        polling for its input in that phase."""
+        of which is that own chunk and does nothing; where the owner's own push takes its
+        inbox, N pushes and then serving and the pull of the own chunk as one) the time,
+        in ms from the first CTA's start, at which the last CTA finished it, and the mean
+        time a CTA spent polling for its input in that phase."""
         if self.trace is None:
             return None
         phases = 2 * self.nranks

@@ -189,3 +189,11 @@ def test_fused_kernel_gives_up_cleanly_when_a_peer_never_sends():
     b1.launch([g], [torch.zeros_like(g)], [g])
     torch.cuda.synchronize()
     b1.check_status()
+
+
+@pytest.mark.parametrize("ctas", [4, 5, 6])
+@pytest.mark.parametrize("name,kw", ALGS)
+def test_ps_own_push_here_or_through_the_inbox(name, kw, ctas):
+    """A chunk of five tiles, the last one ragged, around the number of CTAs at which the
+    owner's own push changes its way."""
+    _run("ps", name, kw, 4, [4 * 4096 * 5 - 4099], steps=2, ctas=ctas)
