@@ -837,9 +837,12 @@ __device__ __forceinline__ uint32_t emit_slices(uint32_t L, uint32_t most) {
 
 // Slice x of nx of one array's candidates.  True in thread 0 of the CTA that finished
 // last, behind the headers.
+// A CTA whose barrier expired goes on, and may have read another count than the others:
+// their slices then overlap, and together hold more than the lists have room for.  So a
+// list is read up to its room and no further, and so is the second one written.
 static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const ListState& ls, const EmitDst& dst,
                                                SelSmem& sm, uint32_t x, uint32_t nx) {
-  const uint32_t L = ls.count, low = ls.low;   // no overflow: the list holds all of them
+  const uint32_t L = min(ls.count, s.cap), low = ls.low;   // no overflow: the list holds all of them
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
   const bool every = L <= s.k;                 // all candidates are sent
   uint32_t bin0 = 0, rem = 0, least = 0xFFFFFFFFu;
@@ -878,9 +881,12 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
       if (at[q] == kNone) continue;
-      if (at[q] & kKeep) {   // never more than the first list holds
-        list2_values(s)[sm.base2 + (at[q] & ~kKeep)] = v[q];
-        list2_indices(s)[sm.base2 + (at[q] & ~kKeep)] = idx[q];
+      if (at[q] & kKeep) {
+        const uint32_t pos = sm.base2 + (at[q] & ~kKeep);
+        if (pos < s.cap) {
+          list2_values(s)[pos] = v[q];
+          list2_indices(s)[pos] = idx[q];
+        }
       } else if (idx[q] < s.n) {
         put_pair(dst, val_off, s.kmax, sm.base + at[q], idx[q], v[q]);
         s.a[idx[q]] = 0.0f;
@@ -903,7 +909,7 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
   // The last CTA: among the elements of the k-th's bin, `rem` are sent.  What is left of
   // their keys is 10 bits in a fine bin, 19 in a bin of the leading bits, and up to 31 in
   // the last fine bin.
-  const uint32_t L2 = every ? 0u : __ldcg(s.ws + kWsCand2Count);
+  const uint32_t L2 = every ? 0u : min(__ldcg(s.ws + kWsCand2Count), s.cap);
   if (threadIdx.x == 0) sm.sent = __ldcg(s.ws + kWsOutCount), sm.ties = 0;
   const uint32_t start = low <= 1u ? bin0 << 19 : low + (bin0 << 10);
   int shift = low <= 1u ? 7 : (bin0 == (uint32_t)kBins - 1u ? 19 : 0), bits = 12;

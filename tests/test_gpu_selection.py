@@ -82,3 +82,39 @@ def test_selection_with_a_workspace_off_alignment():
     ic, vc = sparse_pairs(c.encode(g, c.new_state(n, "cpu")), c.kmax(n))
     ig, vg = sparse_pairs(c.encode(g.cuda(), c.new_state(n, "cuda"), workspace=ws), c.kmax(n))
     assert torch.equal(ic, ig) and torch.equal(vc, vg)
+
+
+# the list's true length, 2048, cut by CTAs that each read another one: five slices that
+# overlap and hold 2452 elements together; and a length beyond the list's room
+@pytest.mark.parametrize("counts", [[511, 1023, 1535, 2047, 2048], [4096] * 8, [511, 4096, 1535, 4096, 2048, 4096]])
+def test_emit_stays_in_its_lists_when_ctas_disagree_about_the_length(tmp_path, counts):
+    import ctypes as C
+    import subprocess
+    from pathlib import Path
+    from hipress_b200._native.build import CSRC, nvcc_path
+    so = tmp_path / "emit_views.so"
+    subprocess.run([nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17", "-fmad=false",
+                    "-Xcompiler", "-fPIC", "-shared", "-I", str(CSRC / "include"), "-I", str(CSRC / "cuda"),
+                    str(Path(__file__).parent / "native/emit_views.cu"), "-o", str(so)], check=True)
+    L = C.CDLL(str(so))
+    n, cap, k = 8192, 2048, 1000
+    # all candidates alike: every one is a tie and goes to the second list
+    a = torch.ones(n, device="cuda")
+    key = int(torch.ones(1).view(torch.int32).item())
+    ws = torch.zeros(L.emit_workspace_words(), dtype=torch.int32, device="cuda")
+    ws[0] = cap                            # histogram: all in the first bin above the bound
+    # two lists of `cap` pairs, and behind them room for whatever the CTAs hold together
+    guard = 0x5A5A5A5A
+    lists = torch.full((4 * cap + 8 * max(counts),), guard, dtype=torch.int32, device="cuda")
+    lists[:cap] = key
+    lists[cap:2 * cap] = torch.arange(cap, dtype=torch.int32, device="cuda")
+    out = torch.zeros(16 + 2 * 4 * (k + 4), dtype=torch.uint8, device="cuda")
+    c = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    p = [C.c_void_p(t.data_ptr()) for t in (a, ws, lists, c, out)]
+    rc = L.emit_views(p[0], C.c_uint32(n), C.c_uint32(k), p[1], p[2], C.c_uint32(cap), C.c_uint32(key), p[3],
+                      C.c_int(len(counts)), p[4], C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert bool((lists[4 * cap:] == guard).all()), "the second list was written past its end"
+    assert bool((lists[cap:2 * cap] == torch.arange(cap, dtype=torch.int32, device="cuda")).all())
+    assert bool((a[cap:] == 1).all())
