@@ -174,17 +174,27 @@ def fast_cuda():
 
 
 class OrderEvent:
-    """An event that orders one stream behind another (``stream_order``)."""
+    """The event behind one ``stream_order``.  An event records on streams of the device it
+    was made on, and that may be another than is current here: one for each device, made
+    when it is first needed."""
 
     def __init__(self):
-        e = C.c_void_p()
-        check(cuda().hp_cuda_event_create(C.byref(e)), "event create")
-        self.handle = e.value
+        self._handles = {}
+        self.on(current_device())
+
+    def on(self, device: int) -> int:
+        h = self._handles.get(device)
+        if h is None:
+            e = C.c_void_p()
+            with torch.cuda.device(device):
+                check(cuda().hp_cuda_event_create(C.byref(e)), "event create")
+            h = self._handles[device] = e.value
+        return h
 
     def __del__(self):
-        h, self.handle = getattr(self, "handle", None), None
-        if h is not None and _cuda is not None:
-            _cuda.hp_cuda_event_destroy(h)
+        for h in self.__dict__.pop("_handles", {}).values():
+            if _cuda is not None:
+                _cuda.hp_cuda_event_destroy(h)
 
 
 def check(code: int, what: str = "native call", device_call: bool = True):
@@ -205,8 +215,12 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
+def current_device() -> int:
+    return torch._C._cuda_getDevice()
+
+
 def stream_ptr(stream=None):
     """Handle of ``stream``, or of the current stream of the current device."""
     if stream is not None:
         return stream.cuda_stream
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch._C._cuda_getCurrentRawStream(current_device())

@@ -38,7 +38,7 @@ from dataclasses import dataclass, field
 import torch
 import torch.distributed as dist
 
-from .._native.lib import check, stream_ptr
+from .._native.lib import check, current_device, stream_ptr
 from ..config import HipressConfig
 from ..ops.algorithms import get_algorithm
 from ..ops.compressor import TILE, Compressor
@@ -454,9 +454,10 @@ class GradSyncEngine:
             p.grad = g = g.contiguous()
         return g
 
-    def _order_streams(self, i: int, src: int, dst: int):
-        """Work launched on ``dst`` from here on runs behind what ``src`` holds now."""
-        rc = self._fast.stream_order(self._order[i].handle, src, dst)
+    def _order_streams(self, i: int, device: int, src: int, dst: int):
+        """Work launched on ``dst`` from here on runs behind what ``src``, a stream of
+        ``device``, holds now."""
+        rc = self._fast.stream_order(self._order[i].on(device), src, dst)
         if rc:   # an ordering that failed must not pass as one that holds
             check(rc, "stream order")
 
@@ -466,7 +467,7 @@ class GradSyncEngine:
             # fused kernels take the raw stream: no stream context switch on the
             # autograd thread, which is busy launching backward
             st = b.stream or self.comm_stream
-            self._order_streams(b.index, stream_ptr(), st.cuda_stream)
+            self._order_streams(b.index, current_device(), stream_ptr(), st.cuda_stream)
             tok = self.timeline.begin(f"bucket{b.index}", st) if self.timeline.enabled else None
             self._launch_fused(b)
             if self.outer is not None:
@@ -625,7 +626,7 @@ class GradSyncEngine:
                             self._finish_plain(b)
                             if self.on_bucket_done is not None:
                                 self.on_bucket_done(b)
-            self._order_streams(-1, self.comm_stream.cuda_stream, stream_ptr())
+            self._order_streams(-1, self.comm_stream.device_index, self.comm_stream.cuda_stream, stream_ptr())
             if self.arena is not None:
                 if self.cfg.strict_status:
                     # the host waits for this step's kernels and raises before the

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import hipress_b200 as hp
+from hipress_b200._native import lib
 from hipress_b200._native.lib import NativeLibraryError
 from hipress_b200.config import HipressConfig
 from hipress_b200.parallel import engine as engine_module
@@ -13,12 +14,20 @@ from hipress_b200.parallel.engine import GradSyncEngine
 HERE, COMM = 11, 22     # stream handles
 
 
+class Event:
+    """Stands for an OrderEvent: its handle names the device it was made on."""
+
+    def on(self, device):
+        return 1000 + device
+
+
 class Native:
     def __init__(self, rc=0):
-        self.rc, self.calls = rc, []
+        self.rc, self.calls, self.events = rc, [], []
 
     def stream_order(self, event, src, dst):
         self.calls.append(("order", src, dst))
+        self.events.append(event)
         return self.rc
 
 
@@ -26,10 +35,11 @@ def _engine(monkeypatch, native):
     """An engine of CPU parameters dressed up as one with a fused bucket on a GPU."""
     hp.init()
     monkeypatch.setattr(engine_module, "stream_ptr", lambda stream=None: HERE)
+    monkeypatch.setattr(engine_module, "current_device", lambda: 1, raising=False)
     named = [("w", torch.nn.Parameter(torch.zeros(300))), ("b", torch.nn.Parameter(torch.zeros(20)))]
     eng = GradSyncEngine(named, HipressConfig(algorithm="tbq", comp_threshold=1, overlap=False))
-    eng._fast, eng._order = native, [SimpleNamespace(handle=100 + i) for i in range(len(eng.buckets) + 1)]
-    eng.comm_stream = SimpleNamespace(cuda_stream=COMM)
+    eng._fast, eng._order = native, [Event() for _ in range(len(eng.buckets) + 1)]
+    eng.comm_stream = SimpleNamespace(cuda_stream=COMM, device_index=3)
     eng.on_cuda = True
     for b in eng.buckets:
         b.impl = SimpleNamespace(launch_ptrs=lambda *a, **k: native.calls.append(("launch",)))
@@ -59,3 +69,40 @@ def test_a_failed_ordering_behind_the_launches_raises(monkeypatch):
     with pytest.raises(NativeLibraryError, match="stream order"):
         eng.synchronize()
     assert native.calls[-1] == ("order", COMM, HERE)
+
+
+def test_events_belong_to_the_device_of_the_stream_they_record(monkeypatch):
+    """The device that is current at a step may be another than the communication
+    stream's, and than the one that was current when the engine was built."""
+    native = Native()
+    _engine(monkeypatch, native).synchronize()
+    assert native.calls == [("order", HERE, COMM), ("launch",), ("order", COMM, HERE)]
+    assert native.events == [1001, 1003]
+
+
+def test_an_order_event_is_made_once_on_each_device(monkeypatch):
+    made, current = [], [0]
+
+    class Device:
+        def __init__(self, d):
+            self.d = d
+
+        def __enter__(self):
+            self.before, current[0] = current[0], self.d
+
+        def __exit__(self, *a):
+            current[0] = self.before
+
+    def create(out):
+        made.append(current[0])
+        out._obj.value = 500 + current[0]
+        return 0
+    native = SimpleNamespace(hp_cuda_event_create=create, hp_cuda_event_destroy=lambda h: made.append(-h))
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(lib, "current_device", lambda: current[0], raising=False)
+    monkeypatch.setattr(lib, "cuda", lambda: native)
+    monkeypatch.setattr(lib, "_cuda", native)
+    e = lib.OrderEvent()
+    assert [e.on(0), e.on(2), e.on(2), e.on(0)] == [500, 502, 502, 500] and made == [0, 2]
+    del e
+    assert sorted(made[2:]) == [-502, -500]
