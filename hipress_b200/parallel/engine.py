@@ -467,9 +467,11 @@ class GradSyncEngine:
             # fused kernels take the raw stream: no stream context switch on the
             # autograd thread, which is busy launching backward
             st = b.stream or self.comm_stream
+            # before the ordering: a gradient may be made or copied here, on this stream
+            g = [self._grad(e).data_ptr() for e in b.entries]
             self._order_streams(b.index, current_device(), stream_ptr(), st.cuda_stream)
             tok = self.timeline.begin(f"bucket{b.index}", st) if self.timeline.enabled else None
-            self._launch_fused(b)
+            self._launch_fused(b, g)
             if self.outer is not None:
                 with torch.cuda.stream(st):
                     self._between_machines(b)
@@ -506,9 +508,9 @@ class GradSyncEngine:
             if b.fused and self.on_bucket_done is not None:
                 self.on_bucket_done(b)
 
-    def _launch_fused(self, b: Bucket):
+    def _launch_fused(self, b: Bucket, g: list | None = None):
+        """``g``: the gradients' addresses, for a bucket with a fused kernel."""
         if b.impl is not None:
-            g = [self._grad(e).data_ptr() for e in b.entries]
             if not b.in_order:
                 g = [g[i] + off for i, off in b.at]
             st = b.stream or self.comm_stream

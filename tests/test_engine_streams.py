@@ -106,3 +106,22 @@ def test_an_order_event_is_made_once_on_each_device(monkeypatch):
     assert [e.on(0), e.on(2), e.on(2), e.on(0)] == [500, 502, 502, 500] and made == [0, 2]
     del e
     assert sorted(made[2:]) == [-502, -500]
+
+
+def test_missing_gradients_are_made_before_the_ordering(monkeypatch):
+    """A gradient that does not exist yet is filled on the caller's stream; the kernel on
+    the communication stream must run behind that fill."""
+    native = Native()
+    eng = _engine(monkeypatch, native)
+    grad = eng._grad
+
+    def recorded(e):
+        native.calls.append(("grad", e.name))
+        return grad(e)
+    eng._grad = recorded
+    for e in eng.entries:
+        e.param.grad = None
+    eng.synchronize()
+    kinds = [c[0] for c in native.calls]
+    assert kinds == ["grad"] * len(eng.entries) + ["order", "launch", "order"]
+    assert all(e.param.grad is not None for e in eng.entries)
