@@ -654,20 +654,25 @@ static __device__ __noinline__ void sample_body(const SelUnit& s, float momentum
   if (threadIdx.x == 0) s.ws[kWsLow] = low;
 }
 
-// Items [0, total).  Below 32 per CTA in equal shares: the tickets of all CTAs follow one
-// another, 25 ns each, and took longer than the SMs' unequal speed costs (24 us instead
-// of 23 for 1600 tiles, 33 instead of 30 for 5844).  Above, seven eighths in equal
-// shares, the rest in short stretches taken from
+// Items [0, total).  Below kShareAll per CTA in equal shares: the tickets of all CTAs
+// follow one another, 25 ns each, and took longer than the SMs' unequal speed costs.
+// Above, seven eighths in equal shares, the rest in short stretches taken from
 // *word by whichever of the ctas CTAs is free -- SMs do not run at one speed, and equal
 // shares alone leave the fast ones waiting, while handing out everything made the ticket
-// word the bottleneck.  The next stretch is asked for before the current one is worked
+// word the bottleneck.  One array, 296 CTAs, us per launch with equal shares / handed out:
+//   tiles per CTA          5.4        20.8       32.4       54         108         216
+//   GradDrop encode      48.1/49.2  85.0/87.0  110/113    167/171    292/288     538/536
+//   GradDrop, PS bucket  94.2/99.3  171/179    221/229    342/347    605/597    1142/1121
+//   DGC, ring bucket     70.7/75.7  144/146    198/202    319/321    601/587    1160/1144
+// At 81 tiles the two are within 2 % of one another, either way.  The next stretch is asked for before the current one is worked
 // on, by predicated instructions (an `if` around them split thread 0 from its warp, and
 // the two halves then counted twice at the barriers that follow).  f(lo, hi) runs with
 // the whole CTA; `slot` is shared memory.
+constexpr uint32_t kShareAll = 96;
 template <typename F>
 __device__ __forceinline__ void hand_out(uint32_t* word, uint32_t total, uint32_t cta, uint32_t ctas, uint32_t& slot,
                                          F f) {
-  if (total < 32u * ctas) {
+  if (total < kShareAll * ctas) {
     const uint32_t lo = (uint32_t)((uint64_t)total * cta / ctas), hi = (uint32_t)((uint64_t)total * (cta + 1) / ctas);
     if (lo < hi) f(lo, hi);
     return;

@@ -44,6 +44,15 @@ def test_selection_with_few_ctas():
     _check("dgc", torch.randn(500000) * torch.randn(500000), 0.002, max_ctas=3)
 
 
+# around 96 tiles per CTA, where a CTA's tiles stop being one equal share of all
+@pytest.mark.parametrize("tiles", [191, 192, 193, 400])
+@pytest.mark.parametrize("name", ["dgc", "graddrop"])
+def test_selection_with_tiles_that_are_handed_out(name, tiles):
+    torch.manual_seed(tiles)
+    n = tiles * 4096 - 5
+    _check(name, torch.randn(n) * torch.randn(n), 0.002, max_ctas=2)
+
+
 def test_selection_of_arrays_the_sample_misjudges():
     """Almost everything zero, the few large values in one place: the sample sees none of
     them, so the list is all that is not zero; and magnitudes the sample sees in full
