@@ -553,8 +553,10 @@ __global__ void __launch_bounds__(256{bound}) {name}_{self.tag}_kernel({em.kerne
         coop = len(self.plan.phases) > 1
         if coop:
             # all blocks resident; no more per SM than keep it busy, because every one of them
-            # arrives at the same barrier word, 10 ns each (TernGradEncode of 1 M elements 16.4 us
-            # with six blocks per SM, 12.4 with four; 17.2 with eight and one polled word)
+            # arrives at the same barrier word, 10 ns each.  TernGradEncode, 2 bits, us with
+            # what fits / four / two blocks per SM: 0.5 M elements 14.3 / 14.3 / 12.3, 1 M
+            # 18.4 / 16.4 / 14.3, 4 M 28.1 / 26.6 / 26.6, 8 M 41.0 / 38.9 / 41.0, 16 M 65.5 /
+            # 63.5 / 73.7, 32 M 117 / 117 / 147, 64 M 215 / 219 / 274: four lose little anywhere
             most = "kMaxBlocks" if any(_ordered(s.expr) for s in self.em.reduces) else "kMaxBlocks / 2"
             rows = ("    if (blocks > (uint64_t)cap[dev]) blocks = cap[dev];\n"
                     f"    if (blocks > {most}) blocks = {most};")
