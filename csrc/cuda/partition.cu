@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "hipress/capi.h"
+#include "partition.cuh"
 
 namespace {
 
@@ -30,6 +31,29 @@ bool resolve(const char* name, F& fn) {
 }
 
 }  // namespace
+
+namespace hipress {
+
+int stream_sms(cudaStream_t stream, int device_sms) {
+  typedef CUresult (*StreamGetGreenCtx_t)(CUstream, CUgreenCtx*);
+  typedef CUresult (*GreenCtxGetDevResource_t)(CUgreenCtx, CUdevResource*, CUdevResourceType);
+  struct Entry {
+    StreamGetGreenCtx_t of_stream = nullptr;
+    GreenCtxGetDevResource_t resource = nullptr;
+    bool ok = resolve("cuStreamGetGreenCtx", of_stream) && resolve("cuGreenCtxGetDevResource", resource);
+  };
+  static const Entry entry;
+  // the default streams (null, and the handles 1 and 2) belong to the primary context
+  if (!entry.ok || reinterpret_cast<uintptr_t>(stream) <= 2) return device_sms;
+  CUgreenCtx g = nullptr;
+  if (entry.of_stream((CUstream)stream, &g) != CUDA_SUCCESS || !g) return device_sms;
+  CUdevResource res;
+  if (entry.resource(g, &res, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS) return device_sms;
+  const int sms = (int)res.sm.smCount;
+  return sms > 0 && sms < device_sms ? sms : device_sms;
+}
+
+}  // namespace hipress
 
 extern "C" {
 

@@ -1,7 +1,12 @@
 // Sparse (top-k) compression for DGC and GradDrop on sm_100a.
 //
 // With room for a candidate list (the usual call) an encode is ONE cooperative launch:
-// sample, update + collect, finish (sparse_core.cuh), with grid barriers in between.
+// sample, update + collect, finish (sparse_core.cuh), with grid barriers in between.  Its
+// CTAs wait for one another, so all of them must be resident at once: the grid is sized
+// for the SMs that the stream may use, and where kernels on other streams keep those
+// occupied the launch waits for room.  Each barrier is bounded (kGridBarrierNs); if a
+// kernel that holds SMs for longer than that comes between this one's CTAs, the payload may
+// lack elements, and the workspace's status word (kWsStatus) is set.
 // It was a chain of eight launches that read the array three times behind the update:
 // GradDrop's encode of 23.9 M elements at 0.1 % took 138 us and takes 87, of 1 M elements
 // 63 and takes 33 (B200, states rotating through more than L2 holds).
@@ -22,6 +27,7 @@
 // mark14wu/hipress (README.md:9; --comp_alg dgc README.md:180); CompLL planned
 // sort/copy_if for them (src/CompLL/GCGen/unit.py:24-29) but has no translation
 // rule, so there is no reference kernel to compare with.
+#include "partition.cuh"
 #include "sparse_core.cuh"
 #include "sync.cuh"
 #include "hipress/noalloc.h"
@@ -208,22 +214,24 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
   if (e != cudaSuccess) return (int)e;
   if (listed) {
     const size_t smem = sizeof(SelOrPassSmem);
-    static int resident[64] = {};   // CTAs the GPU holds at once, per device
+    static int per_sm[64] = {}, all_sms[64] = {};   // CTAs an SM holds at once and SMs, per device
     int dev = 0;
     e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    int cap = dev >= 0 && dev < 64 ? resident[dev] : 0;
-    if (cap == 0) {
-      int sms = 0, per = 0;
+    int per = dev >= 0 && dev < 64 ? per_sm[dev] : 0, sms = per ? all_sms[dev] : 0;
+    if (per == 0) {
       e = cudaFuncSetAttribute((const void*)sparse_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sparse_encode_kernel, kSpThreads, smem);
       if (e != cudaSuccess) return (int)e;
-      cap = per * sms;
-      if (cap < 1) return HP_ERR_RESIDENCY;
-      if (dev >= 0 && dev < 64) resident[dev] = cap;
+      if (per < 1 || sms < 1) return HP_ERR_RESIDENCY;
+      if (dev >= 0 && dev < 64) {
+        all_sms[dev] = sms;
+        per_sm[dev] = per;
+      }
     }
+    int cap = per * stream_sms(st, sms);   // the stream may own only some of the SMs
     if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
     const int grid = (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
     SelArgs A;
@@ -248,7 +256,10 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
     A.momentum = momentum;
     A.out = out;
     void* args[] = {(void*)&A};
-    return (int)cudaLaunchCooperativeKernel((const void*)sparse_encode_kernel, dim3(grid), dim3(kSpThreads), args, smem, st);
+    e = cudaLaunchCooperativeKernel((const void*)sparse_encode_kernel, dim3(grid), dim3(kSpThreads), args, smem, st);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return (int)e;
+    // less of the GPU is ours than the queries said: the launches that need no co-residency
+    cudaGetLastError();
   }
   if (max_ctas <= 0) max_ctas = 148 * 4;
   const int grid = (int)(tiles < (uint64_t)max_ctas ? tiles : (uint64_t)max_ctas);

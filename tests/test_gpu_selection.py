@@ -127,3 +127,29 @@ def test_emit_stays_in_its_lists_when_ctas_disagree_about_the_length(tmp_path, c
     assert bool((lists[4 * cap:] == guard).all()), "the second list was written past its end"
     assert bool((lists[cap:2 * cap] == torch.arange(cap, dtype=torch.int32, device="cuda")).all())
     assert bool((a[cap:] == 1).all())
+
+
+@pytest.mark.parametrize("name", ["dgc", "graddrop"])
+def test_selection_on_a_stream_that_owns_a_few_sms(name):
+    """The launch is sized for the stream's SMs: its CTAs wait for one another."""
+    import ctypes as C
+    from hipress_b200._native import lib
+    st, sms, green = C.c_void_p(), C.c_int(), C.c_void_p()
+    L = lib.cuda()
+    if L.hp_cuda_partition_stream_create(torch.cuda.current_device(), 16, 0, C.byref(st), C.byref(sms), C.byref(green)):
+        pytest.skip("the driver refuses SM partitions")
+    assert 0 < sms.value < torch.cuda.get_device_properties(0).multi_processor_count
+    stream = torch.cuda.ExternalStream(st.value)
+    torch.manual_seed(7)
+    n = 3000001
+    g, c = torch.randn(n) * torch.randn(n), Compressor(name, ratio=0.001)
+    gg, state, ws = g.cuda(), c.new_state(n, "cuda"), c.new_workspace("cuda", n)
+    torch.cuda.synchronize()
+    out = c.encode(gg, state, workspace=ws, stream=stream)
+    stream.synchronize()
+    ic, vc = sparse_pairs(c.encode(g, c.new_state(n, "cpu")), c.kmax(n))
+    ig, vg = sparse_pairs(out, c.kmax(n))
+    assert torch.equal(ic, ig) and torch.equal(vc, vg)
+    assert int(ws[3 * 4096 + 9]) == 0, "a barrier expired"     # kWsStatus
+    torch.cuda.synchronize()
+    L.hp_cuda_partition_stream_destroy(st, green)
