@@ -173,26 +173,24 @@ def fast_cuda():
     return _fast_cuda
 
 
-class OrderEvent:
+class OrderEvent(dict):
     """The event behind one ``stream_order``.  An event records on streams of the device it
     was made on, and that may be another than is current here: one for each device, made
-    when it is first needed."""
+    when it is first looked up."""
 
     def __init__(self):
-        self._handles = {}
-        self.on(current_device())
+        super().__init__()
+        self[current_device()]
 
-    def on(self, device: int) -> int:
-        h = self._handles.get(device)
-        if h is None:
-            e = C.c_void_p()
-            with torch.cuda.device(device):
-                check(cuda().hp_cuda_event_create(C.byref(e)), "event create")
-            h = self._handles[device] = e.value
-        return h
+    def __missing__(self, device: int) -> int:
+        e = C.c_void_p()
+        with torch.cuda.device(device):
+            check(cuda().hp_cuda_event_create(C.byref(e)), "event create")
+        self[device] = e.value
+        return e.value
 
     def __del__(self):
-        for h in self.__dict__.pop("_handles", {}).values():
+        for h in self.values():
             if _cuda is not None:
                 _cuda.hp_cuda_event_destroy(h)
 
@@ -215,8 +213,7 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def current_device() -> int:
-    return torch._C._cuda_getDevice()
+current_device = getattr(torch._C, "_cuda_getDevice", None)   # index of the current device
 
 
 def stream_ptr(stream=None):

@@ -454,13 +454,6 @@ class GradSyncEngine:
             p.grad = g = g.contiguous()
         return g
 
-    def _order_streams(self, i: int, device: int, src: int, dst: int):
-        """Work launched on ``dst`` from here on runs behind what ``src``, a stream of
-        ``device``, holds now."""
-        rc = self._fast.stream_order(self._order[i].on(device), src, dst)
-        if rc:   # an ordering that failed must not pass as one that holds
-            check(rc, "stream order")
-
     def _launch(self, b: Bucket):
         b.launched = True
         if b.impl is not None:
@@ -469,7 +462,9 @@ class GradSyncEngine:
             st = b.stream or self.comm_stream
             # before the ordering: a gradient may be made or copied here, on this stream
             g = [self._grad(e).data_ptr() for e in b.entries]
-            self._order_streams(b.index, current_device(), stream_ptr(), st.cuda_stream)
+            rc = self._fast.stream_order(self._order[b.index][current_device()], stream_ptr(), st.cuda_stream)
+            if rc:   # an ordering that failed must not pass as one that holds
+                check(rc, "stream order")
             tok = self.timeline.begin(f"bucket{b.index}", st) if self.timeline.enabled else None
             self._launch_fused(b, g)
             if self.outer is not None:
@@ -628,7 +623,10 @@ class GradSyncEngine:
                             self._finish_plain(b)
                             if self.on_bucket_done is not None:
                                 self.on_bucket_done(b)
-            self._order_streams(-1, self.comm_stream.device_index, self.comm_stream.cuda_stream, stream_ptr())
+            done = self.comm_stream
+            rc = self._fast.stream_order(self._order[-1][done.device_index], done.cuda_stream, stream_ptr())
+            if rc:
+                check(rc, "stream order")
             if self.arena is not None:
                 if self.cfg.strict_status:
                     # the host waits for this step's kernels and raises before the

@@ -14,10 +14,10 @@ from hipress_b200.parallel.engine import GradSyncEngine
 HERE, COMM = 11, 22     # stream handles
 
 
-class Event:
+class Event(dict):
     """Stands for an OrderEvent: its handle names the device it was made on."""
 
-    def on(self, device):
+    def __missing__(self, device):
         return 1000 + device
 
 
@@ -103,7 +103,7 @@ def test_an_order_event_is_made_once_on_each_device(monkeypatch):
     monkeypatch.setattr(lib, "cuda", lambda: native)
     monkeypatch.setattr(lib, "_cuda", native)
     e = lib.OrderEvent()
-    assert [e.on(0), e.on(2), e.on(2), e.on(0)] == [500, 502, 502, 500] and made == [0, 2]
+    assert [e[0], e[2], e[2], e[0]] == [500, 502, 502, 500] and made == [0, 2]
     del e
     assert sorted(made[2:]) == [-502, -500]
 
