@@ -776,7 +776,8 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 // kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us; TernGrad is bound by instruction
 // issue and latency (ring 195 -> 124 us, PS 378 -> 173 us, with six CTAs per SM where
 // no state is kept).
-// RES: some tensor of the bucket keeps error-feedback state.
+// RES: some tensor of the bucket keeps error-feedback state (TernGrad's buckets keep none,
+// but the entry point takes some).
 template <int ALG, int B, int TOPO, bool RES>
 __global__ void __launch_bounds__(kThreads, RES ? (TOPO == HP_TOPO_PS ? 3 : 4) : 6)
 local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
@@ -990,6 +991,9 @@ uint64_t hp_fused_chunk_elems(uint64_t n, int nranks) {
   return align_up((n + nranks - 1) / nranks, kTile);
 }
 
+// One synchronisation of a bucket.  ctas: the grid of the persistent kernels; with one
+// rank nothing waits and the grid is one CTA per tile (local_dense_kernel), ctas is only
+// checked.
 int hp_cuda_fused_dense(int topo, int alg, int bits, const HpSeg* segs, int nseg,
                         const HpComm* comm, float tau, uint64_t seed, uint32_t step, uint32_t salt,
                         int ctas, void* stream) {

@@ -26,7 +26,9 @@ class HipressConfig:
     backend: str = "auto"             # auto | fused | host | allreduce
     bucket_bytes: int = 256 << 20     # gradient bytes per fused launch
     plain_bucket_bytes: int = 32 << 20
-    ctas: int = 444                   # CTAs of a fused kernel (3 per SM on a 148-SM B200)
+    # CTAs of a quantiser's fused kernel (3 per SM on a 148-SM B200).  A job of one rank waits
+    # for nobody and takes one CTA per tile instead, whatever this and partition_ctas say
+    ctas: int = 444
     partition_sms: int = 0            # SMs reserved (green context) for fused kernels that overlap backward; 0 = off
     partition_ctas: int = 48          # CTAs of a fused kernel on the SM partition
     timeout_s: float = 10.0           # bound of every device-side wait

@@ -41,6 +41,9 @@ def decode_status(word: int) -> str:
 class FusedDenseBucket:
     """One bucket = up to 40 tensors synchronised by one launch.
 
+    ``ctas``: grid of the persistent kernel; with one rank the kernel takes one CTA per
+    tile instead and ``ctas`` does nothing.
+
     ``inbox_ptrs`` / ``flag_ptrs``: per-rank device addresses of this bucket's
     regions as mapped into this process (from a symmetric arena), ``status``: a
     local int32 tensor of 4 words per emulated rank.
