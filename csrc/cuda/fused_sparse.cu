@@ -384,7 +384,7 @@ static __device__ __noinline__ void select_units(const SpBucket& bk, const HpCom
       } else if (pass == 0) {
         pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.sh, x, nx);
       } else if (pass < 3) {
-        pass_body_rt(pass, s.a, s.n, s.k, s.ws, sm.sh, sm.fs, x, nx);
+        pass_body(pass, s.a, s.n, s.k, s.ws, sm.sh, sm.fs, x, nx);
       } else {
         unit_dst(bk, cm, cx, ph, (uint32_t)y, sm);
         if (emit_body(bk.alg, s.a, s.u, s.n, s.k, s.kmax, sm.dst.out, s.ws, sm.fs, sm.es, x, nx)) unit_release(cm, sm);

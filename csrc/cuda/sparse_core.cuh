@@ -195,7 +195,7 @@ static __device__ __noinline__ void pass0_body(const float* __restrict__ g, floa
 // One copy of the code for both digit passes (PASS is a run-time value) and one per
 // body below: the persistent kernels call every body from several phases, and inlined
 // copies made them so large that cold instruction fetches showed in the phase times.
-static __device__ __noinline__ void pass_body_rt(int PASS, const float* __restrict__ a, uint64_t n,
+static __device__ __noinline__ void pass_body(int PASS, const float* __restrict__ a, uint64_t n,
                                           uint32_t k, uint32_t* __restrict__ ws, uint32_t* sh,
                                           FindSmem& fs, uint32_t cta, uint32_t nctas) {
   for (int i = threadIdx.x; i < kBins; i += kSpThreads) sh[i] = 0;
@@ -226,13 +226,6 @@ static __device__ __noinline__ void pass_body_rt(int PASS, const float* __restri
   __syncthreads();
   flush_hist(sh, ws + PASS * kBins);
 }
-template <int PASS>
-__device__ __forceinline__ void pass_body(const float* __restrict__ a, uint64_t n, uint32_t k,
-                                          uint32_t* __restrict__ ws, uint32_t* sh, FindSmem& fs,
-                                          uint32_t cta, uint32_t nctas) {
-  pass_body_rt(PASS, a, n, k, ws, sh, fs, cta, nctas);
-}
-
 struct EmitSmem {
   uint32_t warp_tot[kSpThreads / 32];
   uint32_t base_gt;

@@ -48,7 +48,7 @@ sparse_pass_kernel(const float* __restrict__ a, uint64_t n, uint32_t k,
                    uint32_t* __restrict__ ws) {
   __shared__ __align__(16) uint32_t sh[kBins];
   __shared__ FindSmem fs;
-  pass_body<PASS>(a, n, k, ws, sh, fs, blockIdx.x, gridDim.x);
+  pass_body(PASS, a, n, k, ws, sh, fs, blockIdx.x, gridDim.x);
 }
 
 __global__ void __launch_bounds__(kSpThreads)
@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(kSpThreads, 2) sparse_encode_kernel(const __gr
   barrier();
   pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
   barrier();
-  pass_body<1>(s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
+  pass_body(1, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
   barrier();
-  pass_body<2>(s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
+  pass_body(2, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
   barrier();
   emit_body(A.alg, s.a, s.u, s.n, s.k, s.kmax, d, s.ws, fs, sm.emit, c, G);
 }
