@@ -449,6 +449,11 @@ __device__ __forceinline__ void feed_top_up(const BucketDev& bk, const HpComm& c
   }
 }
 
+// Bound of a CTA's wait for its own copies once it has given up on a peer: they read this
+// GPU's memory and arrive within microseconds, and the CTA must not end, nor a stage be
+// filled again, while one is under way.
+constexpr uint64_t kOwnCopyNs = 10000000ull;
+
 // the next tile's gradient into x; returns its stage, or -1 when it was not prefetched
 __device__ __forceinline__ int feed_take(const HpComm& cm, FusedSmem& sm, const float* gp, const float* rp, int m,
                                          uint32_t* status, Feed& f, float (&x)[kIter][4]) {
@@ -457,8 +462,8 @@ __device__ __forceinline__ int feed_take(const HpComm& cm, FusedSmem& sm, const 
     return -1;
   }
   const int st = f.consumed % kStages;
-  if (!sm.ws.poisoned && !mbar_wait_bounded(&sm.full[st], (f.consumed / kStages) & 1, cm.timeout_ns, status,
-                                            HP_STATUS_TIMEOUT | (3u << 16) | (blockIdx.x & 255)))
+  if (!mbar_wait_bounded(&sm.full[st], (f.consumed / kStages) & 1, sm.ws.poisoned ? kOwnCopyNs : cm.timeout_ns, status,
+                         HP_STATUS_TIMEOUT | (3u << 16) | (blockIdx.x & 255)))
     sm.ws.poisoned = 1;
   ++f.consumed;
   load_tile_smem(sm.g[st], x);
