@@ -89,8 +89,11 @@ class FlatSyncer:
 
     def _sync_fused(self, flat, key, stream=None):
         n = flat.numel()
-        s, server, _ = self._state(key, n, flat.device)
-        impl, _, _ = self._fused_impl(key, n, flat.device)
+        # what a first call makes is filled on the stream that the kernel runs on
+        first = key not in self._fused or self._fused[key][0].sizes[0] != n
+        with torch.cuda.stream(stream) if first and stream is not None else _null():
+            s, server, _ = self._state(key, n, flat.device)
+            impl, _, _ = self._fused_impl(key, n, flat.device)
         sp = self.comp.spec
         g = flat.data_ptr()
         if sp.sparse:
@@ -98,12 +101,11 @@ class FlatSyncer:
             u = s.get("momentum_u")
             sr = server.get("residual")
             if sr is None and self.cfg.topology == "ps":   # the owner always needs an accumulator
-                sr = server.setdefault("_scratch", torch.zeros(
-                    chunk_elems(n, comm.group_size(self.group)), dtype=torch.float32, device=flat.device))
-                if stream is not None:
-                    with torch.cuda.stream(stream):
-                        sr.zero_()
-                else:
+                with torch.cuda.stream(stream) if stream is not None else _null():
+                    sr = server.get("_scratch")
+                    if sr is None:
+                        sr = server["_scratch"] = torch.empty(
+                            chunk_elems(n, comm.group_size(self.group)), dtype=torch.float32, device=flat.device)
                     sr.zero_()
             impl.launch_ptrs([g], [acc.data_ptr()], None if u is None else [u.data_ptr()], [g],
                              [None if sr is None else sr.data_ptr()], stream=stream)

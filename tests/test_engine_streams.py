@@ -125,3 +125,38 @@ def test_missing_gradients_are_made_before_the_ordering(monkeypatch):
     kinds = [c[0] for c in native.calls]
     assert kinds == ["grad"] * len(eng.entries) + ["order", "launch", "order"]
     assert all(e.param.grad is not None for e in eng.entries)
+
+
+def test_flat_syncer_fills_new_state_on_the_kernels_stream(monkeypatch):
+    """The caller orders `stream` behind the gradient, not behind state that the first call
+    makes: that has to be filled on the same stream."""
+    import contextlib
+    from hipress_b200.parallel import hooks
+    current, made = [None], []
+
+    @contextlib.contextmanager
+    def on(stream):
+        before, current[0] = current[0], stream
+        yield
+        current[0] = before
+    hp.init()
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    for name in ("zeros", "empty"):
+        def recorded(*a, _make=getattr(torch, name), **k):
+            made.append(current[0])
+            return _make(*a, **k)
+        monkeypatch.setattr(hooks.torch, name, recorded)
+    fs = hooks.FlatSyncer(HipressConfig(algorithm="dgc", topology="ps", comp_threshold=0, server_residual=False))
+    launched = []
+    impl = SimpleNamespace(sizes=[5000], launch_ptrs=lambda *a, **k: launched.append(k["stream"]))
+
+    def fused_impl(key, n, device):
+        if key not in fs._fused:
+            made.append(current[0])
+        return fs._fused.setdefault(key, (impl, None, None))
+    fs._fused_impl = fused_impl
+    flat = torch.ones(5000)
+    for _ in range(2):
+        fs._sync_fused(flat, 0, COMM)
+    # momentum, accumulator, kernel scratch, the owner's accumulator: once each
+    assert launched == [COMM, COMM] and made == [COMM] * 4
