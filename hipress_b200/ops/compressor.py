@@ -107,7 +107,12 @@ class Compressor:
         a = state["accum_v"] if "accum_v" in state else state["residual"]
         u = state.get("momentum_u")
         if g.is_cuda:
-            ws = workspace if workspace is not None else self.new_workspace(g.device, n)
+            ws = workspace
+            if ws is None and stream is None:
+                ws = self.new_workspace(g.device, n)
+            elif ws is None:    # filled, and given back after the call, in that stream's order
+                with torch.cuda.stream(stream):
+                    ws = self.new_workspace(g.device, n)
             if incoming is not None:
                 # the accumulator must hold the updated local value before the merge
                 raise ValueError("merge incoming sparse payloads with decode(accumulate=True) "

@@ -160,3 +160,25 @@ def test_flat_syncer_fills_new_state_on_the_kernels_stream(monkeypatch):
         fs._sync_fused(flat, 0, COMM)
     # momentum, accumulator, kernel scratch, the owner's accumulator: once each
     assert launched == [COMM, COMM] and made == [COMM] * 4
+
+
+def test_an_encode_on_another_stream_makes_its_workspace_there(monkeypatch):
+    import contextlib
+    from hipress_b200.ops import compressor
+    current, made = [None], []
+
+    @contextlib.contextmanager
+    def on(stream):
+        before, current[0] = current[0], stream
+        yield
+        current[0] = before
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    monkeypatch.setattr(compressor._lib, "fast_cuda", lambda: SimpleNamespace(sparse_encode=lambda *a: 0))
+    monkeypatch.setattr(compressor._lib, "stream_ptr", lambda stream=None: HERE)
+    c = compressor.Compressor("graddrop", ratio=0.1)
+    c.new_workspace = lambda device, n=None: made.append(current[0]) or torch.zeros(8, dtype=torch.int32)
+    g = SimpleNamespace(numel=lambda: 100, is_cuda=True, device="cuda", data_ptr=lambda: 0)
+    state = {"residual": torch.zeros(100)}
+    for stream in (None, COMM):
+        c._encode_sparse(g, state, None, torch.zeros(200, dtype=torch.uint8), True, None, None, stream, 0)
+    assert made == [None, COMM]
