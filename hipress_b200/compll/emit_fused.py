@@ -562,9 +562,13 @@ __global__ void __launch_bounds__(256{bound}) {name}_{self.tag}_kernel({em.kerne
                     f"    if (blocks > {most}) blocks = {most};")
         else:
             # nothing waits: a few thousand blocks, which the hardware gives to whichever SM is
-            # free (a fixed share for every resident block costs about a tenth of the bandwidth)
+            # free (a fixed share for every resident block costs about a tenth of the bandwidth),
+            # and of a small array as many as fit (TbqDecodeAccumulate of 64 K elements 8.2 us
+            # with several groups per thread, 6.2 with one)
             unroll = f"compll_gen_{name}::{name}_{self.tag}_groups"
-            rows = (f"    blocks = (blocks + {unroll} - 1) / {unroll};\n"
+            rows = ("    const uint64_t fit = blocks < (uint64_t)cap[dev] ? blocks : cap[dev];\n"
+                    f"    blocks = (blocks + {unroll} - 1) / {unroll};\n"
+                    "    if (blocks < fit) blocks = fit;\n"
                     "    if (blocks > 0x7FFFFFFFull) blocks = 0x7FFFFFFFull;")
         most_rows = "\n".join(f"    if (n_{pname} > most) most = n_{pname};"
                               for ty, pname in self.em.fn.params if ty.vector)
