@@ -354,9 +354,16 @@ class FusedGen:
         # it also writes, so hoisting the loads over the stores is safe).
         # Four groups where nothing but packed fragments comes in or nothing goes out.  A phase
         # that streams floats in and out has enough loads with one group, but behind a header
-        # (whose fields every block has to read first) or a barrier two pay.
+        # (whose fields every block has to read first) or a barrier two pay: not where 32
+        # registers are the limit (a sum, see _ordered: OnebitEncode of 64 M elements 244 us
+        # with two, 228 with one) nor beside single bits (OnebitDecodeAccumulate 100 with two,
+        # 90 with one; TernGradDecodeAccumulate 90 and 92).
         headed = bool(em.extracts) or len(self.plan.phases) > 1
-        U = 4 if not need_in or not stores else (2 if headed else 1)
+        bits = [em.syms[v].bits for v in need_frag]
+        two = headed and not any(isinstance(b, F.Num) and b.text == "1" for b in bits)
+        U = 4 if not need_in or not stores else (2 if two else 1)
+        if any(_ordered(r.expr) for r in em.reduces):
+            U = 1
         # groups of a block in a grid that is not limited: a block that reads a header is
         # worth more of them (TernGradDecodeAccumulate of 16.8 M elements 28.8 us with one
         # group per thread and block, 25.4 with four)
