@@ -366,8 +366,13 @@ class FusedGen:
             U = 1
         # groups of a block in a grid that is not limited: a block that reads a header is
         # worth more of them (TernGradDecodeAccumulate of 16.8 M elements 28.8 us with one
-        # group per thread and block, 25.4 with four)
-        self.unroll = 4 if headed else U
+        # group per thread and block, 25.4 with four), and a decode, whose loads are few,
+        # still more (64 M elements, OnebitDecode 57 us with four and 53 with sixteen, TbqDecode
+        # 59 and 57; the decode-accumulates lose up to 28 % with sixteen)
+        self.unroll = (4 if need_in else 16) if headed else U
+        # one test for the four elements of nearly every group, where loads of floats are to
+        # overlap; the decodes are faster without it (TbqDecode of 64 M elements 65 us, now 59)
+        skip = "!full && i >= count" if need_in else "i >= count"
         larr = [f"      {C_TYPES[em.syms[v].type.name]} in_{v}[{U}][4];" for v in need_in] + \
                [f"      uint32_t fr_{v}[{U}];" for v in need_frag]
         loads = [f"        compll_load4(c.v_{v}, i0, count, in_{v}[u]);" for v in need_in]
@@ -404,14 +409,14 @@ class FusedGen:
       if (qb >= groups) break;
       const uint64_t q = qb + threadIdx.x;
       const uint64_t i0 = q * 4;
-      const bool full = i0 + 3 < count;   // one test for the four elements of nearly every group
+      const bool full = i0 + 3 < count;
       (void)full;
 {nl.join(rngs)}
 {nl.join(decls)}
 #pragma unroll
       for (int e = 0; e < 4; ++e) {{
         const uint64_t i = i0 + e;
-        if (!full && i >= count) continue;
+        if ({skip}) continue;
 {nl.join(body)}
       }}
 {nl.join(stores)}
