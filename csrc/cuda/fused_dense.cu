@@ -778,9 +778,11 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 // run at one speed (a plain in-place streaming kernel reaches 6.15 TB/s with a fixed
 // share per CTA and 6.7 TB/s with one block per tile).  Bound by HBM
 // for onebit and TBQ: 102.8 M elements, TBQ ring 278 us (5.92 TB/s) in the persistent
-// kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us; TernGrad is bound by instruction
-// issue and latency (ring 195 -> 124 us, PS 378 -> 173 us, with six CTAs per SM where
-// no state is kept).
+// kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us.  TernGrad, six CTAs per SM where no
+// state is kept: the ring is near HBM's speed (195 -> 124 us; at 67 M elements issue slots
+// 65 % used, DRAM 74 % of ncu's peak), PS quantises every tile twice and is bound by
+// instruction issue (378 -> 173 us; issue slots 79 % used, the integer pipe 60 %, DRAM 51 %,
+// warps ready but not selected 5.6 cycles per issue, waiting for memory 1.8).
 // RES: some tensor of the bucket keeps error-feedback state (TernGrad's buckets keep none,
 // but the entry point takes some).
 template <int ALG, int B, int TOPO, bool RES>

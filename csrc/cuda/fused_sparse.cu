@@ -16,9 +16,9 @@
 //            result, which the update pass cleared.
 //
 // All units of a bucket are batched in every phase, which is the "bulk
-// synchronisation" of many small tensors: the update pass hands out the bucket's tiles
-// in stretches to whichever CTA is free, whatever the tensors' sizes (equal shares of
-// CTAs per tensor left ResNet-50's largest tensors on 15 CTAs each).  An earlier
+// synchronisation" of many small tensors: the update pass splits the bucket's tiles, not
+// its tensors, over the CTAs (equal shares of the CTAs per tensor left ResNet-50's largest
+// tensors on 15 CTAs each; see hand_out for how the tiles are split).  An earlier
 // version ran every stage as a launch of its own: 19 launches per bucket for PS and
 // 9 per ring hop, with a floor of about 0.2 ms per bucket from launch latency alone.
 //

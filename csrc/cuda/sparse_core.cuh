@@ -16,7 +16,8 @@ namespace hipress {
 // barrier counter, adds to the same histograms and reserves room in the same lists, and
 // such an access to one address takes 10 to 25 ns of its own, so 444 CTAs of 256 threads
 // spent 4.5 us per barrier.  One CTA per SM leaves HBM idle while it waits at its tile's
-// end: ResNet-50's bucket took 184 us instead of 173.
+// end: the kernel of ResNet-50's compressed tensors through DGC and PS takes 197 us
+// instead of 180.
 constexpr int kSpThreads = 512;
 constexpr uint32_t kSpTile = 16 * kSpThreads;   // elements per tile of the whole-array passes
 constexpr int kBins = 4096;
@@ -401,10 +402,11 @@ static __device__ __noinline__ bool emit_body(int alg, float* __restrict__ a, fl
 //            writes the header.
 //
 // State is read and written once: HBM bound at 20 bytes per element for DGC, 12 for
-// GradDrop (3.3 and 4.4 TB/s of those bytes at 23.9 M and 67 M elements and 0.1 %; a bucket
-// of ResNet-50 with its serving pass takes 180 us, three passes over the arrays took 500).  A list that came out shorter than k or longer than its room (a sample that
-// misled, or massive ties) makes the launch fall back to histogram passes over the
-// whole array.
+// GradDrop (encodes at 0.1 %: DGC 5.2 TB/s of those bytes at 67 M elements, GradDrop 3.6
+// and 4.8 at 25 M and 67 M; the kernel of a PS bucket with ResNet-50's 25.5 M elements takes
+// 182 us, 98 of them this pass over its arrays).  A list that came out shorter than k or
+// longer than its room (a sample that misled, or massive ties) makes the launch fall back
+// to histogram passes over the whole array.
 //
 // Up to a few million elements the time is a chain of latencies instead: two grid
 // barriers, and steps of a few dependent L2 accesses each (about 0.7 us an atomic).  So

@@ -8,8 +8,8 @@
 // kernel that holds SMs for longer than that comes between this one's CTAs, the payload may
 // lack elements, and the workspace's status word (kWsStatus) is set.
 // It was a chain of eight launches that read the array three times behind the update:
-// GradDrop's encode of 23.9 M elements at 0.1 % took 138 us and takes 87, of 1 M elements
-// 63 and takes 33 (B200, states rotating through more than L2 holds).
+// GradDrop's encode of 16.8 M elements at 0.1 % took 130 us and takes 67, of 1 M elements
+// 68 and takes 34 (B200, L2 flushed in between).
 //
 // Without it (the allocation-free entry point) four launches read the array once each:
 //   pass 0   state update fused with the first radix histogram

@@ -94,7 +94,8 @@ def sweep_fused(sizes, iters, ranks, ctas, out):
 
 def run_single(alg, topo, mbytes, ctas, iters, out, flush_l2=True, in_place=False):
     """One rank, one tensor, one fused launch per iteration (the case to hand to
-    a profiler): encode + local hand-off + decode of `mbytes` of fp32 gradient."""
+    a profiler): encode + decode of `mbytes` of fp32 gradient, without owner state for
+    the quantisers' PS."""
     peaks = measured_peaks()
     flush = L2Flusher() if flush_l2 else None
     c = Compressor(alg)
@@ -171,8 +172,7 @@ def sweep_generated(mbytes, iters, out):
             out.append(row)
             print(json.dumps(row), flush=True)
     # DGC encode: the generated function is one kernel for both state updates plus the
-    # run-time library's exact top-k; the hand-written path folds the updates into the
-    # selection's histogram pass
+    # run-time library's exact top-k; the hand-written path selects in the updates' pass
     ratio, m = 0.001, 0.9
     k = int(n * ratio) + 16      # the function rounds ratio * n up in fp32; the buffer may be larger
     hand = Compressor("dgc", ratio=ratio)

@@ -48,8 +48,8 @@ class Compressor:
 
     def new_workspace(self, device, n: int | None = None):
         """Scratch of the sparse CUDA encoder: radix histograms and counters, plus
-        (when the tensor size ``n`` is given) room for the candidate list that lets
-        the encoder read the array once instead of three times after the update."""
+        (when the tensor size ``n`` is given) room for the candidate lists with which the
+        encoder selects in the update's pass, instead of reading the array three times more."""
         if self.spec.sparse and torch.device(device).type == "cuda":
             L = _lib.cuda()
             nb = int(L.hp_sparse_workspace_bytes()) if n is None else \

@@ -2,7 +2,8 @@
 
 :class:`FusedDenseBucket` owns the symmetric inbox / flag regions of one bucket of
 tensors and launches ONE persistent kernel per synchronisation that performs
-encode, peer-to-peer transfer and decode-aggregate for every tensor of the bucket.
+encode, peer-to-peer transfer and decode-aggregate for every tensor of the bucket (one
+rank, which has nobody to exchange with, a kernel that encodes and decodes a tile per CTA).
 With ``emulate=N`` a single GPU plays all N ranks in one cooperative launch
 (gridDim.y = N): kernels that wait on one another must not run as separate
 launches on one GPU, so this is how the multi-rank protocol is tested on one GPU.
