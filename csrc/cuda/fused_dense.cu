@@ -641,7 +641,7 @@ __device__ __forceinline__ void serve_phase(const BucketDev& bk, const HpComm& c
       decode_average<ALG, B>(frag, meta, fp, x);
       store_checked(sg.out + E * cm.emu_stride_out + tr.off, m, x);
     }
-    if (OWN_HERE) __syncthreads();  // the prefetch stage of this tile may be refilled from here on
+    __syncthreads();  // the tile's prefetch stage and the reduction's shared words are free from here on
   }
   trace_phase(cm, E, pushes, sm.ws);
 }
