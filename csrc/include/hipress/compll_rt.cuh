@@ -49,6 +49,35 @@ COMPLL_FN float compll_rand01(uint64_t seed, uint64_t elem, uint32_t site) {
   return hipress::u01(compll_rand4(seed, elem >> 2, site).v[elem & 3]);
 }
 
+// Quotients with one divisor, rounded as `/` rounds them, from a product and three fused
+// multiply-adds.  hi + lo is 1/b to about 47 bits (hi rounded to nearest), so q is within
+// one unit of a/b, the remainder a - b*q is exact, and q + remainder * hi rounds to the
+// nearest float (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990; the two-part reciprocal is from N. Brisebarre, J.-M. Muller
+// and S. K. Raina, "Accelerating correctly rounded floating-point division when the divisor
+// is known in advance", 2004).  Holds while nothing overflows or gets subnormal: for b in
+// [2^-60, 2^61) (`ok`) and |a| in [2^-63, 2^65) -- of anything else, zero included,
+// compll_div sets the top bit of `bad`, and the caller divides instead.
+struct CompllDivisor {
+  float b, hi, lo;
+  bool ok;
+};
+COMPLL_FN CompllDivisor compll_divisor(float b) {
+  CompllDivisor d;
+  d.b = b;
+  d.hi = 1.0f / b;
+  d.lo = fmaf(-b, d.hi, 1.0f) * d.hi;
+  d.ok = b >= 0x1p-60f && b < 0x1p61f;
+  return d;
+}
+COMPLL_FN float compll_div(float a, const CompllDivisor& d, uint32_t& bad) {
+  uint32_t bits;
+  memcpy(&bits, &a, 4);
+  bad |= (bits << 1) - (64u << 24);   // its exponent, from 0 where the quotient is exact
+  const float q = fmaf(a, d.hi, a * d.lo);
+  return fmaf(fmaf(-d.b, q, a), d.hi, q);
+}
+
 #if defined(__CUDACC__)
 // ---- support of the fused (one launch per function) target --------------------
 // a bit width known when the code is compiled
@@ -56,6 +85,43 @@ template <uint32_t W>
 struct CompllWidth {
   __device__ constexpr operator uint32_t() const { return W; }
 };
+template <bool V>
+struct CompllFlag {
+  __device__ constexpr operator bool() const { return V; }
+};
+// Philox4x32-7 of one seed: the keys of the rounds are made once, not for every call (two
+// additions a round, a tenth of TernGradEncode's instructions)
+struct CompllRand {
+  uint32_t k0[hipress::kPhiloxRounds], k1[hipress::kPhiloxRounds];
+  __device__ __forceinline__ explicit CompllRand(uint64_t seed) {
+#pragma unroll
+    for (int r = 0; r < hipress::kPhiloxRounds; ++r) {
+      k0[r] = (uint32_t)seed + r * 0x9E3779B9u;
+      k1[r] = (uint32_t)(seed >> 32) + r * 0xBB67AE85u;
+    }
+  }
+  // compll_rand4 of a group below 2^32
+  __device__ __forceinline__ hipress::Philox4 operator()(uint32_t group, uint32_t site) const {
+    uint32_t c0 = group, c1 = 0u, c2 = site, c3 = 0u;
+#pragma unroll
+    for (int r = 0; r < hipress::kPhiloxRounds; ++r) {
+      uint32_t hi0, lo0, hi1, lo1;
+      hipress::philox_mulhilo(0xD2511F53u, c0, hi0, lo0);
+      hipress::philox_mulhilo(0xCD9E8D57u, c2, hi1, lo1);
+      c0 = hi1 ^ c1 ^ k0[r];
+      c1 = lo1;
+      c2 = hi0 ^ c3 ^ k1[r];
+      c3 = lo0;
+    }
+    return hipress::Philox4{{c0, c1, c2, c3}};
+  }
+};
+// Groups of four elements that lie in whole blocks of 256 groups, where every vector can
+// be read and written 16 bytes at a time; none when a vector is off alignment or a group's
+// number does not fit 31 bits.
+__device__ __forceinline__ uint32_t compll_whole(uint64_t count, uint64_t addresses) {
+  return (addresses & 15) == 0 && count < (1ull << 33) ? (uint32_t)(count / 1024) * 256u : 0u;
+}
 // four consecutive floats starting at element i0 (a multiple of 4) of a vector of n
 __device__ __forceinline__ void compll_load4(const float* p, uint64_t i0, uint64_t n, float (&v)[4]) {
   if (i0 + 3 < n && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
@@ -150,6 +216,26 @@ __device__ __forceinline__ void compll_pack_store(uint8_t* dst, uint64_t nbytes,
     *reinterpret_cast<uint32_t*>(p) = w;
   } else {
     for (uint32_t b = 0; b < 4 && off + b < nbytes; ++b) p[b] = (uint8_t)(w >> (8 * b));
+  }
+}
+
+// The same for a warp whose groups are all complete: no bounds.
+__device__ __forceinline__ void compll_pack_full(uint8_t* dst, uint32_t q, uint32_t frag, uint32_t bits) {
+  const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(dst) & 3u;
+  if (bits == 8 && low == 0) {
+    reinterpret_cast<uint32_t*>(dst)[q] = frag;
+  } else if (bits >= 4 && (low & 1u) == 0) {
+    uint16_t* p = reinterpret_cast<uint16_t*>(dst + (uint64_t)q * (bits / 2));
+    p[0] = (uint16_t)frag;
+    if (bits == 8) p[1] = (uint16_t)(frag >> 16);
+  } else if (bits == 1 || low == 0) {
+    const uint32_t lanes = low == 0 ? 8u / bits : 2u;   // whose bits go out together
+    for (uint32_t s = 1, sh = 4u * bits; s < lanes; s <<= 1, sh <<= 1) frag |= __shfl_down_sync(0xffffffffu, frag, s) << sh;
+    if ((q & (lanes - 1)) != 0) return;
+    if (low == 0) reinterpret_cast<uint32_t*>(dst)[q / lanes] = frag;
+    else dst[q / 2] = (uint8_t)frag;
+  } else {
+    for (uint32_t b = 0; b < bits / 2; ++b) dst[(uint64_t)q * (bits / 2) + b] = (uint8_t)(frag >> (8 * b));
   }
 }
 

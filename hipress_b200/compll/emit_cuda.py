@@ -221,6 +221,11 @@ class Emitter:
         if isinstance(e, F.Binary):
             if e.op == "%":
                 return f"({X(e.a)} % {X(e.b)})"
+            hook = getattr(self, "_binary_hook", None)
+            if hook is not None:      # fused target: cheaper forms with the same bits
+                got = hook(e, local, X)
+                if got is not None:
+                    return got
             return f"({X(e.a)} {e.op} {X(e.b)})"
         if isinstance(e, F.Ternary):
             return f"({X(e.c)} ? {X(e.a)} : {X(e.b)})"
@@ -272,7 +277,9 @@ class Emitter:
             elif isinstance(st, F.Assign):
                 out.append(f"{indent}{self.expr(st.target, local)} = {self.expr(st.value, local)};")
             elif isinstance(st, F.If):
-                out.append(f"{indent}if ({self.expr(st.cond, local)}) {{")
+                hook = getattr(self, "_cond_hook", None)
+                cond = (hook(st.cond, local) if hook is not None else None) or self.expr(st.cond, local)
+                out.append(f"{indent}if ({cond}) {{")
                 out.append(self.stmts(st.then, set(local), ret_partial, indent + "  "))
                 if st.other:
                     out.append(f"{indent}}} else {{")

@@ -232,6 +232,10 @@ def _ordered(r: F.Reduce) -> bool:
     return not (isinstance(r.fn, F.Name) and r.fn.id in ("smaller", "greater"))
 
 
+def _is_num(e, value: float) -> bool:
+    return isinstance(e, F.Num) and float(e.text) == value
+
+
 class FusedGen:
     """Emits the fused kernel and its launch for a plan that is ``ok``."""
 
@@ -293,8 +297,51 @@ class FusedGen:
                 return f"in_{vec}[u][e]"
             return frag_value(s)
 
+        reducing = any(it.kind == "reduce" for it in ph.items)
+        divisors: dict[str, None] = {}
+        flags: list[str] = []
+
+        def float_scalar(e, local):
+            return isinstance(e, F.Name) and e.id not in local and e.id in em.syms and \
+                em.syms[e.id].kind in ("param_scalar", "reduced", "derived", "extracted") and \
+                em.syms[e.id].type.name == "float"
+
+        def unit_draw(e):
+            return isinstance(e, F.Random) and e.type == "float" and _is_num(e.lo, 0) and _is_num(e.hi, 1)
+
+        def binary_hook(e, local, expr):
+            if e.op == "/" and float_scalar(e.b, local) and not reducing:
+                # one divisor for the whole phase; the elements run a second time, with `/`,
+                # where a quotient may have come out wrong, so nothing may be accumulated
+                divisors[e.b.id] = None
+                num = f"(float)({expr(e.a)})"
+                return f"(exact ? {num} / c.v_{e.b.id} : compll_div({num}, dv_{e.b.id}, bad))"
+            if e.op == "+" and (unit_draw(e.a) or unit_draw(e.b)):
+                # the draw is a multiple of 2^-24: exact, so one rounding either way
+                first = None if unit_draw(e.a) else expr(e.a)     # sites count in source order
+                site, em.rand_sites = em.rand_sites, em.rand_sites + 1
+                sites.append(site)
+                other = expr(e.b) if first is None else first
+                return f"fmaf((float)(rg{site}.v[e] >> 8), 1.0f / 16777216.0f, (float)({other}))"
+            return None
+
+        def cond_hook(cond, local):
+            # a condition on scalars alone: the loop is compiled for both of its values
+            names = [n for n in _walk(cond) if isinstance(n, (F.Name, F.Index, F.Random, F.Call, F.SizeOf))]
+            if not names or any(not isinstance(n, F.Name) or n.id in local or
+                                em.syms[n.id].kind not in ("param_scalar", "reduced", "derived", "extracted")
+                                for n in names):
+                return None
+            text = em.expr(cond, set())
+            if text not in flags:
+                if flags:
+                    return None
+                flags.append(text)
+            return "flag"
+
         em._index_hook, em._random_hook = index_hook, random_hook
-        decls, stores = [], []
+        em._binary_hook, em._cond_hook = binary_hook, cond_hook
+        decls, stores, whole_stores = [], [], []
         try:
             for k, it in enumerate(ph.items):
                 if it.kind == "reduce":
@@ -343,10 +390,16 @@ class FusedGen:
         const uint32_t frag = {var}[0] | ({var}[1] << bits) | ({var}[2] << (2 * bits)) | ({var}[3] << (3 * bits));
         compll_pack_store(c.v_{it.target}, (count * bits + 7) / 8, q, frag, bits);
       }}""")
+                        whole_stores.append(stores[-1].replace(
+                            f"compll_pack_store(c.v_{it.target}, (count * bits + 7) / 8, q, frag, bits)",
+                            f"compll_pack_full(c.v_{it.target}, q, frag, bits)"))
                     else:
                         stores.append(f"      compll_store4(c.v_{it.target}, i0, count, {var});")
+                        whole_stores.append(stores[-1] if rty != "float" else
+                                            f"      reinterpret_cast<float4*>(c.v_{it.target})[q] = "
+                                            f"make_float4({var}[0], {var}[1], {var}[2], {var}[3]);")
         finally:
-            em._index_hook = em._random_hook = None
+            em._index_hook = em._random_hook = em._binary_hook = em._cond_hook = None
             em._own = None
             em._return_to = None
         # U groups of four elements per thread and trip, every load of a trip issued before
@@ -394,7 +447,25 @@ class FusedGen:
                                 f"(p_{tname}) + {off}, c.v_{fname});")
             if rows:
                 header = "    if (blockIdx.x == 0 && threadIdx.x == 0) {\n" + nl.join(rows) + "\n    }\n"
-        main = f"""    for (uint64_t qb0 = (uint64_t)blockIdx.x * blockDim.x; qb0 < groups; qb0 += stride * {U}) {{
+        def elements(skip_test: str) -> str:
+            loop = f"""#pragma unroll
+      for (int e = 0; e < 4; ++e) {{
+        const uint64_t i = i0 + e;
+        (void)i;
+{skip_test}{nl.join(body)}
+      }}"""
+            if not divisors:
+                return loop
+            ok = " && ".join(f"dv_{d}.ok" for d in divisors)
+            return f"""      auto elements = [&](auto exact_) {{
+        constexpr bool exact = decltype(exact_)();
+        uint32_t bad = 0;
+{loop}
+        return bad >> 31;
+      }};
+      if (!({ok}) || elements(CompllFlag<false>())) elements(CompllFlag<true>());"""
+
+        main = f"""    for (; qb0 < groups; qb0 += stride * {U}) {{
 {nl.join(larr)}
 #pragma unroll
       for (int u = 0; u < {U}; ++u) {{   // past the end the loads return zeros and touch nothing
@@ -413,45 +484,100 @@ class FusedGen:
       (void)full;
 {nl.join(rngs)}
 {nl.join(decls)}
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {{
-        const uint64_t i = i0 + e;
-        if ({skip}) continue;
-{nl.join(body)}
-      }}
+{elements(f"        if ({skip}) continue;{nl}")}
 {nl.join(stores)}
       }}
     }}
 """
-        main = self._per_width(main, need_frag, ph)
+        start = "    uint64_t qb0 = (uint64_t)blockIdx.x * blockDim.x;\n"
+        # Blocks whose groups are all complete run without bounds tests and with 32-bit
+        # indices.  TernGradEncode of 16.8 M elements took 56 us, of 67 M 207, and takes 37
+        # and 139 with these loops: 36 instructions per element of its second phase were the
+        # bound, 27 are left, 10 of them the random draws.  A trip of loads ahead cost more
+        # in registers than it gained (39 and 148 us).  Functions with sums gain 1 to 3 % and
+        # lose 7 % at 100 K elements, those of a single phase nothing: they keep one loop.
+        whole = bool(need_in) and len(self.plan.phases) > 1 and not any(_ordered(r.expr) for r in em.reduces)
+        if whole:
+            floats = [v for v in need_in if em.syms[v].type.name == "float"]
+            touched = sorted(set(floats) | {it.target for it in ph.items if it.kind == "map" and
+                                            em.syms[it.target].bits is None and em.syms[it.target].type.name == "float"})
+            address = " | ".join(f"reinterpret_cast<uint64_t>(c.v_{v})" for v in touched) or "0"
+            wloads = [f"""        {{
+          const float4 t = reinterpret_cast<const float4*>(c.v_{v})[q];
+          in_{v}[u][0] = t.x; in_{v}[u][1] = t.y; in_{v}[u][2] = t.z; in_{v}[u][3] = t.w;
+        }}""" if v in floats else f"        compll_load4(c.v_{v}, (uint64_t)q * 4, count, in_{v}[u]);" for v in need_in]
+            wloads += [ld.replace(", q, ", ", (uint64_t)q, ") for ld in loads[len(need_in):]]
+            wrngs = [f"      const hipress::Philox4 rg{s} = rand(q, {s}u);" for s in sorted(set(sites))]
+            start += f"""    const uint32_t whole = compll_whole(count, {address});
+    if (whole) {{
+      const uint32_t step = (uint32_t)stride;
+      for (uint32_t qw = (uint32_t)qb0; qw < whole; qw += step * {U}) {{
+{nl.join(larr)}
+#pragma unroll
+      for (int u = 0; u < {U}; ++u) {{
+        const uint32_t q = qw + u * step + threadIdx.x;
+        if (u > 0 && qw + u * step >= whole) break;
+{nl.join(wloads)}
+      }}
+#pragma unroll
+      for (int u = 0; u < {U}; ++u) {{
+      if (u > 0 && qw + u * step >= whole) break;
+      const uint32_t q = qw + u * step + threadIdx.x;
+      const uint64_t i0 = (uint64_t)q * 4;
+      (void)i0;
+{nl.join(wrngs)}
+{nl.join(decls)}
+{elements("")}
+{nl.join(whole_stores)}
+      }}
+      }}
+      // the block whose turn it is takes the groups that are left
+      qb0 = whole / 256u % gridDim.x == blockIdx.x ? whole : groups;
+    }}
+"""
+        main = self._per_width(start + main, need_frag, ph, flags)
+        once = [f"    const CompllDivisor dv_{d} = compll_divisor(c.v_{d});" for d in divisors]
+        if whole and sites:
+            once.append("    const CompllRand rand(c.seed);")
         out = f"""  {{  // ---- phase {pi}: {', '.join((it.target if it.kind == 'map' else 'reduce ' + it.sym.name) for it in ph.items)}
 {header}    const uint64_t count = {ph.count};
     const uint64_t groups = (count + 3) / 4;
-{nl.join(acc_init)}
+{nl.join(acc_init + once)}
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 {main}{self._block_reduce(reds)}  }}
 """
         return out
 
-    def _per_width(self, main: str, need_frag, ph: Phase) -> str:
+    def _per_width(self, main: str, need_frag, ph: Phase, flags: list) -> str:
         """A width that is a scalar of the function (a parameter, a header field) makes every
         shift and mask of the packing a run-time one: the loop is compiled for the widths
-        1, 2, 4 and 8 as well, and the kernel takes the one that applies."""
+        1, 2, 4 and 8 as well, and the kernel takes the one that applies.  So it is for both
+        values of a condition on scalars (`flags`): as a branch in the loop
+        TernGradEncode's cost 7 instructions per element."""
         em = self.em
         names = set()
         for v in list(need_frag) + [it.target for it in ph.items if it.kind == "map"]:
             bits = em.syms[v].bits
             if isinstance(bits, F.Name) and em.syms[bits.id].kind in ("param_scalar", "extracted"):
                 names.add(bits.id)
-        if len(names) != 1:
-            return main
-        name = f"c.v_{names.pop()}"
-        body = main.replace(name, "width")
-        cases = " ".join(f"case {w}: loop(CompllWidth<{w}>()); break;" for w in (1, 2, 4, 8))
-        return f"""    auto loop = [&](auto width_) {{
-      const uint32_t width = width_;
-{body}    }};
-    switch ({name}) {{ {cases} default: loop((uint32_t){name}); }}
+        name = f"c.v_{names.pop()}" if len(names) == 1 else None
+        if name is None and not flags:
+            return "    {\n" + main + "    }\n"
+        body = main if name is None else main.replace(name, "width")
+        params = (["auto width_"] if name else []) + (["auto flag_"] if flags else [])
+        head = ("      const uint32_t width = width_;\n" if name else "") + \
+            ("      constexpr bool flag = decltype(flag_)();\n" if flags else "")
+
+        def call(width):
+            one = lambda f: f"loop({', '.join(([width] if name else []) + ([f'CompllFlag<{f}>()'] if flags else []))});"  # noqa: E731
+            return f"if ({flags[0]}) {one('true')} else {one('false')}" if flags else one("")
+
+        cases = call("") if name is None else \
+            f"switch ({name}) {{ " + " ".join(f"case {w}: {call(f'CompllWidth<{w}>()')} break;" for w in (1, 2, 4, 8)) + \
+            f" default: {call(f'(uint32_t){name}')} }}"
+        return f"""    auto loop = [&]({', '.join(params)}) {{
+{head}{body}    }};
+    {cases}
 """
 
     def _block_reduce(self, reds) -> str:
