@@ -605,13 +605,35 @@ class FusedGen:
     def _fold(self, reds) -> str:
         """Behind the barrier: every block folds the per-block partials itself."""
         rows = []
+        free = [s for s in reds if not _ordered(s.expr)]
+        if free:
+            # all together: every thread ends with the results, behind one barrier
+            types = [C_TYPES[s.type.name] for s in free]
+            part = lambda s, ty: f"({ty})__ldcg(&partials[{s.slot} * gridDim.x + w])"  # noqa: E731
+            rows.append("  {")
+            rows += [f"    {ty} f_{s.name} = ({ty})({self.em.expr(s.expr.init, set())});" for s, ty in zip(free, types)]
+            rows.append("    for (unsigned w = threadIdx.x; w < gridDim.x; w += blockDim.x) {")
+            rows += [f"      f_{s.name} = {self._apply(s.expr, 'f_' + s.name, part(s, ty))};" for s, ty in zip(free, types)]
+            rows.append("    }\n    for (int off = 16; off > 0; off >>= 1) {")
+            rows += [f"      {{ {ty} o = __shfl_xor_sync(0xffffffffu, f_{s.name}, off); "
+                     f"f_{s.name} = {self._apply(s.expr, 'f_' + s.name, 'o')}; }}" for s, ty in zip(free, types)]
+            rows.append("    }\n    if ((threadIdx.x & 31) == 0) {")
+            rows += [f"      sh[{s.slot}][threadIdx.x >> 5] = (float)f_{s.name};" for s in free]
+            rows.append("    }\n    __syncthreads();")
+            for s, ty in zip(free, types):
+                rows.append(f"    f_{s.name} = ({ty})sh[{s.slot}][0];\n    for (int w = 1; w < 8; ++w) f_{s.name} = "
+                            f"{self._apply(s.expr, 'f_' + s.name, '(' + ty + ')sh[' + str(s.slot) + '][w]')};\n"
+                            f"    red[{s.slot}] = (float)f_{s.name};\n"
+                            f"    if (blockIdx.x == 0 && threadIdx.x == 0) scalars[{s.slot}] = red[{s.slot}];")
+            rows.append("  }")
         for s in reds:
+            if not _ordered(s.expr):
+                continue
             ty = C_TYPES[s.type.name]
             init = self.em.expr(s.expr.init, set())
             load = '(' + ty + ')__ldcg(&partials[' + str(s.slot) + ' * gridDim.x + w])'
-            if _ordered(s.expr):
-                # one warp, every lane in a fixed order; eight loads in flight
-                fold = f"""    if (threadIdx.x < 32) {{
+            # one warp, every lane in a fixed order; eight loads in flight
+            fold = f"""    if (threadIdx.x < 32) {{
 #pragma unroll 8
       for (unsigned w = threadIdx.x; w < gridDim.x; w += 32)
         a = {self._apply(s.expr, 'a', load)};
@@ -621,20 +643,6 @@ class FusedGen:
       }}
       if (threadIdx.x == 0) sh[{s.slot}][0] = (float)a;
     }}
-    __syncthreads();"""
-            else:
-                fold = f"""    for (unsigned w = threadIdx.x; w < gridDim.x; w += blockDim.x)
-      a = {self._apply(s.expr, 'a', load)};
-    for (int off = 16; off > 0; off >>= 1) {{
-      {ty} o = __shfl_xor_sync(0xffffffffu, a, off);
-      a = {self._apply(s.expr, 'a', 'o')};
-    }}
-    if ((threadIdx.x & 31) == 0) sh[{s.slot}][threadIdx.x >> 5] = (float)a;
-    __syncthreads();
-    a = ({ty})sh[{s.slot}][0];
-    for (int w = 1; w < 8; ++w) a = {self._apply(s.expr, 'a', '(' + ty + ')sh[' + str(s.slot) + '][w]')};
-    __syncthreads();
-    if (threadIdx.x == 0) sh[{s.slot}][0] = (float)a;
     __syncthreads();"""
             rows.append(f"""  {{
     {ty} a = ({ty})({init});
