@@ -780,9 +780,9 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 // for onebit and TBQ: 102.8 M elements, TBQ ring 278 us (5.92 TB/s) in the persistent
 // kernel, 244 us (6.74 TB/s) here, PS 400 -> 363 us.  TernGrad, six CTAs per SM where no
 // state is kept: the ring is near HBM's speed (195 -> 124 us; at 67 M elements issue slots
-// 65 % used, DRAM 74 % of ncu's peak), PS quantises every tile twice and is bound by
-// instruction issue (378 -> 173 us; issue slots 79 % used, the integer pipe 60 %, DRAM 51 %,
-// warps ready but not selected 5.6 cycles per issue, waiting for memory 1.8).
+// 65 % used, DRAM 74 % of ncu's peak).  Through PS every tile is quantised twice, which was
+// bound by instruction issue (378 -> 173 us; issue slots 79 % used) until the server's
+// pass was made from the push's codes (tern_requantise).
 // RES: some tensor of the bucket keeps error-feedback state (TernGrad's buckets keep none,
 // but the entry point takes some).
 template <int ALG, int B, int TOPO, bool RES>
@@ -831,6 +831,9 @@ local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
       else store_tile(state, m, x);
     }
     if (TOPO == HP_TOPO_RING || pass == 1) break;
+    if (ALG == kTernGrad && !sp && m == kTile &&
+        tern_requantise<B>(frag, meta, fp.P, sg.id, off, fp.P.salt + 1u, s))
+      break;
 #pragma unroll
     for (int j = 0; j < kIter; ++j) decode_frag<ALG, B>(frag[j], meta, fp.P.tau, x[j]);
   }
