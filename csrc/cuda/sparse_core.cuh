@@ -835,19 +835,18 @@ __device__ __forceinline__ uint32_t emit_slices(uint32_t L, uint32_t most) {
   return n < most ? n : most;
 }
 
-// Slice x of nx of one array's candidates.  True in thread 0 of the CTA that finished
+// Places [lo, hi) of one array's candidate list, one of nx spans.  True in thread 0 of the CTA that finished
 // last, behind the headers.
 // A CTA whose barrier expired goes on, and may have read another count than the others:
 // their slices then overlap, and together hold more than the lists have room for.  So a
 // list is read up to its room and no further, and so is the second one written.
-static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const ListState& ls, const EmitDst& dst,
-                                               SelSmem& sm, uint32_t x, uint32_t nx) {
+static __device__ __noinline__ bool emit_span(int alg, const SelUnit& s, const ListState& ls, const EmitDst& dst,
+                                              SelSmem& sm, uint32_t lo, uint32_t hi, uint32_t nx) {
   const uint32_t L = min(ls.count, s.cap), low = ls.low;   // no overflow: the list holds all of them
   const size_t val_off = 16 + align_up(4ull * s.kmax, 16);
   const bool every = L <= s.k;                 // all candidates are sent
   uint32_t bin0 = 0, rem = 0, least = 0xFFFFFFFFu;
   if (!every) find_bin(s.ws, s.k, sm.fs, bin0, rem);
-  const uint32_t per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
   // four candidates per thread: the reservations of all CTAs on the two counters follow
   // one another, 25 ns each
   constexpr int kPer = 4;
@@ -960,6 +959,13 @@ static __device__ __noinline__ bool emit_slice(int alg, const SelUnit& s, const 
 #pragma unroll 1
   for (int d = 0; d < dst.n; ++d) *reinterpret_cast<uint4*>(dst.out[d]) = *reinterpret_cast<const uint4*>(&h);
   return true;
+}
+
+// slice x of nx of a list without gaps
+__device__ __forceinline__ bool emit_slice(int alg, const SelUnit& s, const ListState& ls, const EmitDst& dst, SelSmem& sm,
+                                           uint32_t x, uint32_t nx) {
+  const uint32_t L = min(ls.count, s.cap), per = (L + nx - 1) / nx, lo = min(x * per, L), hi = min(lo + per, L);
+  return emit_span(alg, s, ls, dst, sm, lo, hi, nx);
 }
 
 // out[idx] (+)= val * scale ; indices come from another rank: bounds-checked

@@ -1,15 +1,16 @@
 // Sparse (top-k) compression for DGC and GradDrop on sm_100a.
 //
-// With room for a candidate list (the usual call) an encode is ONE cooperative launch:
-// sample, update + collect, finish (sparse_core.cuh), with grid barriers in between.  Its
-// CTAs wait for one another, so all of them must be resident at once: the grid is sized
-// for the SMs that the stream may use, and where kernels on other streams keep those
-// occupied the launch waits for room.  Each barrier is bounded (kGridBarrierNs); if a
-// kernel that holds SMs for longer than that comes between this one's CTAs, the payload may
-// lack elements, and the workspace's status word (kWsStatus) is set.
-// It was a chain of eight launches that read the array three times behind the update:
-// GradDrop's encode of 16.8 M elements at 0.1 % took 130 us and takes 67, of 1 M elements
-// 68 and takes 34 (B200, L2 flushed in between).
+// With room for a candidate list (the usual call) an encode is three launches, of which
+// each begins while the one before it ends: sample, update + collect with a CTA per half
+// tile, emit (sparse_chain.cuh).  One persistent kernel with grid barriers did the same and
+// is kept for calls that limit the CTAs (max_ctas): equal shares left the faster SMs idle,
+// and the arrays stood still while the sample was worked out.  DGC encode and decode at
+// 0.1 %, us, persistent / chain (B200): 64 K elements 28.3 / 26.2, 1 M 37.9 / 30.8, 3 M
+// 52.4 / 45.2, 10 M at 1 % 93.8 / 81.1, 20 M 123.3 / 119.6.
+// The emitting launch is cooperative, because where a list came out short its CTAs count
+// the digits together, and sized for the SMs that the stream may use.  Barriers are
+// bounded (kGridBarrierNs); if a kernel that holds SMs for longer than that comes between
+// the CTAs, the payload may lack elements, and the workspace's status word (kWsStatus) is set.
 //
 // Without it (the allocation-free entry point) four launches read the array once each:
 //   pass 0   state update fused with the first radix histogram
@@ -28,6 +29,7 @@
 // sort/copy_if for them (src/CompLL/GCGen/unit.py:24-29) but has no translation
 // rule, so there is no reference kernel to compare with.
 #include "partition.cuh"
+#include "sparse_chain.cuh"
 #include "sparse_core.cuh"
 #include "sync.cuh"
 #include "hipress/noalloc.h"
@@ -62,7 +64,7 @@ sparse_emit_kernel(int alg, float* __restrict__ a, float* __restrict__ u, uint64
   emit_body(alg, a, u, n, k, kmax, d, ws, fs, es, blockIdx.x, gridDim.x);
 }
 
-// ---- the whole encode in one cooperative launch
+// ---- the whole encode in one cooperative launch, as wide as the caller allows
 struct SelArgs {
   SelUnit unit;
   int alg, mode;
@@ -189,7 +191,7 @@ extern "C" {
 // 4 * kmax pairs each on top, the encoder reads the state once, in the update
 uint64_t hp_sparse_workspace_bytes() { return (uint64_t)kWsWords * 4; }
 uint64_t hp_sparse_workspace_bytes_for(uint64_t kmax) {
-  return (uint64_t)(kWsWords + kBarrierWords) * 4 + (8 * kmax + 4096) * 8;
+  return (uint64_t)(kWsWords + kBarrierWords + 32 * kChainLists) * 4 + (8 * kmax + 4096) * 8;
 }
 
 // ws_bytes beyond the histogram block is used for the candidate lists; when there
@@ -207,7 +209,8 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
   float* uu = alg == kDgc ? u : nullptr;
   const int mode = !update ? 0 : (alg == kGradDrop ? 1 : 2);
   // histograms and counters, then the barrier words and the candidate lists
-  const uint64_t head = (uint64_t)(kWsWords + kBarrierWords) * 4;
+  constexpr uint32_t kParts = 32 * kChainLists;   // counts of a list's parts
+  const uint64_t head = (uint64_t)(kWsWords + kBarrierWords + kParts) * 4;
   const uint64_t pairs = ws_bytes > head ? (ws_bytes - head) / 8 : 0;
   const bool listed = pairs >= 1024 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0;   // counters are read as uint4
   cudaError_t e = cudaMemsetAsync(ws, 0, listed ? head : (size_t)kWsWords * 4, st);
@@ -232,16 +235,41 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
       }
     }
     int cap = per * stream_sms(st, sms);   // the stream may own only some of the SMs
+    if (max_ctas <= 0 && chain_per_sm(dev) > 0) {
+      ChainArgs C = {};
+      SelUnit& V = C.unit[0].s;
+      V.g = g;
+      V.a = a;
+      V.u = uu;
+      V.ws = ws;
+      V.cv = reinterpret_cast<float*>(ws + kWsWords + kBarrierWords + kParts);
+      V.n = (uint32_t)n;
+      V.k = (uint32_t)k;
+      V.kmax = (uint32_t)kmax;
+      V.cap = list_cap(pairs);
+      const Sampling cs = sampling((uint32_t)tiles, tiles, (uint32_t)cap, n, k);
+      V.stride = cs.stride;
+      V.top = cs.top;
+      C.unit[0].counts = ws + kWsWords + kBarrierWords;
+      C.units = 1;
+      C.alg = alg;
+      C.momentum = momentum;
+      C.payload = out;
+      C.barrier = ws + kWsWords;
+      C.status = ws + kWsStatus;
+      if (chain_place(C, chain_per_sm(dev) * stream_sms(st, sms)))
+        return (int)(mode == 0 ? chain_select<0>(C, st) : (mode == 1 ? chain_select<1>(C, st) : chain_select<2>(C, st)));
+    }
     if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
     const int grid = (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);
-    SelArgs A;
+    SelArgs A = {};
     SelUnit& U = A.unit;
     U.g = g;
     U.a = a;
     U.u = uu;
     U.clear = nullptr;
     U.ws = ws;
-    U.cv = reinterpret_cast<float*>(ws + kWsWords + kBarrierWords);
+    U.cv = reinterpret_cast<float*>(ws + kWsWords + kBarrierWords + kParts);
     U.n = (uint32_t)n;
     U.k = (uint32_t)k;
     U.kmax = (uint32_t)kmax;

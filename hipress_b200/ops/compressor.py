@@ -68,10 +68,11 @@ class Compressor:
         ``state`` is the dict from :meth:`new_state` (views of it for chunks).
 
         On a GPU a sparse encode with the workspace of :meth:`new_workspace` for this
-        size is one cooperative launch, as wide as the SMs that ``stream`` may use: it
-        starts when all its CTAs find room at once, and must not share the GPU with a
-        kernel that holds SMs for seconds.  ``max_ctas`` makes it narrower; a workspace
-        without a size runs plain launches instead, which need no such room.
+        size is three launches, the last one cooperative, as wide as the SMs that ``stream``
+        may use: it starts when all its CTAs find room at once, and must not share the GPU
+        with a kernel that holds SMs for seconds.  With ``max_ctas`` it is one cooperative
+        launch of that many CTAs; a workspace without a size runs plain launches instead,
+        which need no such room.
         """
         sp = self.spec
         n = g.numel()
