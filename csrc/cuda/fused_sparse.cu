@@ -15,6 +15,8 @@
 //   pull   : every rank waits for each owner's flag and scatters value / N into the
 //            result, which the update pass cleared.
 //
+// A job of one rank takes neither: its bucket is a chain of launches (launch_chain).
+//
 // All units of a bucket are batched in every phase, which is the "bulk
 // synchronisation" of many small tensors: the update pass splits the bucket's tiles, not
 // its tensors, over the CTAs (equal shares of the CTAs per tensor left ResNet-50's largest
@@ -28,6 +30,8 @@
 #include <cuda_runtime.h>
 
 #include "hipress/capi.h"
+#include "partition.cuh"
+#include "sparse_chain.cuh"
 #include "sparse_core.cuh"
 #include "sync.cuh"
 
@@ -583,8 +587,73 @@ static uint64_t sp_hist_words(int nseg, int nranks) {
   return (uint64_t)(nseg * nranks + nseg) * kWsWords;   // the ring uses nseg * nranks of them
 }
 
+// words behind the control words that a job of one rank uses: the counts of its lists'
+// parts, push and server, and the server selection's barrier
+static uint64_t sp_chain_words(int nseg, int nranks) {
+  return nranks == 1 ? 2ull * nseg * 32 * kChainLists + kBarrierWords : 0;
+}
+static uint64_t sp_cleared_words(int nseg, int nranks) {
+  return sp_hist_words(nseg, nranks) + kCtlWords + sp_chain_words(nseg, nranks);
+}
+
+// A job of one rank waits for nobody: its selections run as chains of launches, in a PS the
+// owner's sum behind the push.  The persistent kernels that follow do the same with grid
+// barriers; us per step or bucket, persistent / chain (B200): ResNet-50, DGC, PS 199.6 /
+// 187.6; GradDrop ring 6.6 M elements 55.1 / 43.1, 20 M at 1 % 134 / 97; DGC ring 3 M 49.4 /
+// 34.2; DGC PS 64 K 51.9 / 39.5, 20 M 173 / 147; 24 arrays of 1 M in all, PS 60.7 / 48.7.
+// False when the arrays do not fit a chain (and always with a limit on the CTAs).
+static bool launch_chain(int topo, const SpBucket& bk, const HpComm& cm, uint8_t* ws, cudaStream_t st, int& rc) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || chain_per_sm(dev) == 0) return false;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int resident = chain_per_sm(dev) * stream_sms(st, sms);
+  uint32_t* words = reinterpret_cast<uint32_t*>(ws);
+  uint32_t* ctl = words + sp_hist_words(bk.nseg, 1);
+  uint8_t* lists = ws + align_up(sp_cleared_words(bk.nseg, 1) * 4, 256);
+  auto arrays = [&](ChainArgs& A, bool serve) {
+    A.units = bk.nseg;
+    A.alg = bk.alg;
+    A.momentum = bk.momentum;
+    A.scale = bk.inv_n;
+    A.barrier = serve ? ctl + kCtlWords + 2 * bk.nseg * 32 * kChainLists : ctl + kCtlBarrier;
+    A.status = reinterpret_cast<uint32_t*>(cm.status);
+    A.code = HP_STATUS_TIMEOUT | (8u << 16);
+    for (int i = 0; i < bk.nseg; ++i) {
+      const SpSeg& sg = bk.seg[i];
+      const int y = serve ? bk.nseg + i : i;
+      ChainUnit& u = A.unit[i];
+      u.s.g = serve ? nullptr : sg.g;
+      u.s.a = serve ? sg.sr : sg.a;
+      u.s.u = serve ? nullptr : sg.u;
+      u.s.clear = serve ? nullptr : sg.out;
+      u.s.ws = words + (size_t)y * kWsWords;
+      u.s.cv = reinterpret_cast<float*>(lists + (serve ? sg.cand_srv : sg.cand_push) * 8);
+      u.s.n = sg.n;
+      u.s.k = sg.n == sg.chunk ? sg.kmax : sg.k_last;
+      u.s.kmax = sg.kmax;
+      u.s.cap = list_cap(sg.cap);
+      const Sampling p = sampling(sg.tiles, bk.tiles_total, (uint32_t)resident, sg.chunk, sg.kmax);
+      u.s.stride = p.stride;
+      u.s.top = p.top;
+      u.counts = ctl + kCtlWords + (size_t)y * 32 * kChainLists;
+      u.add = topo == HP_TOPO_PS && !serve ? sg.sr : nullptr;
+      u.set = topo == HP_TOPO_PS && !serve ? nullptr : sg.out;
+    }
+    return chain_place(A, resident);
+  };
+  ChainArgs push = {}, sum = {};
+  if (!arrays(push, false) || (topo == HP_TOPO_PS && !arrays(sum, true))) return false;
+  cudaError_t e = cudaMemsetAsync(ws, 0, sp_cleared_words(bk.nseg, 1) * 4, st);
+  if (e == cudaSuccess) e = chain_select(bk.alg == kDgc ? 2 : 1, push, st);
+  if (e == cudaSuccess && topo == HP_TOPO_PS) e = chain_select(0, sum, st);
+  rc = (int)e;
+  return true;
+}
+
 static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int ctas,
                          cudaStream_t st) {
+  int chained = 0;
+  if (cm.nranks == 1 && ctas <= 0 && launch_chain(topo, bk, cm, static_cast<uint8_t*>(ws), st, chained)) return chained;
   const void* kern = topo == HP_TOPO_RING ? (const void*)sp_ring_kernel : (const void*)sp_ps_kernel;
   const int N = cm.nranks, nseg = bk.nseg;
   static int resident[2][64] = {};   // CTAs the GPU holds at once, per (topology, device)
@@ -618,7 +687,7 @@ static int launch_sparse(int topo, SpBucket& bk, const HpComm& cm, void* ws, int
   SpLaunch L;
   L.ws = static_cast<uint8_t*>(ws);
   L.hist_words = sp_hist_words(nseg, N);
-  L.hist_bytes = align_up((L.hist_words + kCtlWords) * 4, 256);
+  L.hist_bytes = align_up(sp_cleared_words(nseg, N) * 4, 256);
   L.ws_rank_bytes = L.hist_bytes + bk.cand_pairs * 8;
   for (int r = 0; r < ranks_here; ++r) {  // histograms, counters and control words start at zero
     e = cudaMemsetAsync(L.ws + (size_t)r * L.ws_rank_bytes, 0, (L.hist_words + kCtlWords) * 4, st);
@@ -650,7 +719,7 @@ int hp_fused_sparse_layout(float ratio, const uint64_t* ns, int nseg, int nranks
   // per rank played by a launch: histogram blocks of the push (nseg * nranks) and
   // server (nseg) units, control words, candidate lists
   if (ws_bytes)
-    *ws_bytes = align_up((sp_hist_words(nseg, nranks) + kCtlWords) * 4, 256) + bk.cand_pairs * 8;
+    *ws_bytes = align_up(sp_cleared_words(nseg, nranks) * 4, 256) + bk.cand_pairs * 8;
   return 0;
 }
 

@@ -1,5 +1,5 @@
 // The selection of sparse_core.cuh as a chain of launches, for callers that wait for nobody
-// (the stand-alone encode): sample, collect with a CTA per half tile, emit.  SMs do not run
+// (the stand-alone encode, buckets of a job of one rank): sample, collect with a CTA per half tile, emit.  SMs do not run
 // at one speed, and equal shares of a persistent grid leave the fast ones idle for a tenth
 // of the pass; a new CTA goes to whichever SM is free.  A launch begins while the one
 // before it ends, and the collecting CTAs that start ahead of the bound update their tile
@@ -10,9 +10,9 @@
 
 namespace hipress {
 
-constexpr int kChainThreads = 256;
-constexpr uint32_t kChainTile = kSelTile / 2;   // two float4 of each array per thread
-constexpr uint32_t kChainLists = 8;             // an array's list in parts: its counter takes 20 ns a reservation
+// An array's list is in parts, because its counter takes 20 ns a reservation; a CTA emits
+// each, and those of a bucket's forty arrays fit the GPU at once.
+constexpr uint32_t kChainLists = 7;
 
 struct ChainUnit {
   SelUnit s;
@@ -22,289 +22,24 @@ struct ChainUnit {
   float* add;           // where its pairs go, besides a payload (EmitDst)
   float* set;
 };
-__device__ __forceinline__ void after_launches_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// Half tile h of an array: update, and what reaches the bound into part `part` of its list.
-// HBM bound on large arrays; 256 threads and two vectors of each array per thread leave room
-// for five CTAs on an SM, whose starts and ends overlap (six: no change).
-template <int MODE>
-__device__ __forceinline__ void chain_collect(const SelUnit& s, uint32_t* counts, float momentum, uint32_t h, uint32_t part) {
-  __shared__ float val[kChainTile];
-  __shared__ uint32_t idx[kChainTile];
-  __shared__ uint32_t count, base;
-  const bool vec = ((reinterpret_cast<uintptr_t>(s.a) | (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.g) : 0) |
-                     (MODE >= 1 ? reinterpret_cast<uintptr_t>(s.clear) : 0) |
-                     (MODE == 2 ? reinterpret_cast<uintptr_t>(s.u) : 0)) & 15) == 0;
-  const uint64_t i0 = (uint64_t)h * kChainTile + threadIdx.x * 4;
-  const bool full = vec && (uint64_t)(h + 1) * kChainTile <= s.n;
-  constexpr int kStep = kChainThreads * 4;
-  float4 av[2], gv[2], uv[2];
-  if (threadIdx.x == 0) count = 0;
-  if (full) {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      av[j] = *reinterpret_cast<const float4*>(s.a + i0 + j * kStep);
-      if (MODE >= 1) gv[j] = *reinterpret_cast<const float4*>(s.g + i0 + j * kStep);
-      if (MODE == 2) uv[j] = *reinterpret_cast<const float4*>(s.u + i0 + j * kStep);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      av[j] = ld4(s.a, i0 + j * kStep, s.n, vec);
-      if (MODE >= 1) gv[j] = ld4(s.g, i0 + j * kStep, s.n, vec);
-      if (MODE == 2) uv[j] = ld4(s.u, i0 + j * kStep, s.n, vec);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint64_t i = i0 + j * kStep;
-    float4& v = av[j];
-    if (MODE == 1) {
-      v.x = v.x + gv[j].x; v.y = v.y + gv[j].y; v.z = v.z + gv[j].z; v.w = v.w + gv[j].w;
-    } else if (MODE == 2) {
-      float4& w = uv[j];
-      w.x = __fmaf_rn(momentum, w.x, gv[j].x);
-      w.y = __fmaf_rn(momentum, w.y, gv[j].y);
-      w.z = __fmaf_rn(momentum, w.z, gv[j].z);
-      w.w = __fmaf_rn(momentum, w.w, gv[j].w);
-      v.x = v.x + w.x; v.y = v.y + w.y; v.z = v.z + w.z; v.w = v.w + w.w;
-      if (full) *reinterpret_cast<float4*>(s.u + i) = w;
-      else st4(s.u, i, s.n, vec, w);
-    }
-    if (MODE >= 1) {
-      if (full) *reinterpret_cast<float4*>(s.a + i) = v;
-      else st4(s.a, i, s.n, vec, v);
-      if (s.clear) {
-        if (full) *reinterpret_cast<float4*>(s.clear + i) = make_float4(0.f, 0.f, 0.f, 0.f);
-        else st4(s.clear, i, s.n, vec, make_float4(0.f, 0.f, 0.f, 0.f));
-      }
-    }
-  }
-  after_launches_before();   // the bound
-  const uint32_t low = __ldcg(s.ws + kWsLow), room = s.cap / kChainLists;
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const float e[4] = {av[j].x, av[j].y, av[j].z, av[j].w};
-    if (max(max(abs_key(e[0]), abs_key(e[1])), max(abs_key(e[2]), abs_key(e[3]))) < low) continue;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (abs_key(e[q]) < low) continue;
-      const uint32_t p = atomicAdd(&count, 1u);
-      val[p] = e[q];
-      idx[p] = (uint32_t)i0 + j * kStep + q;
-    }
-  }
-  __syncthreads();
-  const uint32_t n = count;
-  if (n == 0) return;
-  if (threadIdx.x == 0) {
-    base = atomicAdd(counts + 32 * part, n);
-    if (base + n > room) s.ws[kWsOverflow] = 1u;
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (uint32_t p = threadIdx.x; p < n; p += kChainThreads) {
-    const float v = val[p];
-    atomicAdd(s.ws + cand_digit(abs_key(v), low), 1u);
-    if (base + p < room) {
-      s.cv[part * room + base + p] = v;
-      list_indices(s)[part * room + base + p] = idx[p];
-    }
-  }
-}
-
-constexpr int kChainUnits = 36;   // eight emitting CTAs for each of them fit the GPU at once
+constexpr int kChainUnits = HP_MAX_SEGS;
 struct ChainArgs {
   ChainUnit unit[kChainUnits];
   int units, alg;
   float momentum, scale;
   uint8_t* payload;      // of the only unit, or null
   uint32_t* barrier;     // kBarrierWords of zeros
-  uint32_t* status;
+  uint32_t *status, code;   // what a barrier that expires records, and where
   uint32_t emitters;     // CTAs that share the list of a unit: a multiple of kChainLists
 };
 
-__device__ __forceinline__ uint32_t chain_unit(const ChainArgs& A, uint32_t ChainUnit::* first, uint32_t i) {
-  uint32_t lo = 0, hi = (uint32_t)A.units;
-#pragma unroll 1
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) / 2;
-    if (A.unit[mid].*first <= i) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kSpThreads, 2) chain_sample_kernel(const __grid_constant__ ChainArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SelSmem& sm = *reinterpret_cast<SelSmem*>(smem_raw);
-  __shared__ SelUnit s;
-  const uint32_t y = chain_unit(A, &ChainUnit::sample0, blockIdx.x);
-  if (threadIdx.x == 0) s = A.unit[y].s;
-  __syncthreads();
-  after_launches_before();
-  let_next_launch_begin();   // what lies before this launch is complete: the next one may read it too
-  sample_body<MODE>(s, A.momentum, sm, blockIdx.x - A.unit[y].sample0, sm.stash[0]);
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kChainThreads, 5) chain_collect_kernel(const __grid_constant__ ChainArgs A) {
-  const uint32_t t = blockIdx.x / 2, y = chain_unit(A, &ChainUnit::tile0, t);
-  const ChainUnit& u = A.unit[y];
-  const uint32_t h = blockIdx.x - 2 * u.tile0, part = blockIdx.x % kChainLists;
-  if (MODE != 0 && (t - u.tile0) % u.s.stride == 0) {
-    after_launches_before();   // the sample's update
-    chain_collect<0>(u.s, u.counts, 0.0f, h, part);
-  } else {
-    chain_collect<MODE>(u.s, u.counts, A.momentum, h, part);
-  }
-}
-
-__device__ __forceinline__ ListState chain_state(const ChainUnit& u) {
-  ListState l = {0u, __ldcg(u.s.ws + kWsOverflow), __ldcg(u.s.ws + kWsLow)};
-#pragma unroll
-  for (uint32_t p = 0; p < kChainLists; ++p) l.count += __ldcg(u.counts + 32 * p);
-  return l;
-}
-
-union ChainSmem {
-  SelSmem sel;
-  uint32_t hist[kBins];
-  EmitSmem emit;
-};
-
-__global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_constant__ ChainArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ChainSmem& sm = *reinterpret_cast<ChainSmem*>(smem_raw);
-  __shared__ SelUnit s;
-  __shared__ EmitDst dst;
-  __shared__ WaitState wst;
-  __shared__ FindSmem fs;
-  const uint32_t y = blockIdx.x / A.emitters, x = blockIdx.x - y * A.emitters;
-  const ChainUnit& u = A.unit[y];
-  auto aim = [&](const ChainUnit& to) {
-    if (threadIdx.x == 0) {
-      s = to.s;
-      dst.n = A.payload ? 1 : 0;
-      dst.out[0] = A.payload;
-      dst.add = to.add;
-      dst.set = to.set;
-      dst.scale = A.scale;
-    }
-    __syncthreads();
-  };
-  wait_init(wst);
-  aim(u);
-  const ListState ls = chain_state(u);
-  if (!selection_failed(s, ls)) {
-    // the spans of a part: CTAs part, part + kChainLists, ...
-    const uint32_t part = x % kChainLists, sub = x / kChainLists, subs = A.emitters / kChainLists;
-    const uint32_t room = s.cap / kChainLists, n = min(__ldcg(u.counts + 32 * part), room);
-    const uint32_t per = (n + subs - 1) / subs, lo = min(sub * per, n), hi = min(lo + per, n);
-    emit_span(A.alg, s, ls, dst, sm.sel, part * room + lo, part * room + hi, A.emitters);
-  }
-  // whole-array passes for the units whose list is not complete; every CTA decides the same
-  int bad = 0;
-  for (int q = threadIdx.x; q < A.units; q += kSpThreads) bad |= selection_failed(A.unit[q].s, chain_state(A.unit[q]));
-  if (!__syncthreads_or(bad)) return;
-  uint32_t gen = 0;
-#pragma unroll 1
-  for (int pass = -1; pass <= 3; ++pass) {
-#pragma unroll 1
-    for (int q = 0; q < A.units; ++q) {
-      const ChainUnit& f = A.unit[q];
-      if (!selection_failed(f.s, chain_state(f))) continue;
-      __syncthreads();
-      aim(f);
-      const uint32_t c = blockIdx.x, G = gridDim.x;
-      if (pass < 0) {
-        for (uint32_t i = c * kSpThreads + threadIdx.x; i < 3u * kBins; i += G * kSpThreads) s.ws[i] = 0;
-      } else if (pass == 0) {
-        pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
-      } else if (pass < 3) {
-        pass_body(pass, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
-      } else {
-        emit_body(A.alg, s.a, s.u, s.n, s.k, s.kmax, dst, s.ws, fs, sm.emit, c, G);
-      }
-      __syncthreads();
-    }
-    if (pass < 3) grid_barrier(A.barrier, gen, gridDim.x, kGridBarrierNs, A.status, 1u, wst);
-  }
-}
-
-// ------------------------------------------------------------------ host side
 // CTAs of the emitting launch that an SM holds at once, 0 when the kernels cannot run
-inline int chain_per_sm(int dev) {
-  static int known[64] = {};
-  if (dev < 0 || dev >= 64) return 0;
-  if (known[dev]) return known[dev] - 1;
-  int per = 0;
-  const void* big[] = {(const void*)chain_sample_kernel<0>, (const void*)chain_sample_kernel<1>,
-                       (const void*)chain_sample_kernel<2>, (const void*)chain_emit_kernel};
-  bool ok = true;
-  for (const void* k : big)
-    ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChainSmem)) == cudaSuccess;
-  ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, chain_emit_kernel, kSpThreads, sizeof(ChainSmem)) == cudaSuccess;
-  if (!ok) {
-    cudaGetLastError();
-    per = 0;
-  }
-  known[dev] = per + 1;
-  return per;
-}
-
+int chain_per_sm(int dev);
 // Places the units' tiles and samples behind one another; `resident`: emitting CTAs that
 // run at once.  False when the lists cannot be shared out.
-inline bool chain_place(ChainArgs& A, int resident) {
-  uint64_t tiles = 0, samples = 0;
-  uint32_t longest = 1;
-  for (int i = 0; i < A.units; ++i) {
-    SelUnit& s = A.unit[i].s;
-    if (s.n == 0) return false;
-    const uint32_t t = (s.n - 1) / kSelTile + 1;
-    s.sampled = (t + s.stride - 1) / s.stride;
-    A.unit[i].tile0 = (uint32_t)tiles;
-    A.unit[i].sample0 = (uint32_t)samples;
-    tiles += t;
-    samples += s.sampled;
-    const uint32_t spans = (s.kmax + s.kmax / 2) / (4 * kSpThreads * kChainLists) + 1;
-    longest = longest > spans ? longest : spans;
-  }
-  const uint32_t most = (uint32_t)(resident / A.units) / kChainLists;
-  if (most < 1 || tiles > 0x3FFFFFFFull) return false;
-  A.emitters = kChainLists * (longest < most ? longest : most);
-  return true;
-}
-
-template <typename K>
-static cudaError_t chain_launch(K kern, uint32_t grid, int threads, size_t smem, bool early, cudaStream_t st, const ChainArgs& A) {
-  cudaLaunchAttribute at;
-  at.id = early ? cudaLaunchAttributeProgrammaticStreamSerialization : cudaLaunchAttributeCooperative;
-  if (early) at.val.programmaticStreamSerializationAllowed = 1;
-  else at.val.cooperative = 1;
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(threads);
-  c.dynamicSmemBytes = smem;
-  c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kern, A);
-}
-
-// The three launches; counters, lists' counts and barrier words are zero before them.
-template <int MODE>
-static cudaError_t chain_select(const ChainArgs& A, cudaStream_t st) {
-  const ChainUnit& last = A.unit[A.units - 1];
-  const uint32_t tiles = last.tile0 + (last.s.n - 1) / kSelTile + 1, samples = last.sample0 + last.s.sampled;
-  cudaError_t e = chain_launch(chain_sample_kernel<MODE>, samples, kSpThreads, sizeof(SelSmem), true, st, A);
-  if (e == cudaSuccess) e = chain_launch(chain_collect_kernel<MODE>, 2 * tiles, kChainThreads, 0, true, st, A);
-  if (e == cudaSuccess)
-    e = chain_launch(chain_emit_kernel, A.units * A.emitters, kSpThreads, sizeof(ChainSmem), false, st, A);
-  return e;
-}
+bool chain_place(ChainArgs& A, int resident);
+// The three launches (mode of the update: see pass0_body); counters, lists' counts and
+// barrier words are zero before them.
+cudaError_t chain_select(int mode, const ChainArgs& A, cudaStream_t st);
 
 }  // namespace hipress

@@ -257,8 +257,9 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
       C.payload = out;
       C.barrier = ws + kWsWords;
       C.status = ws + kWsStatus;
+      C.code = 1u;
       if (chain_place(C, chain_per_sm(dev) * stream_sms(st, sms)))
-        return (int)(mode == 0 ? chain_select<0>(C, st) : (mode == 1 ? chain_select<1>(C, st) : chain_select<2>(C, st)));
+        return (int)chain_select(mode, C, st);
     }
     if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
     const int grid = (int)(tiles < (uint64_t)cap ? tiles : (uint64_t)cap);

@@ -1,7 +1,8 @@
 """Python face of the fused sparse kernels (csrc/cuda/fused_sparse.cu): a DGC /
 GradDrop bucket is synchronised by ONE persistent cooperative launch that selects,
 stores (index, value) pairs into peer GPUs' inboxes, re-selects (at the owner for
-PS, at every hop for the ring) and scatters the result -- no NCCL call."""
+PS, at every hop for the ring) and scatters the result -- no NCCL call.  A job of one
+rank, which waits for nobody, runs its selections as chains of plain launches instead."""
 from __future__ import annotations
 
 import ctypes as C
@@ -92,7 +93,8 @@ class FusedSparseBucket:
     def last_phase_times(self):
         """Device-side profile of the last launch (rank 0 of an emulated launch): the
         time in ms, from the kernel's start, at which CTA 0 left each phase barrier,
-        and last its own end.  %globaltimer stamps written by the kernel."""
+        and last its own end.  %globaltimer stamps written by the persistent kernels (a
+        chain of launches, see above, writes none)."""
         WS_WORDS, STAMPS = 3 * 4096 + 16, 8      # kWsWords, kCtlStamps of the kernels
         nseg = len(self.sizes)
         ctl = (nseg * self.nranks + nseg) * WS_WORDS

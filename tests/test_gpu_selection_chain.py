@@ -60,3 +60,36 @@ def test_chain_where_the_list_does_not_hold_them(what):
     left = g.clone()
     left[idx] = 0.0
     assert torch.equal(st["residual"].cpu(), left)
+
+
+@pytest.mark.parametrize("topology", ["ps", "ring"])
+@pytest.mark.parametrize("name", ["dgc", "graddrop"])
+# one array; arrays of very different sizes; as many as a bucket holds, the smallest of one element
+@pytest.mark.parametrize("sizes", [[300003], [200003, 8192, 300, 1 << 18, 4096], [1, 7000] + [3000 + 37 * i for i in range(38)]])
+def test_buckets_of_one_rank(name, topology, sizes):
+    from hipress_b200.parallel.fused_sparse import FusedSparseBucket
+    from hipress_b200.parallel.simulate import chunk_elems, simulate_ps, simulate_ring
+    gen = torch.Generator().manual_seed(len(sizes))
+    c = Compressor(name, ratio=0.01)
+    b = FusedSparseBucket(c.spec, sizes, 1, 0, topology=topology).bind_local("cuda")
+    acc = "accum_v" if name == "dgc" else "residual"
+    cpu = [c.new_state(s, "cpu") for s in sizes]
+    srv = [{"residual": torch.zeros(chunk_elems(s, 1))} for s in sizes]
+    gpu = [{k: v.cuda() for k, v in st.items()} for st in cpu]
+    sums = [x["residual"].cuda() for x in srv]
+    for step in range(3):
+        grads = [torch.randn(s, generator=gen) * torch.randn(s, generator=gen) for s in sizes]
+        dev = [g.cuda() for g in grads]       # the result takes the gradient's place
+        b.launch_ptrs([g.data_ptr() for g in dev], [s[acc].data_ptr() for s in gpu],
+                      [s["momentum_u"].data_ptr() for s in gpu] if name == "dgc" else None,
+                      [g.data_ptr() for g in dev], [s.data_ptr() if topology == "ps" else None for s in sums])
+        torch.cuda.synchronize()
+        b.check_status()
+        for i in range(len(sizes)):
+            ref = simulate_ps(c, [grads[i]], [cpu[i]], [srv[i]]) if topology == "ps" else \
+                simulate_ring(c, [grads[i]], [cpu[i]])
+            assert torch.allclose(dev[i].cpu(), ref[0], rtol=1e-5, atol=1e-7), (step, i)
+            for k in cpu[i]:
+                assert torch.allclose(gpu[i][k].cpu(), cpu[i][k], rtol=1e-5, atol=1e-7), (step, i, k)
+            if topology == "ps":
+                assert torch.allclose(sums[i].cpu(), srv[i]["residual"], rtol=1e-5, atol=1e-7), (step, i)
