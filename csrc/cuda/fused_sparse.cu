@@ -723,7 +723,8 @@ int hp_fused_sparse_layout(float ratio, const uint64_t* ns, int nseg, int nranks
   return 0;
 }
 
-// One synchronisation of a bucket through the PS topology: one cooperative launch.
+// One synchronisation of a bucket through the PS topology: one cooperative launch, or with
+// one rank and ctas <= 0 two chains of three launches.
 // segs[i].r is the accumulator (DGC v / GradDrop residual), us[i] the DGC momentum
 // (or NULL), segs[i].sr the server accumulator of the owned chunk.  ws: scratch of
 // hp_fused_sparse_layout().ws_bytes per rank played by this call.  ctas <= 0: the
@@ -738,7 +739,8 @@ int hp_cuda_fused_sparse_ps(int alg, float ratio, float momentum, const HpSeg* s
   return launch_sparse(HP_TOPO_PS, bk, *comm, ws, ctas, (cudaStream_t)stream);
 }
 
-// One synchronisation of a bucket through the ring topology: one cooperative launch.
+// One synchronisation of a bucket through the ring topology: one cooperative launch, or with
+// one rank and ctas <= 0 a chain of three.
 // Same arguments as hp_cuda_fused_sparse_ps (segs[i].sr is not used).
 int hp_cuda_fused_sparse_ring(int alg, float ratio, float momentum, const HpSeg* segs,
                               void* const* us, int nseg, const HpComm* comm, void* ws, int ctas,
