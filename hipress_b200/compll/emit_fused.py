@@ -267,6 +267,14 @@ class FusedGen:
         body = []
         last_writer = {it.target: k for k, it in enumerate(ph.items) if it.kind == "map"}
 
+        def scalar(e) -> str:
+            # for use outside the loop over elements too, which the hooked forms belong to
+            hook, em._binary_hook = em._binary_hook, None
+            try:
+                return em.expr(e, set())
+            finally:
+                em._binary_hook = hook
+
         def index_hook(sym, idx, local):
             own = em._own
             if own is None or not (isinstance(idx, F.Name) and idx.id == own and idx.id in local):
@@ -281,7 +289,7 @@ class FusedGen:
         def frag_value(sym):
             # a packed input read at the own index: the group's fragment is loaded once
             need_frag[sym.name] = None
-            b = f"(uint32_t)({em.expr(sym.bits, set())})"
+            b = f"(uint32_t)({scalar(sym.bits)})"
             return f"((fr_{sym.name}[u] >> (e * {b})) & ((1u << {b}) - 1u))"
 
         def random_hook(site):
@@ -332,7 +340,7 @@ class FusedGen:
                                 em.syms[n.id].kind not in ("param_scalar", "reduced", "derived", "extracted")
                                 for n in names):
                 return None
-            text = em.expr(cond, set())
+            text = scalar(cond)
             if text not in flags:
                 if flags:
                     return None
@@ -372,7 +380,7 @@ class FusedGen:
                 em._return_to = None
                 mask = ""
                 if sub:
-                    mask = f" & ((1u << (uint32_t)({em.expr(tgt.bits, set())})) - 1u)"
+                    mask = f" & ((1u << (uint32_t)({scalar(tgt.bits)})) - 1u)"
                 body.append(f"""        {{  // {it.target} = map(..., {lam_sym.name})
           const {C_TYPES[pty.name]} l_{pname} = {pinit};
           {lret} res = 0;
@@ -384,7 +392,7 @@ class FusedGen:
                 fwd[it.target] = f"{var}[e]"
                 if last_writer[it.target] == k:
                     if sub:
-                        bits = f"(uint32_t)({em.expr(tgt.bits, set())})"
+                        bits = f"(uint32_t)({scalar(tgt.bits)})"
                         stores.append(f"""      {{
         const uint32_t bits = {bits};
         const uint32_t frag = {var}[0] | ({var}[1] << bits) | ({var}[2] << (2 * bits)) | ({var}[3] << (3 * bits));

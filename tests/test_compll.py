@@ -94,6 +94,22 @@ def test_generated_code_compiles_for_sm100a(tmp_path):
         assert files[-1].name.startswith("lib") and files[-1].exists()
 
 
+# scalars divided outside the loop over elements: a condition compiled for both of its values,
+# a ternary inside one, the width of the codes
+@pytest.mark.skipif(not HAVE_NVCC, reason="nvcc not available")
+@pytest.mark.parametrize("old,new", [("gap > 0.0", "hi / gap > 0.5"),
+                                     ("gap > 0.0", "(gap > 0.0 ? hi / gap : lo) > 0.0"),
+                                     ("uint<bitwidth>* Q", "uint<8 / gap>* Q")])
+def test_divisions_of_scalars_compile(tmp_path, old, new):
+    source = (PSE / "TernGradEncode.pse").read_text()
+    assert old in source
+    (tmp_path / "x.pse").write_text(source.replace(old, new))
+    files = generate_files(tmp_path / "x.pse", tmp_path, build=True, target="cuda")
+    assert files[-1].exists()
+    body = (tmp_path / "TernGradEncode" / "TernGradEncode_body.cuh").read_text()
+    assert "compll_div" in body      # the elements' own quotient
+
+
 def test_topk_and_scatter_lower_to_library_stages():
     em = generate((PSE / "DgcEncode.pse").read_text())
     assert [s[0] for s in em.stages] == ["map", "map", "topk"] and em.uses_library
