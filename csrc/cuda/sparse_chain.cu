@@ -149,6 +149,34 @@ union ChainSmem {
   EmitSmem emit;
 };
 
+// Where the pairs of an array go; thread 0 fills `s` and `dst` in.
+__device__ __forceinline__ void chain_aim(const ChainArgs& A, const ChainUnit& to, SelUnit& s, EmitDst& dst) {
+  if (threadIdx.x == 0) {
+    s = to.s;
+    dst.n = A.payload ? 1 : 0;
+    dst.out[0] = A.payload;
+    dst.add = to.add;
+    dst.set = to.set;
+    dst.scale = A.scale;
+  }
+  __syncthreads();
+}
+
+// The passes over a whole array: -1 clears the histograms, 0 to 2 count a digit each, 3
+// sends.  Between two of them all of its G CTAs are done with the one before.
+__device__ __forceinline__ void chain_pass(int pass, int alg, const SelUnit& s, const EmitDst& dst, ChainSmem& sm,
+                                           FindSmem& fs, uint32_t c, uint32_t G) {
+  if (pass < 0) {
+    for (uint32_t i = c * kSpThreads + threadIdx.x; i < 3u * kBins; i += G * kSpThreads) s.ws[i] = 0;
+  } else if (pass == 0) {
+    pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
+  } else if (pass < 3) {
+    pass_body(pass, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
+  } else {
+    emit_body(alg, s.a, s.u, s.n, s.k, s.kmax, dst, s.ws, fs, sm.emit, c, G);
+  }
+}
+
 __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_constant__ ChainArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ChainSmem& sm = *reinterpret_cast<ChainSmem*>(smem_raw);
@@ -158,19 +186,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_
   __shared__ FindSmem fs;
   const uint32_t y = blockIdx.x / A.emitters, x = blockIdx.x - y * A.emitters;
   const ChainUnit& u = A.unit[y];
-  auto aim = [&](const ChainUnit& to) {
-    if (threadIdx.x == 0) {
-      s = to.s;
-      dst.n = A.payload ? 1 : 0;
-      dst.out[0] = A.payload;
-      dst.add = to.add;
-      dst.set = to.set;
-      dst.scale = A.scale;
-    }
-    __syncthreads();
-  };
   wait_init(wst);
-  aim(u);
+  chain_aim(A, u, s, dst);
   const ListState ls = chain_state(u);
   if (!selection_failed(s, ls)) {
     // the spans of a part: CTAs part, part + kChainLists, ...
@@ -191,20 +208,26 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_
       const ChainUnit& f = A.unit[q];
       if (!selection_failed(f.s, chain_state(f))) continue;
       __syncthreads();
-      aim(f);
-      const uint32_t c = blockIdx.x, G = gridDim.x;
-      if (pass < 0) {
-        for (uint32_t i = c * kSpThreads + threadIdx.x; i < 3u * kBins; i += G * kSpThreads) s.ws[i] = 0;
-      } else if (pass == 0) {
-        pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
-      } else if (pass < 3) {
-        pass_body(pass, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
-      } else {
-        emit_body(A.alg, s.a, s.u, s.n, s.k, s.kmax, dst, s.ws, fs, sm.emit, c, G);
-      }
+      chain_aim(A, f, s, dst);
+      chain_pass(pass, A.alg, s, dst, sm, fs, blockIdx.x, gridDim.x);
       __syncthreads();
     }
     if (pass < 3) grid_barrier(A.barrier, gen, gridDim.x, kGridBarrierNs, A.status, A.code, wst);
+  }
+}
+
+// One of those passes for all arrays, as a launch of its own.
+__global__ void __launch_bounds__(kSpThreads, 2) chain_pass_kernel(const __grid_constant__ ChainArgs A, int pass) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ChainSmem& sm = *reinterpret_cast<ChainSmem*>(smem_raw);
+  __shared__ SelUnit s;
+  __shared__ EmitDst dst;
+  __shared__ FindSmem fs;
+#pragma unroll 1
+  for (int q = 0; q < A.units; ++q) {
+    chain_aim(A, A.unit[q], s, dst);
+    chain_pass(pass, A.alg, s, dst, sm, fs, blockIdx.x, gridDim.x);
+    __syncthreads();
   }
 }
 
@@ -215,7 +238,8 @@ int chain_per_sm(int dev) {
   if (known[dev]) return known[dev] - 1;
   int per = 0;
   const void* big[] = {(const void*)chain_sample_kernel<0>, (const void*)chain_sample_kernel<1>,
-                       (const void*)chain_sample_kernel<2>, (const void*)chain_emit_kernel};
+                       (const void*)chain_sample_kernel<2>, (const void*)chain_emit_kernel,
+                       (const void*)chain_pass_kernel};
   bool ok = true;
   for (const void* k : big)
     ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChainSmem)) == cudaSuccess;
@@ -273,7 +297,13 @@ static cudaError_t chain_select_mode(const ChainArgs& A, cudaStream_t st) {
   if (e == cudaSuccess) e = chain_launch(chain_collect_kernel<MODE>, 2 * tiles, kChainThreads, 0, true, st, A);
   if (e == cudaSuccess)
     e = chain_launch(chain_emit_kernel, A.units * A.emitters, kSpThreads, sizeof(ChainSmem), false, st, A);
-  return e;
+  if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+  // Less of the GPU is ours than the queries said, and the arrays are updated by now: what
+  // the emitting CTAs do together, in launches that need no co-residency.
+  cudaGetLastError();
+  const uint32_t grid = tiles < 148u * 2u ? tiles : 148u * 2u;
+  for (int pass = -1; pass <= 3; ++pass) chain_pass_kernel<<<grid, kSpThreads, sizeof(ChainSmem), st>>>(A, pass);
+  return cudaGetLastError();
 }
 
 cudaError_t chain_select(int mode, const ChainArgs& A, cudaStream_t st) {

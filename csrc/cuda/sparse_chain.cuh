@@ -39,7 +39,8 @@ int chain_per_sm(int dev);
 // run at once.  False when the lists cannot be shared out.
 bool chain_place(ChainArgs& A, int resident);
 // The three launches (mode of the update: see pass0_body); counters, lists' counts and
-// barrier words are zero before them.
+// barrier words are zero before them.  Where the emitting launch is refused (less of the GPU
+// is ours than the queries said) five plain ones make up for it.
 cudaError_t chain_select(int mode, const ChainArgs& A, cudaStream_t st);
 
 }  // namespace hipress
