@@ -588,9 +588,9 @@ static uint64_t sp_hist_words(int nseg, int nranks) {
 }
 
 // words behind the control words that a job of one rank uses: the counts of its lists'
-// parts, push and server, and the server selection's barrier
+// parts, push and server, the server selection's barrier, and whether one expired
 static uint64_t sp_chain_words(int nseg, int nranks) {
-  return nranks == 1 ? 2ull * nseg * 32 * kChainLists + kBarrierWords : 0;
+  return nranks == 1 ? 2ull * nseg * 32 * kChainLists + kBarrierWords + 1 : 0;
 }
 static uint64_t sp_cleared_words(int nseg, int nranks) {
   return sp_hist_words(nseg, nranks) + kCtlWords + sp_chain_words(nseg, nranks);
@@ -615,7 +615,9 @@ static bool launch_chain(int topo, const SpBucket& bk, const HpComm& cm, uint8_t
     A.alg = bk.alg;
     A.momentum = bk.momentum;
     A.scale = bk.inv_n;
-    A.barrier = serve ? ctl + kCtlWords + 2 * bk.nseg * 32 * kChainLists : ctl + kCtlBarrier;
+    uint32_t* behind = ctl + kCtlWords + 2 * bk.nseg * 32 * kChainLists;
+    A.barrier = serve ? behind : ctl + kCtlBarrier;
+    A.gave_up = behind + kBarrierWords;
     A.status = reinterpret_cast<uint32_t*>(cm.status);
     A.code = HP_STATUS_TIMEOUT | (8u << 16);
     for (int i = 0; i < bk.nseg; ++i) {

@@ -149,14 +149,15 @@ union ChainSmem {
   EmitSmem emit;
 };
 
-// Where the pairs of an array go; thread 0 fills `s` and `dst` in.
-__device__ __forceinline__ void chain_aim(const ChainArgs& A, const ChainUnit& to, SelUnit& s, EmitDst& dst) {
+// Where the pairs of an array go; thread 0 fills `s` and `dst` in.  A CTA that has given up
+// on a barrier may pick other elements than the largest, and leaves the result alone.
+__device__ __forceinline__ void chain_aim(const ChainArgs& A, const ChainUnit& to, bool gave_up, SelUnit& s, EmitDst& dst) {
   if (threadIdx.x == 0) {
     s = to.s;
     dst.n = A.payload ? 1 : 0;
     dst.out[0] = A.payload;
     dst.add = to.add;
-    dst.set = to.set;
+    dst.set = gave_up ? nullptr : to.set;
     dst.scale = A.scale;
   }
   __syncthreads();
@@ -186,9 +187,11 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_
   __shared__ FindSmem fs;
   const uint32_t y = blockIdx.x / A.emitters, x = blockIdx.x - y * A.emitters;
   const ChainUnit& u = A.unit[y];
-  wait_init(wst);
-  chain_aim(A, u, s, dst);
+  const uint32_t before = A.gave_up ? __ldcg(A.gave_up) : 0u;   // the chain before this one
   const ListState ls = chain_state(u);
+  wait_init(wst);
+  if (threadIdx.x == 0) wst.poisoned = before != 0;
+  chain_aim(A, u, before != 0, s, dst);
   if (!selection_failed(s, ls)) {
     // the spans of a part: CTAs part, part + kChainLists, ...
     const uint32_t part = x % kChainLists, sub = x / kChainLists, subs = A.emitters / kChainLists;
@@ -208,12 +211,13 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_
       const ChainUnit& f = A.unit[q];
       if (!selection_failed(f.s, chain_state(f))) continue;
       __syncthreads();
-      chain_aim(A, f, s, dst);
+      chain_aim(A, f, wst.poisoned, s, dst);
       chain_pass(pass, A.alg, s, dst, sm, fs, blockIdx.x, gridDim.x);
       __syncthreads();
     }
     if (pass < 3) grid_barrier(A.barrier, gen, gridDim.x, kGridBarrierNs, A.status, A.code, wst);
   }
+  if (A.gave_up && threadIdx.x == 0 && wst.poisoned) *A.gave_up = 1u;
 }
 
 // One of those passes for all arrays, as a launch of its own.
@@ -225,7 +229,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_pass_kernel(const __grid_
   __shared__ FindSmem fs;
 #pragma unroll 1
   for (int q = 0; q < A.units; ++q) {
-    chain_aim(A, A.unit[q], s, dst);
+    chain_aim(A, A.unit[q], A.gave_up && __ldcg(A.gave_up), s, dst);
     chain_pass(pass, A.alg, s, dst, sm, fs, blockIdx.x, gridDim.x);
     __syncthreads();
   }

@@ -30,6 +30,7 @@ struct ChainArgs {
   uint8_t* payload;      // of the only unit, or null
   uint32_t* barrier;     // kBarrierWords of zeros
   uint32_t *status, code;   // what a barrier that expires records, and where
+  uint32_t* gave_up;     // zero until a CTA's barrier expires, for the chains of one bucket; or null
   uint32_t emitters;     // CTAs that share the list of a unit: a multiple of kChainLists
 };
 

@@ -1,6 +1,7 @@
-"""The top-k chain of launches where its cooperative launch is refused.  The library is
-linked with a copy of the chain that refuses it on the host, and runs in a child process
-because the choice of library is made once per process."""
+"""The top-k chain of launches where its cooperative launch is refused, and where a barrier
+of that launch expires.  The library is linked with a copy of the chain whose host refuses
+the launch, or whose barrier waits, 20 us, for one CTA more than there are.  It runs in a
+child process because the choice of library is made once per process."""
 import os
 import subprocess
 import sys
@@ -99,3 +100,36 @@ def _child(d, source, code):
 def test_a_refused_launch_is_made_up_for(tmp_path):
     """The arrays are updated when the last launch is refused: the call ends as it would have."""
     _child(tmp_path, "chain_refused.cu", REFUSED)
+
+
+EXPIRED = """
+from hipress_b200.parallel.fused import HipressTimeoutError
+sizes = [200003, 8192]
+c = Compressor("graddrop", ratio=0.01)
+for topology in ("ps", "ring"):
+    b = FusedSparseBucket(c.spec, sizes, 1, 0, topology=topology).bind_local("cuda")
+    # equal values: the list overflows and the CTAs meet at the barrier
+    grads = [torch.full((sizes[0],), 0.5), values(sizes[1])]
+    out = [g.cuda() for g in grads]
+    acc = [torch.zeros(s, device="cuda") for s in sizes]
+    sums = [torch.zeros(s, device="cuda") for s in sizes]
+    b.launch_ptrs([g.data_ptr() for g in out], [a.data_ptr() for a in acc], None, [g.data_ptr() for g in out],
+                  [s.data_ptr() for s in sums])
+    torch.cuda.synchronize()
+    assert not out[0].any(), (topology, int(out[0].count_nonzero()))
+    if topology == "ps":    # nor from the sum of a push that was not complete
+        assert not out[1].any(), int(out[1].count_nonzero())
+    else:                   # its list was complete
+        assert torch.equal(out[1].cpu(), simulate_ring(c, [grads[1]], [c.new_state(sizes[1], "cpu")])[0])
+    try:
+        b.check_status()
+    except HipressTimeoutError:
+        pass
+    else:
+        raise AssertionError("no status")
+print("OK")
+"""
+
+
+def test_a_result_is_left_alone_behind_a_barrier_that_expired(tmp_path):
+    _child(tmp_path, "chain_expired.cu", EXPIRED)
