@@ -5,11 +5,13 @@ namespace hipress {
 
 constexpr int kChainThreads = 256;
 constexpr uint32_t kChainTile = kSelTile / 2;   // two float4 of each array per thread
+constexpr uint32_t kNoBase = 0xFFFFFFFFu;       // no places of a list
 
 __device__ __forceinline__ void after_launches_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Half tile h of an array: update, and what reaches the bound into part `part` of its list.
+// Half tile h of an array: update, and what reaches the bound into its list, from part
+// `part` on.
 // HBM bound on large arrays; 256 threads and two vectors of each array per thread leave room
 // for five CTAs on an SM, whose starts and ends overlap (six: no change).
 template <int MODE>
@@ -83,19 +85,32 @@ __device__ __forceinline__ void chain_collect(const SelUnit& s, uint32_t* counts
   __syncthreads();
   const uint32_t n = count;
   if (n == 0) return;
-  if (threadIdx.x == 0) {
-    base = atomicAdd(counts + 32 * part, n);
-    if (base + n > room) s.ws[kWsOverflow] = 1u;
-  }
-  __syncthreads();
+  // What finds no room in its part goes to the next one, so that an array whose large values
+  // lie together (the rows of an embedding that a batch touched, a block of a matrix's
+  // columns) fills all of the list: it overflowed at a seventh.
+  uint32_t done = 0, of = part;
 #pragma unroll 1
-  for (uint32_t p = threadIdx.x; p < n; p += kChainThreads) {
-    const float v = val[p];
-    atomicAdd(s.ws + cand_digit(abs_key(v), low), 1u);
-    if (base + p < room) {
-      s.cv[part * room + base + p] = v;
-      list_indices(s)[part * room + base + p] = idx[p];
+  for (uint32_t t = 0; done < n; ++t) {
+    if (threadIdx.x == 0) {
+      const bool lost = t == kChainLists || (t > 0 && __ldcg(s.ws + kWsOverflow) != 0u);
+      if (lost) s.ws[kWsOverflow] = 1u;
+      base = lost ? kNoBase : atomicAdd(counts + 32 * of, n - done);
     }
+    __syncthreads();
+    const uint32_t at = base;
+    if (at == kNoBase) return;
+    const uint32_t end = at < room ? min(n, done + room - at) : done;
+#pragma unroll 1
+    for (uint32_t p = done + threadIdx.x; p < end; p += kChainThreads) {
+      const float v = val[p];
+      const uint32_t to = of * room + at + p - done;
+      atomicAdd(s.ws + cand_digit(abs_key(v), low), 1u);
+      s.cv[to] = v;
+      list_indices(s)[to] = idx[p];
+    }
+    done = end;
+    of = of + 1 == kChainLists ? 0 : of + 1;
+    __syncthreads();
   }
 }
 
@@ -139,7 +154,7 @@ __global__ void __launch_bounds__(kChainThreads, 5) chain_collect_kernel(const _
 __device__ __forceinline__ ListState chain_state(const ChainUnit& u) {
   ListState l = {0u, __ldcg(u.s.ws + kWsOverflow), __ldcg(u.s.ws + kWsLow)};
 #pragma unroll
-  for (uint32_t p = 0; p < kChainLists; ++p) l.count += __ldcg(u.counts + 32 * p);
+  for (uint32_t p = 0; p < kChainLists; ++p) l.count += min(__ldcg(u.counts + 32 * p), u.s.cap / kChainLists);
   return l;
 }
 

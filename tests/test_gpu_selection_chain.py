@@ -34,6 +34,41 @@ def test_chain_at_its_edges(name, n, ratio, off):
             assert torch.equal(st_g[key].cpu(), st_c[key]), key
 
 
+# large values that lie together: one row of 1024; a block of columns of a matrix whose rows
+# are as long as the parts' turns; one half tile; the first hundredth; an array of one half
+# tile, most of which is sent
+@pytest.mark.parametrize("what", ["row", "columns", "half tile", "hundredth", "small"])
+def test_concentrated_values_fit_the_list(what):
+    n, ratio = 1 << 20, 0.001
+    gen = torch.Generator().manual_seed(3)
+    if what == "hundredth":
+        n, ratio = 6553600, 0.0005
+    elif what == "small":
+        n, ratio = 2048, 0.9
+    c = Compressor("graddrop", ratio=ratio)
+    k = c.kmax(n)
+    g = torch.randn(n, generator=gen)
+    if what == "row":
+        g[:300 * 1024] = 0.0
+        g[301 * 1024:] = 0.0
+    elif what == "columns":
+        g *= 1e-3
+        g[:n // 14336 * 14336].view(-1, 14336)[:, :20] += 1.0
+    elif what == "half tile":
+        g *= 1e-3
+        g[6 * 2048:6 * 2048 + 1500] += 3.0
+    elif what == "hundredth":
+        g *= 1e-3
+        g[:2 * k] *= 1e3
+    st, ws = c.new_state(n, "cuda"), c.new_workspace("cuda", n)
+    idx, val = sparse_pairs(c.encode(g.cuda(), st, workspace=ws), k)
+    ic, vc = sparse_pairs(c.encode(g, c.new_state(n, "cpu")), k)
+    assert torch.equal(idx, ic) and torch.equal(val, vc)
+    # the word that says that the list did not hold them (kWsOverflow): no pass over the
+    # whole array behind the update
+    assert int(ws.view(torch.int32)[3 * 4096 + 5]) == 0
+
+
 @pytest.mark.parametrize("what", ["equal", "clustered", "zeros", "infinite"])
 def test_chain_where_the_list_does_not_hold_them(what):
     """Lists that overflow or come out short: the digits are counted over the whole array."""
