@@ -606,7 +606,8 @@ static bool launch_chain(int topo, const SpBucket& bk, const HpComm& cm, uint8_t
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || chain_per_sm(dev) == 0) return false;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int resident = chain_per_sm(dev) * stream_sms(st, sms);
+  sms = stream_sms(st, sms);
+  const int resident = chain_per_sm(dev) * sms;
   uint32_t* words = reinterpret_cast<uint32_t*>(ws);
   uint32_t* ctl = words + sp_hist_words(bk.nseg, 1);
   uint8_t* lists = ws + align_up(sp_cleared_words(bk.nseg, 1) * 4, 256);
@@ -641,7 +642,7 @@ static bool launch_chain(int topo, const SpBucket& bk, const HpComm& cm, uint8_t
       u.add = topo == HP_TOPO_PS && !serve ? sg.sr : nullptr;
       u.set = topo == HP_TOPO_PS && !serve ? nullptr : sg.out;
     }
-    return chain_place(A, resident);
+    return chain_place(A, chain_per_sm(dev), sms);
   };
   ChainArgs push = {}, sum = {};
   if (!arrays(push, false) || (topo == HP_TOPO_PS && !arrays(sum, true))) return false;

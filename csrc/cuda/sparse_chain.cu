@@ -178,18 +178,27 @@ __device__ __forceinline__ void chain_aim(const ChainArgs& A, const ChainUnit& t
   __syncthreads();
 }
 
-// The passes over a whole array: -1 clears the histograms, 0 to 2 count a digit each, 3
-// sends.  Between two of them all of its G CTAs are done with the one before.
-__device__ __forceinline__ void chain_pass(int pass, int alg, const SelUnit& s, const EmitDst& dst, ChainSmem& sm,
-                                           FindSmem& fs, uint32_t c, uint32_t G) {
-  if (pass < 0) {
-    for (uint32_t i = c * kSpThreads + threadIdx.x; i < 3u * kBins; i += G * kSpThreads) s.ws[i] = 0;
-  } else if (pass == 0) {
-    pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
-  } else if (pass < 3) {
-    pass_body(pass, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
-  } else {
-    emit_body(alg, s.a, s.u, s.n, s.k, s.kmax, dst, s.ws, fs, sm.emit, c, G);
+// One of the passes over whole arrays, of the n arrays listed in `which` (or the first n):
+// -1 clears the histograms, 0 to 2 count a digit each, 3 sends.  Between two of them all CTAs
+// are done with the one before.  The arrays share the CTAs: each has histograms of its own,
+// and its passes are short.
+__device__ __forceinline__ void chain_pass(const ChainArgs& A, int pass, const uint8_t* which, uint32_t n, bool gave_up,
+                                           SelUnit& s, EmitDst& dst, ChainSmem& sm, FindSmem& fs) {
+  const uint32_t G = max(gridDim.x / n, 1u);
+#pragma unroll 1
+  for (uint32_t v = blockIdx.x; v < n * G; v += gridDim.x) {
+    const uint32_t c = v % G;
+    chain_aim(A, A.unit[which ? which[v / G] : v / G], gave_up, s, dst);
+    if (pass < 0) {
+      for (uint32_t i = c * kSpThreads + threadIdx.x; i < 3u * kBins; i += G * kSpThreads) s.ws[i] = 0;
+    } else if (pass == 0) {
+      pass0_body<0>(nullptr, s.a, nullptr, s.n, 0.0f, s.ws, sm.hist, c, G);
+    } else if (pass < 3) {
+      pass_body(pass, s.a, s.n, s.k, s.ws, sm.hist, fs, c, G);
+    } else {
+      emit_body(A.alg, s.a, s.u, s.n, s.k, s.kmax, dst, s.ws, fs, sm.emit, c, G);
+    }
+    __syncthreads();   // s and dst
   }
 }
 
@@ -200,36 +209,39 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_
   __shared__ EmitDst dst;
   __shared__ WaitState wst;
   __shared__ FindSmem fs;
+  __shared__ uint8_t failed[kChainUnits];
+  __shared__ uint32_t nfailed;
   const uint32_t y = blockIdx.x / A.emitters, x = blockIdx.x - y * A.emitters;
-  const ChainUnit& u = A.unit[y];
   const uint32_t before = A.gave_up ? __ldcg(A.gave_up) : 0u;   // the chain before this one
-  const ListState ls = chain_state(u);
-  wait_init(wst);
-  if (threadIdx.x == 0) wst.poisoned = before != 0;
-  chain_aim(A, u, before != 0, s, dst);
-  if (!selection_failed(s, ls)) {
-    // the spans of a part: CTAs part, part + kChainLists, ...
-    const uint32_t part = x % kChainLists, sub = x / kChainLists, subs = A.emitters / kChainLists;
-    const uint32_t room = s.cap / kChainLists, n = min(__ldcg(u.counts + 32 * part), room);
-    const uint32_t per = (n + subs - 1) / subs, lo = min(sub * per, n), hi = min(lo + per, n);
-    emit_span(A.alg, s, ls, dst, sm.sel, part * room + lo, part * room + hi, A.emitters);
+  if (y < (uint32_t)A.units) {
+    const ChainUnit& u = A.unit[y];
+    const ListState ls = chain_state(u);
+    chain_aim(A, u, before != 0, s, dst);
+    if (!selection_failed(s, ls)) {
+      // the spans of a part: CTAs part, part + kChainLists, ...
+      const uint32_t part = x % kChainLists, sub = x / kChainLists, subs = A.emitters / kChainLists;
+      const uint32_t room = s.cap / kChainLists, n = min(__ldcg(u.counts + 32 * part), room);
+      const uint32_t per = (n + subs - 1) / subs, lo = min(sub * per, n), hi = min(lo + per, n);
+      emit_span(A.alg, s, ls, dst, sm.sel, part * room + lo, part * room + hi, A.emitters);
+    }
   }
   // whole-array passes for the units whose list is not complete; every CTA decides the same
-  int bad = 0;
-  for (int q = threadIdx.x; q < A.units; q += kSpThreads) bad |= selection_failed(A.unit[q].s, chain_state(A.unit[q]));
+  const bool bad = threadIdx.x < (uint32_t)A.units &&
+                   selection_failed(A.unit[threadIdx.x].s, chain_state(A.unit[threadIdx.x]));
   if (!__syncthreads_or(bad)) return;
+  if (threadIdx.x < (uint32_t)A.units) failed[threadIdx.x] = bad;
+  wait_init(wst);
+  if (threadIdx.x == 0) {
+    wst.poisoned = before != 0;
+    nfailed = 0;
+    for (int q = 0; q < A.units; ++q)
+      if (failed[q]) failed[nfailed++] = (uint8_t)q;
+  }
+  __syncthreads();
   uint32_t gen = 0;
 #pragma unroll 1
   for (int pass = -1; pass <= 3; ++pass) {
-#pragma unroll 1
-    for (int q = 0; q < A.units; ++q) {
-      const ChainUnit& f = A.unit[q];
-      if (!selection_failed(f.s, chain_state(f))) continue;
-      __syncthreads();
-      chain_aim(A, f, wst.poisoned, s, dst);
-      chain_pass(pass, A.alg, s, dst, sm, fs, blockIdx.x, gridDim.x);
-      __syncthreads();
-    }
+    chain_pass(A, pass, failed, nfailed, wst.poisoned, s, dst, sm, fs);
     if (pass < 3) grid_barrier(A.barrier, gen, gridDim.x, kGridBarrierNs, A.status, A.code, wst);
   }
   if (A.gave_up && threadIdx.x == 0 && wst.poisoned) *A.gave_up = 1u;
@@ -242,12 +254,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_pass_kernel(const __grid_
   __shared__ SelUnit s;
   __shared__ EmitDst dst;
   __shared__ FindSmem fs;
-#pragma unroll 1
-  for (int q = 0; q < A.units; ++q) {
-    chain_aim(A, A.unit[q], A.gave_up && __ldcg(A.gave_up), s, dst);
-    chain_pass(pass, A.alg, s, dst, sm, fs, blockIdx.x, gridDim.x);
-    __syncthreads();
-  }
+  chain_pass(A, pass, nullptr, (uint32_t)A.units, A.gave_up && __ldcg(A.gave_up), s, dst, sm, fs);
 }
 
 // ------------------------------------------------------------------ host side
@@ -271,7 +278,7 @@ int chain_per_sm(int dev) {
   return per;
 }
 
-bool chain_place(ChainArgs& A, int resident) {
+bool chain_place(ChainArgs& A, int per_sm, int sms) {
   uint64_t tiles = 0, samples = 0;
   uint32_t longest = 1;
   for (int i = 0; i < A.units; ++i) {
@@ -286,9 +293,15 @@ bool chain_place(ChainArgs& A, int resident) {
     const uint32_t spans = (s.kmax + s.kmax / 2) / (4 * kSpThreads * kChainLists) + 1;
     longest = longest > spans ? longest : spans;
   }
-  const uint32_t most = (uint32_t)(resident / A.units) / kChainLists;
+  const uint32_t most = (uint32_t)(per_sm * sms / A.units) / kChainLists;
   if (most < 1 || tiles > 0x3FFFFFFFull) return false;
   A.emitters = kChainLists * (longest < most ? longest : most);
+  // One CTA per SM for the passes over whole arrays, up to a tile each.  Of 6.6 M elements,
+  // 40 rows of 1024 not zero, GradDrop at 0.1 % (encode, us): the emitters alone 658, one per
+  // SM 88, two 78; but where no list comes out short two cost the 25 MB bucket 1.9 us, one
+  // nothing.
+  const uint64_t busy = (uint64_t)A.units * A.emitters, wide = tiles < (uint64_t)sms ? tiles : (uint64_t)sms;
+  A.ctas = (uint32_t)(busy > wide ? busy : wide);
   return true;
 }
 
@@ -315,7 +328,7 @@ static cudaError_t chain_select_mode(const ChainArgs& A, cudaStream_t st) {
   cudaError_t e = chain_launch(chain_sample_kernel<MODE>, samples, kSpThreads, sizeof(SelSmem), true, st, A);
   if (e == cudaSuccess) e = chain_launch(chain_collect_kernel<MODE>, 2 * tiles, kChainThreads, 0, true, st, A);
   if (e == cudaSuccess)
-    e = chain_launch(chain_emit_kernel, A.units * A.emitters, kSpThreads, sizeof(ChainSmem), false, st, A);
+    e = chain_launch(chain_emit_kernel, A.ctas, kSpThreads, sizeof(ChainSmem), false, st, A);
   if (e != cudaErrorCooperativeLaunchTooLarge) return e;
   // Less of the GPU is ours than the queries said, and the arrays are updated by now: what
   // the emitting CTAs do together, in launches that need no co-residency.

@@ -22,7 +22,7 @@ struct ChainUnit {
   float* add;           // where its pairs go, besides a payload (EmitDst)
   float* set;
 };
-constexpr int kChainUnits = HP_MAX_SEGS;
+constexpr int kChainUnits = HP_MAX_SEGS;   // at most kSpThreads: a thread looks at each
 struct ChainArgs {
   ChainUnit unit[kChainUnits];
   int units, alg;
@@ -32,13 +32,14 @@ struct ChainArgs {
   uint32_t *status, code;   // what a barrier that expires records, and where
   uint32_t* gave_up;     // zero until a CTA's barrier expires, for the chains of one bucket; or null
   uint32_t emitters;     // CTAs that share the list of a unit: a multiple of kChainLists
+  uint32_t ctas;         // of the emitting launch; those behind the emitters wait for a list that came out short
 };
 
 // CTAs of the emitting launch that an SM holds at once, 0 when the kernels cannot run
 int chain_per_sm(int dev);
-// Places the units' tiles and samples behind one another; `resident`: emitting CTAs that
-// run at once.  False when the lists cannot be shared out.
-bool chain_place(ChainArgs& A, int resident);
+// Places the units' tiles and samples behind one another; per_sm: what chain_per_sm says,
+// sms: those of the stream.  False when the lists cannot be shared out.
+bool chain_place(ChainArgs& A, int per_sm, int sms);
 // The three launches (mode of the update: see pass0_body); counters, lists' counts and
 // barrier words are zero before them.  Where the emitting launch is refused (less of the GPU
 // is ours than the queries said) five plain ones make up for it.

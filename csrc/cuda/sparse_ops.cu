@@ -258,7 +258,7 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
       C.barrier = ws + kWsWords;
       C.status = ws + kWsStatus;
       C.code = 1u;
-      if (chain_place(C, chain_per_sm(dev) * stream_sms(st, sms)))
+      if (chain_place(C, chain_per_sm(dev), stream_sms(st, sms)))
         return (int)chain_select(mode, C, st);
     }
     if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;

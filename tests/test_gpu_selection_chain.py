@@ -128,3 +128,45 @@ def test_buckets_of_one_rank(name, topology, sizes):
                 assert torch.allclose(gpu[i][k].cpu(), cpu[i][k], rtol=1e-5, atol=1e-7), (step, i, k)
             if topology == "ps":
                 assert torch.allclose(sums[i].cpu(), srv[i]["residual"], rtol=1e-5, atol=1e-7), (step, i)
+
+
+@pytest.mark.parametrize("topology", ["ps", "ring"])
+@pytest.mark.parametrize("name", ["dgc", "graddrop"])
+# which arrays' lists overflow: the largest; some, of different sizes; all
+@pytest.mark.parametrize("full", [[0], [1, 3, 6], list(range(8))])
+def test_buckets_where_some_arrays_take_the_whole_array_passes(name, topology, full):
+    from hipress_b200.parallel.fused_sparse import FusedSparseBucket
+    gen = torch.Generator().manual_seed(len(full))
+    sizes = [600007, 70001, 9000, 1 << 17, 20480, 33333, 16384, 50000]
+    c = Compressor(name, ratio=0.001)
+    b = FusedSparseBucket(c.spec, sizes, 1, 0, topology=topology).bind_local("cuda")
+    acc = "accum_v" if name == "dgc" else "residual"
+    st = [c.new_state(s, "cuda") for s in sizes]
+    sums = [torch.zeros(s, device="cuda") for s in sizes]
+    left = [torch.zeros(s) for s in sizes]
+    for step in range(2 if name == "graddrop" else 1):
+        grads = [torch.randn(s, generator=gen) * torch.randn(s, generator=gen) for s in sizes]
+        for i in full:      # two values: far more ties than a list holds, but for the first few
+            grads[i] = torch.where(torch.rand(sizes[i], generator=gen) < 0.5, -1.0, 1.0)
+            grads[i][:3] = 5.0
+        out = [g.cuda() for g in grads]       # the result takes the gradient's place
+        b.launch_ptrs([g.data_ptr() for g in out], [s[acc].data_ptr() for s in st],
+                      [s["momentum_u"].data_ptr() for s in st] if name == "dgc" else None,
+                      [g.data_ptr() for g in out], [s.data_ptr() for s in sums])
+        torch.cuda.synchronize()
+        b.check_status()
+        for i, n in enumerate(sizes):
+            # kWsOverflow of the push's unit
+            assert (int(b.ws[i * (3 * 4096 + 16) + 3 * 4096 + 5]) != 0) == (i in full), (step, i)
+            total, got = left[i] + grads[i], out[i].cpu()
+            sent = got.nonzero().flatten()
+            want = total.abs().topk(c.kmax(n)).values
+            assert torch.equal(got[sent].abs().sort(descending=True).values, want), (step, i)
+            assert torch.equal(got[sent], total[sent]), (step, i)
+            left[i] = total
+            left[i][sent] = 0.0
+            assert torch.equal(st[i][acc].cpu(), left[i]), (step, i)
+            if name == "dgc":                 # the momentum of what was sent starts anew
+                assert torch.equal(st[i]["momentum_u"].cpu(), left[i]), i
+            if topology == "ps":              # the owner sent all it was given
+                assert not sums[i].any(), (step, i)
