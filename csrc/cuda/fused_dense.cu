@@ -783,10 +783,13 @@ ps_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
 // 65 % used, DRAM 74 % of ncu's peak).  Through PS every tile is quantised twice, which was
 // bound by instruction issue (378 -> 173 us; issue slots 79 % used) until the server's
 // pass was made from the push's codes (tern_requantise).
-// RES: some tensor of the bucket keeps error-feedback state (TernGrad's buckets keep none,
-// but the entry point takes some).
-template <int ALG, int B, int TOPO, bool RES>
-__global__ void __launch_bounds__(kThreads, RES ? (TOPO == HP_TOPO_PS ? 3 : 4) : 6)
+// STATE: some tensor of the bucket keeps error-feedback state, 1 the sender's alone, 2 the
+// owner's too (TernGrad's buckets keep none, but the entry point takes some).  With the
+// owner's the server quantises a sum, which the push's codes do not give: the code that
+// makes them does not fit in the registers beside that sum, and its spills cost a bucket of
+// 60 M elements with both states a seventh (2 bits: 258 us with it, 226 without).
+template <int ALG, int B, int TOPO, int STATE>
+__global__ void __launch_bounds__(kThreads, STATE ? (TOPO == HP_TOPO_PS ? 3 : 4) : 6)
 local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   __shared__ TileSmem s;
   int seg = 0;
@@ -797,8 +800,8 @@ local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
   const uint32_t left = sg.n - t * kTile;
   const int m = (int)(left < (uint32_t)kTile ? left : (uint32_t)kTile);
   const float* gp = sg.g + off;
-  float* rp = RES && sg.r ? sg.r + off : nullptr;
-  float* sp = RES && TOPO == HP_TOPO_PS && sg.sr ? sg.sr + off : nullptr;
+  float* rp = STATE >= 1 && sg.r ? sg.r + off : nullptr;
+  float* sp = STATE == 2 && sg.sr ? sg.sr + off : nullptr;
   float* op = sg.out + off;
   const bool full = m == kTile && ((reinterpret_cast<uintptr_t>(gp) | reinterpret_cast<uintptr_t>(rp) |
                                     reinterpret_cast<uintptr_t>(sp) | reinterpret_cast<uintptr_t>(op)) & 15) == 0;
@@ -831,7 +834,7 @@ local_dense_kernel(const BucketDev bk, const HpComm cm, const FusedParams fp) {
       else store_tile(state, m, x);
     }
     if (TOPO == HP_TOPO_RING || pass == 1) break;
-    if (ALG == kTernGrad && !sp && m == kTile &&
+    if (ALG == kTernGrad && STATE < 2 && m == kTile &&
         tern_requantise<B>(frag, meta, fp.P, sg.id, off, fp.P.salt + 1u, s))
       break;
 #pragma unroll
@@ -903,12 +906,15 @@ template <int ALG, int B>
 static int launch_fused(int topo, const BucketDev& bk, const HpComm& cm, const FusedParams& fp,
                         int ctas, cudaStream_t st) {
   if (cm.nranks == 1) {
-    bool res = false;
-    for (int i = 0; i < bk.nseg; ++i) res = res || bk.seg[i].r || bk.seg[i].sr;
-    auto kern = topo == HP_TOPO_RING ? (res ? local_dense_kernel<ALG, B, HP_TOPO_RING, true>
-                                            : local_dense_kernel<ALG, B, HP_TOPO_RING, false>)
-                                     : (res ? local_dense_kernel<ALG, B, HP_TOPO_PS, true>
-                                            : local_dense_kernel<ALG, B, HP_TOPO_PS, false>);
+    bool r = false, sr = false;
+    for (int i = 0; i < bk.nseg; ++i) {
+      r = r || bk.seg[i].r;
+      sr = sr || bk.seg[i].sr;
+    }
+    auto kern = local_dense_kernel<ALG, B, HP_TOPO_RING, 0>;
+    if (topo == HP_TOPO_RING) kern = r ? local_dense_kernel<ALG, B, HP_TOPO_RING, 1> : kern;
+    else kern = sr ? local_dense_kernel<ALG, B, HP_TOPO_PS, 2>
+                   : (r ? local_dense_kernel<ALG, B, HP_TOPO_PS, 1> : local_dense_kernel<ALG, B, HP_TOPO_PS, 0>);
     kern<<<bk.tiles_total, kThreads, 0, st>>>(bk, cm, fp);
     return (int)cudaGetLastError();
   }

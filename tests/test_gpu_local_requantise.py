@@ -49,3 +49,32 @@ def test_server_codes_from_push_codes(bits, what):
         got = out.cpu()
         same = (got == ref) | (got.isnan() & ref.isnan())
         assert bool(same.all()), (step, int((~same).sum()), got[~same][:4], ref[~same][:4])
+
+
+@pytest.mark.parametrize("bits", [1, 2, 4, 8])
+# which of two tensors keep state: the sender's; the owner's; both; one tensor each; one both, one none
+@pytest.mark.parametrize("sender,owner", [((1, 1), (0, 0)), ((0, 0), (1, 1)), ((1, 1), (1, 1)), ((1, 0), (0, 1)),
+                                          ((0, 1), (0, 0)), ((0, 1), (0, 1))])
+def test_state_of_either_side(bits, sender, owner):
+    gen = torch.Generator().manual_seed(bits)
+    sizes = [6 * 4096 + 77, 3 * 4096]
+    plain, kept = Compressor("terngrad", bitwidth=bits), Compressor("terngrad", bitwidth=bits, error_feedback=True)
+    b = FusedDenseBucket(plain.spec, "ps", sizes, 1, 0).bind_local("cuda")
+    state = [[torch.randn(n, generator=gen) * 0.01 if on else None for n, on in zip(sizes, side)] for side in (sender, owner)]
+    dev = [[None if t is None else t.cuda() for t in side] for side in state]
+    for step in range(2):
+        grads = [torch.randn(n, generator=gen) for n in sizes]
+        outs = [torch.empty(n, device="cuda") for n in sizes]
+        b.launch([g.cuda() for g in grads], dev[0], outs, dev[1], step=step, tensor_ids=[4, 5])
+        torch.cuda.synchronize()
+        for i, n in enumerate(sizes):
+            # the push, then the owner's pass over what it decodes to, as the oracle does one encode
+            x = grads[i]
+            for side in range(2):
+                st = state[side][i]
+                pay = (plain if st is None else kept).encode(x, {} if st is None else {"residual": st}, step=step, salt=side,
+                                                             tensor_id=4 + i)
+                x = plain.decode(pay, torch.zeros(n))
+                if st is not None:
+                    assert torch.equal(dev[side][i].cpu(), st), (step, i, side)
+            assert torch.equal(outs[i].cpu(), x), (step, i)
