@@ -144,7 +144,9 @@ def main(argv=None):
                         fused.enable_trace(False)
                     if a.trace and comp.spec.sparse:
                         torch.cuda.synchronize()
-                        row["phase_end_ms_rank0"] = [round(x, 4) for x in fused.last_phase_times()]
+                        phases = fused.last_phase_times()
+                        if phases:      # one rank: a chain of launches, which has none
+                            row["phase_end_ms_rank0"] = [round(x, 4) for x in phases]
                     if int(status.abs().sum()) != 0:
                         row["status"] = [w & 0xFFFFFFFF for w in status.tolist()]
                         status.zero_()

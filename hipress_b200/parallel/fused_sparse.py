@@ -93,14 +93,17 @@ class FusedSparseBucket:
     def last_phase_times(self):
         """Device-side profile of the last launch (rank 0 of an emulated launch): the
         time in ms, from the kernel's start, at which CTA 0 left each phase barrier,
-        and last its own end.  %globaltimer stamps written by the persistent kernels (a
-        chain of launches, see above, writes none)."""
+        and last its own end.  %globaltimer stamps written by the persistent kernels; a
+        chain of launches (one rank, see above) writes none, and the list is empty."""
         WS_WORDS, STAMPS = 3 * 4096 + 16, 8      # kWsWords, kCtlStamps of the kernels
         nseg = len(self.sizes)
         ctl = (nseg * self.nranks + nseg) * WS_WORDS
         w = self.ws[ctl:ctl + 128].cpu().tolist()
         gen = w[1]
         st = [(x & 0xFFFFFFFF) for x in w[STAMPS:STAMPS + min(gen + 2, 64 - STAMPS)]]
+        if st[0] == 0:
+            self.last_marks = []
+            return []
         self.last_marks = [((x & 0xFFFFFFFF) - st[0]) % (1 << 32) * 1e-6 for x in w[64:72]]
         return [((x - st[0]) & 0xFFFFFFFF) * 1e-6 for x in st[1:]]
 
