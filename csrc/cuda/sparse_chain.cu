@@ -211,18 +211,18 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_emit_kernel(const __grid_
   __shared__ FindSmem fs;
   __shared__ uint8_t failed[kChainUnits];
   __shared__ uint32_t nfailed;
-  const uint32_t y = blockIdx.x / A.emitters, x = blockIdx.x - y * A.emitters;
   const uint32_t before = A.gave_up ? __ldcg(A.gave_up) : 0u;   // the chain before this one
-  if (y < (uint32_t)A.units) {
-    const ChainUnit& u = A.unit[y];
+  if (blockIdx.x < A.emitting) {
+    const ChainEmitters em = A.emitters[blockIdx.x / kChainLists];
+    const ChainUnit& u = A.unit[em.unit];
     const ListState ls = chain_state(u);
     chain_aim(A, u, before != 0, s, dst);
     if (!selection_failed(s, ls)) {
-      // the spans of a part: CTAs part, part + kChainLists, ...
-      const uint32_t part = x % kChainLists, sub = x / kChainLists, subs = A.emitters / kChainLists;
+      // a part each; of several groups each takes a span of all parts
+      const uint32_t part = blockIdx.x % kChainLists, sub = em.group, subs = em.groups;
       const uint32_t room = s.cap / kChainLists, n = min(__ldcg(u.counts + 32 * part), room);
       const uint32_t per = (n + subs - 1) / subs, lo = min(sub * per, n), hi = min(lo + per, n);
-      emit_span(A.alg, s, ls, dst, sm.sel, part * room + lo, part * room + hi, A.emitters);
+      emit_span(A.alg, s, ls, dst, sm.sel, part * room + lo, part * room + hi, kChainLists * subs);
     }
   }
   // whole-array passes for the units whose list is not complete; every CTA decides the same
@@ -278,9 +278,11 @@ int chain_per_sm(int dev) {
   return per;
 }
 
+// groups of kChainLists CTAs that emit a list in one round, four candidates a thread
+static uint64_t groups_for(uint64_t kmax) { return (kmax + kmax / 2) / (4 * kSpThreads * kChainLists) + 1; }
+
 bool chain_place(ChainArgs& A, int per_sm, int sms) {
-  uint64_t tiles = 0, samples = 0;
-  uint32_t longest = 1;
+  uint64_t tiles = 0, samples = 0, wanted = 0;
   for (int i = 0; i < A.units; ++i) {
     SelUnit& s = A.unit[i].s;
     if (s.n == 0) return false;
@@ -290,17 +292,27 @@ bool chain_place(ChainArgs& A, int per_sm, int sms) {
     A.unit[i].sample0 = (uint32_t)samples;
     tiles += t;
     samples += s.sampled;
-    const uint32_t spans = (s.kmax + s.kmax / 2) / (4 * kSpThreads * kChainLists) + 1;
-    longest = longest > spans ? longest : spans;
+    wanted += groups_for(s.kmax) - 1;
   }
-  const uint32_t most = (uint32_t)(per_sm * sms / A.units) / kChainLists;
-  if (most < 1 || tiles > 0x3FFFFFFFull) return false;
-  A.emitters = kChainLists * (longest < most ? longest : most);
+  const uint32_t fit = (uint32_t)(per_sm * sms) / kChainLists, most = fit < kChainGroups ? fit : kChainGroups;
+  if (most < (uint32_t)A.units || tiles > 0x3FFFFFFFull) return false;
+  // A group for each list, and of those that are left as many more as its length asks for,
+  // or where they are too few its share of them.  In equal shares the longest list kept few
+  // CTAs busy: 20 M elements and 30 arrays of 500, DGC, ring, us, equal / by length
+  // (persistent kernels): 0.1 % 129 / 120 (138), 1 % 230 / 137 (256), 10 % 1218 / 288 (1033).
+  const uint64_t spare = most - (uint32_t)A.units;
+  uint32_t group = 0;
+  for (int i = 0; i < A.units; ++i) {
+    const uint64_t more = groups_for(A.unit[i].s.kmax) - 1;
+    const uint32_t n = 1 + (uint32_t)(wanted <= spare ? more : more * spare / wanted);
+    for (uint32_t q = 0; q < n; ++q) A.emitters[group++] = {(uint8_t)i, (uint8_t)q, (uint8_t)n};
+  }
+  A.emitting = kChainLists * group;
   // One CTA per SM for the passes over whole arrays, up to a tile each.  Of 6.6 M elements,
   // 40 rows of 1024 not zero, GradDrop at 0.1 % (encode, us): the emitters alone 658, one per
   // SM 88, two 78; but where no list comes out short two cost the 25 MB bucket 1.9 us, one
   // nothing.
-  const uint64_t busy = (uint64_t)A.units * A.emitters, wide = tiles < (uint64_t)sms ? tiles : (uint64_t)sms;
+  const uint64_t busy = A.emitting, wide = tiles < (uint64_t)sms ? tiles : (uint64_t)sms;
   A.ctas = (uint32_t)(busy > wide ? busy : wide);
   return true;
 }
