@@ -5,6 +5,7 @@ namespace hipress {
 
 constexpr int kChainThreads = 256;
 constexpr uint32_t kChainTile = kSelTile / 2;   // two float4 of each array per thread
+constexpr uint32_t kStretches = 16;
 constexpr uint32_t kNoBase = 0xFFFFFFFFu;       // no places of a list
 
 __device__ __forceinline__ void after_launches_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -140,9 +141,14 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_sample_kernel(const __gri
 
 template <int MODE>
 __global__ void __launch_bounds__(kChainThreads, 5) chain_collect_kernel(const __grid_constant__ ChainArgs A) {
-  const uint32_t t = blockIdx.x / 2, y = chain_unit(A, &ChainUnit::tile0, t);
+  uint32_t b = blockIdx.x;
+  if (MODE == 0 && A.stretch != 0u) {
+    b = b % kStretches * A.stretch + b / kStretches;
+    if (b >= 2 * A.tiles) return;
+  }
+  const uint32_t t = b / 2, y = chain_unit(A, &ChainUnit::tile0, t);
   const ChainUnit& u = A.unit[y];
-  const uint32_t h = blockIdx.x - 2 * u.tile0, part = blockIdx.x % kChainLists;
+  const uint32_t h = b - 2 * u.tile0, part = b % kChainLists;
   if (MODE != 0 && (t - u.tile0) % u.s.stride == 0) {
     after_launches_before();   // the sample's update
     chain_collect<0>(u.s, u.counts, 0.0f, h, part);
@@ -308,6 +314,13 @@ bool chain_place(ChainArgs& A, int per_sm, int sms) {
     for (uint32_t q = 0; q < n; ++q) A.emitters[group++] = {(uint8_t)i, (uint8_t)q, (uint8_t)n};
   }
   A.emitting = kChainLists * group;
+  // The owner's sum holds little but what was pushed, so its candidates' digits are a few
+  // leading bits, and an array's CTAs wait for one another at a few words.  Several arrays
+  // are taken at a time, by their half tiles in sixteen stretches side by side: two arrays
+  // of 10 M elements, PS, DGC / GradDrop, us, one stretch / sixteen (persistent kernels):
+  // 1 % 222 / 197 (240), 159 / 149 (193); 3 % 355 / 290 (334), 362 / 303 (313).
+  A.tiles = (uint32_t)tiles;
+  A.stretch = A.units > 1 ? (uint32_t)((2 * tiles + kStretches - 1) / kStretches) : 0u;
   // One CTA per SM for the passes over whole arrays, up to a tile each.  Of 6.6 M elements,
   // 40 rows of 1024 not zero, GradDrop at 0.1 % (encode, us): the emitters alone 658, one per
   // SM 88, two 78; but where no list comes out short two cost the 25 MB bucket 1.9 us, one
@@ -338,7 +351,8 @@ static cudaError_t chain_select_mode(const ChainArgs& A, cudaStream_t st) {
   const ChainUnit& last = A.unit[A.units - 1];
   const uint32_t tiles = last.tile0 + (last.s.n - 1) / kSelTile + 1, samples = last.sample0 + last.s.sampled;
   cudaError_t e = chain_launch(chain_sample_kernel<MODE>, samples, kSpThreads, sizeof(SelSmem), true, st, A);
-  if (e == cudaSuccess) e = chain_launch(chain_collect_kernel<MODE>, 2 * tiles, kChainThreads, 0, true, st, A);
+  const uint32_t halves = MODE == 0 && A.stretch ? kStretches * A.stretch : 2 * tiles;
+  if (e == cudaSuccess) e = chain_launch(chain_collect_kernel<MODE>, halves, kChainThreads, 0, true, st, A);
   if (e == cudaSuccess)
     e = chain_launch(chain_emit_kernel, A.ctas, kSpThreads, sizeof(ChainSmem), false, st, A);
   if (e != cudaErrorCooperativeLaunchTooLarge) return e;

@@ -40,6 +40,8 @@ struct ChainArgs {
   uint32_t* gave_up;     // zero until a CTA's barrier expires, for the chains of one bucket; or null
   ChainEmitters emitters[kChainGroups];
   uint32_t emitting;     // CTAs of these groups
+  uint32_t tiles;
+  uint32_t stretch;      // half tiles that lie between those of two neighbouring CTAs, 0 with one array
   uint32_t ctas;         // of the emitting launch; those behind the emitters wait for a list that came out short
 };
 
