@@ -601,9 +601,18 @@ static uint64_t sp_cleared_words(int nseg, int nranks) {
 // barriers; us per step or bucket, persistent / chain (B200): ResNet-50, DGC, PS 199.6 /
 // 187.6; GradDrop ring 6.6 M elements 55.1 / 43.1, 20 M at 1 % 134 / 97; DGC ring 3 M 49.4 /
 // 34.2; DGC PS 64 K 51.9 / 39.5, 20 M 173 / 147; 24 arrays of 1 M in all, PS 60.7 / 48.7.
-// False when the arrays do not fit a chain (and always with a limit on the CTAs).
+// False when the arrays do not fit a chain (and always with a limit on the CTAs), and for the
+// DGC ring of more than 67 M elements with few candidates (see chain_is_slower; 0.1 %: 80 M
+// 377 / 383, 134 M 591 / 627; the others gain up to there: GradDrop 134 M 410 / 415, DGC PS
+// 134 M 790 / 768).
 static bool launch_chain(int topo, const SpBucket& bk, const HpComm& cm, uint8_t* ws, cudaStream_t st, int& rc) {
   int dev = 0, sms = 0;
+  uint64_t n = 0, k = 0;
+  for (int i = 0; i < bk.nseg; ++i) {
+    n += bk.seg[i].n;
+    k += bk.seg[i].kmax;
+  }
+  if (topo == HP_TOPO_RING && bk.alg == kDgc && n > (1ull << 26) && chain_is_slower(2, n, k)) return false;
   if (cudaGetDevice(&dev) != cudaSuccess || chain_per_sm(dev) == 0) return false;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   sms = stream_sms(st, sms);

@@ -1,10 +1,11 @@
 // Sparse (top-k) compression for DGC and GradDrop on sm_100a.
 //
-// With room for a candidate list (the usual call) an encode is three launches, of which
-// each begins while the one before it ends: sample, update + collect with a CTA per half
-// tile, emit (sparse_chain.cuh).  One persistent kernel with grid barriers did the same and
-// is kept for calls that limit the CTAs (max_ctas): equal shares left the faster SMs idle,
-// and the arrays stood still while the sample was worked out.  DGC encode and decode at
+// With room for a candidate list (the usual call) an encode is three launches: sample, update
+// + collect with a CTA per half tile, which begins while the sample ends, and emit
+// (sparse_chain.cuh).  One persistent kernel with grid barriers does the same for calls that
+// limit the CTAs (max_ctas), and for those that it is better at (chain_is_slower); in the
+// others equal shares leave the faster SMs idle, and the arrays stand still while the sample
+// is worked out.  DGC encode and decode at
 // 0.1 %, us, persistent / chain (B200): 64 K elements 28.3 / 26.2, 1 M 37.9 / 30.8, 3 M
 // 52.4 / 45.2, 10 M at 1 % 93.8 / 81.1, 20 M 123.3 / 119.6.
 // The emitting launch is cooperative, because where a list came out short its CTAs count
@@ -235,7 +236,7 @@ static int sparse_encode_impl(int alg, const float* g, float* a, float* u, uint6
       }
     }
     int cap = per * stream_sms(st, sms);   // the stream may own only some of the SMs
-    if (max_ctas <= 0 && chain_per_sm(dev) > 0) {
+    if (max_ctas <= 0 && !chain_is_slower(mode, n, k) && chain_per_sm(dev) > 0) {
       ChainArgs C = {};
       SelUnit& V = C.unit[0].s;
       V.g = g;

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from hipress_b200.ops import Compressor
+from hipress_b200.ops import Compressor, sparse_pairs
 from hipress_b200.parallel.fused_sparse import FusedSparseBucket
 
 pytestmark = pytest.mark.gpu
@@ -38,3 +38,29 @@ def test_chain_of_large_arrays_is_no_slower_than_the_persistent_kernels(name):
         for i in range(2):
             best[i] = min(best[i], _us(runs[i], 10))
     assert best[0] < 1.05 * best[1], best
+
+
+# around one tile; around 42 M elements, where the share of the elements that are sent decides
+@pytest.mark.parametrize("name,n,ratio,chain,chain_without_update", [
+    ("dgc", 1, 0.5, 0, 0), ("dgc", 4096, 0.01, 0, 0), ("dgc", 4097, 0.01, 1, 1), ("graddrop", 4096, 0.5, 0, 0),
+    ("graddrop", 4097, 0.001, 1, 1), ("dgc", 10240 * 4096, 0.0002, 1, 1), ("dgc", 10240 * 4096 + 1, 0.0002, 0, 0),
+    ("dgc", 10240 * 4096 + 1, 0.001, 0, 1), ("dgc", 10240 * 4096 + 1, 0.003, 1, 1),
+    ("graddrop", 10240 * 4096 + 1, 0.001, 0, 1), ("graddrop", 10240 * 4096 + 1, 0.002, 1, 1)])
+def test_routes_of_an_encode(name, n, ratio, chain, chain_without_update):
+    """Sizes at which the persistent kernel is the faster one are its own again.  The counts
+    of a chain's list parts are words of the workspace that the persistent kernel leaves zero."""
+    c = Compressor(name, ratio=ratio)
+    ws, k = c.new_workspace("cuda", n), c.kmax(n)
+    for update in (True, False):
+        g = torch.randn(n, device="cuda")
+        st = c.new_state(n, "cuda")
+        if not update:
+            st["accum_v" if name == "dgc" else "residual"].copy_(g)
+        pay = c.encode(g, st, workspace=ws, update=update)
+        words = ws.view(torch.int32)
+        head = 3 * 4096 + 16 + 160            # kWsWords, then kBarrierWords
+        assert bool(words[head:head + 32 * 7].any()) == bool(chain if update else chain_without_update)
+        idx, val = sparse_pairs(pay, k)
+        want = g.abs().topk(k).values
+        assert torch.equal(val.abs().sort(descending=True).values, want.cpu())
+        assert torch.equal(g.cpu()[idx], val)
