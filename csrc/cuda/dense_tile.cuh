@@ -351,7 +351,7 @@ __device__ __forceinline__ void tern_encode_full(float (&x)[kIter][4], const Den
 // are the values of levels 0 and qmax, and the position of level L is 65536*L plus a
 // rounding error `off` that is the same for the whole tile: the new code is L unless the
 // draw u16 is within `off` of its end of the range.  A thread whose sixteen draws stay clear
-// of both ends keeps its codes; the others (1 in 2000 when off is -1) take the element-wise
+// of both ends keeps its codes; the others (1 in 4096 when off is -1) take the element-wise
 // way.  Instead of a decode, a minimum and maximum and sixteen roundings that is a pair of
 // packed minima per draw, and no draw at all where every level is exact.  One rank, PS,
 // 60 M elements, us per bucket: 1 bit 100.5 -> 74.8, 2 bits 103.6 -> 77.9, 8 bits 98.5 -> 90.9

@@ -15,7 +15,8 @@
 //   pull   : every rank waits for each owner's flag and scatters value / N into the
 //            result, which the update pass cleared.
 //
-// A job of one rank takes neither: its bucket is a chain of launches (launch_chain).
+// A job of one rank takes neither: its bucket is a chain of launches, but for a few that are
+// better served by the kernels here (launch_chain).
 //
 // All units of a bucket are batched in every phase, which is the "bulk
 // synchronisation" of many small tensors: the update pass splits the bucket's tiles, not
@@ -736,7 +737,7 @@ int hp_fused_sparse_layout(float ratio, const uint64_t* ns, int nseg, int nranks
 }
 
 // One synchronisation of a bucket through the PS topology: one cooperative launch, or with
-// one rank and ctas <= 0 two chains of three launches.
+// one rank and ctas <= 0 usually two chains of three launches (launch_chain).
 // segs[i].r is the accumulator (DGC v / GradDrop residual), us[i] the DGC momentum
 // (or NULL), segs[i].sr the server accumulator of the owned chunk.  ws: scratch of
 // hp_fused_sparse_layout().ws_bytes per rank played by this call.  ctas <= 0: the
@@ -752,7 +753,7 @@ int hp_cuda_fused_sparse_ps(int alg, float ratio, float momentum, const HpSeg* s
 }
 
 // One synchronisation of a bucket through the ring topology: one cooperative launch, or with
-// one rank and ctas <= 0 a chain of three.
+// one rank and ctas <= 0 usually a chain of three (launch_chain).
 // Same arguments as hp_cuda_fused_sparse_ps (segs[i].sr is not used).
 int hp_cuda_fused_sparse_ring(int alg, float ratio, float momentum, const HpSeg* segs,
                               void* const* us, int nseg, const HpComm* comm, void* ws, int ctas,

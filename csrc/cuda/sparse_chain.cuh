@@ -1,9 +1,9 @@
 // The selection of sparse_core.cuh as a chain of launches, for callers that wait for nobody
 // (the stand-alone encode, buckets of a job of one rank): sample, collect with a CTA per half tile, emit.  SMs do not run
 // at one speed, and equal shares of a persistent grid leave the fast ones idle for a tenth
-// of the pass; a new CTA goes to whichever SM is free.  A launch begins while the one
-// before it ends, and the collecting CTAs that start ahead of the bound update their tile
-// before they wait for it.
+// of the pass; a new CTA goes to whichever SM is free.  The collect begins while the sample
+// ends, and its CTAs that start ahead of the bound update their tile before they wait for
+// it; the emit is cooperative, and begins when the collect has ended.
 #pragma once
 #include "sparse_core.cuh"
 #include "sync.cuh"

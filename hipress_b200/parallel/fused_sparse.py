@@ -2,7 +2,7 @@
 GradDrop bucket is synchronised by ONE persistent cooperative launch that selects,
 stores (index, value) pairs into peer GPUs' inboxes, re-selects (at the owner for
 PS, at every hop for the ring) and scatters the result -- no NCCL call.  A job of one
-rank, which waits for nobody, runs its selections as chains of plain launches instead."""
+rank, which waits for nobody, runs its selections as chains of three launches instead."""
 from __future__ import annotations
 
 import ctypes as C
