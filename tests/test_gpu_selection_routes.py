@@ -64,3 +64,20 @@ def test_routes_of_an_encode(name, n, ratio, chain, chain_without_update):
         want = g.abs().topk(k).values
         assert torch.equal(val.abs().sort(descending=True).values, want.cpu())
         assert torch.equal(g.cpu()[idx], val)
+
+
+def test_chain_whose_list_overflows_is_no_slower_than_the_persistent_kernel():
+    """Large values that lie together in a hundredth of the array: the sample sees few of them."""
+    n, c = 6553600, Compressor("graddrop", ratio=0.001)
+    g = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) * 1e-3
+    g[:n // 100] *= 1e3
+    st, ws = c.new_state(n, "cuda"), c.new_workspace("cuda", n)
+    pay = torch.empty(c.payload_bytes(n), dtype=torch.uint8, device="cuda")
+    times = [[], []]
+    for _ in range(15):        # in turn
+        for i, ctas in enumerate((0, 10 ** 6)):
+            st["residual"].zero_()
+            times[i].append(_us(lambda: c.encode(g, st, workspace=ws, out=pay, max_ctas=ctas), 1))
+            assert int(ws.view(torch.int32)[3 * 4096 + 5]) != 0      # kWsOverflow
+    mid = [sorted(t)[len(t) // 2] for t in times]
+    assert mid[0] < 1.1 * mid[1], mid
