@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) chain_sample_kernel(const __gri
 template <int MODE>
 __global__ void __launch_bounds__(kChainThreads, 5) chain_collect_kernel(const __grid_constant__ ChainArgs A) {
   uint32_t b = blockIdx.x;
-  if (MODE == 0 && A.stretch != 0u) {
+  if (A.stretch != 0u) {
     b = b % kStretches * A.stretch + b / kStretches;
     if (b >= 2 * A.tiles) return;
   }
@@ -290,7 +290,7 @@ int chain_per_sm(int dev) {
 static uint64_t groups_for(uint64_t kmax) { return (kmax + kmax / 2) / (4 * kSpThreads * kChainLists) + 1; }
 
 bool chain_place(ChainArgs& A, int per_sm, int sms) {
-  uint64_t tiles = 0, samples = 0, wanted = 0;
+  uint64_t tiles = 0, samples = 0, wanted = 0, n = 0, k = 0;
   for (int i = 0; i < A.units; ++i) {
     SelUnit& s = A.unit[i].s;
     if (s.n == 0) return false;
@@ -301,6 +301,8 @@ bool chain_place(ChainArgs& A, int per_sm, int sms) {
     tiles += t;
     samples += s.sampled;
     wanted += groups_for(s.kmax) - 1;
+    n += s.n;
+    k += s.kmax;
   }
   const uint32_t fit = (uint32_t)(per_sm * sms) / kChainLists, most = fit < kChainGroups ? fit : kChainGroups;
   if (most < (uint32_t)A.units || tiles > 0x3FFFFFFFull) return false;
@@ -312,17 +314,22 @@ bool chain_place(ChainArgs& A, int per_sm, int sms) {
   uint32_t group = 0;
   for (int i = 0; i < A.units; ++i) {
     const uint64_t more = groups_for(A.unit[i].s.kmax) - 1;
-    const uint32_t n = 1 + (uint32_t)(wanted <= spare ? more : more * spare / wanted);
-    for (uint32_t q = 0; q < n; ++q) A.emitters[group++] = {(uint8_t)i, (uint8_t)q, (uint8_t)n};
+    const uint32_t own = 1 + (uint32_t)(wanted <= spare ? more : more * spare / wanted);
+    for (uint32_t q = 0; q < own; ++q) A.emitters[group++] = {(uint8_t)i, (uint8_t)q, (uint8_t)own};
   }
   A.emitting = kChainLists * group;
-  // The owner's sum holds little but what was pushed, so its candidates' digits are a few
-  // leading bits, and an array's CTAs wait for one another at a few words.  Several arrays
-  // are taken at a time, by their half tiles in sixteen stretches side by side: two arrays
-  // of 10 M elements, PS, DGC / GradDrop, us, one stretch / sixteen (persistent kernels):
-  // 1 % 222 / 197 (240), 159 / 149 (193); 3 % 355 / 290 (334), 362 / 303 (313).
+  // An array's CTAs wait for one another where they count its candidates' first digits: at a
+  // few words in an owner's sum, which holds little but what was pushed, and else where many
+  // are sent.  Several arrays are taken at a time then, by the bucket's half tiles in sixteen
+  // stretches side by side.  Two arrays of 10 M elements, us, one stretch / sixteen
+  // (persistent kernels): PS, the sums alone, DGC, 1 % 222 / 197 (240), 3 % 355 / 290 (334);
+  // ring, GradDrop, 0.1 % 81.2 / 82.0 (96), 1 % 93.9 / 93.2 (115), 3 % 170 / 129 (159), 10 %
+  // 412 / 267 (303).  Half tiles of an update are fastest in order: one of 16 M elements, one
+  // of 8 M and so on, DGC, ring, 0.1 % 150 / 152 (188), 1 % 185 / 186 (237), 3 % 241 / 232
+  // (309).
+  const bool sums = A.unit[0].s.g == nullptr;
   A.tiles = (uint32_t)tiles;
-  A.stretch = A.units > 1 ? (uint32_t)((2 * tiles + kStretches - 1) / kStretches) : 0u;
+  A.stretch = A.units > 1 && (sums || k * 50 >= n) ? (uint32_t)((2 * tiles + kStretches - 1) / kStretches) : 0u;
   // One CTA per SM for the passes over whole arrays, up to a tile each.  Of 6.6 M elements,
   // 40 rows of 1024 not zero, GradDrop at 0.1 % (encode, us): the emitters alone 658, one per
   // SM 88, two 78; but where no list comes out short two cost the 25 MB bucket 1.9 us, one
@@ -353,7 +360,7 @@ static cudaError_t chain_select_mode(const ChainArgs& A, cudaStream_t st) {
   const ChainUnit& last = A.unit[A.units - 1];
   const uint32_t tiles = last.tile0 + (last.s.n - 1) / kSelTile + 1, samples = last.sample0 + last.s.sampled;
   cudaError_t e = chain_launch(chain_sample_kernel<MODE>, samples, kSpThreads, sizeof(SelSmem), true, st, A);
-  const uint32_t halves = MODE == 0 && A.stretch ? kStretches * A.stretch : 2 * tiles;
+  const uint32_t halves = A.stretch ? kStretches * A.stretch : 2 * tiles;
   if (e == cudaSuccess) e = chain_launch(chain_collect_kernel<MODE>, halves, kChainThreads, 0, true, st, A);
   if (e == cudaSuccess)
     e = chain_launch(chain_emit_kernel, A.ctas, kSpThreads, sizeof(ChainSmem), false, st, A);

@@ -41,7 +41,7 @@ struct ChainArgs {
   ChainEmitters emitters[kChainGroups];
   uint32_t emitting;     // CTAs of these groups
   uint32_t tiles;
-  uint32_t stretch;      // half tiles that lie between those of two neighbouring CTAs, 0 with one array
+  uint32_t stretch;      // half tiles that lie between those of two neighbouring CTAs, or 0: in order
   uint32_t ctas;         // of the emitting launch; those behind the emitters wait for a list that came out short
 };
 

@@ -18,21 +18,25 @@ def _us(f, reps):
     return a.elapsed_time(e) * 1e3 / reps
 
 
-# two large arrays, of which many elements are sent: the owner's sums count the same few words
-@pytest.mark.parametrize("name", ["dgc", "graddrop"])
-def test_chain_of_large_arrays_is_no_slower_than_the_persistent_kernels(name):
-    sizes, c = [10_000_000] * 2, Compressor(name, ratio=0.03)
+# two large arrays, of which many elements are sent: an array's CTAs count the same words
+@pytest.mark.parametrize("name,topology,ratio", [("dgc", "ps", 0.03), ("graddrop", "ps", 0.03), ("graddrop", "ring", 0.05)])
+def test_chain_of_large_arrays_is_no_slower_than_the_persistent_kernels(name, topology, ratio):
+    sizes, c = [10_000_000] * 2, Compressor(name, ratio=ratio)
     runs = []
     for ctas in (0, 1024):     # 0: a chain of launches
-        b = FusedSparseBucket(c.spec, sizes, 1, 0, topology="ps", ctas=ctas).bind_local("cuda")
+        b = FusedSparseBucket(c.spec, sizes, 1, 0, topology=topology, ctas=ctas).bind_local("cuda")
         g = [torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)) for n in sizes]
         out, sums = [torch.empty_like(x) for x in g], [torch.zeros_like(x) for x in g]
         st = [c.new_state(n, "cuda") for n in sizes]
         acc = "accum_v" if name == "dgc" else "residual"
-        args = ([x.data_ptr() for x in g], [s[acc].data_ptr() for s in st],
-                [s["momentum_u"].data_ptr() for s in st] if name == "dgc" else None, [x.data_ptr() for x in out],
-                [x.data_ptr() for x in sums])
-        runs.append(lambda b=b, args=args, keep=(g, out, sums, st): b.launch_ptrs(*args))
+        args = ([s[acc].data_ptr() for s in st], [s["momentum_u"].data_ptr() for s in st] if name == "dgc" else None,
+                [x.data_ptr() for x in out], [x.data_ptr() for x in sums])
+        h = [-x for x in g]     # gradients that cancel, so that the state stays as it is
+
+        def run(b=b, args=args, g=g, h=h, keep=(out, sums, st)):
+            b.launch_ptrs([x.data_ptr() for x in g], *args)
+            b.launch_ptrs([x.data_ptr() for x in h], *args)
+        runs.append(run)
     best = [1e9, 1e9]
     for _ in range(5):         # in turn
         for i in range(2):
