@@ -15,8 +15,7 @@
 //   pull   : every rank waits for each owner's flag and scatters value / N into the
 //            result, which the update pass cleared.
 //
-// A job of one rank takes neither: its bucket is a chain of launches, but for a few that are
-// better served by the kernels here (launch_chain).
+// A job of one rank takes neither: its bucket is a chain of launches (launch_chain).
 //
 // All units of a bucket are batched in every phase, which is the "bulk
 // synchronisation" of many small tensors: the update pass splits the bucket's tiles, not
@@ -599,21 +598,12 @@ static uint64_t sp_cleared_words(int nseg, int nranks) {
 
 // A job of one rank waits for nobody: its selections run as chains of launches, in a PS the
 // owner's sum behind the push.  The persistent kernels that follow do the same with grid
-// barriers; us per step or bucket, persistent / chain (B200): ResNet-50, DGC, PS 199.6 /
-// 187.6; GradDrop ring 6.6 M elements 55.1 / 43.1, 20 M at 1 % 134 / 97; DGC ring 3 M 49.4 /
-// 34.2; DGC PS 64 K 51.9 / 39.5, 20 M 173 / 147; 24 arrays of 1 M in all, PS 60.7 / 48.7.
-// False when the arrays do not fit a chain (and always with a limit on the CTAs), and for the
-// DGC ring of more than 67 M elements with few candidates (see chain_is_slower; 0.1 %: 80 M
-// 377 / 383, 134 M 591 / 627; the others gain up to there: GradDrop 134 M 410 / 415, DGC PS
-// 134 M 790 / 768).
+// barriers; us per step or bucket, persistent / chain (B200): ResNet-50, DGC, PS 203 / 171;
+// GradDrop ring 6.6 M elements 56.0 / 39.8, 20 M at 1 % 128 / 95; DGC ring 3 M 49.0 / 34.4; DGC
+// PS 64 K 52.1 / 37.7, 20 M 176 / 132; 24 arrays of 1 M in all, PS 61.7 / 47.6.
+// False when the arrays do not fit a chain (and always with a limit on the CTAs).
 static bool launch_chain(int topo, const SpBucket& bk, const HpComm& cm, uint8_t* ws, cudaStream_t st, int& rc) {
   int dev = 0, sms = 0;
-  uint64_t n = 0, k = 0;
-  for (int i = 0; i < bk.nseg; ++i) {
-    n += bk.seg[i].n;
-    k += bk.seg[i].kmax;
-  }
-  if (topo == HP_TOPO_RING && bk.alg == kDgc && n > (1ull << 26) && chain_is_slower(2, n, k)) return false;
   if (cudaGetDevice(&dev) != cudaSuccess || chain_per_sm(dev) == 0) return false;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   sms = stream_sms(st, sms);
@@ -737,7 +727,7 @@ int hp_fused_sparse_layout(float ratio, const uint64_t* ns, int nseg, int nranks
 }
 
 // One synchronisation of a bucket through the PS topology: one cooperative launch, or with
-// one rank and ctas <= 0 usually two chains of three launches (launch_chain).
+// one rank and ctas <= 0 two chains of three launches (launch_chain).
 // segs[i].r is the accumulator (DGC v / GradDrop residual), us[i] the DGC momentum
 // (or NULL), segs[i].sr the server accumulator of the owned chunk.  ws: scratch of
 // hp_fused_sparse_layout().ws_bytes per rank played by this call.  ctas <= 0: the
@@ -753,7 +743,7 @@ int hp_cuda_fused_sparse_ps(int alg, float ratio, float momentum, const HpSeg* s
 }
 
 // One synchronisation of a bucket through the ring topology: one cooperative launch, or with
-// one rank and ctas <= 0 usually a chain of three (launch_chain).
+// one rank and ctas <= 0 a chain of three (launch_chain).
 // Same arguments as hp_cuda_fused_sparse_ps (segs[i].sr is not used).
 int hp_cuda_fused_sparse_ring(int alg, float ratio, float momentum, const HpSeg* segs,
                               void* const* us, int nseg, const HpComm* comm, void* ws, int ctas,

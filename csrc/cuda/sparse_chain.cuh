@@ -50,18 +50,16 @@ int chain_per_sm(int dev);
 // Whether an array of n elements, of which k are sent, is better served by the persistent
 // kernels.  Of at most one tile: a single CTA of theirs meets no barrier, and is one launch
 // instead of three (encode, us, persistent / chain: 300 elements, 10 % 17.0 / 19.6, 4096
-// elements, 1 % 18.1 / 20.0; 4097 elements 19.8 / 18.1).  Of more than 42 M, when few of a
-// tile's elements are candidates: a CTA per half tile spends longer on the bound, its barriers
-// and its reservation than on them, where theirs look after several tiles (DGC, 0.1 %,
-// normal values: 33 M 147 / 147, 50 M 204 / 211, 67 M 261 / 274, 134 M 472 / 525; GradDrop
-// 33 M 96 / 97, 67 M 163 / 174, 134 M 296 / 322).  With more candidates their list's one
-// counter is the longer wait, the sooner the fewer bytes an element moves: 67 M, DGC, 0.3 %
-// 279 / 288 with normal, 290 / 285 with heavy-tailed values, 0.5 % 300 / 299, 328 / 295;
-// GradDrop, 0.15 % 168 / 174, 186 / 175, 0.2 % 180 / 176, 202 / 175; without an update 0.02 %
-// 79 / 85, 0.1 % 98 / 84.  mode: of the update (see pass0_body).
+// elements, 1 % 18.1 / 20.0; 4097 elements 19.8 / 18.1).  Without DGC's momentum, of more than
+// 42 M, when few of a tile's elements are candidates: a CTA per half tile spends longer on the
+// bound, its barriers and its reservation than on them, where theirs look after several tiles
+// (GradDrop, 0.1 %, normal values: 33 M 96 / 97, 67 M 163 / 171, 134 M 297 / 319).  With more
+// candidates their list's one counter is the longer wait (67 M, GradDrop, 0.2 % 181 / 174 with
+// normal, 201 / 174 with heavy-tailed values; without an update 0.02 % 79 / 85, 0.1 % 98 / 84),
+// and DGC, which moves more bytes, gains throughout (0.1 %: 20 M 103 / 84, 67 M 262 / 224,
+// 134 M 474 / 426).  mode: of the update (see pass0_body).
 inline bool chain_is_slower(int mode, uint64_t n, uint64_t k) {
-  const uint64_t few = mode == 2 ? 400 : (mode == 1 ? 900 : 2000);
-  return n <= (uint64_t)kSelTile || (n > 10240ull * kSelTile && k * few <= n);
+  return n <= (uint64_t)kSelTile || (mode != 2 && n > 10240ull * kSelTile && k * (mode == 1 ? 900 : 2000) <= n);
 }
 // Places the units' tiles and samples behind one another; per_sm: what chain_per_sm says,
 // sms: those of the stream.  False when the lists cannot be shared out.

@@ -5,9 +5,8 @@
 // (sparse_chain.cuh).  One persistent kernel with grid barriers does the same for calls that
 // limit the CTAs (max_ctas), and for those that it is better at (chain_is_slower); in the
 // others equal shares leave the faster SMs idle, and the arrays stand still while the sample
-// is worked out.  DGC encode and decode at
-// 0.1 %, us, persistent / chain (B200): 64 K elements 28.3 / 26.2, 1 M 36.8 / 30.1, 3 M
-// 52.4 / 45.2, 10 M at 1 % 93.8 / 81.1, 20 M 123.3 / 119.6.
+// is worked out.  DGC encode and decode at 0.1 %, us, persistent / chain (B200): 64 K elements
+// 26.7 / 24.8, 1 M 36.8 / 30.3, 3 M 51.4 / 42.1, 10 M at 1 % 98.4 / 75.9, 20 M 122.7 / 104.7.
 // The emitting launch is cooperative, because where a list came out short its CTAs count
 // the digits together, and sized for the SMs that the stream may use.  Barriers are
 // bounded (kGridBarrierNs); if a kernel that holds SMs for longer than that comes between

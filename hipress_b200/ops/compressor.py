@@ -72,7 +72,7 @@ class Compressor:
         may use: it starts when all its CTAs find room at once, and must not share the GPU
         with a kernel that holds SMs for seconds.  With ``max_ctas`` it is one cooperative
         launch of that many CTAs, and one as wide as there is room for arrays of at most 4096
-        elements and for the largest (over 42 M, few of them sent); a workspace without a size runs plain launches instead,
+        elements and for GradDrop's largest (over 42 M, few of them sent); a workspace without a size runs plain launches instead,
         which need no such room.
         """
         sp = self.spec
