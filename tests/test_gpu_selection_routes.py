@@ -85,3 +85,17 @@ def test_chain_whose_list_overflows_is_no_slower_than_the_persistent_kernel():
             assert int(ws.view(torch.int32)[3 * 4096 + 5]) != 0      # kWsOverflow
     mid = [sorted(t)[len(t) // 2] for t in times]
     assert mid[0] < 1.1 * mid[1], mid
+
+
+@pytest.mark.parametrize("name", ["dgc", "graddrop"])
+@pytest.mark.parametrize("max_ctas", [1, 40, 10 ** 6])     # the last: as wide as the GPU is
+def test_persistent_kernel_at_its_widths(name, max_ctas):
+    n, c = 300 * 4096 + 5, Compressor(name, ratio=0.01)
+    gen = torch.Generator().manual_seed(max_ctas)
+    cpu, dev, ws = c.new_state(n, "cpu"), c.new_state(n, "cuda"), c.new_workspace("cuda", n)
+    for _ in range(2):
+        g = torch.randn(n, generator=gen) * torch.randn(n, generator=gen)
+        want = sparse_pairs(c.encode(g, cpu), c.kmax(n))
+        got = sparse_pairs(c.encode(g.cuda(), dev, workspace=ws, max_ctas=max_ctas), c.kmax(n))
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+        assert all(torch.equal(dev[k].cpu(), cpu[k]) for k in cpu)
